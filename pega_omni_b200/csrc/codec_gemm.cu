@@ -20,6 +20,7 @@
 #include "codec.h"
 #include "gemm.h"
 #include "sm100.cuh"
+#include "pdl.cuh"
 
 namespace omni {
 
@@ -51,7 +52,6 @@ __global__ void __launch_bounds__(kConvThreads, 1)
     conv_gemm_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap wmap,
                      const ConvArgs a) {
   using namespace sm100;
-  if (*reinterpret_cast<volatile uint32_t*>(a.err) != 0) return;
   extern __shared__ unsigned char conv_smem_raw[];
   const uint32_t raw = smem_addr(conv_smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
@@ -87,6 +87,13 @@ __global__ void __launch_bounds__(kConvThreads, 1)
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot_ptr;
+  grid_trigger();  // not before this CTA holds its TMEM columns: the next kernel could take them and wait for this one
+  grid_wait();
+  if (*reinterpret_cast<volatile uint32_t*>(a.err) != 0) {
+    __syncthreads();
+    if (warp == 1) tmem_dealloc(tmem_base, 2 * a.acc_cols);
+    return;
+  }
 
   if (warp == 0) {
     if (lane == 0) {
@@ -308,8 +315,7 @@ cudaError_t conv_launch(const ConvGemmPlan& p, uint32_t* err, cudaStream_t strea
   a.tn = p.tn, a.kbs = p.kbs, a.cpb = p.cpb, a.ragged = p.ragged, a.stages = p.stages, a.kind = p.kind;
   a.t_tiles = p.T / p.TB, a.n_tiles = p.n_tiles, a.tiles = p.n_tiles * p.row_tiles;
   a.acc_cols = p.tn <= 32 ? 32u : p.tn <= 64 ? 64u : p.tn <= 128 ? 128u : 256u;
-  conv_gemm_kernel<<<p.ctas, kConvThreads, kConvSmem, stream>>>(p.xmap, p.wmap, a);
-  return cudaGetLastError();
+  return launch_pdl(conv_gemm_kernel, dim3(p.ctas), dim3(kConvThreads), kConvSmem, stream, p.xmap, p.wmap, a);
 }
 
 }  // namespace omni

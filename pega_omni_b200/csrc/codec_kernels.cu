@@ -12,6 +12,7 @@
 #include <algorithm>
 
 #include "codec.h"
+#include "pdl.cuh"
 
 namespace omni {
 
@@ -31,6 +32,8 @@ __device__ __forceinline__ void ldf8(const float* p, float* v) {
 // One stream per block: [codebook 0 | sum of codebooks 1..15], the sum in f32 in codebook order.
 __global__ void codec_rvq_kernel(const int32_t* __restrict__ codes, const bf16* __restrict__ books, bf16* __restrict__ out,
                                  int half, int book_rows) {
+  grid_trigger();
+  grid_wait();
   const int s = blockIdx.x;
   for (int c = threadIdx.x * 8; c < half; c += blockDim.x * 8) {
     const int32_t* code = codes + s * 16;
@@ -50,7 +53,9 @@ __global__ void codec_rvq_kernel(const int32_t* __restrict__ codes, const bf16* 
 
 // A warp per row, dim a multiple of 256 up to 1024.
 __global__ void codec_add_norm_kernel(const bf16* add, int64_t add_stride, bf16* __restrict__ res,
-                                      const bf16* __restrict__ w, bf16* out, int rows, int dim, float eps) {  // out may be add
+                                      const bf16* __restrict__ w, bf16* out, int rows, int dim, float eps) {
+  grid_trigger();
+  grid_wait();  // out may be add
   const int r = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (r >= rows) return;
   const bf16* a = add + r * add_stride;
@@ -92,6 +97,8 @@ __global__ void codec_add_norm_kernel(const bf16* add, int64_t add_stride, bf16*
 __global__ void __launch_bounds__(128)
     codec_window_attend_kernel(const bf16* __restrict__ qkv, CodecStateRef st, int64_t ring_offset, bf16* __restrict__ out,
                                int heads, float theta) {
+  grid_trigger();
+  grid_wait();
   __shared__ float sq[4][kHeadDim];
   __shared__ float sp[4][kWindow + 8];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -153,6 +160,8 @@ __global__ void __launch_bounds__(128)
 }
 
 __global__ void codec_silu_mul_kernel(const bf16* __restrict__ gate_up, bf16* __restrict__ out, int inter, int64_t total) {
+  grid_trigger();
+  grid_wait();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= total) return;
   const int per = inter / 8;
@@ -166,6 +175,8 @@ __global__ void codec_silu_mul_kernel(const bf16* __restrict__ gate_up, bf16* __
 }
 
 __global__ void codec_bias_gelu_kernel(bf16* __restrict__ x, const bf16* __restrict__ bias, int cols, int64_t total) {
+  grid_trigger();
+  grid_wait();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= total) return;
   float v[8], b[8];
@@ -191,6 +202,8 @@ __device__ __forceinline__ void bias_snake8(float* v, const bf16* bias, const fl
 __global__ void codec_bias_snake_kernel(const bf16* __restrict__ x, const bf16* __restrict__ bias,
                                         const float* __restrict__ alpha, const float* __restrict__ inv_b,
                                         bf16* __restrict__ out, int cols, int64_t total) {
+  grid_trigger();
+  grid_wait();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= total) return;
   float v[8];
@@ -204,6 +217,8 @@ __global__ void codec_bias_snake_kernel(const bf16* __restrict__ x, const bf16* 
 __global__ void codec_stage_kernel(const bf16* __restrict__ x, const bf16* __restrict__ bias, const float* __restrict__ alpha,
                                    const float* __restrict__ inv_b, CodecStateRef st, int64_t hist_offset,
                                    bf16* __restrict__ padded, int T, int C, int H, int64_t total) {
+  grid_trigger();
+  grid_wait();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= total) return;
   const int per = C / 8, P = H + T;
@@ -235,6 +250,8 @@ __global__ void codec_stage_kernel(const bf16* __restrict__ x, const bf16* __res
 
 __global__ void codec_gather_taps_kernel(const bf16* __restrict__ padded, bf16* __restrict__ col, int T, int C, int taps,
                                          int dil, int64_t total) {
+  grid_trigger();
+  grid_wait();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= total) return;
   const int per = C / 8, P = (taps - 1) * dil + T;
@@ -249,6 +266,8 @@ __global__ void codec_gather_taps_kernel(const bf16* __restrict__ padded, bf16* 
 
 __global__ void codec_overlap_add_kernel(const bf16* __restrict__ z, const bf16* __restrict__ bias, CodecStateRef st,
                                          int64_t prev_offset, bf16* __restrict__ out, int L, int r, int C, int64_t total) {
+  grid_trigger();
+  grid_wait();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= total) return;
   const int per = C / 8;
@@ -281,6 +300,8 @@ __global__ void codec_dwconv_ln_kernel(const bf16* __restrict__ z, const bf16* _
                                        const bf16* __restrict__ b, const bf16* __restrict__ ln_w,
                                        const bf16* __restrict__ ln_b, CodecStateRef st, int64_t hist_offset,
                                        bf16* __restrict__ xin, bf16* __restrict__ out, int T, int r, int C, float eps) {
+  grid_trigger();
+  grid_wait();
   constexpr int H = kTaps - 1;
   __shared__ float scratch[32];
   const int64_t g = blockIdx.x;
@@ -352,6 +373,8 @@ __global__ void __launch_bounds__(256)
     codec_out_conv_kernel(const bf16* __restrict__ x, const bf16* __restrict__ bias, const float* __restrict__ alpha,
                           const float* __restrict__ inv_b, const bf16* __restrict__ w, const bf16* __restrict__ wb,
                           CodecStateRef st, int64_t hist_offset, float* __restrict__ wav, int T, int C) {
+  grid_trigger();
+  grid_wait();
   constexpr int H = kTaps - 1, kPer = 4;  // samples per thread
   extern __shared__ __align__(16) float out_smem[];
   const int ld = C + 4, per = C / 8;
@@ -408,78 +431,64 @@ inline unsigned blocks_for(int64_t total, int threads) { return (unsigned)((tota
 
 cudaError_t launch_codec_rvq(const int32_t* codes, const bf16* books, bf16* out, int n, int half, int book_rows,
                              cudaStream_t stream) {
-  codec_rvq_kernel<<<n, std::min(256, std::max(32, half / 8)), 0, stream>>>(codes, books, out, half, book_rows);
-  return cudaGetLastError();
+  return launch_pdl(codec_rvq_kernel, dim3(n), dim3(std::min(256, std::max(32, half / 8))), 0, stream, codes, books, out, half, book_rows);
 }
 
 cudaError_t launch_codec_add_norm(const bf16* add, int64_t add_stride, bf16* res, const bf16* w, bf16* out, int rows,
                                   int dim, float eps, cudaStream_t stream) {
-  codec_add_norm_kernel<<<(rows + 3) / 4, 128, 0, stream>>>(add, add_stride, res, w, out, rows, dim, eps);
-  return cudaGetLastError();
+  return launch_pdl(codec_add_norm_kernel, dim3((rows + 3) / 4), dim3(128), 0, stream, add, add_stride, res, w, out, rows, dim, eps);
 }
 
 cudaError_t launch_codec_window_attend(const bf16* qkv, CodecStateRef st, int64_t ring_offset, bf16* out, int n, int heads,
                                        float theta, cudaStream_t stream) {
-  codec_window_attend_kernel<<<dim3(n, (heads + 3) / 4), 128, 0, stream>>>(qkv, st, ring_offset, out, heads, theta);
-  return cudaGetLastError();
+  return launch_pdl(codec_window_attend_kernel, dim3(n, (heads + 3) / 4), dim3(128), 0, stream, qkv, st, ring_offset, out, heads, theta);
 }
 
 cudaError_t launch_codec_silu_mul(const bf16* gate_up, bf16* out, int rows, int inter, cudaStream_t stream) {
   const int64_t total = (int64_t)rows * inter / 8;
-  codec_silu_mul_kernel<<<blocks_for(total, 256), 256, 0, stream>>>(gate_up, out, inter, total);
-  return cudaGetLastError();
+  return launch_pdl(codec_silu_mul_kernel, dim3(blocks_for(total, 256)), dim3(256), 0, stream, gate_up, out, inter, total);
 }
 
 cudaError_t launch_codec_bias_gelu(bf16* x, const bf16* bias, int64_t rows, int cols, cudaStream_t stream) {
   const int64_t total = rows * cols / 8;
-  codec_bias_gelu_kernel<<<blocks_for(total, 256), 256, 0, stream>>>(x, bias, cols, total);
-  return cudaGetLastError();
+  return launch_pdl(codec_bias_gelu_kernel, dim3(blocks_for(total, 256)), dim3(256), 0, stream, x, bias, cols, total);
 }
 
 cudaError_t launch_codec_bias_snake(const bf16* x, const bf16* bias, const float* alpha, const float* inv_b, bf16* out,
                                     int64_t rows, int cols, cudaStream_t stream) {
   const int64_t total = rows * cols / 8;
-  codec_bias_snake_kernel<<<blocks_for(total, 256), 256, 0, stream>>>(x, bias, alpha, inv_b, out, cols, total);
-  return cudaGetLastError();
+  return launch_pdl(codec_bias_snake_kernel, dim3(blocks_for(total, 256)), dim3(256), 0, stream, x, bias, alpha, inv_b, out, cols, total);
 }
 
 cudaError_t launch_codec_stage(const bf16* x, const bf16* bias, const float* alpha, const float* inv_b, CodecStateRef st,
                                int64_t hist_offset, bf16* padded, int n, int T, int C, int H, cudaStream_t stream) {
   const int64_t total = (int64_t)n * (H + T) * (C / 8);
-  codec_stage_kernel<<<blocks_for(total, 256), 256, 0, stream>>>(x, bias, alpha, inv_b, st, hist_offset, padded, T, C, H,
-                                                                 total);
-  return cudaGetLastError();
+  return launch_pdl(codec_stage_kernel, dim3(blocks_for(total, 256)), dim3(256), 0, stream, x, bias, alpha, inv_b, st, hist_offset, padded, T, C, H, total);
 }
 
 cudaError_t launch_codec_gather_taps(const bf16* padded, bf16* col, int n, int T, int C, int taps, int dil,
                                      cudaStream_t stream) {
   const int64_t total = (int64_t)n * T * taps * (C / 8);
-  codec_gather_taps_kernel<<<blocks_for(total, 256), 256, 0, stream>>>(padded, col, T, C, taps, dil, total);
-  return cudaGetLastError();
+  return launch_pdl(codec_gather_taps_kernel, dim3(blocks_for(total, 256)), dim3(256), 0, stream, padded, col, T, C, taps, dil, total);
 }
 
 cudaError_t launch_codec_overlap_add(const bf16* z, const bf16* bias, CodecStateRef st, int64_t prev_offset, bf16* out,
                                      int n, int L, int r, int C, cudaStream_t stream) {
   const int64_t total = (int64_t)n * L * r * (C / 8);
-  codec_overlap_add_kernel<<<blocks_for(total, 256), 256, 0, stream>>>(z, bias, st, prev_offset, out, L, r, C, total);
-  return cudaGetLastError();
+  return launch_pdl(codec_overlap_add_kernel, dim3(blocks_for(total, 256)), dim3(256), 0, stream, z, bias, st, prev_offset, out, L, r, C, total);
 }
 
 cudaError_t launch_codec_dwconv_ln(const bf16* z, const bf16* zb, const bf16* w, const bf16* b, const bf16* ln_w,
                                    const bf16* ln_b, CodecStateRef st, int64_t hist_offset, bf16* xin, bf16* out, int n,
                                    int T, int r, int C, float eps, cudaStream_t stream) {
-  codec_dwconv_ln_kernel<<<(unsigned)((int64_t)n * T), (C / 8 + 31) / 32 * 32, 0, stream>>>(z, zb, w, b, ln_w, ln_b, st, hist_offset, xin,
-                                                                          out, T, r, C, eps);
-  return cudaGetLastError();
+  return launch_pdl(codec_dwconv_ln_kernel, dim3((unsigned)((int64_t)n * T)), dim3((C / 8 + 31) / 32 * 32), 0, stream, z, zb, w, b, ln_w, ln_b, st, hist_offset, xin, out, T, r, C, eps);
 }
 
 cudaError_t launch_codec_out_conv(const bf16* x, const bf16* bias, const float* alpha, const float* inv_b, const bf16* w,
                                   const bf16* wb, CodecStateRef st, int64_t hist_offset, float* wav, int n, int T, int C,
                                   cudaStream_t stream) {
   const size_t smem = ((size_t)(kOutTile + kTaps - 1) * (C + 4) + (size_t)kTaps * C) * sizeof(float);
-  codec_out_conv_kernel<<<dim3(T / kOutTile, n), 256, smem, stream>>>(x, bias, alpha, inv_b, w, wb, st, hist_offset, wav,
-                                                                      T, C);
-  return cudaGetLastError();
+  return launch_pdl(codec_out_conv_kernel, dim3(T / kOutTile, n), dim3(256), smem, stream, x, bias, alpha, inv_b, w, wb, st, hist_offset, wav, T, C);
 }
 
 }  // namespace omni

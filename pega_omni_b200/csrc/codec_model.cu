@@ -16,6 +16,7 @@
 #include <vector>
 
 #include "../../include/omni_b200_codec.h"
+#include "chain.h"
 #include "codec.h"
 #include "gemm.h"
 
@@ -114,6 +115,8 @@ struct omni_codec {
   std::map<std::tuple<const void*, const void*, const void*, int>, TcGemmPlan> plans;
   std::map<std::tuple<const void*, const void*, const void*, int>, RmGemmPlan> rm_plans;
   std::map<std::tuple<const void*, const void*, const void*, int, int>, ConvGemmPlan> conv_plans;
+  std::map<std::tuple<const void*, const void*, const void*, int, int>, StreamGemmPlan> stream_plans;
+  Chain chain() { return Chain{stream, err, sm_count, scratch.partials, scratch.partial_floats, &launches, &stream_plans}; }
   struct StepGraph {
     cudaGraphExec_t exec = nullptr;
     int seen = 0, nodes = 0;
@@ -448,6 +451,10 @@ size_t elems_per_stream(const omni_codec_config& c) {
 
 // y[rows, N] = x[rows, K] . w[N, K]^T on the library's dense GEMMs (K a multiple of 64).
 int dense(omni_codec* m, const bf16* w, int N, int K, const bf16* x, int rows, bf16* y) {
+  if (rows <= kChainRows && stream_supports(N, K, rows)) {
+    CCUDA(m, m->chain().gemm(w, N, K, x, rows, kStreamBf16, y, N));
+    return OMNI_OK;
+  }
   if (rows <= 8 || !tc_supports(N, K, rows)) {
     CLAUNCH(m, gemv_launch(w, N, K, x, rows, y, N, Epilogue{}, m->sm_count, m->stream));
     return OMNI_OK;
@@ -665,6 +672,7 @@ int create_impl(omni_codec* m, const omni_tensor* tensors, int n_tensors) {
   m->sm_count = prop.multiProcessorCount;
   if (tc_init() != 0) return m->fail(OMNI_ERR_CUDA, "cuTensorMapEncodeTiled entry point not found");
   tc_configure();
+  stream_configure();
   conv_configure();
   CCUDA(m, cudaStreamCreateWithFlags(&m->stream, cudaStreamNonBlocking));
   CCUDA(m, cudaEventCreate(&m->ev0));

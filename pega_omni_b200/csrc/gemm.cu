@@ -8,6 +8,7 @@
 #include <cstdio>
 
 #include "sm100.cuh"
+#include "pdl.cuh"
 
 namespace omni {
 
@@ -32,6 +33,8 @@ __global__ void __launch_bounds__(kGemvWarps * 32) gemv_kernel(const bf16* __res
                                                                 const bf16* __restrict__ x, int rows,
                                                                 bf16* __restrict__ y, int ldy, const bf16* bias,
                                                                 int kind, int cols_per_warp) {
+  grid_trigger();
+  grid_wait();
   extern __shared__ __align__(16) unsigned char gemv_smem[];
   bf16* xs = reinterpret_cast<bf16*>(gemv_smem);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -80,8 +83,7 @@ static cudaError_t gemv_launch_r(const bf16* w, int N, int K, const bf16* x, int
   int cpw = N / (kGemvWarps * sm_count * 4);
   cpw = std::max(1, std::min(cpw, 4));
   const int blocks = (N + kGemvWarps * cpw - 1) / (kGemvWarps * cpw);
-  gemv_kernel<R><<<blocks, kGemvWarps * 32, smem, stream>>>(w, N, K, x, rows, y, ldy, epi.bias, epi.kind, cpw);
-  return cudaGetLastError();
+  return launch_pdl(gemv_kernel<R>, dim3(blocks), dim3(kGemvWarps * 32), smem, stream, w, N, K, x, rows, y, ldy, epi.bias, epi.kind, cpw);
 }
 
 cudaError_t gemv_launch(const bf16* w, int N, int K, const bf16* x, int rows, bf16* y, int ldy, Epilogue epi,
@@ -177,7 +179,6 @@ __global__ void __launch_bounds__(128, 1)
   const int n_stages = S::kStages / kbs;
   const uint32_t stage_bytes = (uint32_t)kbs * S::kStageBytes, x_base = (uint32_t)kbs * kTileW * kTileK * 2;
   using namespace sm100;
-  if (*reinterpret_cast<volatile uint32_t*>(err) != 0) return;  // an earlier kernel failed: do not wait on hardware
 
   extern __shared__ unsigned char tc_smem_raw[];
   const uint32_t raw = smem_addr(tc_smem_raw);
@@ -213,6 +214,13 @@ __global__ void __launch_bounds__(128, 1)
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot_ptr;
+  grid_trigger();  // not before this CTA holds its TMEM columns: the next kernel could take them and wait for this one
+  grid_wait();
+  if (*reinterpret_cast<volatile uint32_t*>(err) != 0) {  // an earlier kernel failed: do not wait on hardware
+    __syncthreads();
+    if (warp == 1) tmem_dealloc(tmem_base, S::kTmemCols);
+    return;
+  }
 
   bool ok = true;
   if (warp == 0) {
@@ -383,7 +391,6 @@ __global__ void __launch_bounds__(128, 1)
                    uint32_t tmem_cols,
                    const bf16* bias, int kind, uint32_t* err) {
   using namespace sm100;
-  if (*reinterpret_cast<volatile uint32_t*>(err) != 0) return;
   extern __shared__ unsigned char rm_smem_raw[];
   const uint32_t raw = smem_addr(rm_smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
@@ -415,6 +422,13 @@ __global__ void __launch_bounds__(128, 1)
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot_ptr;
+  grid_trigger();  // not before this CTA holds its TMEM columns: the next kernel could take them and wait for this one
+  grid_wait();
+  if (*reinterpret_cast<volatile uint32_t*>(err) != 0) {  // an earlier kernel failed: do not wait on hardware
+    __syncthreads();
+    if (warp == 1) tmem_dealloc(tmem_base, tmem_cols);
+    return;
+  }
 
   if (warp == 0) {
     if (lane == 0) {
@@ -601,9 +615,7 @@ template <int BN>
 static cudaError_t tc_launch_bn(const TcGemmPlan& p, const GemmScratch& s, uint32_t* err, cudaStream_t stream) {
   using S = TcShape<BN>;
   const dim3 grid(p.tiles_n(), p.splits, p.row_tiles);
-  gemm_tc_kernel<BN><<<grid, 128, S::kSmemBytes, stream>>>(p.wmap, p.xmap, p.y, p.ldy, p.N, p.K, p.rows, p.splits,
-                                                           p.kbs, s.partials, s.counters, p.epi.bias, p.epi.kind, err);
-  return cudaGetLastError();
+  return launch_pdl(gemm_tc_kernel<BN>, grid, dim3(128), S::kSmemBytes, stream, p.wmap, p.xmap, p.y, p.ldy, p.N, p.K, p.rows, p.splits, p.kbs, s.partials, s.counters, p.epi.bias, p.epi.kind, err);
 }
 
 // Raises the dynamic shared-memory limit of every instantiation up front, so no
@@ -673,12 +685,7 @@ int rm_plan(RmGemmPlan* plan, const bf16* w, int N, int K, const bf16* x, int ro
 
 cudaError_t rm_launch(const RmGemmPlan& p, uint32_t* err, cudaStream_t stream) {
   if (p.TN < 16 || p.TN > 256 || p.TN % 16) return cudaErrorInvalidValue;
-  gemm_rm_kernel<<<(p.N + p.TN - 1) / p.TN, 128, RmShape::kSmemBytes, stream>>>(
-      p.wmap, p.xmap, p.y, p.ldy, p.N, p.K, p.rows, p.TN, p.kbs, p.bn, RmShape::stages(p.TN, p.kbs, p.bn),
-      RmShape::tmem_cols(p.TN),
-      p.epi.bias,
-      p.epi.kind, err);
-  return cudaGetLastError();
+  return launch_pdl(gemm_rm_kernel, dim3((p.N + p.TN - 1) / p.TN), dim3(128), RmShape::kSmemBytes, stream, p.wmap, p.xmap, p.y, p.ldy, p.N, p.K, p.rows, p.TN, p.kbs, p.bn, RmShape::stages(p.TN, p.kbs, p.bn), RmShape::tmem_cols(p.TN), p.epi.bias, p.epi.kind, err);
 }
 
 // ---------------------------------------------------------------------------

@@ -5,6 +5,7 @@
 // association order of their block scan (higgs.cu:66-183, talker.cu:108-257).
 #include "kernels.h"
 #include "sampler.cuh"
+#include "pdl.cuh"
 
 namespace omni {
 
@@ -14,6 +15,8 @@ constexpr int kHiggsBooks = 8;
 // b * vocab + code of the fused table), rounded once.
 __global__ void higgs_frame_embed_kernel(SlotState st, const bf16* __restrict__ table, bf16* __restrict__ out, int dim,
                                          int vocab, uint32_t* err) {
+  grid_trigger();
+  grid_wait();
   const int s = blockIdx.x, c = threadIdx.x * 8;
   const int32_t* codes =
       reinterpret_cast<const int32_t*>(static_cast<const char*>(st.state) + (int64_t)st.lines[s] * st.stride);
@@ -37,6 +40,8 @@ __global__ void __launch_bounds__(1024)
     higgs_sample_kernel(const bf16* __restrict__ logits, int vocab, float temperature, int top_k,
                         const float* __restrict__ uniforms, const int32_t* __restrict__ force, SlotState st,
                         int32_t* __restrict__ codes) {
+  grid_trigger();
+  grid_wait();
   using Team = sampler::Team<1024, sampler::CtaSync>;
   __shared__ sampler::Shared sh;
   const int s = blockIdx.x, b = blockIdx.y;
@@ -57,16 +62,13 @@ __global__ void __launch_bounds__(1024)
 cudaError_t launch_higgs_frame_embed(SlotState st, const bf16* table, bf16* out, int rows, int dim, int vocab,
                                      uint32_t* err, cudaStream_t s) {
   if (dim % 8 || dim / 8 > 1024) return cudaErrorInvalidValue;
-  higgs_frame_embed_kernel<<<rows, dim / 8, 0, s>>>(st, table, out, dim, vocab, err);
-  return cudaGetLastError();
+  return launch_pdl(higgs_frame_embed_kernel, dim3(rows), dim3(dim / 8), 0, s, st, table, out, dim, vocab, err);
 }
 
 cudaError_t launch_higgs_sample(const bf16* logits, int vocab, float temperature, int top_k, const float* uniforms,
                                 const int32_t* force, SlotState st, int32_t* codes, int rows, cudaStream_t s) {
   if (vocab < 1 || vocab > sampler::kVocabMax) return cudaErrorInvalidValue;
-  higgs_sample_kernel<<<dim3(rows, kHiggsBooks), 1024, 0, s>>>(logits, vocab, temperature, top_k, uniforms, force, st,
-                                                               codes);
-  return cudaGetLastError();
+  return launch_pdl(higgs_sample_kernel, dim3(rows, kHiggsBooks), dim3(1024), 0, s, logits, vocab, temperature, top_k, uniforms, force, st, codes);
 }
 
 }  // namespace omni

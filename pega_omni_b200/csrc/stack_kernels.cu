@@ -5,6 +5,8 @@
 // every tensor that crosses HBM is bf16, arithmetic is f32.
 #include "attend.cuh"
 #include "kernels.h"
+#include "pdl.cuh"
+#include "rope.cuh"
 #include "sampler.cuh"
 
 namespace omni {
@@ -15,6 +17,8 @@ namespace omni {
 // (qwen3.cu:18-31).
 __global__ void norm_copy_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, bf16* __restrict__ out,
                                  bf16* __restrict__ res, int dim, float eps) {
+  grid_trigger();
+  grid_wait();
   __shared__ float scratch[32];
   const int64_t at = (int64_t)blockIdx.x * dim + threadIdx.x * 8;
   float v[8], g[8];
@@ -34,6 +38,8 @@ __global__ void norm_copy_kernel(const bf16* __restrict__ x, const bf16* __restr
 // rounded, the norm is taken over the unrounded sum.
 __global__ void add_norm_kernel(const bf16* __restrict__ x, bf16* __restrict__ res, const bf16* __restrict__ w,
                                 bf16* __restrict__ out, int dim, float eps, int every, int which) {
+  grid_trigger();
+  grid_wait();
   __shared__ float scratch[32];
   const int n = blockIdx.x;
   const int64_t at = (int64_t)n * dim + threadIdx.x * 8;
@@ -59,12 +65,14 @@ __global__ void add_norm_kernel(const bf16* __restrict__ x, bf16* __restrict__ r
 // g up channels (the weight layout the tensor-core SwiGLU epilogue wants) instead of [all gate | all up].
 __global__ void silu_mul_kernel(const bf16* __restrict__ gate_up, bf16* __restrict__ act, int inter, int total,
                                 int interleaved) {
+  grid_trigger();
+  grid_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= total) return;
   const int64_t n = i / (inter / 8), c = i % (inter / 8) * 8;
   float g[8], u[8];
   const int64_t g_at = interleaved ? (c / interleaved) * 2 * interleaved + c % interleaved : c;
-  const int64_t u_at = interleaved ? g_at + interleaved : inter + c;
+  const int64_t u_at = interleaved ? g_at + min((int64_t)interleaved, inter - c / interleaved * interleaved) : inter + c;
   ld8(gate_up + n * 2 * inter + g_at, g);
   ld8(gate_up + n * 2 * inter + u_at, u);
 #pragma unroll
@@ -72,25 +80,78 @@ __global__ void silu_mul_kernel(const bf16* __restrict__ gate_up, bf16* __restri
   st8(act + (int64_t)i * 8, g);
 }
 
+// add_norm over a GEMM's summands: a thread owns eight columns, and all its loads - up to eight partial sums, the
+// residual, the gain - are under way together, so the kernel is one L2 round trip and one block reduction long.
+__global__ void add_norm_sum_kernel(const Summands x, bf16* __restrict__ res, const bf16* __restrict__ w,
+                                    bf16* __restrict__ out, int dim, float eps, int every, int which) {
+  grid_trigger();
+  __shared__ float scratch[32];
+  const int n = blockIdx.x, c = threadIdx.x * 8;
+  float g[8], v[8], rv[8];
+  ld8(w + c, g);
+  grid_wait();
+  ld8cg(res + (int64_t)n * dim + c, rv);
+  load_sum8(x, n, c, v);
+  float ss = 0.f;
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    v[k] += rv[k];
+    ss += v[k] * v[k];
+  }
+  ss = warp_add(ss);
+  if ((threadIdx.x & 31) == 0) scratch[threadIdx.x >> 5] = ss;
+  st8(res + (int64_t)n * dim + c, v);
+  if (n % every != which) return;
+  __syncthreads();
+  float total = 0.f;
+  for (int i = 0; i < (int)(blockDim.x + 31) >> 5; ++i) total += scratch[i];
+  const float r = rsqrtf(total / dim + eps);
+#pragma unroll
+  for (int k = 0; k < 8; ++k) v[k] = v[k] * r * g[k];
+  st8(out + (int64_t)(n / every) * dim + c, v);
+}
+
+cudaError_t launch_add_norm_sum(const Summands& x, bf16* res, const bf16* w, bf16* out, int rows, int dim, float eps,
+                                int every, int which, cudaStream_t s) {
+  if (dim % 8 || dim / 8 > 1024 || x.splits > 8) return cudaErrorInvalidValue;
+  return launch_pdl(add_norm_sum_kernel, dim3(rows), dim3(dim / 8), 0, s, x, res, w, out, dim, eps, every, which);
+}
+
+__global__ void interleave_gate_up_kernel(const bf16* __restrict__ src, bf16* __restrict__ dst, int inter, int k,
+                                          int granule) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;  // one 16-byte piece
+  const int64_t per_row = k / 8, total = (int64_t)2 * inter * per_row;
+  if (i >= total) return;
+  const int64_t row = i / per_row, piece = i % per_row;
+  const bool up = row >= inter;
+  const int c = (int)(up ? row - inter : row), group = c / granule;
+  const int64_t out_row = (int64_t)group * 2 * granule + (up ? min(granule, inter - group * granule) : 0) + c % granule;
+  *reinterpret_cast<uint4*>(dst + out_row * k + piece * 8) = *reinterpret_cast<const uint4*>(src + row * k + piece * 8);
+}
+
+cudaError_t launch_interleave_gate_up(const bf16* src, bf16* dst, int inter, int k, int granule, cudaStream_t s) {
+  if (k % 8 || granule < 1) return cudaErrorInvalidValue;
+  const int64_t pieces = (int64_t)2 * inter * (k / 8);
+  interleave_gate_up_kernel<<<(unsigned)((pieces + 255) / 256), 256, 0, s>>>(src, dst, inter, k, granule);
+  return cudaGetLastError();
+}
+
 cudaError_t launch_norm_copy(const bf16* x, const bf16* w, bf16* out, bf16* res, int rows, int dim, float eps,
                              cudaStream_t s) {
   if (dim % 8 || dim / 8 > 1024) return cudaErrorInvalidValue;
-  norm_copy_kernel<<<rows, dim / 8, 0, s>>>(x, w, out, res, dim, eps);
-  return cudaGetLastError();
+  return launch_pdl(norm_copy_kernel, dim3(rows), dim3(dim / 8), 0, s, x, w, out, res, dim, eps);
 }
 
 cudaError_t launch_add_norm(const bf16* x, bf16* res, const bf16* w, bf16* out, int rows, int dim, float eps,
                             int every, int which, cudaStream_t s) {
   if (dim % 8 || dim / 8 > 1024) return cudaErrorInvalidValue;
-  add_norm_kernel<<<rows, dim / 8, 0, s>>>(x, res, w, out, dim, eps, every, which);
-  return cudaGetLastError();
+  return launch_pdl(add_norm_kernel, dim3(rows), dim3(dim / 8), 0, s, x, res, w, out, dim, eps, every, which);
 }
 
 cudaError_t launch_silu_mul(const bf16* gate_up, bf16* act, int rows, int inter, int interleaved, cudaStream_t s) {
   const int total = rows * (inter / 8);
-  if (interleaved && (inter % interleaved || interleaved % 8)) return cudaErrorInvalidValue;
-  silu_mul_kernel<<<(total + 255) / 256, 256, 0, s>>>(gate_up, act, inter, total, interleaved);
-  return cudaGetLastError();
+  if (interleaved && (inter % 8 || interleaved % 8)) return cudaErrorInvalidValue;
+  return launch_pdl(silu_mul_kernel, dim3((total + 255) / 256), dim3(256), 0, s, gate_up, act, inter, total, interleaved);
 }
 
 // ---- row -> (sequence, position, page) -----------------------------------------
@@ -129,6 +190,8 @@ __global__ void __launch_bounds__(256) rope_kv_kernel(bf16* __restrict__ qkv, co
                                                       const bf16* __restrict__ k_norm, bf16* __restrict__ kv,
                                                       RowMap map, int hq, int hk, float eps, float theta,
                                                       int kv_pages, uint32_t* err) {
+  grid_trigger();
+  grid_wait();
   constexpr int E = D / 64;  // elements of each half a lane owns
   const int n = blockIdx.x;
   const int head = blockIdx.y * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -176,14 +239,12 @@ cudaError_t launch_rope_kv(bf16* qkv, const bf16* q_norm, const bf16* k_norm, bf
   const int heads = a.q_heads + 2 * a.kv_heads;
   const dim3 grid(rows, (heads + 7) / 8);
   if (a.head_dim == 128)
-    rope_kv_kernel<128><<<grid, 256, 0, s>>>(qkv, q_norm, k_norm, kv, map, a.q_heads, a.kv_heads, a.rms_eps,
-                                             a.rope_theta, kv_pages, err);
-  else if (a.head_dim == 64)
-    rope_kv_kernel<64><<<grid, 256, 0, s>>>(qkv, q_norm, k_norm, kv, map, a.q_heads, a.kv_heads, a.rms_eps,
-                                            a.rope_theta, kv_pages, err);
-  else
-    return cudaErrorInvalidValue;
-  return cudaGetLastError();
+    return launch_pdl(rope_kv_kernel<128>, grid, dim3(256), 0, s, qkv, q_norm, k_norm, kv, map, a.q_heads, a.kv_heads,
+                      a.rms_eps, a.rope_theta, kv_pages, err);
+  if (a.head_dim == 64)
+    return launch_pdl(rope_kv_kernel<64>, grid, dim3(256), 0, s, qkv, q_norm, k_norm, kv, map, a.q_heads, a.kv_heads,
+                      a.rms_eps, a.rope_theta, kv_pages, err);
+  return cudaErrorInvalidValue;
 }
 
 // ---- decode attention -------------------------------------------------------------
@@ -197,6 +258,8 @@ template <int D, int G>
 __global__ void __launch_bounds__(kAttnWarps * 32) attend_kernel(const bf16* __restrict__ qkv,
                                                                  const bf16* __restrict__ kv, bf16* __restrict__ out,
                                                                  RowMap map, int hq, int hk, float scale, uint32_t* err) {
+  grid_trigger();
+  grid_wait();
   extern __shared__ __align__(128) unsigned char attend_slots[];
   __shared__ AttnShared<D, G> sh;
   __shared__ __align__(8) uint64_t bars[kAttnWarps * kAttnSlots];
@@ -227,8 +290,8 @@ static cudaError_t launch_attend_dg(const bf16* qkv, const bf16* kv, bf16* out, 
       raised[device] = true;
     }
   }
-  attend_kernel<D, G><<<dim3(rows, hk), kAttnWarps * 32, smem, s>>>(qkv, kv, out, map, hq, hk, 1.f / sqrtf((float)D), err);
-  return cudaGetLastError();
+  return launch_pdl(attend_kernel<D, G>, dim3(rows, hk), dim3(kAttnWarps * 32), smem, s, qkv, kv, out, map, hq, hk,
+                    1.f / sqrtf((float)D), err);
 }
 
 template <int D>
@@ -250,6 +313,196 @@ cudaError_t launch_attend(const bf16* qkv, const bf16* kv, bf16* out, const RowM
   if (a.q_heads % a.kv_heads) return cudaErrorInvalidValue;
   if (a.head_dim == 128) return launch_attend_d<128>(qkv, kv, out, map, rows, a, err, s);
   if (a.head_dim == 64) return launch_attend_d<64>(qkv, kv, out, map, rows, a, err, s);
+  return cudaErrorInvalidValue;
+}
+
+// ---- decode: q/k norm + RoPE + KV write + attention in one kernel ------------------------------------------------
+// One CTA of W warps per (sequence, kv head). The G query heads, the key and the value of a row are dealt to the warps;
+// q goes to shared memory, k and v to the row's slot, and the same CTA then attends to them. The pages that earlier
+// calls filled are asked for before grid_wait(): they come through bulk copies into the warps' staging slots while
+// the projection before this kernel still runs. The row's own page is read with ordinary loads after the write.
+// W: enough warps that one wave of CTAs has every page of a long context under way.
+
+template <int D, int G, int W>
+__global__ void __launch_bounds__(W * 32)
+    rope_attend_kernel(const bf16* __restrict__ qkv, const QkvTable lookup, const bf16* __restrict__ q_norm,
+                       const bf16* __restrict__ k_norm, bf16* kv, bf16* __restrict__ out, RowMap map, int hq, int hk,
+                       float eps, float theta, float scale, int kv_pages, uint32_t* err) {
+  constexpr int E = D / 64, VE = D / 32, PV = D / 32;
+  grid_trigger();
+  extern __shared__ __align__(128) unsigned char ra_slots[];
+  __shared__ AttnShared<D, G, W> sh;
+  __shared__ __align__(8) uint64_t bars[W];
+  const int seq = blockIdx.x, kh = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int per = map.pages ? 1 : map.per;
+  const int32_t* pages = map.pages ? map.pages + map.indptr[map.seq ? map.seq[seq] : seq] : nullptr;
+  float qwl[E], qwh[E], kwl[E], kwh[E];
+#pragma unroll
+  for (int e = 0; e < E; ++e) {
+    qwl[e] = __bfloat162float(q_norm[lane * E + e]), qwh[e] = __bfloat162float(q_norm[D / 2 + lane * E + e]);
+    kwl[e] = __bfloat162float(k_norm[lane * E + e]), kwh[e] = __bfloat162float(k_norm[D / 2 + lane * E + e]);
+  }
+  if (lane == 0) {
+    sm100::mbar_init(sm100::smem_addr(&bars[warp]), 1);
+    sm100::mbar_init_fence();
+  }
+  __syncwarp();
+  bf16* mine = reinterpret_cast<bf16*>(ra_slots + (size_t)warp * kv_block_bytes<D>());
+  auto issue = [&](int pi) {
+    int64_t page = pages[pi];
+    if (page < 0 || page >= kv_pages) {
+      raise(err, kErrBadIndex);
+      page = 0;
+    }
+    sm100::mbar_expect_tx(sm100::smem_addr(&bars[warp]), kv_block_bytes<D>());
+    sm100::bulk_load(sm100::smem_addr(mine), kv + kv_offset<D>(page, hk, kh, 0, 0), kv_block_bytes<D>(), sm100::smem_addr(&bars[warp]));
+  };
+  uint32_t parity = 0;
+  for (int r = 0; r < per; ++r) {
+    const int n = seq * per + r;
+    const int pos = map.pages ? map.pos[n] : map.base + r;
+    const int len = pos + 1, npages = (len + 15) >> 4, last = npages - 1;
+    float cs[E], sn[E];
+    rope_angles<D>(lane, pos, theta, cs, sn);
+    const int64_t slot = map.pages ? map.slot[n] : (int64_t)seq * 16 + pos;
+    int64_t page = slot >> 4;
+    const int tok = (int)(slot & 15);
+    if (page < 0 || page >= kv_pages) {
+      if (tid == 0) raise(err, kErrBadIndex);
+      page = 0;
+    }
+    if (warp < last && lane == 0) issue(warp);  // (map.pages only: a dense sequence has one page)
+    if (r == 0) grid_wait();
+    const bf16* row = lookup.table ? lookup.table + (int64_t)lookup.codes[n * 16 + lookup.group] * ((hq + 2 * hk) * D)
+                                   : qkv + (int64_t)n * ((hq + 2 * hk) * D);
+    for (int job = warp; job < G + 2; job += W) {
+      if (job == G + 1) {  // value: a plain copy
+        bf16* dst = kv + kv_offset<D>(page, hk, kh, 1, tok);
+        const bf16* src = row + (hq + hk + kh) * D;
+        if constexpr (VE == 4) *reinterpret_cast<uint2*>(dst + lane * 4) = __ldcg(reinterpret_cast<const uint2*>(src + lane * 4));
+        else *reinterpret_cast<uint32_t*>(dst + lane * 2) = __ldcg(reinterpret_cast<const uint32_t*>(src + lane * 2));
+        continue;
+      }
+      const bool is_q = job < G;
+      const bf16* src = row + (is_q ? kh * G + job : hq + kh) * D;
+      float lo[E], hi[E];
+      if constexpr (E == 2) {
+        const uint32_t a2 = __ldcg(reinterpret_cast<const uint32_t*>(src) + lane), b2 = __ldcg(reinterpret_cast<const uint32_t*>(src + D / 2) + lane);
+        lo[0] = __uint_as_float(a2 << 16), lo[1] = __uint_as_float(a2 & 0xffff0000u);
+        hi[0] = __uint_as_float(b2 << 16), hi[1] = __uint_as_float(b2 & 0xffff0000u);
+      } else {
+        lo[0] = __uint_as_float((uint32_t)__ldcg(reinterpret_cast<const uint16_t*>(src) + lane) << 16);
+        hi[0] = __uint_as_float((uint32_t)__ldcg(reinterpret_cast<const uint16_t*>(src + D / 2) + lane) << 16);
+      }
+      if (is_q) rope_head<D>(lo, hi, qwl, qwh, cs, sn, eps);
+      else rope_head<D>(lo, hi, kwl, kwh, cs, sn, eps);
+      bf16* kdst = kv + kv_offset<D>(page, hk, kh, 0, tok);
+#pragma unroll
+      for (int e = 0; e < E; ++e) {
+        const int i = lane * E + e;
+        if (is_q) {
+          sh.qs[job][i] = lo[e], sh.qs[job][D / 2 + i] = hi[e];
+        } else {
+          kdst[i] = __float2bfloat16(lo[e]), kdst[D / 2 + i] = __float2bfloat16(hi[e]);
+        }
+      }
+    }
+    __threadfence_block();
+    __syncthreads();
+    float m[G], l[G], acc[G][PV];
+#pragma unroll
+    for (int g = 0; g < G; ++g) {
+      m[g] = -INFINITY, l[g] = 0.f;
+#pragma unroll
+      for (int d = 0; d < PV; ++d) acc[g][d] = 0.f;
+    }
+    for (int pi = warp; pi < npages; pi += W) {
+      KvBlock<D> blk;
+      if (pi < last) {
+        sm100::mbar_wait(sm100::smem_addr(&bars[warp]), parity, err);
+        parity ^= 1u;
+        blk.load(mine, lane);
+        __syncwarp();  // the block is in registers: its slot takes the warp's next one
+        if (lane == 0 && pi + W < last) issue(pi + W);
+      } else {
+        blk.load(kv + kv_offset<D>(page, hk, kh, 0, 0), lane);
+      }
+      page_update<D, G>(blk, sh.qs, min(16, len - pi * 16), scale, lane, m, l, acc);
+    }
+#pragma unroll
+    for (int g = 0; g < G; ++g) {
+      if (lane == 0) sh.ms[warp][g] = m[g], sh.ls[warp][g] = l[g];
+#pragma unroll
+      for (int d = 0; d < PV; ++d) sh.os[warp][g][lane * PV + d] = acc[g][d];
+    }
+    __syncthreads();
+    const int live = min(W, npages);  // warps that held a page
+    for (int i = tid; i < G * D; i += W * 32) {
+      const int g = i / D, d = i % D;
+      float top = -INFINITY;
+      for (int w = 0; w < live; ++w) top = fmaxf(top, sh.ms[w][g]);
+      float num = 0.f, den = 0.f;
+      for (int w = 0; w < live; ++w) {
+        const float e = __expf(sh.ms[w][g] - top);
+        num += sh.os[w][g][d] * e;
+        den += sh.ls[w][g] * e;
+      }
+      out[((int64_t)n * hq + kh * G) * D + i] = __float2bfloat16(num / den);
+    }
+    if (r + 1 < per) __syncthreads();  // q and the warps' states are free for the next row
+  }
+}
+
+template <int D, int G, int W>
+static cudaError_t launch_rope_attend_dgw(const bf16* qkv, const QkvTable& lookup, const bf16* q_norm, const bf16* k_norm,
+                                          bf16* kv, bf16* out, const RowMap& map, int seqs, const AttnShape& a,
+                                          int kv_pages, uint32_t* err, cudaStream_t s) {
+  const size_t smem = map.pages ? (size_t)W * kv_block_bytes<D>() : 0;
+  if (smem + sizeof(AttnShared<D, G, W>) > 40 * 1024) {  // per device and instantiation: above the default limit of dynamic shared memory
+    static bool raised[64] = {};
+    int device = 0;
+    if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= 64) return cudaErrorInvalidDevice;
+    if (!raised[device]) {
+      const cudaError_t e = cudaFuncSetAttribute(rope_attend_kernel<D, G, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      if (e != cudaSuccess) return e;
+      raised[device] = true;
+    }
+  }
+  return launch_pdl(rope_attend_kernel<D, G, W>, dim3(seqs, a.kv_heads), dim3(W * 32), smem, s, qkv, lookup, q_norm, k_norm,
+                    kv, out, map, a.q_heads, a.kv_heads, a.rms_eps, a.rope_theta, 1.f / sqrtf((float)D), kv_pages, err);
+}
+
+template <int D, int G>
+static cudaError_t launch_rope_attend_dg(const bf16* qkv, const QkvTable& lookup, const bf16* q_norm, const bf16* k_norm,
+                                         bf16* kv, bf16* out, const RowMap& map, int rows, const AttnShape& a,
+                                         int kv_pages, uint32_t* err, cudaStream_t s) {
+  const int seqs = map.pages ? rows : rows / map.per;
+  // a few sequences: eight warps each (more would not leave a thread the registers of a page); many: four, several CTAs per SM
+  if (map.pages && seqs * a.kv_heads <= 148)
+    return launch_rope_attend_dgw<D, G, 8>(qkv, lookup, q_norm, k_norm, kv, out, map, seqs, a, kv_pages, err, s);
+  return launch_rope_attend_dgw<D, G, 4>(qkv, lookup, q_norm, k_norm, kv, out, map, seqs, a, kv_pages, err, s);
+}
+
+template <int D>
+static cudaError_t launch_rope_attend_d(const bf16* qkv, const QkvTable& lookup, const bf16* q_norm, const bf16* k_norm,
+                                        bf16* kv, bf16* out, const RowMap& map, int rows, const AttnShape& a,
+                                        int kv_pages, uint32_t* err, cudaStream_t s) {
+  switch (a.q_heads / a.kv_heads) {
+    case 1: return launch_rope_attend_dg<D, 1>(qkv, lookup, q_norm, k_norm, kv, out, map, rows, a, kv_pages, err, s);
+    case 2: return launch_rope_attend_dg<D, 2>(qkv, lookup, q_norm, k_norm, kv, out, map, rows, a, kv_pages, err, s);
+    case 4: return launch_rope_attend_dg<D, 4>(qkv, lookup, q_norm, k_norm, kv, out, map, rows, a, kv_pages, err, s);
+    case 5: return launch_rope_attend_dg<D, 5>(qkv, lookup, q_norm, k_norm, kv, out, map, rows, a, kv_pages, err, s);
+    case 8: return launch_rope_attend_dg<D, 8>(qkv, lookup, q_norm, k_norm, kv, out, map, rows, a, kv_pages, err, s);
+    default: return cudaErrorInvalidValue;
+  }
+}
+
+cudaError_t launch_rope_attend(const bf16* qkv, const QkvTable& lookup, const bf16* q_norm, const bf16* k_norm, bf16* kv,
+                               bf16* out, const RowMap& map, int rows, const AttnShape& a, int kv_pages, uint32_t* err,
+                               cudaStream_t s) {
+  if (a.q_heads % a.kv_heads) return cudaErrorInvalidValue;
+  if (a.head_dim == 128) return launch_rope_attend_d<128>(qkv, lookup, q_norm, k_norm, kv, out, map, rows, a, kv_pages, err, s);
+  if (a.head_dim == 64) return launch_rope_attend_d<64>(qkv, lookup, q_norm, k_norm, kv, out, map, rows, a, kv_pages, err, s);
   return cudaErrorInvalidValue;
 }
 

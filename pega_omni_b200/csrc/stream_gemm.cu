@@ -1,0 +1,334 @@
+// The decode-sized GEMM of the kernel chains (see stream_gemm.h).
+#include "stream_gemm.h"
+
+#include <algorithm>
+
+#include "pdl.cuh"
+#include "sm100.cuh"
+
+namespace omni {
+namespace {
+
+constexpr int kKb = 64;  // K elements per k-block: one 128-byte swizzle row
+constexpr int kMaxSlots = 8, kIssuers = 4;
+constexpr int kThreads = 32 * (2 + kIssuers);  // W producer, X producer, four MMA issuers that are also the epilogue
+
+struct StreamArgs {
+  bf16* y;
+  float* part;
+  const bf16* bias;
+  uint32_t* err;
+  int N, rows, M, bn, tn, splits, kbs, stages, slots, issuers, ldy, kind, vec;
+  uint32_t acc_cols, tmem_cols;
+};
+
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}\n"
+      : "=r"(p));
+  return p != 0;
+}
+
+__device__ __forceinline__ void tmem_ld8_issue(uint32_t taddr, uint32_t (&r)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "r"(taddr)
+               : "memory");
+}
+template <int NR>
+__device__ __forceinline__ void tmem_ld8_fence(uint32_t (&r)[NR][8]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+  for (int i = 0; i < NR; ++i)
+    asm volatile("" : "+r"(r[i][0]), "+r"(r[i][1]), "+r"(r[i][2]), "+r"(r[i][3]), "+r"(r[i][4]), "+r"(r[i][5]), "+r"(r[i][6]), "+r"(r[i][7])::"memory");
+}
+
+// Eight columns of the accumulators, summed in issuer order.
+__device__ __forceinline__ void acc_cols8(uint32_t lane_addr, int col, const StreamArgs& a, float (&v)[8]) {
+  uint32_t r[kIssuers][8];
+#pragma unroll
+  for (int i = 0; i < kIssuers; ++i)
+    if (i < a.issuers) tmem_ld8_issue(lane_addr + (uint32_t)i * a.acc_cols + col, r[i]);
+    else {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) r[i][j] = 0u;
+    }
+  tmem_ld8_fence<kIssuers>(r);
+#pragma unroll
+  for (int j = 0; j < 8; ++j) v[j] = (__uint_as_float(r[0][j]) + __uint_as_float(r[1][j])) + (__uint_as_float(r[2][j]) + __uint_as_float(r[3][j]));
+}
+
+template <int OUT>
+__global__ void __launch_bounds__(kThreads, 1)
+    stream_gemm_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap xmap,
+                       const StreamArgs a) {
+  using namespace sm100;
+  extern __shared__ unsigned char stream_smem_raw[];
+  __shared__ __align__(8) uint64_t bars_s[3 * kMaxSlots + 1];
+  __shared__ uint32_t tmem_slot_s;
+  const uint32_t base = (smem_addr(stream_smem_raw) + 1023u) & ~1023u;
+  const uint32_t bars = smem_addr(bars_s);
+  auto full_w = [&](int s) { return bars + 8u * s; };
+  auto full_x = [&](int s) { return bars + 8u * (kMaxSlots + s); };
+  auto empty = [&](int s) { return bars + 8u * (2 * kMaxSlots + s); };
+  const uint32_t acc_bar = bars + 8u * (3 * kMaxSlots);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int tile = blockIdx.x, split = blockIdx.y, m0 = blockIdx.z * 128;
+  const int st0 = (int)((int64_t)a.stages * split / a.splits), st1 = (int)((int64_t)a.stages * (split + 1) / a.splits);
+  const int n_st = st1 - st0;
+  const uint32_t x_slice = (uint32_t)a.bn * 128u, w_slice = (uint32_t)a.tn * 128u;
+  const uint32_t x_bytes = x_slice * (uint32_t)a.kbs, w_bytes = w_slice * (uint32_t)a.kbs, slot_bytes = x_bytes + w_bytes;
+
+  auto load_w = [&](int i, int slot) {  // stage st0 + i's weights
+    mbar_expect_tx(full_w(slot), w_bytes);
+    tma_load_3d(base + (uint32_t)slot * slot_bytes + x_bytes, &wmap, full_w(slot), 0, tile * a.tn, (st0 + i) * a.kbs, kEvictFirst);
+  };
+  // after an abort: no copy may land in shared memory once the CTA has left
+  auto drain = [&](uint32_t first_bar, int issued) {
+    for (int i = max(0, issued - a.slots); i < issued; ++i)
+      mbar_wait(first_bar + 8u * (i % a.slots), (uint32_t)(i / a.slots) & 1u, a.err);
+  };
+
+  if (threadIdx.x == 0) {
+    prefetch_tensormap(&wmap);
+    for (int s = 0; s < a.slots; ++s) mbar_init(full_w(s), 1), mbar_init(full_x(s), 1), mbar_init(empty(s), 1);
+    mbar_init(acc_bar, a.issuers);
+    mbar_init_fence();
+    for (int i = 0; i < min(a.slots, n_st); ++i) load_w(i, i);
+    prefetch_tensormap(&xmap);
+  }
+  if (warp == 2) tmem_alloc(smem_addr(&tmem_slot_s), a.tmem_cols);
+  tc_fence_before_sync();
+  __syncthreads();
+  tc_fence_after_sync();
+  const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(&tmem_slot_s);
+  // only now: were the next kernel let in before this CTA has its TMEM columns, it could take them and then wait for
+  // this kernel to complete
+  grid_trigger();
+
+  if (warp == 0) {
+    if (lane == 0) {
+      int slot = 0;
+      uint32_t phase = 0;
+      for (int i = a.slots; i < n_st; ++i) {
+        if (!mbar_wait(empty(slot), phase, a.err)) {
+          drain(full_w(0), i);
+          break;
+        }
+        load_w(i, slot);
+        if (++slot == a.slots) slot = 0, phase ^= 1u;
+      }
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {
+      grid_wait();
+      asm volatile("fence.proxy.async.global;" ::: "memory");  // rows written by ordinary stores, read by TMA
+      int slot = 0;
+      uint32_t phase = 0;
+      for (int i = 0; i < n_st; ++i) {
+        if (i >= a.slots && !mbar_wait(empty(slot), phase ^ 1u, a.err)) {
+          drain(full_x(0), i);
+          break;
+        }
+        mbar_expect_tx(full_x(slot), x_bytes);
+        tma_load_3d(base + (uint32_t)slot * slot_bytes, &xmap, full_x(slot), 0, m0, (st0 + i) * a.kbs, kEvictLast);
+        if (++slot == a.slots) slot = 0, phase ^= 1u;
+      }
+    }
+  } else {
+    // issuer `me` takes stages me, me + issuers, ... into its own accumulator: one thread issues an MMA only every
+    // 80 cycles or so, half of what the tensor pipe takes at these shapes
+    const int me = warp - 2;
+    grid_wait();
+    if (me < a.issuers) {
+      const uint32_t idesc = idesc_bf16_f32(a.M, a.tn), acc = tmem + (uint32_t)me * a.acc_cols;
+      bool alive = true;
+      int slot = me % a.slots;
+      uint32_t phase = (uint32_t)(me / a.slots) & 1u;
+      for (int i = me; i < n_st; i += a.issuers) {
+        alive = mbar_wait(full_w(slot), phase, a.err) && mbar_wait(full_x(slot), phase, a.err);
+        if (!alive) break;
+        tc_fence_after_sync();
+        const uint64_t adesc = kmajor_sw128_desc(base + (uint32_t)slot * slot_bytes);
+        const uint64_t bdesc = kmajor_sw128_desc(base + (uint32_t)slot * slot_bytes + x_bytes);
+        if (elect_one()) {
+          for (int j = 0; j < a.kbs; ++j) {
+            const uint64_t ad = adesc + (uint64_t)((uint32_t)j * (x_slice >> 4)), bd = bdesc + (uint64_t)((uint32_t)j * (w_slice >> 4));
+#pragma unroll
+            for (int k = 0; k < kKb / 16; ++k)
+              mma_bf16(acc, ad + (uint64_t)(k * 2), bd + (uint64_t)(k * 2), idesc, (i > me || j > 0 || k > 0) ? 1u : 0u);
+          }
+          mma_commit(empty(slot));
+        }
+        __syncwarp();
+        slot += a.issuers;
+        while (slot >= a.slots) slot -= a.slots, phase ^= 1u;
+      }
+      if (alive && elect_one()) mma_commit(acc_bar);
+      __syncwarp();
+    }
+    const bool ok = mbar_wait(acc_bar, 0, a.err);
+    tc_fence_after_sync();
+    const int quad = warp & 3;
+    const uint32_t lane_addr = tmem + ((uint32_t)(quad * 32) << 16);
+    // M = 128: row = TMEM lane; M = 64: rows 16 q .. 16 q + 15 sit in the first sixteen lanes of quadrant q
+    const int r = a.M == 128 ? quad * 32 + lane : quad * 16 + lane;
+    const int m = m0 + r;
+    const bool row_live = m < a.rows && (a.M == 128 || lane < 16);
+    const bool warp_live = m0 + (a.M == 128 ? quad * 32 : quad * 16) < a.rows;
+    if (ok && warp_live) {
+      if constexpr (OUT == kStreamSwiglu) {
+        // the tile's rows are `half` gate channels, then their up channels (the last tile may hold fewer)
+        const int ch0 = tile * (a.tn >> 1), half = min(a.tn >> 1, (a.N >> 1) - ch0);
+        for (int c = 0; c < half; c += 8) {
+          float g[8], u[8];
+          acc_cols8(lane_addr, c, a, g);
+          acc_cols8(lane_addr, half + c, a, u);
+          if (!row_live) continue;
+          float o[8];
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            const float gg = bf16_round(g[j]);
+            // the fast division is within 2 ulp of an f32 that is rounded to bf16 next
+            o[j] = bf16_round(__fdividef(gg, 1.f + __expf(-gg))) * bf16_round(u[j]);
+          }
+          st8(a.y + (size_t)m * a.ldy + ch0 + c, o);
+        }
+      } else {
+        const int n0 = tile * a.tn;
+        for (int c = 0; c < a.tn; c += 8) {
+          float v[8];
+          acc_cols8(lane_addr, c, a, v);
+          if (!row_live || n0 + c >= a.N) continue;
+          if constexpr (OUT == kStreamPartials) {
+            float* dst = a.part + ((size_t)split * a.rows + m) * a.N + n0 + c;
+            *reinterpret_cast<float4*>(dst) = make_float4(v[0], v[1], v[2], v[3]);
+            *reinterpret_cast<float4*>(dst + 4) = make_float4(v[4], v[5], v[6], v[7]);
+          } else {
+            bf16* dst = a.y + (size_t)m * a.ldy + n0 + c;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+              v[j] = bf16_round(v[j]);
+              if (a.kind != kEpiNone && n0 + c + j < a.N) {
+                v[j] = bf16_round(v[j] + __bfloat162float(a.bias[n0 + c + j]));
+                if (a.kind == kEpiBiasSilu) v[j] = v[j] / (1.f + __expf(-v[j]));
+              }
+            }
+            if (a.vec) st8(dst, v);
+            else
+              for (int j = 0; j < 8 && n0 + c + j < a.N; ++j) dst[j] = __float2bfloat16(v[j]);
+          }
+        }
+      }
+    }
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  if (warp == 2) tmem_dealloc(tmem, a.tmem_cols);
+}
+
+// More than half of an SM's shared memory whatever the ring needs: kernels of a chain start on whichever SM has room, so
+// CTAs small enough to share an SM would pile up on the first ones free and leave the rest of the chip idle.
+constexpr int kMinSmem = 116 * 1024, kMaxSmem = 200 * 1024;
+
+}  // namespace
+
+void stream_configure() {
+  cudaFuncSetAttribute(stream_gemm_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
+  cudaFuncSetAttribute(stream_gemm_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
+  cudaFuncSetAttribute(stream_gemm_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
+}
+
+bool stream_supports(int N, int K, int rows) { return K % kKb == 0 && K >= kKb && N >= 1 && rows >= 1; }
+
+int stream_granule(int inter, int sm_count) {
+  int waves = 1;
+  auto width = [&](int w) { return (2 * inter + sm_count * w - 1) / (sm_count * w); };
+  while (width(waves) > 256) ++waves;
+  return std::max(16, (width(waves) + 15) / 16 * 16) / 2;
+}
+
+// Weight rows per tile (tn) and K splits: the shape with the shortest estimated time after the inputs are there. A CTA
+// pulls its tile's inputs at about 170 GB/s whatever the number of CTAs (they all read the same rows), the tensor pipe
+// takes (M + tn) / 4 cycles per 16 elements of K, stores leave an SM at 57 GB/s, and weights only count where a shape
+// loads some SMs more than others, since they were asked for before the inputs were there.
+static double stream_cost(int N, int K, int rows, int M, int bn, int tn, int S, int out, int sms, int row_tiles) {
+  const int ctas = (N + tn - 1) / tn * S * row_tiles;
+  const double per_sm = (ctas + sms - 1) / sms, kc = (double)K / S;
+  const double t_x = kc * 2 * bn * per_sm / 170e3;
+  const double t_w = kc * 2 * tn * per_sm / std::min(170e3, 6.5e6 / std::min(ctas, sms));
+  const double t_mma = kc / 16 * std::max(0.25 * (M + tn), tn > 128 ? 40.0 : 20.0) * per_sm / 1900;
+  const double t_out = std::min(rows, 128) * tn * (out == kStreamPartials ? 4.0 : 2.0) * per_sm / 57e3;
+  return std::max({t_x + 0.3 * t_mma, t_mma, 0.5 * t_x + t_w}) + t_out + 0.1 * S;
+}
+
+int stream_plan(StreamGemmPlan* plan, const bf16* w, int N, int K, const bf16* x, int rows, int out, bf16* y, int ldy,
+                float* part, Epilogue epi, int sm_count, int granule, int force_splits) {
+  if (!stream_supports(N, K, rows)) return -2;
+  if (out == kStreamPartials && N % 8) return -2;
+  if (out == kStreamSwiglu && (granule < 8 || granule % 8 || granule > 128 || N % 16 || ldy % 8)) return -2;
+  if ((reinterpret_cast<uintptr_t>(w) & 15) || (reinterpret_cast<uintptr_t>(x) & 15)) return -3;
+  StreamGemmPlan& p = *plan;
+  p.N = N, p.K = K, p.rows = rows, p.out = out, p.y = y, p.ldy = ldy, p.part = part, p.epi = epi;
+  p.M = rows <= 64 ? 64 : 128;
+  p.bn = std::min(128, (rows + 7) / 8 * 8);
+  const int nkb = K / kKb, row_tiles = (rows + 127) / 128;
+  if (out == kStreamSwiglu) {
+    p.tn = 2 * granule, p.splits = 1;
+  } else {
+    double best = 1e30;
+    for (int tn = 16; tn <= 256; tn += 16)
+      for (int S : {1, 2, 4, 8}) {
+        if (S > 1 && (out != kStreamPartials || S * 2 > nkb)) break;
+        if (force_splits > 0 && S != force_splits) continue;
+        const double cost = stream_cost(N, K, rows, p.M, p.bn, tn, S, out, sm_count, row_tiles);
+        if (cost < best - 1e-9) best = cost, p.tn = tn, p.splits = S;
+      }
+    if (best > 1e29) return -2;
+  }
+  // k-blocks per stage: as many (up to four) as leave three stages in the ring; a copy costs its thread about 0.16 us
+  const int kb_bytes = (p.bn + p.tn) * 128, room = kMaxSmem - 1024 - (p.M - p.bn) * 128;
+  p.kbs = 1;
+  for (int k : {4, 2})
+    if (k * 2 <= nkb / p.splits && room / (k * kb_bytes) >= 3) {
+      p.kbs = k;
+      break;
+    }
+  p.stages = (nkb + p.kbs - 1) / p.kbs;
+  const int per = (p.stages + p.splits - 1) / p.splits;
+  p.slots = std::min({kMaxSlots, per, room / (p.kbs * kb_bytes)});
+  if (p.slots < 1 || p.stages < p.splits) return -2;
+  p.acc_cols = p.tn <= 32 ? 32 : p.tn <= 64 ? 64 : p.tn <= 128 ? 128 : 256;
+  // a slot belongs to one issuer for good (slots is a multiple of issuers): a wait on a barrier parity means "this phase"
+  // only to a thread that has seen every phase of the barrier. Every split has a stage for each issuer.
+  p.issuers = std::min({kIssuers, p.stages / p.splits, 512 / p.acc_cols, p.slots});
+  p.slots -= p.slots % p.issuers;
+  const uint64_t wd[3] = {kKb, (uint64_t)N, (uint64_t)nkb}, ws[2] = {(uint64_t)K * 2, kKb * 2};
+  const uint32_t wb[3] = {kKb, (uint32_t)p.tn, (uint32_t)p.kbs};
+  if (tc_encode_bf16(&p.wmap, w, 3, wd, ws, wb) != 0) return -4;
+  const uint64_t xd[3] = {kKb, (uint64_t)rows, (uint64_t)nkb}, xs[2] = {(uint64_t)K * 2, kKb * 2};
+  const uint32_t xb[3] = {kKb, (uint32_t)p.bn, (uint32_t)p.kbs};
+  if (tc_encode_bf16(&p.xmap, x, 3, xd, xs, xb) != 0) return -4;
+  return 0;
+}
+
+cudaError_t stream_launch(const StreamGemmPlan& p, uint32_t* err, cudaStream_t stream) {
+  StreamArgs a;
+  a.y = p.y, a.part = p.part, a.bias = p.epi.bias, a.err = err, a.kind = p.epi.kind;
+  a.N = p.N, a.rows = p.rows, a.M = p.M, a.bn = p.bn, a.tn = p.tn, a.splits = p.splits, a.kbs = p.kbs;
+  a.stages = p.stages, a.slots = p.slots, a.issuers = p.issuers, a.ldy = p.ldy;
+  a.vec = p.ldy % 8 == 0 && p.N % 8 == 0 && (reinterpret_cast<uintptr_t>(p.y) & 15) == 0;
+  a.acc_cols = (uint32_t)p.acc_cols;
+  a.tmem_cols = 32;
+  while (a.tmem_cols < a.acc_cols * (uint32_t)p.issuers) a.tmem_cols *= 2;
+  const size_t smem = std::max<size_t>(kMinSmem, 1024 + (size_t)p.slots * p.kbs * (p.bn + p.tn) * 128 + (size_t)(p.M - p.bn) * 128);
+  const dim3 grid((p.N + p.tn - 1) / p.tn, p.splits, (p.rows + 127) / 128);
+  switch (p.out) {
+    case kStreamBf16: return launch_pdl(stream_gemm_kernel<0>, grid, dim3(kThreads), smem, stream, p.wmap, p.xmap, a);
+    case kStreamPartials: return launch_pdl(stream_gemm_kernel<1>, grid, dim3(kThreads), smem, stream, p.wmap, p.xmap, a);
+    default: return launch_pdl(stream_gemm_kernel<2>, grid, dim3(kThreads), smem, stream, p.wmap, p.xmap, a);
+  }
+}
+
+}  // namespace omni

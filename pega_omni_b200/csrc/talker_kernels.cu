@@ -4,6 +4,7 @@
 // device error word instead of reading out of bounds.
 #include "kernels.h"
 #include "sampler.cuh"
+#include "pdl.cuh"
 
 namespace omni {
 
@@ -11,6 +12,8 @@ constexpr int kGroups = 16;
 
 __global__ void gather_kernel(const int32_t* __restrict__ ids, int stride, const bf16* __restrict__ table,
                               int table_rows, bf16* __restrict__ out, int dim, uint32_t* err) {
+  grid_trigger();
+  grid_wait();
   const int c = threadIdx.x * 8;
   int64_t id = ids[(int64_t)blockIdx.x * stride];
   if (id < 0 || id >= table_rows) {
@@ -25,6 +28,8 @@ __global__ void gather_kernel(const int32_t* __restrict__ ids, int stride, const
 __global__ void prompt_codec_kernel(bf16* __restrict__ x, const bf16* __restrict__ bias,
                                     const bf16* __restrict__ table, int table_rows, const int32_t* __restrict__ ids,
                                     int dim, uint32_t* err) {
+  grid_trigger();
+  grid_wait();
   const int c = threadIdx.x * 8;
   bf16* row = x + (int64_t)blockIdx.x * dim + c;
   int id = ids[blockIdx.x];
@@ -51,12 +56,12 @@ __device__ __forceinline__ int32_t* slot_of(const SlotState& st, int s) {
 
 // `talker_frame_embed` (talker.cu:76-96): f32 sum in the order pad, codebook 0,
 // codebooks 1.., one rounding.
-__global__ void frame_embed_kernel(SlotState st, const bf16* __restrict__ pad, const bf16* __restrict__ codec_emb,
-                                   int vocab, const bf16* __restrict__ p_emb, int p_vocab, int groups,
-                                   bf16* __restrict__ out, int dim, uint32_t* err) {
+__device__ __forceinline__ void frame_embed_row(const SlotState& st, const bf16* pad, const bf16* codec_emb, int vocab,
+                                                const bf16* p_emb, int p_vocab, int groups, int dim, uint32_t* err,
+                                                float (&acc)[8]) {
   const int s = blockIdx.x, c = threadIdx.x * 8;
   const int32_t* codes = slot_of(st, s);
-  float acc[8], e[8];
+  float e[8];
   ld8(pad + c, acc);
 #pragma unroll
   for (int k = 0; k < 8; ++k) acc[k] = 0.f + acc[k];
@@ -68,6 +73,7 @@ __global__ void frame_embed_kernel(SlotState st, const bf16* __restrict__ pad, c
   ld8(codec_emb + (int64_t)c0 * dim + c, e);
 #pragma unroll
   for (int k = 0; k < 8; ++k) acc[k] += e[k];
+#pragma unroll 5
   for (int g = 1; g < groups; ++g) {
     int cg = codes[g];
     if (cg < 0 || cg >= p_vocab) {
@@ -78,12 +84,43 @@ __global__ void frame_embed_kernel(SlotState st, const bf16* __restrict__ pad, c
 #pragma unroll
     for (int k = 0; k < 8; ++k) acc[k] += e[k];
   }
-  st8(out + (int64_t)s * dim + c, acc);
+}
+
+__global__ void frame_embed_kernel(SlotState st, const bf16* __restrict__ pad, const bf16* __restrict__ codec_emb,
+                                   int vocab, const bf16* __restrict__ p_emb, int p_vocab, int groups,
+                                   bf16* __restrict__ out, int dim, uint32_t* err) {
+  grid_trigger();
+  grid_wait();
+  float acc[8];
+  frame_embed_row(st, pad, codec_emb, vocab, p_emb, p_vocab, groups, dim, err, acc);
+  st8(out + (int64_t)blockIdx.x * dim + threadIdx.x * 8, acc);
+}
+
+__global__ void frame_embed_norm_kernel(SlotState st, const bf16* __restrict__ pad, const bf16* __restrict__ codec_emb,
+                                        int vocab, const bf16* __restrict__ p_emb, int p_vocab, int groups,
+                                        const bf16* __restrict__ gain, bf16* __restrict__ res, bf16* __restrict__ x, int dim,
+                                        float eps, uint32_t* err) {
+  grid_trigger();
+  __shared__ float scratch[32];
+  const int64_t at = (int64_t)blockIdx.x * dim + threadIdx.x * 8;
+  float v[8], g[8], ss = 0.f;
+  ld8(gain + threadIdx.x * 8, g);
+  grid_wait();
+  frame_embed_row(st, pad, codec_emb, vocab, p_emb, p_vocab, groups, dim, err, v);
+#pragma unroll
+  for (int k = 0; k < 8; ++k) v[k] = bf16_round(v[k]), ss += v[k] * v[k];
+  const float r = rsqrtf(block_add(ss, scratch) / dim + eps);
+  st8(res + at, v);
+#pragma unroll
+  for (int k = 0; k < 8; ++k) v[k] = v[k] * r * g[k];
+  st8(x + at, v);
 }
 
 // `talker_pred_input` (talker.cu:100-106).
 __global__ void pred_input_kernel(const bf16* __restrict__ hidden, const bf16* __restrict__ codec_emb, int vocab,
                                   const int32_t* __restrict__ codes, bf16* __restrict__ out, int dim, uint32_t* err) {
+  grid_trigger();
+  grid_wait();
   const int s = blockIdx.x, c = threadIdx.x * 8;
   const bf16* src;
   if (blockIdx.y == 0) {
@@ -101,56 +138,99 @@ __global__ void pred_input_kernel(const bf16* __restrict__ hidden, const bf16* _
 
 cudaError_t launch_gather(const int32_t* ids, int stride, const bf16* table, int table_rows, bf16* out, int rows,
                           int dim, uint32_t* err, cudaStream_t s) {
-  gather_kernel<<<rows, dim / 8, 0, s>>>(ids, stride, table, table_rows, out, dim, err);
-  return cudaGetLastError();
+  return launch_pdl(gather_kernel, dim3(rows), dim3(dim / 8), 0, s, ids, stride, table, table_rows, out, dim, err);
 }
 
 cudaError_t launch_prompt_codec(bf16* x, const bf16* bias, const bf16* table, int table_rows, const int32_t* ids,
                                 int rows, int dim, uint32_t* err, cudaStream_t s) {
-  prompt_codec_kernel<<<rows, dim / 8, 0, s>>>(x, bias, table, table_rows, ids, dim, err);
-  return cudaGetLastError();
+  return launch_pdl(prompt_codec_kernel, dim3(rows), dim3(dim / 8), 0, s, x, bias, table, table_rows, ids, dim, err);
 }
 
 cudaError_t launch_frame_embed(SlotState st, const bf16* pad, const bf16* codec_emb, int vocab, const bf16* p_emb,
                                int p_vocab, int groups, bf16* out, int rows, int dim, uint32_t* err, cudaStream_t s) {
-  frame_embed_kernel<<<rows, dim / 8, 0, s>>>(st, pad, codec_emb, vocab, p_emb, p_vocab, groups, out, dim, err);
-  return cudaGetLastError();
+  return launch_pdl(frame_embed_kernel, dim3(rows), dim3(dim / 8), 0, s, st, pad, codec_emb, vocab, p_emb, p_vocab, groups, out, dim, err);
+}
+
+cudaError_t launch_frame_embed_norm(SlotState st, const bf16* pad, const bf16* codec_emb, int vocab, const bf16* p_emb,
+                                    int p_vocab, int groups, const bf16* gain, bf16* res, bf16* x, int rows, int dim,
+                                    float eps, uint32_t* err, cudaStream_t s) {
+  return launch_pdl(frame_embed_norm_kernel, dim3(rows), dim3(dim / 8), 0, s, st, pad, codec_emb, vocab, p_emb, p_vocab, groups,
+                    gain, res, x, dim, eps, err);
 }
 
 cudaError_t launch_pred_input(const bf16* hidden, const bf16* codec_emb, int vocab, const int32_t* codes, bf16* out,
                               int rows, int dim, uint32_t* err, cudaStream_t s) {
-  pred_input_kernel<<<dim3(rows, 2), dim / 8, 0, s>>>(hidden, codec_emb, vocab, codes, out, dim, err);
-  return cudaGetLastError();
+  return launch_pdl(pred_input_kernel, dim3(rows, 2), dim3(dim / 8), 0, s, hidden, codec_emb, vocab, codes, out, dim, err);
 }
 
 // ---- token selection ----------------------------------------------------------
-// One 1024-thread block per row; the algorithm lives in sampler.cuh.
+// One 512-thread block per row; the algorithm lives in sampler.cuh.
 
-__global__ void __launch_bounds__(1024) sample_kernel(const bf16* __restrict__ logits, sampler::Params prm,
-                                                      const int32_t* __restrict__ frames,
-                                                      const float* __restrict__ uniforms,
-                                                      const int32_t* __restrict__ force, SlotState st,
-                                                      int32_t* __restrict__ codes) {
-  using Team = sampler::Team<1024, sampler::CtaSync>;
+template <int THREADS>
+__global__ void __launch_bounds__(THREADS)
+    sample_kernel(const bf16* __restrict__ logits, sampler::Params prm, const int32_t* __restrict__ frames,
+                  const float* __restrict__ uniforms, const int32_t* __restrict__ force, SlotState st,
+                  int32_t* __restrict__ codes, NextRow next) {
+  using Team = sampler::Team<THREADS, sampler::CtaSync>;
+  grid_trigger();
   __shared__ sampler::Shared sh;
-  const int s = blockIdx.x;
+  const int s = blockIdx.x, tid = threadIdx.x;
   const bf16* l = logits + (int64_t)s * prm.vocab;
   int32_t* slot = slot_of(st, s);
-  Team::sample_row([&](int i, int) { return __bfloat162float(l[i]); }, prm, frames[s], uniforms[s * kGroups + prm.group],
-                   force[s * kGroups + prm.group], slot, Team::seen_word(slot, prm, threadIdx.x),
-                   codes + s * kGroups + prm.group, threadIdx.x, sh);
+  const int frame = frames[s], forced = force[s * kGroups + prm.group];
+  const float uniform = uniforms[s * kGroups + prm.group];
+  grid_wait();
+  float mine[Team::PER];
+  if (prm.vocab % Team::PER == 0) {
+    if (tid * Team::PER < prm.vocab) {
+#pragma unroll
+      for (int j = 0; j < Team::PER; j += 4) {
+        const uint2 u = __ldcg(reinterpret_cast<const uint2*>(l + tid * Team::PER + j));
+        mine[j] = __uint_as_float(u.x << 16), mine[j + 1] = __uint_as_float(u.x & 0xffff0000u);
+        mine[j + 2] = __uint_as_float(u.y << 16), mine[j + 3] = __uint_as_float(u.y & 0xffff0000u);
+      }
+    }
+  } else {
+    for (int j = 0; j < Team::PER; ++j)
+      mine[j] = tid * Team::PER + j < prm.vocab ? __bfloat162float(l[tid * Team::PER + j]) : 0.f;
+  }
+  const int token = Team::sample_row([&](int, int j) { return mine[j]; }, prm, frame, uniform, forced, slot,
+                                     Team::seen_word(slot, prm, tid), codes + s * kGroups + prm.group, tid, sh);
+  if (!next.table) return;
+  const int c = tid * 8;
+  float v[8], g[8], ss = 0.f;
+  const bool on = c < next.dim;
+  if (on) {
+    ld8(next.table + (int64_t)token * next.dim + c, v);
+    ld8(next.gain + c, g);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) ss += v[k] * v[k];
+  }
+  const float r = rsqrtf(block_add(ss, sh.red) / next.dim + next.eps);
+  if (on) {
+    st8(next.res + (int64_t)s * next.dim + c, v);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) v[k] = v[k] * r * g[k];
+    st8(next.x + (int64_t)s * next.dim + c, v);
+  }
 }
 
-cudaError_t launch_sample(const bf16* logits, const SampleParams& p, const int32_t* frames, const float* uniforms,
-                          const int32_t* force, SlotState st, int32_t* codes, int rows, cudaStream_t s) {
+cudaError_t launch_sample_next(const bf16* logits, const SampleParams& p, const int32_t* frames, const float* uniforms,
+                               const int32_t* force, SlotState st, int32_t* codes, const NextRow& next, int rows,
+                               cudaStream_t s) {
   if (p.vocab > sampler::kVocabMax || p.vocab < 1) return cudaErrorInvalidValue;
   // the nucleus filter ranks at most kMaxNucleus survivors of the top-k cut: without a cut that small it would
   // silently drop candidates in arrival order
   if (p.top_p < 1.f && (p.top_k <= 0 || p.top_k > sampler::kMaxNucleus)) return cudaErrorInvalidValue;
   sampler::Params prm{p.vocab,  p.temperature, p.top_k,    p.top_p, p.penalty, p.suppress_lo, p.suppress_hi,
                       p.exempt, p.min_frames,  p.penalize, p.group, p.philox,  p.seen_words};
-  sample_kernel<<<rows, 1024, 0, s>>>(logits, prm, frames, uniforms, force, st, codes);
-  return cudaGetLastError();
+  if (next.table && next.dim > 8 * 512) return cudaErrorInvalidValue;
+  return launch_pdl(sample_kernel<512>, dim3(rows), dim3(512), 0, s, logits, prm, frames, uniforms, force, st, codes, next);
+}
+
+cudaError_t launch_sample(const bf16* logits, const SampleParams& p, const int32_t* frames, const float* uniforms,
+                          const int32_t* force, SlotState st, int32_t* codes, int rows, cudaStream_t s) {
+  return launch_sample_next(logits, p, frames, uniforms, force, st, codes, NextRow{}, rows, s);
 }
 
 }  // namespace omni

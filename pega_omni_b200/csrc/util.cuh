@@ -77,6 +77,9 @@ __device__ __forceinline__ void st8v(bf16* dst, const float* v) { *reinterpret_c
 __device__ __forceinline__ void ld8(const bf16* src, float* v) { ld8v(src, v); }
 __device__ __forceinline__ void st8(bf16* dst, const float* v) { st8v(dst, v); }
 
+// The same past L1, for rows that another SM wrote while this kernel had already started.
+__device__ __forceinline__ void ld8cg(const bf16* src, float* v) { unpack8v(__ldcg(reinterpret_cast<const uint4*>(src)), v); }
+
 __device__ __forceinline__ float warp_add(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
