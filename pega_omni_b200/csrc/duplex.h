@@ -10,6 +10,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "stream_gemm.h"
 #include "util.cuh"
 
 namespace omni {
@@ -40,6 +41,9 @@ cudaError_t launch_lm_norm(const bf16* x, const bf16* alpha, bf16* out, int rows
 // x = bf16(x + y); out = norm(x) (out == nullptr: the add alone)
 cudaError_t launch_lm_add_norm(const bf16* y, bf16* x, const bf16* alpha, bf16* out, int rows, int dim, float eps,
                                cudaStream_t s);
+// The same with y given as the summands of its rows.
+cudaError_t launch_lm_add_norm_sum(const Summands& y, bf16* x, const bf16* alpha, bf16* out, int rows, int dim, float eps,
+                                   cudaStream_t s);
 // The words of a tensor-parallel pair's exchange: `my_flag` lives in this rank's memory and is written by the peer,
 // `peer_flag` is the peer's, mapped here; `counter` numbers the exchanges, `finished` counts a launch's CTAs.
 struct TpLink {
@@ -56,6 +60,10 @@ cudaError_t launch_lm_rope_kv(bf16* qkv, const int32_t* pos, const int32_t* slot
 cudaError_t launch_lm_attend(const bf16* qkv, const void* kv, const int32_t* pos, const int32_t* seq,
                              const int32_t* indptr, const int32_t* pages, bf16* out, int rows, int heads, float scale,
                              int context, int kv_pages, uint32_t* err, cudaStream_t s);
+// launch_lm_rope_kv and launch_lm_attend of one row per session in one kernel.
+cudaError_t launch_lm_rope_attend(const bf16* qkv, void* kv, const int32_t* pos, const int32_t* slots,
+                                  const int32_t* indptr, const int32_t* pages, bf16* out, int rows, int heads, float coef,
+                                  float scale, int context, int kv_pages, uint32_t* err, cudaStream_t s);
 // Depformer step k: x = bf16(projected[s][k] + table[drawn[s][k]]); xn = norm(x).
 cudaError_t launch_lm_dep_embed_norm(const bf16* projected, int k, const bf16* table, int table_rows,
                                      const int32_t* drawn, const bf16* alpha, bf16* x, bf16* xn, int rows, int dim,

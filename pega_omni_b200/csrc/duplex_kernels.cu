@@ -6,6 +6,7 @@
 #include "duplex.h"
 
 #include "sm100.cuh"
+#include "pdl.cuh"
 
 namespace omni {
 namespace {
@@ -41,6 +42,8 @@ __device__ __forceinline__ void embed_row(const int32_t* ids, const DuplexTables
 __global__ void lm_embed_ids_kernel(const int32_t* __restrict__ ids, const int32_t* __restrict__ voice,
                                     const bf16* __restrict__ voices, int voice_rows, DuplexTables t,
                                     bf16* __restrict__ out, int dim, uint32_t* err) {
+  grid_trigger();
+  grid_wait();
   const int64_t r = blockIdx.x;
   if (voice && voice[r] >= 0) {
     int v = voice[r];
@@ -59,6 +62,8 @@ __global__ void lm_embed_ids_kernel(const int32_t* __restrict__ ids, const int32
 __global__ void lm_embed_state_kernel(const void* state, const int32_t* __restrict__ lines, int64_t stride,
                                       DuplexTables t, bf16* __restrict__ out, int32_t* __restrict__ rows_out, int dim,
                                       uint32_t* err) {
+  grid_trigger();
+  grid_wait();
   const int s = blockIdx.x;
   const int32_t* row = state_row(state, lines, s, stride);
   if (threadIdx.x < kDuplexStreams) rows_out[s * kDuplexStreams + threadIdx.x] = row[threadIdx.x];
@@ -80,6 +85,8 @@ __device__ __forceinline__ void norm_row(const float* v, const bf16* alpha, bf16
 
 __global__ void lm_norm_kernel(const bf16* __restrict__ x, const bf16* __restrict__ alpha, bf16* __restrict__ out,
                                int dim, float eps) {
+  grid_trigger();
+  grid_wait();
   __shared__ float scratch[32];
   const int64_t at = (int64_t)blockIdx.x * dim;
   float v[8];
@@ -90,6 +97,8 @@ __global__ void lm_norm_kernel(const bf16* __restrict__ x, const bf16* __restric
 // x = bf16(x + y), out = norm(x) over the rounded sum (lm.cu:95-106; out == nullptr: `lm_add`, lm.cu:109-120)
 __global__ void lm_add_norm_kernel(const bf16* __restrict__ y, bf16* __restrict__ x, const bf16* __restrict__ alpha,
                                    bf16* __restrict__ out, int dim, float eps) {
+  grid_trigger();
+  grid_wait();
   __shared__ float scratch[32];
   const int64_t at = (int64_t)blockIdx.x * dim + threadIdx.x * 8;
   float v[8], u[8];
@@ -99,6 +108,37 @@ __global__ void lm_add_norm_kernel(const bf16* __restrict__ y, bf16* __restrict_
   for (int k = 0; k < 8; ++k) v[k] = bf16_round(v[k] + u[k]);
   st8(x + at, v);
   if (out) norm_row(v, alpha, out + (int64_t)blockIdx.x * dim, dim, eps, scratch);
+}
+
+// The same over a GEMM's summands: every load of a thread's eight columns is under way at once.
+__global__ void lm_add_norm_sum_kernel(const Summands y, bf16* __restrict__ x, const bf16* __restrict__ alpha,
+                                       bf16* __restrict__ out, int dim, float eps) {
+  grid_trigger();
+  __shared__ float scratch[32];
+  const int c = threadIdx.x * 8;
+  const int64_t at = (int64_t)blockIdx.x * dim + c;
+  float v[8], u[8], a[8];
+  if (out) ld8(alpha + c, a);
+  grid_wait();
+  ld8cg(x + at, v);
+  load_sum8(y, blockIdx.x, c, u);
+  float ss = 0.f;
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    v[k] = bf16_round(v[k] + u[k]);
+    ss += v[k] * v[k];
+  }
+  st8(x + at, v);
+  if (!out) return;
+  ss = warp_add(ss);
+  if ((threadIdx.x & 31) == 0) scratch[threadIdx.x >> 5] = ss;
+  __syncthreads();
+  float total = 0.f;
+  for (int i = 0; i < (int)(blockDim.x + 31) >> 5; ++i) total += scratch[i];
+  const float r = rsqrtf(total / dim + eps);
+#pragma unroll
+  for (int k = 0; k < 8; ++k) v[k] = v[k] * (a[k] * r);
+  st8(out + at, v);
 }
 
 // ---- tensor-parallel pair: all-reduce of a projection's partial rows, fused with the add + norm that follows -----
@@ -197,6 +237,8 @@ constexpr int kRopeWarps = 8, kRopeParts = 4;
 __global__ void __launch_bounds__(kRopeWarps * 32)
     lm_rope_kv_kernel(bf16* __restrict__ qkv, const int32_t* __restrict__ pos, const int32_t* __restrict__ slots, void* kv,
                       int heads, float coef, int kv_pages, uint32_t* err) {
+  grid_trigger();
+  grid_wait();
   __shared__ float cs[kHeliumHeadDim / 2], sn[kHeliumHeadDim / 2];
   const int n = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (threadIdx.x < kHeliumHeadDim / 2) {
@@ -258,6 +300,48 @@ __device__ __forceinline__ float4 e4m3x4(uint32_t raw) {
 constexpr int kAttendWarps = 4;
 constexpr int kAttendSlotBytes = ((kDuplexPageHeadBytes + 127) / 128) * 128;
 
+// One page of one warp: lane = (key `tok`, half of its dims), the online softmax over 16 keys, then four output dims a lane.
+__device__ __forceinline__ void page_step(const unsigned char* blk, const float* q, int ntok, float scale, int tok, int half,
+                                          int lane, float& m, float& l, float (&acc)[4]) {
+  float dot = 0.f;
+  {
+    const uint4* krow = reinterpret_cast<const uint4*>(blk + tok * kHeliumHeadDim + half * 64);
+    const float* qh = q + half * 64;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const uint4 raw = krow[c];
+      const float4 k0 = e4m3x4(raw.x), k1 = e4m3x4(raw.y), k2 = e4m3x4(raw.z), k3 = e4m3x4(raw.w);
+      const float* qc = qh + c * 16;
+      dot += qc[0] * k0.x + qc[1] * k0.y + qc[2] * k0.z + qc[3] * k0.w + qc[4] * k1.x + qc[5] * k1.y + qc[6] * k1.z +
+             qc[7] * k1.w;
+      dot += qc[8] * k2.x + qc[9] * k2.y + qc[10] * k2.z + qc[11] * k2.w + qc[12] * k3.x + qc[13] * k3.y +
+             qc[14] * k3.z + qc[15] * k3.w;
+    }
+  }
+  dot += __shfl_xor_sync(0xffffffffu, dot, 16);  // both halves of key `tok`
+  const float ks = reinterpret_cast<const float*>(blk + 2 * 16 * kHeliumHeadDim)[tok];
+  const float vs = reinterpret_cast<const float*>(blk + 2 * 16 * kHeliumHeadDim + 64)[tok];
+  const float sv = tok < ntok ? dot * (ks * scale) : -INFINITY;
+  const float m2 = fmaxf(m, warp_fmax(sv));
+  const float corr = __expf(m - m2);
+  const float p = __expf(sv - m2);
+  float psum = p;  // over the 16 keys (both half-warps hold the same values)
+#pragma unroll
+  for (int o = 8; o > 0; o >>= 1) psum += __shfl_xor_sync(0xffffffffu, psum, o);
+  l = l * corr + psum;
+#pragma unroll
+  for (int d = 0; d < 4; ++d) acc[d] *= corr;
+  m = m2;
+  const float pv = p * vs;  // 0 for keys past the row's length
+  const uint32_t* vrows = reinterpret_cast<const uint32_t*>(blk + 16 * kHeliumHeadDim) + lane;
+#pragma unroll
+  for (int j = 0; j < 16; ++j) {
+    const float pj = __shfl_sync(0xffffffffu, pv, j);
+    const float4 vf = e4m3x4(vrows[j * (kHeliumHeadDim / 4)]);
+    acc[0] += pj * vf.x, acc[1] += pj * vf.y, acc[2] += pj * vf.z, acc[3] += pj * vf.w;
+  }
+}
+
 struct AttendShared {
   float q[kHeliumHeadDim];
   float ms[kAttendWarps], ls[kAttendWarps];
@@ -270,6 +354,8 @@ __global__ void __launch_bounds__(kAttendWarps * 32)
                      const int32_t* __restrict__ seq, const int32_t* __restrict__ indptr,
                      const int32_t* __restrict__ pages, bf16* __restrict__ out, int heads, float scale, int context,
                      int kv_pages, uint32_t* err) {
+  grid_trigger();
+  grid_wait();
   extern __shared__ __align__(128) unsigned char attend_smem[];
   AttendShared& sh = *reinterpret_cast<AttendShared*>(attend_smem);
   unsigned char* slots = attend_smem + ((sizeof(AttendShared) + 127) & ~(size_t)127);
@@ -309,43 +395,7 @@ __global__ void __launch_bounds__(kAttendWarps * 32)
     parity[slot] ^= 1u;
     const unsigned char* blk = mine + (size_t)slot * kAttendSlotBytes;
     const int ntok = min(16, len - pi * 16);
-    float dot = 0.f;
-    {
-      const uint4* krow = reinterpret_cast<const uint4*>(blk + tok * kHeliumHeadDim + half * 64);
-      const float* qh = sh.q + half * 64;
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        const uint4 raw = krow[c];
-        const float4 k0 = e4m3x4(raw.x), k1 = e4m3x4(raw.y), k2 = e4m3x4(raw.z), k3 = e4m3x4(raw.w);
-        const float* qc = qh + c * 16;
-        dot += qc[0] * k0.x + qc[1] * k0.y + qc[2] * k0.z + qc[3] * k0.w + qc[4] * k1.x + qc[5] * k1.y + qc[6] * k1.z +
-               qc[7] * k1.w;
-        dot += qc[8] * k2.x + qc[9] * k2.y + qc[10] * k2.z + qc[11] * k2.w + qc[12] * k3.x + qc[13] * k3.y +
-               qc[14] * k3.z + qc[15] * k3.w;
-      }
-    }
-    dot += __shfl_xor_sync(0xffffffffu, dot, 16);  // both halves of key `tok`
-    const float ks = reinterpret_cast<const float*>(blk + 2 * 16 * kHeliumHeadDim)[tok];
-    const float vs = reinterpret_cast<const float*>(blk + 2 * 16 * kHeliumHeadDim + 64)[tok];
-    const float sv = tok < ntok ? dot * (ks * scale) : -INFINITY;
-    const float m2 = fmaxf(m, warp_fmax(sv));
-    const float corr = __expf(m - m2);
-    const float p = __expf(sv - m2);
-    float psum = p;  // over the 16 keys (both half-warps hold the same values)
-#pragma unroll
-    for (int o = 8; o > 0; o >>= 1) psum += __shfl_xor_sync(0xffffffffu, psum, o);
-    l = l * corr + psum;
-#pragma unroll
-    for (int d = 0; d < 4; ++d) acc[d] *= corr;
-    m = m2;
-    const float pv = p * vs;  // 0 for keys past the row's length
-    const uint32_t* vrows = reinterpret_cast<const uint32_t*>(blk + 16 * kHeliumHeadDim) + lane;
-#pragma unroll
-    for (int j = 0; j < 16; ++j) {
-      const float pj = __shfl_sync(0xffffffffu, pv, j);
-      const float4 vf = e4m3x4(vrows[j * (kHeliumHeadDim / 4)]);
-      acc[0] += pj * vf.x, acc[1] += pj * vf.y, acc[2] += pj * vf.z, acc[3] += pj * vf.w;
-    }
+    page_step(blk, sh.q, ntok, scale, tok, half, lane, m, l, acc);
     __syncwarp();  // every lane is done with this slot before lane 0 refills it in the next round
   }
   if (lane == 0) {
@@ -371,11 +421,126 @@ __global__ void __launch_bounds__(kAttendWarps * 32)
   }
 }
 
+// Decode: rotary embedding, FP8 KV write and ring attention of one row per session in one kernel, a CTA of W warps per
+// (session, head). Warps 0, 1 and 2 take the head's query, key and value; meanwhile every warp already has two pages of
+// the ring on their way - the pages earlier ticks filled do not depend on the projection this kernel waits for. The page
+// the row is written to comes last: its writers' stores are fenced for the bulk copy that reads them back.
+template <int W>
+__global__ void __launch_bounds__(W * 32)
+    lm_rope_attend_kernel(const bf16* __restrict__ qkv, void* kv, const int32_t* __restrict__ pos,
+                          const int32_t* __restrict__ slots, const int32_t* __restrict__ indptr,
+                          const int32_t* __restrict__ pages, bf16* __restrict__ out, int heads, float coef, float scale,
+                          int context, int kv_pages, uint32_t* err) {
+  grid_trigger();
+  extern __shared__ __align__(128) unsigned char lra_slots[];
+  __shared__ float q[kHeliumHeadDim], ms[W], ls[W], os[W][kHeliumHeadDim];
+  __shared__ __align__(8) uint64_t bars[W][2];
+  const int n = blockIdx.x, h = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int at = pos[n], len = min(at + 1, context), npages = (len + 15) >> 4, own = (at % context) >> 4;
+  const int32_t* my_pages = pages + indptr[n];
+  int64_t slot_id = slots[n];
+  if (slot_id < 0 || (slot_id >> 4) >= kv_pages) {
+    if (threadIdx.x == 0) raise(err, kErrBadIndex);
+    slot_id = 0;
+  }
+  if (lane == 0) {
+    sm100::mbar_init(sm100::smem_addr(&bars[warp][0]), 1);
+    sm100::mbar_init(sm100::smem_addr(&bars[warp][1]), 1);
+    sm100::mbar_init_fence();
+  }
+  __syncwarp();
+  unsigned char* mine = lra_slots + (size_t)warp * 2 * kAttendSlotBytes;
+  auto page_of = [&](int v) { return v == npages - 1 ? own : v < own ? v : v + 1; };  // the row's own page last
+  auto fetch = [&](int v, int slot) {  // lane 0: one bulk copy of the v-th page's block for this head
+    int64_t page = v == npages - 1 ? slot_id >> 4 : my_pages[page_of(v)];
+    if (page < 0 || page >= kv_pages) {
+      raise(err, kErrBadIndex);
+      page = 0;
+    }
+    const uint32_t bar = sm100::smem_addr(&bars[warp][slot]);
+    sm100::mbar_expect_tx(bar, kDuplexPageHeadBytes);
+    sm100::bulk_load(sm100::smem_addr(mine + (size_t)slot * kAttendSlotBytes), page_head(kv, page, heads, h), kDuplexPageHeadBytes, bar);
+  };
+  if (lane == 0) {
+    if (warp < npages - 1) fetch(warp, 0);
+    if (warp + W < npages - 1) fetch(warp + W, 1);
+  }
+  float cs[2], sn[2];
+#pragma unroll
+  for (int k = 0; k < 2; ++k) sincosf(expf((float)(2 * lane + k) * coef) * (float)at, &sn[k], &cs[k]);
+  grid_wait();
+  if (warp < 3) {
+    const uint2 raw = __ldcg(reinterpret_cast<const uint2*>(qkv + ((int64_t)n * 3 * heads + warp * heads + h) * kHeliumHeadDim) + lane);
+    const float2 p0 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.x));
+    const float2 p1 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.y));
+    float v[4] = {p0.x, p0.y, p1.x, p1.y};
+    if (warp < 2) {  // pairs (2i, 2i + 1) rotated by angle i
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        const float r = v[2 * k], im = v[2 * k + 1];
+        v[2 * k] = r * cs[k] - im * sn[k];
+        v[2 * k + 1] = r * sn[k] + im * cs[k];
+      }
+    }
+    if (warp == 0) {
+#pragma unroll
+      for (int k = 0; k < 4; ++k) q[lane * 4 + k] = bf16_round(v[k]);
+    } else {
+      const float amax = warp_fmax(fmaxf(fmaxf(fabsf(v[0]), fabsf(v[1])), fmaxf(fabsf(v[2]), fabsf(v[3]))));
+      const float sc = e4m3_scale(amax), inv = 1.f / sc;
+      uint8_t* block = page_head(kv, slot_id >> 4, heads, h);
+      const int tok = (int)(slot_id & 15), is_v = warp - 1;
+      const uint32_t lo = __nv_cvt_float2_to_fp8x2(make_float2(v[0] * inv, v[1] * inv), __NV_SATFINITE, __NV_E4M3);
+      const uint32_t hi = __nv_cvt_float2_to_fp8x2(make_float2(v[2] * inv, v[3] * inv), __NV_SATFINITE, __NV_E4M3);
+      *reinterpret_cast<uint32_t*>(block + (is_v * 16 + tok) * kHeliumHeadDim + lane * 4) = lo | hi << 16;
+      if (lane == 0) reinterpret_cast<float*>(block + 2 * 16 * kHeliumHeadDim + is_v * 64)[tok] = sc;
+      asm volatile("fence.proxy.async.global;" ::: "memory");
+    }
+  }
+  __syncthreads();
+  if (lane == 0) {  // the own page, where it is one of the warp's first two
+    if (warp == npages - 1) fetch(warp, 0);
+    else if (warp + W == npages - 1) fetch(warp + W, 1);
+  }
+  float m = -INFINITY, l = 0.f, acc[4] = {0.f, 0.f, 0.f, 0.f};
+  const int tok = lane & 15, half = lane >> 4;
+  uint32_t parity[2] = {0, 0};
+  int slot = 0;
+  for (int vi = warp; vi < npages; vi += W, slot ^= 1) {
+    if (!sm100::mbar_wait(sm100::smem_addr(&bars[warp][slot]), parity[slot], err)) break;
+    parity[slot] ^= 1u;
+    const unsigned char* blk = mine + (size_t)slot * kAttendSlotBytes;
+    const int ntok = min(16, len - page_of(vi) * 16);
+    page_step(blk, q, ntok, scale, tok, half, lane, m, l, acc);
+    __syncwarp();  // every lane is done with this slot
+    if (lane == 0 && vi + 2 * W < npages) fetch(vi + 2 * W, slot);
+  }
+  if (lane == 0) ms[warp] = m, ls[warp] = l;
+#pragma unroll
+  for (int d = 0; d < 4; ++d) os[warp][lane * 4 + d] = acc[d];
+  __syncthreads();
+  for (int d = threadIdx.x; d < kHeliumHeadDim; d += W * 32) {
+    float top = -INFINITY;
+#pragma unroll
+    for (int w = 0; w < W; ++w) top = fmaxf(top, ms[w]);
+    float num = 0.f, den = 0.f;
+#pragma unroll
+    for (int w = 0; w < W; ++w) {
+      const float e = ms[w] == -INFINITY ? 0.f : __expf(ms[w] - top);
+      num += os[w][d] * e;
+      den += ls[w] * e;
+    }
+    out[((int64_t)n * heads + h) * kHeliumHeadDim + d] = __float2bfloat16(num / den);
+  }
+}
+
 // `lm_dep_embed_norm` (lm.cu:301-313)
 __global__ void lm_dep_embed_norm_kernel(const bf16* __restrict__ projected, int k, const bf16* __restrict__ table,
                                          int table_rows, const int32_t* __restrict__ drawn,
                                          const bf16* __restrict__ alpha, bf16* __restrict__ x, bf16* __restrict__ xn,
                                          int dim, float eps, uint32_t* err) {
+  grid_trigger();
+  grid_wait();
   __shared__ float scratch[32];
   const int s = blockIdx.x, c = threadIdx.x * 8;
   int64_t id = drawn[s * kDuplexDrawn + k];
@@ -396,6 +561,8 @@ __global__ void lm_dep_embed_norm_kernel(const bf16* __restrict__ projected, int
 // and V stay in registers.
 __global__ void lm_dep_kv_attend_kernel(const bf16* __restrict__ qkv, bf16* __restrict__ ws, int step,
                                         bf16* __restrict__ out, int heads, float scale) {
+  grid_trigger();
+  grid_wait();
   const int s = blockIdx.x, h = blockIdx.y * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (h >= heads) return;
   const int width = heads * kDepHeadDim;
@@ -467,6 +634,8 @@ __global__ void __launch_bounds__(kSampleThreads)
     lm_sample_kernel(const bf16* __restrict__ logits, int vocab, int64_t ld, float temperature, int top_k,
                      const int32_t* __restrict__ force, const int32_t* __restrict__ seeds, int col,
                      int32_t* __restrict__ drawn) {
+  grid_trigger();
+  grid_wait();
   const int s = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   __shared__ uint32_t counts[2][kSampleThreads / 32];
   __shared__ unsigned long long best[kSampleThreads / 32];
@@ -544,6 +713,8 @@ __global__ void __launch_bounds__(kSampleThreads)
 __global__ void lm_advance_kernel(void* state, const int32_t* __restrict__ lines, int64_t stride,
                                   const int32_t* __restrict__ drawn, const int32_t* __restrict__ caller,
                                   const int32_t* __restrict__ force_caller, int32_t* __restrict__ emitted, int seqs) {
+  grid_trigger();
+  grid_wait();
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= seqs) return;
   int32_t* row = const_cast<int32_t*>(state_row(state, lines, s, stride));
@@ -572,6 +743,8 @@ __global__ void lm_advance_kernel(void* state, const int32_t* __restrict__ lines
 // `lm_init` (lm.cu:576-581)
 __global__ void lm_init_kernel(void* state, const int32_t* __restrict__ lines, int64_t stride,
                                const int32_t* __restrict__ init) {
+  grid_trigger();
+  grid_wait();
   const int s = blockIdx.x;
   int32_t* own = const_cast<int32_t*>(state_row(state, lines, s, stride));
   if (threadIdx.x < kDuplexStateWords) own[threadIdx.x] = init[s * kDuplexStateWords + threadIdx.x];
@@ -581,6 +754,8 @@ __global__ void lm_init_kernel(void* state, const int32_t* __restrict__ lines, i
 // 128-byte value row and the two scales.
 __global__ void lm_copy_kv_kernel(void* kv, const int32_t* __restrict__ src_slot, const int32_t* __restrict__ dst_slot,
                                   int heads, int kv_pages, uint32_t* err) {
+  grid_trigger();
+  grid_wait();
   const int r = blockIdx.x, h = blockIdx.y * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (h >= heads) return;
   int64_t src = src_slot[r], dst = dst_slot[r];
@@ -606,28 +781,30 @@ bool row_dim_ok(int dim) { return dim % 8 == 0 && dim / 8 <= 1024 && dim / 8 >= 
 cudaError_t launch_lm_embed_ids(const int32_t* ids, const int32_t* voice, const bf16* voices, int voice_rows,
                                 DuplexTables t, bf16* out, int rows, int dim, uint32_t* err, cudaStream_t s) {
   if (!row_dim_ok(dim)) return cudaErrorInvalidValue;
-  lm_embed_ids_kernel<<<rows, dim / 8, 0, s>>>(ids, voice, voices, voice_rows, t, out, dim, err);
-  return cudaGetLastError();
+  return launch_pdl(lm_embed_ids_kernel, dim3(rows), dim3(dim / 8), 0, s, ids, voice, voices, voice_rows, t, out, dim, err);
 }
 
 cudaError_t launch_lm_embed_state(const void* state, const int32_t* lines, int64_t stride, DuplexTables t, bf16* out,
                                   int32_t* rows_out, int rows, int dim, uint32_t* err, cudaStream_t s) {
   if (!row_dim_ok(dim)) return cudaErrorInvalidValue;
-  lm_embed_state_kernel<<<rows, dim / 8, 0, s>>>(state, lines, stride, t, out, rows_out, dim, err);
-  return cudaGetLastError();
+  return launch_pdl(lm_embed_state_kernel, dim3(rows), dim3(dim / 8), 0, s, state, lines, stride, t, out, rows_out, dim, err);
 }
 
 cudaError_t launch_lm_norm(const bf16* x, const bf16* alpha, bf16* out, int rows, int dim, float eps, cudaStream_t s) {
   if (!row_dim_ok(dim)) return cudaErrorInvalidValue;
-  lm_norm_kernel<<<rows, dim / 8, 0, s>>>(x, alpha, out, dim, eps);
-  return cudaGetLastError();
+  return launch_pdl(lm_norm_kernel, dim3(rows), dim3(dim / 8), 0, s, x, alpha, out, dim, eps);
 }
 
 cudaError_t launch_lm_add_norm(const bf16* y, bf16* x, const bf16* alpha, bf16* out, int rows, int dim, float eps,
                                cudaStream_t s) {
   if (!row_dim_ok(dim)) return cudaErrorInvalidValue;
-  lm_add_norm_kernel<<<rows, dim / 8, 0, s>>>(y, x, alpha, out, dim, eps);
-  return cudaGetLastError();
+  return launch_pdl(lm_add_norm_kernel, dim3(rows), dim3(dim / 8), 0, s, y, x, alpha, out, dim, eps);
+}
+
+cudaError_t launch_lm_add_norm_sum(const Summands& y, bf16* x, const bf16* alpha, bf16* out, int rows, int dim, float eps,
+                                   cudaStream_t s) {
+  if (!row_dim_ok(dim) || y.splits > 8) return cudaErrorInvalidValue;
+  return launch_pdl(lm_add_norm_sum_kernel, dim3(rows), dim3(dim / 8), 0, s, y, x, alpha, out, dim, eps);
 }
 
 cudaError_t launch_lm_tp_add_norm(const bf16* mine, const bf16* peer, bf16* x, const bf16* alpha, bf16* out, int rows,
@@ -640,8 +817,7 @@ cudaError_t launch_lm_tp_add_norm(const bf16* mine, const bf16* peer, bf16* x, c
 
 cudaError_t launch_lm_rope_kv(bf16* qkv, const int32_t* pos, const int32_t* slots, void* kv, int rows, int heads,
                               float coef, int kv_pages, uint32_t* err, cudaStream_t s) {
-  lm_rope_kv_kernel<<<dim3(rows, kRopeParts), kRopeWarps * 32, 0, s>>>(qkv, pos, slots, kv, heads, coef, kv_pages, err);
-  return cudaGetLastError();
+  return launch_pdl(lm_rope_kv_kernel, dim3(rows, kRopeParts), dim3(kRopeWarps * 32), 0, s, qkv, pos, slots, kv, heads, coef, kv_pages, err);
 }
 
 cudaError_t launch_lm_attend(const bf16* qkv, const void* kv, const int32_t* pos, const int32_t* seq,
@@ -656,24 +832,47 @@ cudaError_t launch_lm_attend(const bf16* qkv, const void* kv, const int32_t* pos
     if (e != cudaSuccess) return e;
     raised[device] = true;
   }
-  lm_attend_kernel<<<dim3(rows, heads), kAttendWarps * 32, smem, s>>>(qkv, kv, pos, seq, indptr, pages, out, heads, scale,
-                                                                     context, kv_pages, err);
-  return cudaGetLastError();
+  return launch_pdl(lm_attend_kernel, dim3(rows, heads), dim3(kAttendWarps * 32), smem, s, qkv, kv, pos, seq, indptr, pages, out, heads, scale, context, kv_pages, err);
+}
+
+template <int W>
+static cudaError_t launch_lm_rope_attend_w(const bf16* qkv, void* kv, const int32_t* pos, const int32_t* slots,
+                                           const int32_t* indptr, const int32_t* pages, bf16* out, int rows, int heads,
+                                           float coef, float scale, int context, int kv_pages, uint32_t* err, cudaStream_t s) {
+  constexpr size_t smem = (size_t)W * 2 * kAttendSlotBytes;
+  if (smem > 40 * 1024) {
+    static bool raised[64] = {};  // per device: above the default limit of dynamic shared memory
+    int device = 0;
+    if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= 64) return cudaErrorInvalidDevice;
+    if (!raised[device]) {
+      const cudaError_t e = cudaFuncSetAttribute(lm_rope_attend_kernel<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      if (e != cudaSuccess) return e;
+      raised[device] = true;
+    }
+  }
+  return launch_pdl(lm_rope_attend_kernel<W>, dim3(rows, heads), dim3(W * 32), smem, s, qkv, kv, pos, slots, indptr, pages, out,
+                    heads, coef, scale, context, kv_pages, err);
+}
+
+cudaError_t launch_lm_rope_attend(const bf16* qkv, void* kv, const int32_t* pos, const int32_t* slots,
+                                  const int32_t* indptr, const int32_t* pages, bf16* out, int rows, int heads, float coef,
+                                  float scale, int context, int kv_pages, uint32_t* err, cudaStream_t s) {
+  if (rows * heads <= 148)  // one CTA per SM at most: more warps of it
+    return launch_lm_rope_attend_w<16>(qkv, kv, pos, slots, indptr, pages, out, rows, heads, coef, scale, context, kv_pages, err, s);
+  return launch_lm_rope_attend_w<4>(qkv, kv, pos, slots, indptr, pages, out, rows, heads, coef, scale, context, kv_pages, err, s);
 }
 
 cudaError_t launch_lm_dep_embed_norm(const bf16* projected, int k, const bf16* table, int table_rows,
                                      const int32_t* drawn, const bf16* alpha, bf16* x, bf16* xn, int rows, int dim,
                                      float eps, uint32_t* err, cudaStream_t s) {
   if (!row_dim_ok(dim)) return cudaErrorInvalidValue;
-  lm_dep_embed_norm_kernel<<<rows, dim / 8, 0, s>>>(projected, k, table, table_rows, drawn, alpha, x, xn, dim, eps, err);
-  return cudaGetLastError();
+  return launch_pdl(lm_dep_embed_norm_kernel, dim3(rows), dim3(dim / 8), 0, s, projected, k, table, table_rows, drawn, alpha, x, xn, dim, eps, err);
 }
 
 cudaError_t launch_lm_dep_kv_attend(const bf16* qkv, bf16* ws, int step, bf16* out, int rows, int heads, float scale,
                                     cudaStream_t s) {
   if (step < 0 || step >= kDepSteps) return cudaErrorInvalidValue;
-  lm_dep_kv_attend_kernel<<<dim3(rows, (heads + 3) / 4), 128, 0, s>>>(qkv, ws, step, out, heads, scale);
-  return cudaGetLastError();
+  return launch_pdl(lm_dep_kv_attend_kernel, dim3(rows, (heads + 3) / 4), dim3(128), 0, s, qkv, ws, step, out, heads, scale);
 }
 
 cudaError_t launch_lm_sample(const bf16* logits, int vocab, int64_t ld, float temperature, int top_k,
@@ -681,28 +880,24 @@ cudaError_t launch_lm_sample(const bf16* logits, int vocab, int64_t ld, float te
                              cudaStream_t s) {
   if (vocab < 1 || col < 0 || col >= kDuplexDrawn) return cudaErrorInvalidValue;
   if (vocab > 2 * kSampleRegs * kSampleThreads) return cudaErrorInvalidValue;  // a thread keeps 64 keys in registers
-  lm_sample_kernel<<<rows, kSampleThreads, 0, s>>>(logits, vocab, ld, temperature, top_k, force, seeds, col, drawn);
-  return cudaGetLastError();
+  return launch_pdl(lm_sample_kernel, dim3(rows), dim3(kSampleThreads), 0, s, logits, vocab, ld, temperature, top_k, force, seeds, col, drawn);
 }
 
 cudaError_t launch_lm_advance(void* state, const int32_t* lines, int64_t stride, const int32_t* drawn,
                               const int32_t* caller, const int32_t* force_caller, int32_t* emitted, int rows,
                               cudaStream_t s) {
-  lm_advance_kernel<<<(rows + 127) / 128, 128, 0, s>>>(state, lines, stride, drawn, caller, force_caller, emitted, rows);
-  return cudaGetLastError();
+  return launch_pdl(lm_advance_kernel, dim3((rows + 127) / 128), dim3(128), 0, s, state, lines, stride, drawn, caller, force_caller, emitted, rows);
 }
 
 cudaError_t launch_lm_copy_kv(void* kv, const int32_t* src_slot, const int32_t* dst_slot, int tokens, int heads,
                               int kv_pages, uint32_t* err, cudaStream_t s) {
   if (tokens < 1) return cudaSuccess;
-  lm_copy_kv_kernel<<<dim3(tokens, (heads + 3) / 4), 128, 0, s>>>(kv, src_slot, dst_slot, heads, kv_pages, err);
-  return cudaGetLastError();
+  return launch_pdl(lm_copy_kv_kernel, dim3(tokens, (heads + 3) / 4), dim3(128), 0, s, kv, src_slot, dst_slot, heads, kv_pages, err);
 }
 
 cudaError_t launch_lm_init(void* state, const int32_t* lines, int64_t stride, const int32_t* init, int rows,
                            cudaStream_t s) {
-  lm_init_kernel<<<rows, 32, 0, s>>>(state, lines, stride, init);
-  return cudaGetLastError();
+  return launch_pdl(lm_init_kernel, dim3(rows), dim3(32), 0, s, state, lines, stride, init);
 }
 
 }  // namespace omni

@@ -14,6 +14,7 @@
 #include <vector>
 
 #include "../../include/omni_b200_duplex.h"
+#include "chain.h"
 #include "duplex.h"
 #include "gemm.h"
 #include "kernels.h"
@@ -128,6 +129,9 @@ struct omni_duplex {
     int seen = 0, nodes = 0;
   };
   std::map<int, TickGraph> tick_graphs;
+  std::map<std::tuple<const void*, const void*, const void*, int, int>, StreamGemmPlan> stream_plans;
+  int granule = 16, d_granule = 16;  // channels per group of the gate|up rows (launch_interleave_gate_up)
+  Chain chain() { return Chain{stream, err, sm_count, scratch.partials, scratch.partial_floats, &launches, &stream_plans}; }
   bool use_graphs = true;
 
   GemmScratch scratch;
@@ -217,6 +221,10 @@ int weight(omni_duplex* m, const Index& idx, const std::string& name, std::initi
 
 // y[rows, N] = x[rows, K] . w[N, K]^T on the path the row count calls for.
 int gemm(omni_duplex* m, const bf16* w, int N, int K, const bf16* x, int rows, bf16* y, int ldy) {
+  if (rows <= kChainRows && stream_supports(N, K, rows)) {
+    DCUDA(m, m->chain().gemm(w, N, K, x, rows, kStreamBf16, y, ldy));
+    return OMNI_OK;
+  }
   if (rows <= 8 || !tc_supports(N, K, rows)) {
     DLAUNCH(m, gemv_launch(w, N, K, x, rows, y, ldy, Epilogue{}, m->sm_count, m->stream));
     return OMNI_OK;
@@ -279,28 +287,45 @@ int helium_forward(omni_duplex* m, int rows, const int32_t* pos, const int32_t* 
   const bool pair = m->tp > 1;
   if (pair && !m->tp_peer_region) return m->fail(OMNI_ERR_INVALID, "tensor-parallel pair not connected (omni_duplex_tp_connect)");
   const float scale = 1.f / std::sqrt((float)kHeliumHeadDim);
+  // up to kChainRows rows: weight-streaming GEMMs whose partial sums the add + norm kernels take (not in a pair, whose
+  // exchange moves finished rows); one row per session (seq == nullptr): rotation, KV write and attention in one kernel
+  const Chain chain = m->chain();
+  const bool stream = rows <= kChainRows;
+  auto projected = [&](const bf16* w, int K, const bf16* x, int which, const bf16* gain) -> int {
+    if (pair) {
+      bf16* y = m->tp_buf(which);
+      DTRY(gemm(m, w, D, K, x, rows, y, D));
+      DLAUNCH(m, launch_lm_tp_add_norm(y, m->tp_peer_buf(which), m->x, gain, m->xn, rows, D, c.norm_eps, m->tp_link(), m->err, m->stream));
+    } else if (stream) {
+      Summands y;
+      DCUDA(m, chain.gemm(w, D, K, x, rows, kStreamPartials, nullptr, D, &y));
+      DLAUNCH(m, launch_lm_add_norm_sum(y, m->x, gain, m->xn, rows, D, c.norm_eps, m->stream));
+    } else {
+      DTRY(gemm(m, w, D, K, x, rows, m->y, D));
+      DLAUNCH(m, launch_lm_add_norm(m->y, m->x, gain, m->xn, rows, D, c.norm_eps, m->stream));
+    }
+    return OMNI_OK;
+  };
   DLAUNCH(m, launch_lm_norm(m->x, m->h[0].norm1, m->xn, rows, D, c.norm_eps, m->stream));
   for (int i = 0; i < c.layers; ++i) {
     const HeliumLayer& L = m->h[i];
     DTRY(gemm(m, L.qkv, 3 * Dl, D, m->xn, rows, m->qkv, 3 * Dl));
-    DLAUNCH(m, launch_lm_rope_kv(m->qkv, pos, slot, m->kv[i], rows, m->local_heads(), rope_coef(c), m->kv_pages, m->err, m->stream));
-    DLAUNCH(m, launch_lm_attend(m->qkv, m->kv[i], pos, seq, indptr, pages, m->attn, rows, m->local_heads(), scale, c.context,
-                                m->kv_pages, m->err, m->stream));
-    bf16* y_o = pair ? m->tp_buf(0) : m->y;
-    DTRY(gemm(m, L.o, D, Dl, m->attn, rows, y_o, D));
-    if (pair)
-      DLAUNCH(m, launch_lm_tp_add_norm(y_o, m->tp_peer_buf(0), m->x, L.norm2, m->xn, rows, D, c.norm_eps, m->tp_link(), m->err, m->stream));
-    else
-      DLAUNCH(m, launch_lm_add_norm(m->y, m->x, L.norm2, m->xn, rows, D, c.norm_eps, m->stream));
-    DTRY(gemm(m, L.gate_up, 2 * Hl, D, m->xn, rows, m->gu, 2 * Hl));
-    DLAUNCH(m, launch_silu_mul(m->gu, m->act, rows, Hl, 0, m->stream));
-    bf16* y_d = pair ? m->tp_buf(1) : m->y;
-    DTRY(gemm(m, L.down, D, Hl, m->act, rows, y_d, D));
-    const bf16* next = i + 1 < c.layers ? m->h[i + 1].norm1 : m->out_norm;
-    if (pair)
-      DLAUNCH(m, launch_lm_tp_add_norm(y_d, m->tp_peer_buf(1), m->x, next, m->xn, rows, D, c.norm_eps, m->tp_link(), m->err, m->stream));
-    else
-      DLAUNCH(m, launch_lm_add_norm(m->y, m->x, next, m->xn, rows, D, c.norm_eps, m->stream));
+    if (!seq) {
+      DLAUNCH(m, launch_lm_rope_attend(m->qkv, m->kv[i], pos, slot, indptr, pages, m->attn, rows, m->local_heads(),
+                                       rope_coef(c), scale, c.context, m->kv_pages, m->err, m->stream));
+    } else {
+      DLAUNCH(m, launch_lm_rope_kv(m->qkv, pos, slot, m->kv[i], rows, m->local_heads(), rope_coef(c), m->kv_pages, m->err, m->stream));
+      DLAUNCH(m, launch_lm_attend(m->qkv, m->kv[i], pos, seq, indptr, pages, m->attn, rows, m->local_heads(), scale, c.context,
+                                  m->kv_pages, m->err, m->stream));
+    }
+    DTRY(projected(L.o, Dl, m->attn, 0, L.norm2));
+    if (stream) {
+      DCUDA(m, chain.gemm(L.gate_up, 2 * Hl, D, m->xn, rows, kStreamSwiglu, m->act, Hl, nullptr, m->granule));
+    } else {
+      DTRY(gemm(m, L.gate_up, 2 * Hl, D, m->xn, rows, m->gu, 2 * Hl));
+      DLAUNCH(m, launch_silu_mul(m->gu, m->act, rows, Hl, m->granule, m->stream));
+    }
+    DTRY(projected(L.down, Hl, m->act, 1, i + 1 < c.layers ? m->h[i + 1].norm1 : m->out_norm));
   }
   return OMNI_OK;
 }
@@ -310,6 +335,7 @@ int depformer_step(omni_duplex* m, int n, const int32_t* force, const int32_t* s
   const omni_duplex_config& c = m->cfg;
   const int D = c.dep_dim, H = c.dep_hidden, S = c.max_sessions;
   const float scale = 1.f / std::sqrt((float)kDepHeadDim);
+  const Chain chain = m->chain();
   DTRY(gemm(m, m->d_input, kDepSteps * D, c.dim, m->xn, n, m->dproj, kDepSteps * D));
   for (int k = 0; k < kDepSteps; ++k) {
     const bf16* table = k == 0 ? m->d_text_emb : m->d_emb + (size_t)(k - 1) * (c.card + 1) * D;
@@ -320,15 +346,14 @@ int depformer_step(omni_duplex* m, int n, const int32_t* force, const int32_t* s
       const DepLayer& L = m->d[i];
       DTRY(gemm(m, L.qkv + (size_t)k * 3 * D * D, 3 * D, D, m->dxn, n, m->dqkv, 3 * D));
       DLAUNCH(m, launch_lm_dep_kv_attend(m->dqkv, m->dkv[i], k, m->dattn, n, c.dep_heads, scale, m->stream));
-      DTRY(gemm(m, L.out + (size_t)k * D * D, D, D, m->dattn, n, m->dy, D));
-      DLAUNCH(m, launch_lm_add_norm(m->dy, m->dx, L.norm2, m->dxn, n, D, c.norm_eps, m->stream));
-      DTRY(gemm(m, L.gate_in + (size_t)k * 2 * H * D, 2 * H, D, m->dxn, n, m->dgu, 2 * H));
-      DLAUNCH(m, launch_silu_mul(m->dgu, m->dact, n, H, 0, m->stream));
-      DTRY(gemm(m, L.gate_out + (size_t)k * D * H, D, H, m->dact, n, m->dy, D));
-      if (i + 1 < c.dep_layers)
-        DLAUNCH(m, launch_lm_add_norm(m->dy, m->dx, m->d[i + 1].norm1, m->dxn, n, D, c.norm_eps, m->stream));
-      else
-        DLAUNCH(m, launch_lm_add_norm(m->dy, m->dx, nullptr, nullptr, n, D, c.norm_eps, m->stream));
+      Summands y;
+      DCUDA(m, chain.gemm(L.out + (size_t)k * D * D, D, D, m->dattn, n, kStreamPartials, nullptr, D, &y));
+      DLAUNCH(m, launch_lm_add_norm_sum(y, m->dx, L.norm2, m->dxn, n, D, c.norm_eps, m->stream));
+      DCUDA(m, chain.gemm(L.gate_in + (size_t)k * 2 * H * D, 2 * H, D, m->dxn, n, kStreamSwiglu, m->dact, H, nullptr, m->d_granule));
+      DCUDA(m, chain.gemm(L.gate_out + (size_t)k * D * H, D, H, m->dact, n, kStreamPartials, nullptr, D, &y));
+      const bool more = i + 1 < c.dep_layers;
+      DLAUNCH(m, launch_lm_add_norm_sum(y, m->dx, more ? m->d[i + 1].norm1 : nullptr, more ? m->dxn : nullptr, n, D,
+                                        c.norm_eps, m->stream));
     }
     bf16* logits = m->audio_logits + (size_t)k * S * c.card;
     DTRY(gemm(m, m->d_heads + (size_t)k * c.card * D, c.card, D, m->dx, n, logits, c.card));
@@ -389,6 +414,7 @@ int32_t omni_duplex_create(const omni_duplex_config* config, const omni_tensor* 
   DCUDA(m, cudaEventCreate(&m->ev1));
   if (tc_init() != 0) return m->fail(OMNI_ERR_CUDA, "cuTensorMapEncodeTiled entry point not found");
   tc_configure();
+  stream_configure();
 
   Index idx;
   for (int i = 0; i < n_tensors; ++i)
@@ -426,6 +452,24 @@ int32_t omni_duplex_create(const omni_duplex_config* config, const omni_tensor* 
     DTRY(weight(m, idx, p + "norm2", {DD}, &L.norm2));
     DTRY(weight(m, idx, p + "gate_in", {kDepSteps * 2 * DH, DD}, &L.gate_in));
     DTRY(weight(m, idx, p + "gate_out", {kDepSteps * DD, DH}, &L.gate_out));
+  }
+
+  {  // gate|up rows regrouped for the fused SwiGLU
+    m->granule = stream_granule((int)Hl, m->sm_count);
+    m->d_granule = stream_granule((int)DH, m->sm_count);
+    bf16* tmp = nullptr;
+    DCUDA(m, cudaDeviceSynchronize());  // the weights were copied on the default stream
+    DCUDA(m, cudaMalloc((void**)&tmp, (size_t)2 * std::max(Hl * D, DH * DD) * sizeof(bf16)));
+    auto regroup = [&](bf16* rows, int64_t inter, int64_t k, int granule) -> int {
+      DCUDA(m, cudaMemcpyAsync(tmp, rows, (size_t)2 * inter * k * sizeof(bf16), cudaMemcpyDeviceToDevice, m->stream));
+      DCUDA(m, launch_interleave_gate_up(tmp, rows, (int)inter, (int)k, granule, m->stream));
+      return OMNI_OK;
+    };
+    for (const HeliumLayer& L : m->h) DTRY(regroup(L.gate_up, Hl, D, m->granule));
+    for (const DepLayer& L : m->d)
+      for (int k = 0; k < kDepSteps; ++k) DTRY(regroup(L.gate_in + (size_t)k * 2 * DH * DD, DH, DD, m->d_granule));
+    DCUDA(m, cudaStreamSynchronize(m->stream));
+    DCUDA(m, cudaFree(tmp));
   }
 
   // pools: every lease is a ring of `context` positions (model.rs:67) and one state line
