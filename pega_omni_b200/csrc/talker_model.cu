@@ -20,6 +20,7 @@
 
 #include "../../include/omni_b200.h"
 #include "../../include/omni_b200_codec.h"
+#include "chain.h"
 #include "gemm.h"
 #include "kernels.h"
 #include "predictor.h"
@@ -40,20 +41,6 @@ int bucket_of(int n) {
 __global__ void f32_to_bf16_kernel(const float* __restrict__ src, bf16* __restrict__ dst, int64_t n) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) dst[i] = __float2bfloat16(src[i]);
-}
-
-// dst = the fused [gate; up] rows of src regrouped as `granule` gate rows, the matching `granule` up rows, ...:
-// one tensor-core tile of 2 * granule weight rows then holds a channel's gate and up columns for the SwiGLU epilogue.
-__global__ void interleave_gate_up_kernel(const bf16* __restrict__ src, bf16* __restrict__ dst, int inter, int k,
-                                          int granule) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;  // one 16-byte piece
-  const int64_t per_row = k / 8, total = (int64_t)2 * inter * per_row;
-  if (i >= total) return;
-  const int64_t row = i / per_row, piece = i % per_row;
-  const bool up = row >= inter;
-  const int64_t c = up ? row - inter : row;
-  const int64_t out_row = (c / granule) * 2 * granule + (up ? granule : 0) + c % granule;
-  *reinterpret_cast<Pack8*>(dst + out_row * k + piece * 8) = *reinterpret_cast<const Pack8*>(src + row * k + piece * 8);
 }
 
 uint16_t host_f2bf(float f) {
@@ -186,6 +173,9 @@ struct omni_talker {
   GemmScratch gemm_scratch;
 
   std::map<std::tuple<const void*, const void*, const void*, int, int>, TcGemmPlan> plans;
+  std::map<std::tuple<const void*, const void*, const void*, int, int>, StreamGemmPlan> stream_plans;
+  Chain chain() { return Chain{stream, err, sm_count, gemm_scratch.partials, gemm_scratch.partial_floats, &launches, &stream_plans}; }
+  bool use_chain = false;  // programs run as chains of kernels (chain.h) rather than as the persistent kernel
   std::map<std::pair<int, int>, cudaGraphExec_t> graphs;  // (program, bucket)
   std::map<std::pair<int, int>, int> graph_nodes;           // kernel nodes of each captured graph
   // the persistent tick kernel: one compiled phase list per (program, bucket)
@@ -309,6 +299,7 @@ int load_stack(omni_talker* m, const TensorIndex& idx, const std::string& prefix
   // gate and up channels are interleaved in groups of half the tile the persistent kernel will use for this GEMM
   out->granule = choose_tiling(2 * c.inter, c.hidden, std::max(1, m->tick_ctas > 0 ? m->tick_ctas : 148), true).tile_n / 2;
   if (c.inter % out->granule) out->granule = 64;
+  if (m->use_chain) out->granule = stream_granule(c.inter, m->sm_count);
   const int64_t h = c.hidden, d = c.head_dim, q = (int64_t)c.q_heads * d, kv = (int64_t)c.kv_heads * d, I = c.inter;
   out->layers.resize(c.layers);
   for (int i = 0; i < c.layers; ++i) {
@@ -336,9 +327,7 @@ int load_stack(omni_talker* m, const TensorIndex& idx, const std::string& prefix
       int rc = upload(m, idx, p + "mlp.gate_proj.weight", {I, h}, fused);
       if (rc == OMNI_OK) rc = upload(m, idx, p + "mlp.up_proj.weight", {I, h}, fused + I * h);
       if (rc == OMNI_OK) {
-        const int64_t pieces = 2 * I * (h / 8);
-        interleave_gate_up_kernel<<<(unsigned)((pieces + 255) / 256), 256, 0, m->stream>>>(fused, L.gate_up, (int)I, (int)h,
-                                                                                     out->granule);
+        if (launch_interleave_gate_up(fused, L.gate_up, (int)I, (int)h, out->granule, m->stream) != cudaSuccess) rc = m->fail(OMNI_ERR_CUDA, "gate|up regroup failed");
         if (cudaStreamSynchronize(m->stream) != cudaSuccess) rc = m->fail(OMNI_ERR_CUDA, "gate|up regroup failed");
       }
       cudaFree(fused);
@@ -373,6 +362,10 @@ int alloc_scratch(omni_talker* m, const StackW& s, int rows, Scratch* out) {
 
 // y[rows, N] = x[rows, K] . w[N, K]^T on the path the row count calls for.
 int gemm(omni_talker* m, const bf16* w, int N, int K, const bf16* x, int rows, bf16* y, int ldy, Epilogue epi = {}) {
+  if (m->use_chain && rows <= kChainRows && stream_supports(N, K, rows)) {
+    CUDA_TRY(m, m->chain().gemm(w, N, K, x, rows, kStreamBf16, y, ldy, nullptr, 0, epi));
+    return OMNI_OK;
+  }
   const bool vector_path = m->cfg.gemm_path == 1 || rows <= 8 || !tc_supports(N, K, rows);
   if (vector_path) {
     LAUNCH(m, gemv_launch(w, N, K, x, rows, y, ldy, epi, m->sm_count, m->stream));
@@ -393,6 +386,17 @@ int gemm(omni_talker* m, const bf16* w, int N, int K, const bf16* x, int rows, b
   return OMNI_OK;
 }
 
+// The layers of a pass whose normalised input is in s.x and whose residual start is in s.res, as a chain of kernels.
+int chain_layers(omni_talker* m, const StackW& S, const Scratch& s, int rows, const RowMap& map,
+                 const std::vector<bf16*>& kv, int kv_pages, bf16* keep_out, int every, int which, const QkvTable& lookup,
+                 bool prompt) {
+  CUDA_TRY(m, chain_pass(m->chain(), S.layers, [](const StackW::Layer& L) { return L.gate_up; },
+                         [](const StackW::Layer& L) { return L.down; }, S.cfg.hidden, S.cfg.inter, S.granule, S.attn(),
+                         ChainBuffers{s.x, s.res, s.qkv, s.attn, s.act}, rows, map, kv, kv_pages, S.norm, keep_out, every,
+                         which, lookup, prompt));
+  return OMNI_OK;
+}
+
 // One pass of a decoder stack: op order of `Stack::forward`
 // (crates/omni-qwen3/src/stack.rs:152-203).
 int stack_forward(omni_talker* m, const StackW& S, const Scratch& s, const bf16* input, int rows, const RowMap& map,
@@ -401,6 +405,7 @@ int stack_forward(omni_talker* m, const StackW& S, const Scratch& s, const bf16*
   const int h = c.hidden, I = c.inter, qd = c.q_heads * c.head_dim;
   const AttnShape a = S.attn();
   LAUNCH(m, launch_norm_copy(input, S.layers[0].ln1, s.x, s.res, rows, h, c.rms_eps, m->stream));
+  if (m->use_chain && rows <= kChainRows) return chain_layers(m, S, s, rows, map, kv, kv_pages, keep_out, every, which, {}, map.seq != nullptr);
   for (int i = 0; i < c.layers; ++i) {
     const StackW::Layer& L = S.layers[i];
     TRY(gemm(m, L.qkv, S.qkv_width(), h, s.x, rows, s.qkv, S.qkv_width()));
@@ -422,7 +427,7 @@ int stack_forward(omni_talker* m, const StackW& S, const Scratch& s, const bf16*
 SlotState slots(omni_talker* m) { return SlotState{m->seq_state, m->din<int32_t>(m->in.lines), m->seq_stride}; }
 
 // `Talker::sample` (crates/omni-qwen3-tts/src/talker.rs:254-290).
-int sample(omni_talker* m, int group, const bf16* logits, int rows) {
+int sample(omni_talker* m, int group, const bf16* logits, int rows, const NextRow& next = {}) {
   const omni_talker_config& c = m->cfg;
   SampleParams p{};
   p.group = group;
@@ -449,8 +454,8 @@ int sample(omni_talker* m, int group, const bf16* logits, int rows) {
     p.min_frames = 0;
     p.penalize = 0;
   }
-  LAUNCH(m, launch_sample(logits, p, m->din<int32_t>(m->in.pos), m->din<float>(m->in.uniforms),
-                          m->din<int32_t>(m->in.force), slots(m), m->codes, rows, m->stream));
+  LAUNCH(m, launch_sample_next(logits, p, m->din<int32_t>(m->in.pos), m->din<float>(m->in.uniforms),
+                               m->din<int32_t>(m->in.force), slots(m), m->codes, next, rows, m->stream));
   return OMNI_OK;
 }
 
@@ -458,6 +463,16 @@ int sample(omni_talker* m, int group, const bf16* logits, int rows) {
 int enqueue_advance(omni_talker* m, int b) {
   const omni_talker_config& c = m->cfg;
   const int h = c.talker.hidden;
+  if (m->use_chain && b <= kChainRows) {
+    LAUNCH(m, launch_frame_embed_norm(slots(m), m->pad_embed, m->codec_emb, c.talker.vocab, m->p_emb, c.predictor.vocab, c.groups,
+                                      m->talker.layers[0].ln1, m->T.res, m->T.x, b, h, c.talker.rms_eps, m->err, m->stream));
+    RowMap rows;
+    rows.pos = m->din<int32_t>(m->in.d_pos);
+    rows.slot = m->din<int32_t>(m->in.d_slot);
+    rows.indptr = m->din<int32_t>(m->in.indptr);
+    rows.pages = m->din<int32_t>(m->in.pages);
+    return chain_layers(m, m->talker, m->T, b, rows, m->kv, m->pages_total, m->hidden, 1, 0, {}, false);
+  }
   LAUNCH(m, launch_frame_embed(slots(m), m->pad_embed, m->codec_emb, c.talker.vocab, m->p_emb, c.predictor.vocab,
                                c.groups, m->t_e, b, h, m->err, m->stream));
   RowMap map;
@@ -467,6 +482,18 @@ int enqueue_advance(omni_talker* m, int b) {
   map.indptr = m->din<int32_t>(m->in.indptr);
   map.pages = m->din<int32_t>(m->in.pages);
   return stack_forward(m, m->talker, m->T, m->t_e, b, map, m->kv, m->pages_total, m->hidden, 1, 0);
+}
+
+// Head g and the draw of codebook g; `folded`: the draw also leaves the next pass's input row (normalised, and residual).
+int tail_draw(omni_talker* m, int g, int b, bool folded) {
+  const omni_talker_config& c = m->cfg;
+  const int p = c.predictor.hidden, PV = c.predictor.vocab;
+  bf16* lg = m->p_logits + (size_t)(g - 1) * m->max_seqs * PV;
+  TRY(gemm(m, m->lm_heads + (size_t)(g - 1) * PV * p, PV, p, m->p_last, b, lg, PV));
+  NextRow next;
+  if (folded && g + 1 < c.groups)
+    next = NextRow{m->p_emb_proj + (size_t)(g - 1) * PV * p, m->pred.layers[0].ln1, m->P.res, m->P.x, p, c.predictor.rms_eps};
+  return sample(m, g, lg, b, next);
 }
 
 // `Talker::tail` (talker.rs:293-356).
@@ -479,8 +506,20 @@ int enqueue_tail(omni_talker* m, int b) {
   Epilogue bias;
   bias.bias = m->mtp_b;
   bias.kind = kEpiBias;
+  // From the second predictor pass on a pass's one input row per sequence is a function of the code just drawn: its
+  // projection and the first layer's q | k | v of it are rows of tables computed at load (p_emb_proj, p_qkv0)
+  const bool folded = m->use_chain && m->p_emb_proj && m->p_qkv0 && 2 * b <= kChainRows;
+  const int qw = m->pred.qkv_width();
   for (int g = 1; g < c.groups; ++g) {
     const int per = g == 1 ? 2 : 1, rows = b * per;
+    if (g > 1 && folded) {
+      RowMap map;
+      map.base = g;
+      const QkvTable lookup{m->p_qkv0 + (size_t)(g - 2) * PV * qw, m->codes, g - 1};
+      TRY(chain_layers(m, m->pred, m->P, b, map, m->pkv, m->max_seqs, m->p_last, 1, 0, lookup, false));
+      TRY(tail_draw(m, g, b, folded));
+      continue;
+    }
     if (g > 1)
       LAUNCH(m, launch_gather(m->codes + (g - 1), OMNI_GROUPS, m->p_emb + (size_t)(g - 2) * PV * h, PV, m->p_in, b, h,
                               m->err, m->stream));
@@ -489,9 +528,7 @@ int enqueue_tail(omni_talker* m, int b) {
     map.per = per;
     map.base = g == 1 ? 0 : g;
     TRY(stack_forward(m, m->pred, m->P, m->p_h, rows, map, m->pkv, m->max_seqs, m->p_last, per, per - 1));
-    bf16* lg = m->p_logits + (size_t)(g - 1) * m->max_seqs * PV;
-    TRY(gemm(m, m->lm_heads + (size_t)(g - 1) * PV * p, PV, p, m->p_last, b, lg, PV));
-    TRY(sample(m, g, lg, b));
+    TRY(tail_draw(m, g, b, folded));
   }
   return OMNI_OK;
 }
@@ -931,7 +968,7 @@ int run_tick_program(omni_talker* m, int program, int b) {
 // as a replay of their captured graph (or eager launches).
 int run_program(omni_talker* m, int program, int b) {
   m->launches = 0;
-  if (m->cfg.tick_kernel && tick_usable(m, b)) return run_tick_program(m, program, b);
+  if (!m->use_chain && m->cfg.tick_kernel && tick_usable(m, b)) return run_tick_program(m, program, b);
   if (!m->cfg.use_graphs) return enqueue_program(m, program, b);
   auto key = std::make_pair(program, b);
   auto it = m->graphs.find(key);
@@ -1169,6 +1206,19 @@ void omni_talker_destroy(omni_talker* m) {
   delete m;
 }
 
+// Whether a model's programs run as chains of kernels (chain.h) or, with `tick_kernel` set, as the persistent kernel.
+static bool chain_wanted(const omni_talker* m) {
+  const omni_talker_config& c = m->cfg;
+  if (c.tick_kernel != 1 || c.gemm_path != 0) return false;
+  double bytes = 0;
+  for (const omni_stack_config* s : {&c.talker, &c.predictor}) {
+    const int qd = s->q_heads * s->head_dim, kvd = s->kv_heads * s->head_dim;
+    if (!chain_supports(s->hidden, s->inter, qd, s->head_dim)) return false;
+    bytes += 2.0 * s->layers * s->hidden * (2.0 * qd + 2.0 * kvd + 3.0 * s->inter);
+  }
+  return bytes > (getenv("CHAIN_ALL") ? 0 : 126e6);
+}
+
 static int create_impl(omni_talker* m, const omni_tensor* tensors, int32_t n_tensors) {
   const omni_talker_config& c = m->cfg;
   const omni_stack_config &t = c.talker, &pc = c.predictor;
@@ -1195,6 +1245,7 @@ static int create_impl(omni_talker* m, const omni_tensor* tensors, int32_t n_ten
   CUDA_TRY(m, cudaEventCreate(&m->ev1));
   if (tc_init() != 0) return m->fail(OMNI_ERR_CUDA, "cuTensorMapEncodeTiled entry point not found");
   tc_configure();
+  stream_configure();
 
   if (c.tick_kernel) {
     m->tick_ctas = tick_configure(m->device);
@@ -1202,6 +1253,7 @@ static int create_impl(omni_talker* m, const omni_tensor* tensors, int32_t n_ten
     TRY(dev_alloc(m, &m->tick_barrier, 64, true));
   }
 
+  m->use_chain = chain_wanted(m);
   TensorIndex idx;
   for (int i = 0; i < n_tensors; ++i) idx.by_name[tensors[i].name] = &tensors[i];
   const int64_t h = t.hidden, p = pc.hidden, V = t.vocab, PV = pc.vocab, G = c.groups;
@@ -1341,7 +1393,7 @@ static int create_impl(omni_talker* m, const omni_tensor* tensors, int32_t n_ten
       TRY(gemm(m, m->pred.layers[0].qkv, (int)qw, (int)p, xn, rows, m->p_qkv0 + r0 * qw, (int)qw));
     }
     CUDA_TRY(m, cudaStreamSynchronize(m->stream));
-    m->plans.clear();  // the plans of these one-off products are not needed again
+    m->plans.clear(), m->stream_plans.clear();  // the plans of these one-off products are not needed again
   }
   return OMNI_OK;
 }
