@@ -4,6 +4,7 @@
 // (crates/omni-qwen3/kernels/qwen3.cu, crates/omni-kern/kernels/common.cuh):
 // every tensor that crosses HBM is bf16, arithmetic is f32.
 #include "attend.cuh"
+#include "decode_attend.cuh"
 #include "kernels.h"
 #include "pdl.cuh"
 #include "rope.cuh"
@@ -317,170 +318,197 @@ cudaError_t launch_attend(const bf16* qkv, const bf16* kv, bf16* out, const RowM
 }
 
 // ---- decode: q/k norm + RoPE + KV write + attention in one kernel ------------------------------------------------
-// One CTA of W warps per (sequence, kv head). The G query heads, the key and the value of a row are dealt to the warps;
-// q goes to shared memory, k and v to the row's slot, and the same CTA then attends to them. The pages that earlier
-// calls filled are asked for before grid_wait(): they come through bulk copies into the warps' staging slots while
-// the projection before this kernel still runs. The row's own page is read with ordinary loads after the write.
-// W: enough warps that one wave of CTAs has every page of a long context under way.
+// A team of W warps per (sequence, kv head). The G query heads, the key and the value of a row are dealt to the team's
+// warps; q, k and v go to shared memory (k and v also to the row's slot), and the team attends to them with the page step
+// of decode_attend.cuh, each warp on its own pages. A page is 16 loads of 16 bytes a lane, straight into registers.
+// Paged rows: a warp's first page is asked for before grid_wait() - what earlier calls wrote does not depend on the
+// projection this kernel waits for - and the row's own token is patched in from shared memory.
+// Dense frames (the predictor): one page per sequence, W = 1, four sequences' heads per CTA; the page is asked for
+// together with the row, and the tokens this kernel itself writes are patched in.
 
+template <int D, int G>
+struct RopeShared {
+  alignas(16) bf16 q[8][D];
+  alignas(16) bf16 k[2][D];
+  alignas(16) bf16 v[2][D];
+};
 template <int D, int G, int W>
-__global__ void __launch_bounds__(W * 32)
+struct MergeShared {
+  float m[W][8], l[W][8];
+  float o[W][G][D];
+};
+template <int D, int G>
+struct MergeShared<D, G, 1> {};
+
+template <int D, int G, int W, int TEAMS>
+__global__ void __launch_bounds__(W * TEAMS * 32, W == 8 ? 1 : 3)
     rope_attend_kernel(const bf16* __restrict__ qkv, const QkvTable lookup, const bf16* __restrict__ q_norm,
-                       const bf16* __restrict__ k_norm, bf16* kv, bf16* __restrict__ out, RowMap map, int hq, int hk,
-                       float eps, float theta, float scale, int kv_pages, uint32_t* err) {
-  constexpr int E = D / 64, VE = D / 32, PV = D / 32;
+                       const bf16* __restrict__ k_norm, bf16* kv, bf16* __restrict__ out, RowMap map, int items, int hq,
+                       int hk, float eps, float theta, float scale, int kv_pages, uint32_t* err) {
+  static_assert(W == 1 || TEAMS == 1, "a team of several warps is a CTA");
+  constexpr int E = D / 64, VE = D / 32;
   grid_trigger();
-  extern __shared__ __align__(128) unsigned char ra_slots[];
-  __shared__ AttnShared<D, G, W> sh;
-  __shared__ __align__(8) uint64_t bars[W];
-  const int seq = blockIdx.x, kh = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int per = map.pages ? 1 : map.per;
-  const int32_t* pages = map.pages ? map.pages + map.indptr[map.seq ? map.seq[seq] : seq] : nullptr;
+  __shared__ RopeShared<D, G> shared[TEAMS];
+  __shared__ MergeShared<D, G, W> merge;
+  const int lane = threadIdx.x & 31, warp = (threadIdx.x >> 5) % W, team = (threadIdx.x >> 5) / W;
+  const int item = blockIdx.x * TEAMS + team, seq = item / hk, kh = item % hk;
+  const bool live = item < items;
+  RopeShared<D, G>& sh = shared[team];
+  auto team_sync = [&]() {
+    if constexpr (W == 1) __syncwarp();
+    else __syncthreads();
+  };
+  const bool paged = map.pages != nullptr;
+  const int per = paged ? 1 : map.per;
   float qwl[E], qwh[E], kwl[E], kwh[E];
 #pragma unroll
   for (int e = 0; e < E; ++e) {
     qwl[e] = __bfloat162float(q_norm[lane * E + e]), qwh[e] = __bfloat162float(q_norm[D / 2 + lane * E + e]);
     kwl[e] = __bfloat162float(k_norm[lane * E + e]), kwh[e] = __bfloat162float(k_norm[D / 2 + lane * E + e]);
   }
-  if (lane == 0) {
-    sm100::mbar_init(sm100::smem_addr(&bars[warp]), 1);
-    sm100::mbar_init_fence();
-  }
-  __syncwarp();
-  bf16* mine = reinterpret_cast<bf16*>(ra_slots + (size_t)warp * kv_block_bytes<D>());
-  auto issue = [&](int pi) {
-    int64_t page = pages[pi];
-    if (page < 0 || page >= kv_pages) {
-      raise(err, kErrBadIndex);
-      page = 0;
-    }
-    sm100::mbar_expect_tx(sm100::smem_addr(&bars[warp]), kv_block_bytes<D>());
-    sm100::bulk_load(sm100::smem_addr(mine), kv + kv_offset<D>(page, hk, kh, 0, 0), kv_block_bytes<D>(), sm100::smem_addr(&bars[warp]));
-  };
-  uint32_t parity = 0;
+  for (int i = warp * 32 + lane; i < (8 - G) * D / 8; i += W * 32)  // heads past G: zero rows
+    *reinterpret_cast<uint4*>(&sh.q[G][0] + i * 8) = make_uint4(0u, 0u, 0u, 0u);
+  const int32_t* pages = paged && live ? map.pages + map.indptr[seq] : nullptr;
+  dattn::Page<D> pg;
+  dattn::State<D> st;
   for (int r = 0; r < per; ++r) {
-    const int n = seq * per + r;
-    const int pos = map.pages ? map.pos[n] : map.base + r;
-    const int len = pos + 1, npages = (len + 15) >> 4, last = npages - 1;
+    const int n = live ? seq * per + r : 0;
+    const int pos = paged ? map.pos[n] : map.base + r;
+    const int npages = paged ? (pos + 16) >> 4 : 1, last = npages - 1;
     float cs[E], sn[E];
     rope_angles<D>(lane, pos, theta, cs, sn);
-    const int64_t slot = map.pages ? map.slot[n] : (int64_t)seq * 16 + pos;
-    int64_t page = slot >> 4;
+    const int64_t slot = paged ? map.slot[n] : (int64_t)seq * 16 + pos;
+    int64_t own = slot >> 4;
     const int tok = (int)(slot & 15);
-    if (page < 0 || page >= kv_pages) {
-      if (tid == 0) raise(err, kErrBadIndex);
-      page = 0;
+    if (own < 0 || own >= kv_pages) {
+      if (live && warp == 0 && lane == 0) raise(err, kErrBadIndex);
+      own = 0;
     }
-    if (warp < last && lane == 0) issue(warp);  // (map.pages only: a dense sequence has one page)
+    auto load = [&](int pi) {
+      int64_t page = pi == last ? own : pages[pi];
+      if (page < 0 || page >= kv_pages) {
+        if (lane == 0) raise(err, kErrBadIndex);
+        page = 0;
+      }
+      pg.load(kv + kv_offset<D>(page, hk, kh, 0, 0), lane);
+    };
+    if (paged && live && warp < npages) load(warp);
     if (r == 0) grid_wait();
+    if (W == 1 && !live) return;  // (a dead team of several warps does not exist: TEAMS is 1 there)
+    if (!paged) load(0);
     const bf16* row = lookup.table ? lookup.table + (int64_t)lookup.codes[n * 16 + lookup.group] * ((hq + 2 * hk) * D)
                                    : qkv + (int64_t)n * ((hq + 2 * hk) * D);
-    for (int job = warp; job < G + 2; job += W) {
-      if (job == G + 1) {  // value: a plain copy
-        bf16* dst = kv + kv_offset<D>(page, hk, kh, 1, tok);
-        const bf16* src = row + (hq + hk + kh) * D;
-        if constexpr (VE == 4) *reinterpret_cast<uint2*>(dst + lane * 4) = __ldcg(reinterpret_cast<const uint2*>(src + lane * 4));
-        else *reinterpret_cast<uint32_t*>(dst + lane * 2) = __ldcg(reinterpret_cast<const uint32_t*>(src + lane * 2));
-        continue;
-      }
-      const bool is_q = job < G;
-      const bf16* src = row + (is_q ? kh * G + job : hq + kh) * D;
-      float lo[E], hi[E];
-      if constexpr (E == 2) {
-        const uint32_t a2 = __ldcg(reinterpret_cast<const uint32_t*>(src) + lane), b2 = __ldcg(reinterpret_cast<const uint32_t*>(src + D / 2) + lane);
-        lo[0] = __uint_as_float(a2 << 16), lo[1] = __uint_as_float(a2 & 0xffff0000u);
-        hi[0] = __uint_as_float(b2 << 16), hi[1] = __uint_as_float(b2 & 0xffff0000u);
-      } else {
-        lo[0] = __uint_as_float((uint32_t)__ldcg(reinterpret_cast<const uint16_t*>(src) + lane) << 16);
-        hi[0] = __uint_as_float((uint32_t)__ldcg(reinterpret_cast<const uint16_t*>(src + D / 2) + lane) << 16);
-      }
-      if (is_q) rope_head<D>(lo, hi, qwl, qwh, cs, sn, eps);
-      else rope_head<D>(lo, hi, kwl, kwh, cs, sn, eps);
-      bf16* kdst = kv + kv_offset<D>(page, hk, kh, 0, tok);
+    constexpr int JOBS = (G + 2 + W - 1) / W;
+    uint32_t raw[JOBS][2];
 #pragma unroll
-      for (int e = 0; e < E; ++e) {
-        const int i = lane * E + e;
-        if (is_q) {
-          sh.qs[job][i] = lo[e], sh.qs[job][D / 2 + i] = hi[e];
+    for (int jj = 0; jj < JOBS; ++jj) {  // every head of this warp's share is asked for before the first is used
+      const int job = warp + jj * W;
+      const bf16* src = row + (job < G ? kh * G + job : job == G ? hq + kh : hq + hk + kh) * D;
+      if (job < G + 2) {
+        if constexpr (E == 2) {
+          raw[jj][0] = __ldcg(reinterpret_cast<const uint32_t*>(src) + lane), raw[jj][1] = __ldcg(reinterpret_cast<const uint32_t*>(src + D / 2) + lane);
         } else {
-          kdst[i] = __float2bfloat16(lo[e]), kdst[D / 2 + i] = __float2bfloat16(hi[e]);
+          raw[jj][0] = __ldcg(reinterpret_cast<const uint16_t*>(src) + lane), raw[jj][1] = __ldcg(reinterpret_cast<const uint16_t*>(src + D / 2) + lane);
         }
       }
     }
-    __threadfence_block();
-    __syncthreads();
-    float m[G], l[G], acc[G][PV];
 #pragma unroll
-    for (int g = 0; g < G; ++g) {
-      m[g] = -INFINITY, l[g] = 0.f;
+    for (int jj = 0; jj < JOBS; ++jj) {
+      const int job = warp + jj * W;
+      if (job >= G + 2) continue;
+      float lo[E], hi[E];
+      lo[0] = __uint_as_float(raw[jj][0] << 16), hi[0] = __uint_as_float(raw[jj][1] << 16);
+      if constexpr (E == 2) lo[1] = __uint_as_float(raw[jj][0] & 0xffff0000u), hi[1] = __uint_as_float(raw[jj][1] & 0xffff0000u);
+      if (job < G) rope_head<D>(lo, hi, qwl, qwh, cs, sn, eps);
+      else if (job == G) rope_head<D>(lo, hi, kwl, kwh, cs, sn, eps);
+      bf16* dst = job < G ? sh.q[job] : job == G ? sh.k[r & 1] : sh.v[r & 1];
+      bf16* page = job < G ? nullptr : kv + kv_offset<D>(own, hk, kh, job - G, tok);
 #pragma unroll
-      for (int d = 0; d < PV; ++d) acc[g][d] = 0.f;
+      for (int e = 0; e < E; ++e) {
+        const bf16 a = __float2bfloat16(lo[e]), b = __float2bfloat16(hi[e]);
+        dst[lane * E + e] = a, dst[D / 2 + lane * E + e] = b;
+        if (page) page[lane * E + e] = a, page[D / 2 + lane * E + e] = b;
+      }
     }
+    team_sync();
+    uint4 q[D / 32];
+#pragma unroll
+    for (int j = 0; j < D / 32; ++j) q[j] = *reinterpret_cast<const uint4*>(sh.q[lane >> 2] + 8 * (lane & 3) + 32 * j);
+    st.reset();
     for (int pi = warp; pi < npages; pi += W) {
-      KvBlock<D> blk;
-      if (pi < last) {
-        sm100::mbar_wait(sm100::smem_addr(&bars[warp]), parity, err);
-        parity ^= 1u;
-        blk.load(mine, lane);
-        __syncwarp();  // the block is in registers: its slot takes the warp's next one
-        if (lane == 0 && pi + W < last) issue(pi + W);
-      } else {
-        blk.load(kv + kv_offset<D>(page, hk, kh, 0, 0), lane);
+      if (pi != warp) load(pi);
+      if (pi == last) {
+        if (!paged && r > 0) pg.patch(tok - 1, sh.k[(r - 1) & 1], sh.v[(r - 1) & 1], lane);  // (per <= 2)
+        pg.patch(tok, sh.k[r & 1], sh.v[r & 1], lane);
       }
-      page_update<D, G>(blk, sh.qs, min(16, len - pi * 16), scale, lane, m, l, acc);
+      st.step(pg, q, min(16, pos + 1 - pi * 16), scale, lane);
     }
+    st.finish();
+    const int g = lane >> 2, t = lane & 3;
+    if constexpr (W == 1) {
 #pragma unroll
-    for (int g = 0; g < G; ++g) {
-      if (lane == 0) sh.ms[warp][g] = m[g], sh.ls[warp][g] = l[g];
+      for (int h = 0; h < 2; ++h)
+        if (2 * t + h < G) {
+          const float inv = 1.f / st.l[h];
 #pragma unroll
-      for (int d = 0; d < PV; ++d) sh.os[warp][g][lane * PV + d] = acc[g][d];
-    }
-    __syncthreads();
-    const int live = min(W, npages);  // warps that held a page
-    for (int i = tid; i < G * D; i += W * 32) {
-      const int g = i / D, d = i % D;
-      float top = -INFINITY;
-      for (int w = 0; w < live; ++w) top = fmaxf(top, sh.ms[w][g]);
-      float num = 0.f, den = 0.f;
-      for (int w = 0; w < live; ++w) {
-        const float e = __expf(sh.ms[w][g] - top);
-        num += sh.os[w][g][d] * e;
-        den += sh.ls[w][g] * e;
+          for (int i = 0; i < D / 64; ++i) {
+            float v[8];
+            st.dims8(i, h, v);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) v[e] *= inv;
+            st8(out + ((int64_t)n * hq + kh * G + 2 * t + h) * D + 64 * i + 8 * g, v);
+          }
+        }
+      __syncwarp();  // q is free for the next row
+    } else {
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+        if (2 * t + h < G) {
+          if (g == 0) merge.m[warp][2 * t + h] = st.m[h], merge.l[warp][2 * t + h] = st.l[h];
+#pragma unroll
+          for (int i = 0; i < D / 64; ++i) {
+            float v[8];
+            st.dims8(i, h, v);
+            float4* dst = reinterpret_cast<float4*>(&merge.o[warp][2 * t + h][64 * i + 8 * g]);
+            dst[0] = make_float4(v[0], v[1], v[2], v[3]), dst[1] = make_float4(v[4], v[5], v[6], v[7]);
+          }
+        }
+      __syncthreads();
+      const int used = min(W, npages);  // warps that held a page
+      for (int i = threadIdx.x; i < G * D; i += W * 32) {
+        const int h = i / D, d = i % D;
+        float top = -INFINITY;
+        for (int w = 0; w < used; ++w) top = fmaxf(top, merge.m[w][h]);
+        float num = 0.f, den = 0.f;
+        for (int w = 0; w < used; ++w) {
+          const float e = __expf(merge.m[w][h] - top);
+          num += merge.o[w][h][d] * e;
+          den += merge.l[w][h] * e;
+        }
+        out[((int64_t)n * hq + kh * G) * D + i] = __float2bfloat16(num / den);
       }
-      out[((int64_t)n * hq + kh * G) * D + i] = __float2bfloat16(num / den);
-    }
-    if (r + 1 < per) __syncthreads();  // q and the warps' states are free for the next row
-  }
-}
-
-template <int D, int G, int W>
-static cudaError_t launch_rope_attend_dgw(const bf16* qkv, const QkvTable& lookup, const bf16* q_norm, const bf16* k_norm,
-                                          bf16* kv, bf16* out, const RowMap& map, int seqs, const AttnShape& a,
-                                          int kv_pages, uint32_t* err, cudaStream_t s) {
-  const size_t smem = map.pages ? (size_t)W * kv_block_bytes<D>() : 0;
-  if (smem + sizeof(AttnShared<D, G, W>) > 40 * 1024) {  // per device and instantiation: above the default limit of dynamic shared memory
-    static bool raised[64] = {};
-    int device = 0;
-    if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= 64) return cudaErrorInvalidDevice;
-    if (!raised[device]) {
-      const cudaError_t e = cudaFuncSetAttribute(rope_attend_kernel<D, G, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      if (e != cudaSuccess) return e;
-      raised[device] = true;
     }
   }
-  return launch_pdl(rope_attend_kernel<D, G, W>, dim3(seqs, a.kv_heads), dim3(W * 32), smem, s, qkv, lookup, q_norm, k_norm,
-                    kv, out, map, a.q_heads, a.kv_heads, a.rms_eps, a.rope_theta, 1.f / sqrtf((float)D), kv_pages, err);
 }
 
 template <int D, int G>
 static cudaError_t launch_rope_attend_dg(const bf16* qkv, const QkvTable& lookup, const bf16* q_norm, const bf16* k_norm,
                                          bf16* kv, bf16* out, const RowMap& map, int rows, const AttnShape& a,
                                          int kv_pages, uint32_t* err, cudaStream_t s) {
-  const int seqs = map.pages ? rows : rows / map.per;
-  // a few sequences: eight warps each (more would not leave a thread the registers of a page); many: four, several CTAs per SM
-  if (map.pages && seqs * a.kv_heads <= 148)
-    return launch_rope_attend_dgw<D, G, 8>(qkv, lookup, q_norm, k_norm, kv, out, map, seqs, a, kv_pages, err, s);
-  return launch_rope_attend_dgw<D, G, 4>(qkv, lookup, q_norm, k_norm, kv, out, map, seqs, a, kv_pages, err, s);
+  const int items = (map.pages ? rows : rows / map.per) * a.kv_heads;
+  const float scale = 1.f / sqrtf((float)D);
+  if (!map.pages) {
+    if (map.per > 2) return cudaErrorInvalidValue;
+    return launch_pdl(rope_attend_kernel<D, G, 1, 4>, dim3((items + 3) / 4), dim3(128), 0, s, qkv, lookup, q_norm, k_norm, kv, out,
+                      map, items, a.q_heads, a.kv_heads, a.rms_eps, a.rope_theta, scale, kv_pages, err);
+  }
+  if (map.seq) return cudaErrorInvalidValue;  // one row per sequence
+  // items that leave SMs idle: eight warps each, so that 128 keys are one round; many: four, four CTAs per SM
+  if (items <= 148)
+    return launch_pdl(rope_attend_kernel<D, G, 8, 1>, dim3(items), dim3(256), 0, s, qkv, lookup, q_norm, k_norm, kv, out, map,
+                      items, a.q_heads, a.kv_heads, a.rms_eps, a.rope_theta, scale, kv_pages, err);
+  return launch_pdl(rope_attend_kernel<D, G, 4, 1>, dim3(items), dim3(128), 0, s, qkv, lookup, q_norm, k_norm, kv, out, map, items,
+                    a.q_heads, a.kv_heads, a.rms_eps, a.rope_theta, scale, kv_pages, err);
 }
 
 template <int D>
