@@ -600,15 +600,11 @@ __global__ void lm_dep_kv_attend_kernel(const bf16* __restrict__ qkv, bf16* __re
 // the k-th largest key (ties kept), score = logit / T - log(-log u) with u = ((mix(seed ^ mix(index)) >> 8) + 0.5) /
 // 2^24, winner = largest (order_key(score), lowest index).
 //
-// One CTA of 1024 threads per row. The row is read from memory ONCE: every thread keeps its share of the keys in
-// registers (two per register, up to 64 per thread = a vocabulary of 65,536). The cut is then found by bisection on
-// the key's 16 bits, most significant first: a bit stays set when at least k keys are >= the candidate, which takes
-// one count per round over registers, a shuffle sum per warp and one block barrier (the per-warp counts are
-// double-buffered in shared memory, so a round needs no second barrier). The survivors' scores are computed from the
-// same registers and the winner is reduced by shuffles and one pass over the 32 warp results.
-
-constexpr int kSampleThreads = 1024;
-constexpr int kSampleRegs = 32;  // packed key pairs per thread
+// One CTA per row. The row is read from memory ONCE: a thread keeps R packed pairs of keys in registers (256 threads x 4
+// for a codebook of 2,048, 1,024 x 16 or x 32 for a text vocabulary up to 65,536). The cut is then found by bisection on
+// the key's 16 bits, two at a time from the top: the counts of keys >= three candidates take one warp reduction each and
+// one block barrier a round (the per-warp counts are double-buffered in shared memory). The survivors' scores are
+// computed from the same registers and the winner is reduced by shuffles and one pass over the warps' results.
 
 __device__ __forceinline__ uint32_t order_key32(float v) {
   const uint32_t u = __float_as_uint(v);
@@ -630,56 +626,84 @@ __device__ __forceinline__ uint32_t mix32(uint32_t x) {
   return x;
 }
 
-__global__ void __launch_bounds__(kSampleThreads)
+template <int THREADS, int R>
+__global__ void __launch_bounds__(THREADS)
     lm_sample_kernel(const bf16* __restrict__ logits, int vocab, int64_t ld, float temperature, int top_k,
                      const int32_t* __restrict__ force, const int32_t* __restrict__ seeds, int col,
                      int32_t* __restrict__ drawn) {
+  constexpr int WARPS = THREADS / 32;
   grid_trigger();
-  grid_wait();
   const int s = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  __shared__ uint32_t counts[2][kSampleThreads / 32];
-  __shared__ unsigned long long best[kSampleThreads / 32];
+  __shared__ uint32_t counts[2][3][WARPS];
+  __shared__ unsigned long long best[WARPS];
   const int forced = force[s * kDuplexDrawn + col];
+  const uint32_t seed = mix32((uint32_t)seeds[2 * s] ^ mix32((uint32_t)seeds[2 * s + 1] + 0x9e3779b9u * (col + 1)));
+  grid_wait();
   if (forced >= 0) {
     if (tid == 0) drawn[s * kDuplexDrawn + col] = forced;
     return;
   }
-  // element 2 * (r * 1024 + tid) + {0, 1} lives in the low / high half of reg[r]; 0 past the vocabulary (the smallest
+  // element 2 * (r * THREADS + tid) + {0, 1} lives in the low / high half of reg[r]; 0 past the vocabulary (the smallest
   // key there is: -NaN with every mantissa bit set orders lowest, and no count ever includes index >= vocab)
   const uint16_t* row = reinterpret_cast<const uint16_t*>(logits + (int64_t)s * ld);
-  uint32_t reg[kSampleRegs];
+  const bool pairs = (reinterpret_cast<uintptr_t>(row) & 3) == 0;
+  uint32_t reg[R];
 #pragma unroll
-  for (int r = 0; r < kSampleRegs; ++r) {
-    const int i = 2 * (r * kSampleThreads + tid);
-    const uint32_t k0 = i < vocab ? order_key16(row[i]) : 0u, k1 = i + 1 < vocab ? order_key16(row[i + 1]) : 0u;
+  for (int r = 0; r < R; ++r) {
+    const int i = 2 * (r * THREADS + tid);
+    uint32_t two = 0u;
+    if (pairs && i + 1 < vocab) {
+      two = __ldcg(reinterpret_cast<const uint32_t*>(row + i));
+    } else {
+      if (i < vocab) two = __ldcg(row + i);
+      if (i + 1 < vocab) two |= (uint32_t)__ldcg(row + i + 1) << 16;
+    }
+    reg[r] = two;
+  }
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const int i = 2 * (r * THREADS + tid);
+    const uint32_t k0 = i < vocab ? order_key16(reg[r] & 0xffffu) : 0u, k1 = i + 1 < vocab ? order_key16(reg[r] >> 16) : 0u;
     reg[r] = k0 | k1 << 16;
   }
   const float inv_t = temperature > 0.f ? 1.f / temperature : 1.f;
   const int keep = top_k > 0 && top_k < vocab ? top_k : vocab;
   uint32_t cut = 0;
   if (temperature > 0.f && keep < vocab) {
-    for (int bit = 15; bit >= 0; --bit) {
-      const uint32_t cand = cut | 1u << bit;  // cand >= 1: the padding keys (0) never count
-      uint32_t c = 0;
+#pragma unroll 1
+    for (int bit = 14; bit >= 0; bit -= 2) {
+      uint32_t c[3] = {0u, 0u, 0u};
 #pragma unroll
-      for (int r = 0; r < kSampleRegs; ++r) c += ((reg[r] & 0xffffu) >= cand) + ((reg[r] >> 16) >= cand);
+      for (int r = 0; r < R; ++r) {
+        const uint32_t k0 = reg[r] & 0xffffu, k1 = reg[r] >> 16;
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
-      if (lane == 0) counts[bit & 1][warp] = c;
+        for (int q = 0; q < 3; ++q) {  // candidates >= 1: the padding keys (0) never count
+          const uint32_t cand = cut | (uint32_t)(q + 1) << bit;
+          c[q] += (k0 >= cand) + (k1 >= cand);
+        }
+      }
+      const int buf = (bit >> 1) & 1;
+#pragma unroll
+      for (int q = 0; q < 3; ++q) {
+        c[q] = __reduce_add_sync(0xffffffffu, c[q]);
+        if (lane == 0) counts[buf][q][warp] = c[q];
+      }
       __syncthreads();
-      uint32_t total = 0;
+      uint32_t digit = 0;
 #pragma unroll
-      for (int w = 0; w < kSampleThreads / 32; ++w) total += counts[bit & 1][w];
-      if (total >= (uint32_t)keep) cut = cand;
+      for (int q = 0; q < 3; ++q) {
+        const uint32_t total = __reduce_add_sync(0xffffffffu, lane < WARPS ? counts[buf][q][lane] : 0u);
+        if (total >= (uint32_t)keep) digit = q + 1;
+      }
+      cut |= digit << bit;
     }
   }
-  const uint32_t seed = mix32((uint32_t)seeds[2 * s] ^ mix32((uint32_t)seeds[2 * s + 1] + 0x9e3779b9u * (col + 1)));
   unsigned long long mine = 0ull;
 #pragma unroll
-  for (int r = 0; r < kSampleRegs; ++r) {
+  for (int r = 0; r < R; ++r) {
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
-      const int i = 2 * (r * kSampleThreads + tid) + e;
+      const int i = 2 * (r * THREADS + tid) + e;
       const uint32_t key = e ? reg[r] >> 16 : reg[r] & 0xffffu;
       if (i >= vocab || key < cut) continue;
       float score = logit_of(key) * inv_t;
@@ -699,7 +723,7 @@ __global__ void __launch_bounds__(kSampleThreads)
   if (lane == 0) best[warp] = mine;
   __syncthreads();
   if (warp == 0) {
-    mine = best[lane];
+    mine = lane < WARPS ? best[lane] : 0ull;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
       const unsigned long long other = __shfl_xor_sync(0xffffffffu, mine, o);
@@ -879,8 +903,13 @@ cudaError_t launch_lm_sample(const bf16* logits, int vocab, int64_t ld, float te
                              const int32_t* force, const int32_t* seeds, int col, int32_t* drawn, int rows,
                              cudaStream_t s) {
   if (vocab < 1 || col < 0 || col >= kDuplexDrawn) return cudaErrorInvalidValue;
-  if (vocab > 2 * kSampleRegs * kSampleThreads) return cudaErrorInvalidValue;  // a thread keeps 64 keys in registers
-  return launch_pdl(lm_sample_kernel, dim3(rows), dim3(kSampleThreads), 0, s, logits, vocab, ld, temperature, top_k, force, seeds, col, drawn);
+  auto go = [&](auto kernel, int threads) {
+    return launch_pdl(kernel, dim3(rows), dim3(threads), 0, s, logits, vocab, ld, temperature, top_k, force, seeds, col, drawn);
+  };
+  if (vocab <= 2048) return go(lm_sample_kernel<256, 4>, 256);
+  if (vocab <= 32768) return go(lm_sample_kernel<1024, 16>, 1024);
+  if (vocab <= 65536) return go(lm_sample_kernel<1024, 32>, 1024);
+  return cudaErrorInvalidValue;
 }
 
 cudaError_t launch_lm_advance(void* state, const int32_t* lines, int64_t stride, const int32_t* drawn,
