@@ -1,16 +1,26 @@
 // A pass of up to 256 rows of a Qwen3-style decoder stack as a chain of kernels under programmatic dependent launch: per layer
 // seven kernels - q|k|v GEMM, rope + KV write + attention, o GEMM, add + norm, gate|up GEMM with SwiGLU, down GEMM,
-// add + norm - of which every GEMM has its first weights in shared memory by the time its input rows are there.
+// add + norm - of which every GEMM has its first weights in shared memory by the time its input rows are there. For a few
+// rows the add + norm is part of the GEMM behind it: five kernels.
 // Op order and rounding points of `Stack::forward` (crates/omni-qwen3/src/stack.rs:152-203).
 #pragma once
 #include <map>
 #include <tuple>
 #include <vector>
 
+#include "few_rows.h"
 #include "kernels.h"
 #include "stream_gemm.h"
 
 namespace omni {
+
+// A GEMM of a chain is planned once per (weights, inputs, outputs, rows) and kept by the model.
+struct ChainPlan {
+  bool few = false;
+  FewPlan f;
+  StreamGemmPlan s;
+};
+using ChainPlans = std::map<std::tuple<const void*, const void*, const void*, int, int>, ChainPlan>;
 
 struct Chain {
   cudaStream_t stream = nullptr;
@@ -19,22 +29,47 @@ struct Chain {
   float* partials = nullptr;
   size_t partial_floats = 0;
   int* launches = nullptr;
-  std::map<std::tuple<const void*, const void*, const void*, int, int>, StreamGemmPlan>* plans = nullptr;
+  ChainPlans* plans = nullptr;
 
   // y (bf16 rows, SwiGLU activations) or, for kStreamPartials, *sum
   cudaError_t gemm(const bf16* w, int N, int K, const bf16* x, int rows, int out, bf16* y, int ldy, Summands* sum = nullptr,
                    int granule = 0, Epilogue epi = {}) const {
+    ChainPlan* p = plan(w, N, K, x, rows, out, y, ldy, granule, epi);
+    return p ? launch(*p, {}, sum) : cudaErrorInvalidValue;
+  }
+
+  // The same behind the add + norm of `norm.sum` into the residual rows `*res` (then exchanged with `*spare`): in one
+  // kernel where few_rows.h takes the shape, otherwise by `apart`, which updates *res in place and writes x.
+  template <typename Apart>
+  cudaError_t norm_gemm(FewNorm norm, bf16** res, bf16** spare, const Apart& apart, const bf16* w, int N, int K, const bf16* x,
+                        int rows, int out, bf16* y, int ldy, int granule = 0) const {
+    if (few_norm_fits(K, rows) && norm.sum.splits >= 1 && norm.sum.splits <= 4) {
+      if (ChainPlan* p = plan(w, N, K, nullptr, rows, out, y, ldy, granule, {})) {
+        norm.res_in = *res, norm.res_out = *spare;
+        std::swap(*res, *spare);
+        return launch(*p, norm, nullptr);
+      }
+    }
+    ++*launches;
+    const cudaError_t e = apart(norm.sum, *res);
+    return e != cudaSuccess ? e : gemm(w, N, K, x, rows, out, y, ldy, nullptr, granule);
+  }
+
+ private:
+  ChainPlan* plan(const bf16* w, int N, int K, const bf16* x, int rows, int out, bf16* y, int ldy, int granule, Epilogue epi) const {
     const auto key = std::make_tuple((const void*)w, (const void*)x, (const void*)y, rows, out);
     auto it = plans->find(key);
-    if (it == plans->end()) {
-      StreamGemmPlan plan;
-      if (stream_plan(&plan, w, N, K, x, rows, out, y, ldy, partials, epi, sm_count, granule) != 0) return cudaErrorInvalidValue;
-      if (out == kStreamPartials && plan.partial_floats() > partial_floats) return cudaErrorInvalidValue;
-      it = plans->emplace(key, plan).first;
-    }
-    if (sum) *sum = it->second.summands();
+    if (it != plans->end()) return &it->second;
+    ChainPlan p;
+    p.few = few_plan(&p.f, w, N, K, x, rows, out, y, ldy, partials, epi, sm_count, granule) == 0;
+    if (!p.few && (!x || stream_plan(&p.s, w, N, K, x, rows, out, y, ldy, partials, epi, sm_count, granule) != 0)) return nullptr;
+    if (out == kStreamPartials && (p.few ? p.f.partial_floats() : p.s.partial_floats()) > partial_floats) return nullptr;
+    return &plans->emplace(key, p).first->second;
+  }
+  cudaError_t launch(const ChainPlan& p, const FewNorm& norm, Summands* sum) const {
+    if (sum) *sum = p.few ? p.f.summands() : p.s.summands();
     ++*launches;
-    return stream_launch(it->second, err, stream);
+    return p.few ? few_launch(p.f, norm, err, stream) : stream_launch(p.s, err, stream);
   }
 };
 
@@ -45,7 +80,7 @@ struct Chain {
   } while (0)
 
 struct ChainBuffers {
-  bf16 *x, *res, *qkv, *attn, *act;  // x, res: the normalised rows and the residual stream the pass starts from
+  bf16 *x, *res, *spare, *qkv, *attn, *act;  // x, res: the normalised rows and the residual stream the pass starts from
 };
 
 // Whether a stack of this shape can run as a chain (the rest is up to the row count).
@@ -58,15 +93,27 @@ constexpr int kChainRows = 256;  // beyond this the GEMMs are contractions, not 
 // gate_up(l) and down(l) pick a layer's MLP; `inter` is its width, its gate|up rows lie in groups of `granule`.
 template <typename Layer, typename GateUp, typename Down>
 cudaError_t chain_pass(const Chain& c, const std::vector<Layer>& layers, const GateUp& gate_up, const Down& down, int hidden,
-                       int inter, int granule, const AttnShape& a, const ChainBuffers& b, int rows, const RowMap& map,
+                       int inter, int granule, const AttnShape& a, ChainBuffers b, int rows, const RowMap& map,
                        const std::vector<bf16*>& kv, int kv_pages, const bf16* final_gain, bf16* keep_out, int every,
                        int which, const QkvTable& lookup = {}, bool prompt = false) {
   const int qd = a.q_heads * a.head_dim, qw = (a.q_heads + 2 * a.kv_heads) * a.head_dim;
+  Summands sum;
+  FewNorm norm;
+  norm.kind = kNormStack, norm.eps = a.rms_eps;
+  // the add + norm of `sum` by layer gain `gain`, and the GEMM of the rows it makes
+  auto norm_gemm = [&](const bf16* gain, const bf16* w, int N, int out, bf16* y, int ldy, int g) {
+    norm.sum = sum, norm.gain = gain;
+    return c.norm_gemm(norm, &b.res, &b.spare,
+                       [&](const Summands& from, bf16* res) {
+                         return launch_add_norm_sum(from, res, gain, b.x, rows, hidden, a.rms_eps, 1, 0, c.stream);
+                       },
+                       w, N, hidden, b.x, rows, out, y, ldy, g);
+  };
   for (size_t i = 0; i < layers.size(); ++i) {
     const Layer& L = layers[i];
     const QkvTable& from = i == 0 ? lookup : QkvTable{};
-    Summands sum;
-    if (!from.table) OMNI_CHAIN(c.gemm(L.qkv, qw, hidden, b.x, rows, kStreamBf16, b.qkv, qw));
+    if (i > 0) OMNI_CHAIN(norm_gemm(L.ln1, L.qkv, qw, kStreamBf16, b.qkv, qw, 0));
+    else if (!from.table) OMNI_CHAIN(c.gemm(L.qkv, qw, hidden, b.x, rows, kStreamBf16, b.qkv, qw));
     if (prompt) {  // rows of one sequence attend to one another: every key is written before the first is read
       *c.launches += 2;
       OMNI_CHAIN(launch_rope_kv(b.qkv, L.q_norm, L.k_norm, kv[i], map, rows, a, kv_pages, c.err, c.stream));
@@ -76,17 +123,11 @@ cudaError_t chain_pass(const Chain& c, const std::vector<Layer>& layers, const G
       OMNI_CHAIN(launch_rope_attend(b.qkv, from, L.q_norm, L.k_norm, kv[i], b.attn, map, rows, a, kv_pages, c.err, c.stream));
     }
     OMNI_CHAIN(c.gemm(L.o, hidden, qd, b.attn, rows, kStreamPartials, nullptr, hidden, &sum));
-    ++*c.launches;
-    OMNI_CHAIN(launch_add_norm_sum(sum, b.res, L.ln2, b.x, rows, hidden, a.rms_eps, 1, 0, c.stream));
-    OMNI_CHAIN(c.gemm(gate_up(L), 2 * inter, hidden, b.x, rows, kStreamSwiglu, b.act, inter, nullptr, granule));
+    OMNI_CHAIN(norm_gemm(L.ln2, gate_up(L), 2 * inter, kStreamSwiglu, b.act, inter, granule));
     OMNI_CHAIN(c.gemm(down(L), hidden, inter, b.act, rows, kStreamPartials, nullptr, hidden, &sum));
-    ++*c.launches;
-    if (i + 1 < layers.size())
-      OMNI_CHAIN(launch_add_norm_sum(sum, b.res, layers[i + 1].ln1, b.x, rows, hidden, a.rms_eps, 1, 0, c.stream));
-    else
-      OMNI_CHAIN(launch_add_norm_sum(sum, b.res, final_gain, keep_out, rows, hidden, a.rms_eps, every, which, c.stream));
   }
-  return cudaSuccess;
+  ++*c.launches;
+  return launch_add_norm_sum(sum, b.res, final_gain, keep_out, rows, hidden, a.rms_eps, every, which, c.stream);
 }
 
 }  // namespace omni

@@ -115,7 +115,7 @@ struct omni_codec {
   std::map<std::tuple<const void*, const void*, const void*, int>, TcGemmPlan> plans;
   std::map<std::tuple<const void*, const void*, const void*, int>, RmGemmPlan> rm_plans;
   std::map<std::tuple<const void*, const void*, const void*, int, int>, ConvGemmPlan> conv_plans;
-  std::map<std::tuple<const void*, const void*, const void*, int, int>, StreamGemmPlan> stream_plans;
+  ChainPlans stream_plans;
   Chain chain() { return Chain{stream, err, sm_count, scratch.partials, scratch.partial_floats, &launches, &stream_plans}; }
   struct StepGraph {
     cudaGraphExec_t exec = nullptr;

@@ -108,9 +108,10 @@ struct omni_duplex {
 
   // activations (max_rows = max(max_prefill, max_sessions))
   int max_rows = 0;
-  bf16 *x = nullptr, *xn = nullptr, *qkv = nullptr, *attn = nullptr, *y = nullptr, *gu = nullptr, *act = nullptr;
+  bf16 *x = nullptr, *x2 = nullptr, *xn = nullptr,  // x2, dx2: the other residual of a few rows' chain
+      *qkv = nullptr, *attn = nullptr, *y = nullptr, *gu = nullptr, *act = nullptr;
   bf16 *text_logits = nullptr, *audio_logits = nullptr;  // [max_sessions, text_vocab], [8][max_sessions][card]
-  bf16 *dproj = nullptr, *dx = nullptr, *dxn = nullptr, *dqkv = nullptr, *dattn = nullptr, *dy = nullptr,
+  bf16 *dproj = nullptr, *dx = nullptr, *dx2 = nullptr, *dxn = nullptr, *dqkv = nullptr, *dattn = nullptr, *dy = nullptr,
        *dgu = nullptr, *dact = nullptr;
   int32_t *rows_buf = nullptr, *drawn = nullptr, *emitted = nullptr;
 
@@ -129,7 +130,7 @@ struct omni_duplex {
     int seen = 0, nodes = 0;
   };
   std::map<int, TickGraph> tick_graphs;
-  std::map<std::tuple<const void*, const void*, const void*, int, int>, StreamGemmPlan> stream_plans;
+  ChainPlans stream_plans;
   int granule = 16, d_granule = 16;  // channels per group of the gate|up rows (launch_interleave_gate_up)
   Chain chain() { return Chain{stream, err, sm_count, scratch.partials, scratch.partial_floats, &launches, &stream_plans}; }
   bool use_graphs = true;
@@ -277,6 +278,19 @@ float rope_coef(const omni_duplex_config& c) {  // helium.rs:79-81
   return (float)(-std::log((double)c.rope_period) * 2.0 / (double)kHeliumHeadDim);
 }
 
+// A projection behind Helium's add + norm (kAddLm: the add alone, whose rows are then the residual itself).
+static cudaError_t lm_norm_gemm(const Chain& c, int kind, const Summands& sum, bf16** res, bf16** spare, const bf16* gain,
+                                float eps, bf16* xn, const bf16* w, int N, int K, int rows, int out, bf16* y, int ldy,
+                                int granule) {
+  FewNorm norm;
+  norm.kind = kind, norm.sum = sum, norm.gain = gain, norm.eps = eps;
+  return c.norm_gemm(norm, res, spare,
+                     [&](const Summands& from, bf16* x) {
+                       return launch_lm_add_norm_sum(from, x, gain, kind == kAddLm ? nullptr : xn, rows, K, eps, c.stream);
+                     },
+                     w, N, K, kind == kAddLm ? *res : xn, rows, out, y, ldy, granule);
+}
+
 // Every Helium layer over `rows` rows of m->x; the output norm's rows end in m->xn (helium.rs:225-284). In a
 // tensor-parallel pair the projections run on this rank's heads and channels, and the o and down projections' partial
 // rows are summed over the pair inside the add + norm kernel that follows them.
@@ -290,26 +304,32 @@ int helium_forward(omni_duplex* m, int rows, const int32_t* pos, const int32_t* 
   // up to kChainRows rows: weight-streaming GEMMs whose partial sums the add + norm kernels take (not in a pair, whose
   // exchange moves finished rows); one row per session (seq == nullptr): rotation, KV write and attention in one kernel
   const Chain chain = m->chain();
-  const bool stream = rows <= kChainRows;
+  const bool stream = rows <= kChainRows && !pair;
+  bf16 *res = m->x, *spare = m->x2;
+  Summands y;
+  // the o or down projection `which`, whose sums the add + norm in front of the next projection takes
   auto projected = [&](const bf16* w, int K, const bf16* x, int which, const bf16* gain) -> int {
-    if (pair) {
-      bf16* y = m->tp_buf(which);
-      DTRY(gemm(m, w, D, K, x, rows, y, D));
-      DLAUNCH(m, launch_lm_tp_add_norm(y, m->tp_peer_buf(which), m->x, gain, m->xn, rows, D, c.norm_eps, m->tp_link(), m->err, m->stream));
-    } else if (stream) {
-      Summands y;
+    if (stream) {
       DCUDA(m, chain.gemm(w, D, K, x, rows, kStreamPartials, nullptr, D, &y));
-      DLAUNCH(m, launch_lm_add_norm_sum(y, m->x, gain, m->xn, rows, D, c.norm_eps, m->stream));
+    } else if (pair) {
+      bf16* mine = m->tp_buf(which);
+      DTRY(gemm(m, w, D, K, x, rows, mine, D));
+      DLAUNCH(m, launch_lm_tp_add_norm(mine, m->tp_peer_buf(which), m->x, gain, m->xn, rows, D, c.norm_eps, m->tp_link(), m->err, m->stream));
     } else {
       DTRY(gemm(m, w, D, K, x, rows, m->y, D));
       DLAUNCH(m, launch_lm_add_norm(m->y, m->x, gain, m->xn, rows, D, c.norm_eps, m->stream));
     }
     return OMNI_OK;
   };
+  auto behind_norm = [&](const bf16* gain, const bf16* w, int N, int out, bf16* to, int ld, int granule) -> int {
+    DCUDA(m, lm_norm_gemm(chain, kNormLm, y, &res, &spare, gain, c.norm_eps, m->xn, w, N, D, rows, out, to, ld, granule));
+    return OMNI_OK;
+  };
   DLAUNCH(m, launch_lm_norm(m->x, m->h[0].norm1, m->xn, rows, D, c.norm_eps, m->stream));
   for (int i = 0; i < c.layers; ++i) {
     const HeliumLayer& L = m->h[i];
-    DTRY(gemm(m, L.qkv, 3 * Dl, D, m->xn, rows, m->qkv, 3 * Dl));
+    if (stream && i > 0) DTRY(behind_norm(L.norm1, L.qkv, 3 * Dl, kStreamBf16, m->qkv, 3 * Dl, 0));
+    else DTRY(gemm(m, L.qkv, 3 * Dl, D, m->xn, rows, m->qkv, 3 * Dl));
     if (!seq) {
       DLAUNCH(m, launch_lm_rope_attend(m->qkv, m->kv[i], pos, slot, indptr, pages, m->attn, rows, m->local_heads(),
                                        rope_coef(c), scale, c.context, m->kv_pages, m->err, m->stream));
@@ -320,6 +340,8 @@ int helium_forward(omni_duplex* m, int rows, const int32_t* pos, const int32_t* 
     }
     DTRY(projected(L.o, Dl, m->attn, 0, L.norm2));
     if (stream) {
+      DTRY(behind_norm(L.norm2, L.gate_up, 2 * Hl, kStreamSwiglu, m->act, Hl, m->granule));
+    } else if (rows <= kChainRows) {
       DCUDA(m, chain.gemm(L.gate_up, 2 * Hl, D, m->xn, rows, kStreamSwiglu, m->act, Hl, nullptr, m->granule));
     } else {
       DTRY(gemm(m, L.gate_up, 2 * Hl, D, m->xn, rows, m->gu, 2 * Hl));
@@ -327,6 +349,7 @@ int helium_forward(omni_duplex* m, int rows, const int32_t* pos, const int32_t* 
     }
     DTRY(projected(L.down, Hl, m->act, 1, i + 1 < c.layers ? m->h[i + 1].norm1 : m->out_norm));
   }
+  if (stream) DLAUNCH(m, launch_lm_add_norm_sum(y, res, m->out_norm, m->xn, rows, D, c.norm_eps, m->stream));
   return OMNI_OK;
 }
 
@@ -342,21 +365,24 @@ int depformer_step(omni_duplex* m, int n, const int32_t* force, const int32_t* s
     const int table_rows = k == 0 ? c.text_vocab + 1 : c.card + 1;
     DLAUNCH(m, launch_lm_dep_embed_norm(m->dproj, k, table, table_rows, m->drawn, m->d[0].norm1, m->dx, m->dxn, n, D,
                                         c.norm_eps, m->err, m->stream));
+    bf16 *res = m->dx, *spare = m->dx2;
+    Summands y;
+    auto behind_norm = [&](int kind, const bf16* gain, const bf16* w, int N, int out, bf16* to, int granule) -> int {
+      DCUDA(m, lm_norm_gemm(chain, kind, y, &res, &spare, gain, c.norm_eps, m->dxn, w, N, D, n, out, to, out == kStreamSwiglu ? N / 2 : N, granule));
+      return OMNI_OK;
+    };
     for (int i = 0; i < c.dep_layers; ++i) {
       const DepLayer& L = m->d[i];
-      DTRY(gemm(m, L.qkv + (size_t)k * 3 * D * D, 3 * D, D, m->dxn, n, m->dqkv, 3 * D));
+      const bf16* qkv = L.qkv + (size_t)k * 3 * D * D;
+      if (i > 0) DTRY(behind_norm(kNormLm, L.norm1, qkv, 3 * D, kStreamBf16, m->dqkv, 0));
+      else DTRY(gemm(m, qkv, 3 * D, D, m->dxn, n, m->dqkv, 3 * D));
       DLAUNCH(m, launch_lm_dep_kv_attend(m->dqkv, m->dkv[i], k, m->dattn, n, c.dep_heads, scale, m->stream));
-      Summands y;
       DCUDA(m, chain.gemm(L.out + (size_t)k * D * D, D, D, m->dattn, n, kStreamPartials, nullptr, D, &y));
-      DLAUNCH(m, launch_lm_add_norm_sum(y, m->dx, L.norm2, m->dxn, n, D, c.norm_eps, m->stream));
-      DCUDA(m, chain.gemm(L.gate_in + (size_t)k * 2 * H * D, 2 * H, D, m->dxn, n, kStreamSwiglu, m->dact, H, nullptr, m->d_granule));
+      DTRY(behind_norm(kNormLm, L.norm2, L.gate_in + (size_t)k * 2 * H * D, 2 * H, kStreamSwiglu, m->dact, m->d_granule));
       DCUDA(m, chain.gemm(L.gate_out + (size_t)k * D * H, D, H, m->dact, n, kStreamPartials, nullptr, D, &y));
-      const bool more = i + 1 < c.dep_layers;
-      DLAUNCH(m, launch_lm_add_norm_sum(y, m->dx, more ? m->d[i + 1].norm1 : nullptr, more ? m->dxn : nullptr, n, D,
-                                        c.norm_eps, m->stream));
     }
     bf16* logits = m->audio_logits + (size_t)k * S * c.card;
-    DTRY(gemm(m, m->d_heads + (size_t)k * c.card * D, c.card, D, m->dx, n, logits, c.card));
+    DTRY(behind_norm(kAddLm, nullptr, m->d_heads + (size_t)k * c.card * D, c.card, kStreamBf16, logits, 0));
     DLAUNCH(m, launch_lm_sample(logits, c.card, c.card, c.audio_temperature, c.audio_top_k, force, seeds, 1 + k,
                                 m->drawn, n, m->stream));
   }
@@ -490,6 +516,7 @@ int32_t omni_duplex_create(const omni_duplex_config* config, const omni_tensor* 
   m->max_rows = std::max(c.max_prefill, S);
   const size_t R = m->max_rows;
   DTRY(dalloc(m, &m->x, R * D));
+  DTRY(dalloc(m, &m->x2, (size_t)kFewNormRows * D));
   DTRY(dalloc(m, &m->xn, R * D));
   DTRY(dalloc(m, &m->qkv, R * 3 * D));
   DTRY(dalloc(m, &m->attn, R * D));
@@ -504,6 +531,7 @@ int32_t omni_duplex_create(const omni_duplex_config* config, const omni_tensor* 
   DTRY(dalloc(m, &m->audio_logits, (size_t)kDepSteps * S * c.card, true));
   DTRY(dalloc(m, &m->dproj, (size_t)S * kDepSteps * DD));
   DTRY(dalloc(m, &m->dx, (size_t)S * DD));
+  DTRY(dalloc(m, &m->dx2, (size_t)kFewNormRows * DD));
   DTRY(dalloc(m, &m->dxn, (size_t)S * DD));
   DTRY(dalloc(m, &m->dqkv, (size_t)S * 3 * DD));
   DTRY(dalloc(m, &m->dattn, (size_t)S * DD));

@@ -1,0 +1,413 @@
+// The GEMM of the kernel chains for up to sixteen rows (see few_rows.h).
+//
+// A decode node of a few rows is latency: its weights were asked for before its inputs existed, so what counts is the
+// path from the inputs' arrival to the outputs' stores. tcgen05 puts four hand-overs on it (rows to shared memory by TMA,
+// MMA issue, commit, TMEM load); here the weights are M of m16n8k16 and the rows its N, and a warp keeps everything it
+// needs to itself: its eighth of K, its own ring of weight blocks, its rows of x, so that only the final sum over the
+// eight warps crosses a barrier. One m16n8k16 takes 2 cycles of the SM's pipe, which is ten times the rate at which DRAM
+// delivers weights, and up to sixteen rows there is nothing for a larger tile to reuse.
+// The add + norm before a projection is made by every CTA from the summands (L2 broadcast reads, 16 KB to 100 KB), which
+// takes about 1 us where a kernel of its own takes 2.7.
+#include "few_rows.h"
+
+#include <algorithm>
+#include <type_traits>
+
+#include "pdl.cuh"
+#include "sm100.cuh"
+
+namespace omni {
+namespace {
+
+constexpr int kWarps = 8, kKb = 64, kFewSlots = 8;
+constexpr int kNormChunks = 6;  // 8-element pieces of the rows that a lane holds across the norm's sum
+
+struct FewArgs {
+  const bf16* x;
+  bf16* y;
+  float* part;
+  const bf16* bias;
+  uint32_t* err;
+  FewNorm norm;
+  float inv_k;
+  int N, K, rows, R, slots, ldy, kind, nkb, span, per, xk, lanes_log2, rounds;
+};
+
+__device__ __forceinline__ void ldsm4(uint32_t addr, uint32_t (&r)[4]) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(addr)
+               : "memory");
+}
+
+__device__ __forceinline__ void mma_16816(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+
+__device__ __forceinline__ void st_shared16(uint32_t addr, const uint4& v) {
+  asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+}
+
+// Where a lane's pieces of the rows lie: piece first + j * lanes of this warp's share of row n, 16 bytes each.
+struct Share {
+  int warp, lane, n, first, lanes, pieces, c0;  // c0: first column of the warp's share
+  bool live;
+  uint32_t xs;  // row n's share in shared memory
+};
+
+// The add + norm's rows, RD pieces a lane, from S partial sums; `keep`: this CTA stores the residual.
+template <int NORM, int S, int RD>
+__device__ __forceinline__ void norm_rows(const FewArgs& a, const Share& h, bool keep, float (*ss_s)[kWarps], const uint4* gain) {
+  const int64_t at = (int64_t)(h.live ? h.n : 0) * a.K + h.c0 + h.first * 8;
+  const float* part = a.norm.sum.part + at;
+  constexpr int B = S >= 4 ? 2 : RD < 4 ? RD : RD == 4 && S == 1 ? 4 : 2;  // pieces under way at a time
+  float v[RD][8], ss = 0.f;
+#pragma unroll
+  for (int j0 = 0; j0 < RD; j0 += B) {
+    uint4 r[B];
+    float4 f[B][S][2];
+#pragma unroll
+    for (int j = 0; j < B; ++j) {
+      const int o = h.first + (j0 + j) * h.lanes < h.pieces ? (j0 + j) * h.lanes * 8 : 0;
+      r[j] = __ldcg(reinterpret_cast<const uint4*>(a.norm.res_in + at + o));
+#pragma unroll
+      for (int s = 0; s < S; ++s) {
+        const float4* q = reinterpret_cast<const float4*>(part + s * a.norm.sum.split_stride + o);
+        f[j][s][0] = __ldcg(q), f[j][s][1] = __ldcg(q + 1);
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < B; ++j) {
+      float u[8], mine = 0.f;
+      unpack8v(r[j], u);
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        float t = reinterpret_cast<const float*>(&f[j][0][0])[k];
+#pragma unroll
+        for (int s = 1; s < S; ++s) t += reinterpret_cast<const float*>(&f[j][s][0])[k];
+        t = bf16_round(t) + u[k];
+        if constexpr (NORM != kNormStack) t = bf16_round(t);
+        v[j0 + j][k] = t;
+        mine += t * t;
+      }
+      ss += h.first + (j0 + j) * h.lanes < h.pieces ? mine : 0.f;
+    }
+    if (j0 + B < RD) asm volatile("" ::: "memory");
+  }
+  float scale = 1.f;
+  if constexpr (NORM != kAddLm) {
+    for (int o = h.lanes >> 1; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+    if (h.live && h.first == 0) ss_s[h.n][h.warp] = ss;
+    __syncthreads();
+    const float4 s0 = *reinterpret_cast<const float4*>(&ss_s[h.n & 7][0]), s1 = *reinterpret_cast<const float4*>(&ss_s[h.n & 7][4]);
+    scale = rsqrtf((((s0.x + s0.y) + (s0.z + s0.w)) + ((s1.x + s1.y) + (s1.z + s1.w))) * a.inv_k + a.norm.eps);
+  }
+#pragma unroll
+  for (int j = 0; j < RD; ++j) {
+    if (!h.live || h.first + j * h.lanes >= h.pieces) break;
+    if (keep) st8(a.norm.res_out + at + j * h.lanes * 8, v[j]);
+    if constexpr (NORM != kAddLm) {
+      float g[8];
+      unpack8v(gain[j], g);
+#pragma unroll
+      for (int k = 0; k < 8; ++k) v[j][k] = NORM == kNormLm ? v[j][k] * (g[k] * scale) : v[j][k] * scale * g[k];
+    }
+    st_shared16(h.xs + (uint32_t)(h.first + j * h.lanes) * 16u, pack8v(v[j]));
+  }
+}
+
+template <int RD>
+__device__ __forceinline__ void plain_rows(const FewArgs& a, const Share& h) {
+  const uint4* src = reinterpret_cast<const uint4*>(a.x + (int64_t)(h.live ? h.n : 0) * a.K + h.c0) + h.first;
+  for (int j0 = 0; h.first + j0 * h.lanes < h.pieces; j0 += RD) {
+    uint4 v[RD];
+#pragma unroll
+    for (int j = 0; j < RD; ++j) v[j] = __ldcg(src + (h.first + (j0 + j) * h.lanes < h.pieces ? (j0 + j) * h.lanes : 0));
+#pragma unroll
+    for (int j = 0; j < RD; ++j)
+      if (h.live && h.first + (j0 + j) * h.lanes < h.pieces) st_shared16(h.xs + (uint32_t)(h.first + (j0 + j) * h.lanes) * 16u, v[j]);
+  }
+}
+
+// MT: 16-row tiles of weights per CTA (10: up to ten); NT: 8-row tiles of x.
+// Every instruction behind grid_wait() is on the chain's critical path and is executed once: what costs is how many a
+// warp goes through (about 5 cycles each, more when its line has to come from L2), hence the index arithmetic in front of
+// the wait, loops that run as often as there is work and bodies chosen by the number of pieces and sums.
+template <int MT, int NT, int NORM, int OUT>
+__global__ void __launch_bounds__(kWarps * 32, 2) few_rows_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ FewArgs a) {
+  using namespace sm100;
+  extern __shared__ unsigned char few_smem_raw[];
+  __shared__ __align__(8) uint64_t bars_s[kWarps * kFewSlots];
+  __shared__ __align__(16) float ss_s[8][kWarps];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int tile = blockIdx.x, split = blockIdx.y;
+  // k-blocks: `span` per split, `per` per warp, the last of each fewer
+  const int kb0 = split * a.span + warp * a.per;
+  const int nk = max(0, min(min(a.per, a.span - warp * a.per), a.nkb - kb0));
+  const uint32_t slot_bytes = (uint32_t)a.R * 128u;
+  const uint32_t ring0 = (smem_addr(few_smem_raw) + 1023u) & ~1023u;
+  const uint32_t ring = ring0 + (uint32_t)(warp * a.slots) * slot_bytes;
+  // this warp's rows of x: [rows][xk] bf16 (xk = 64 * per, + 8 against bank conflicts)
+  const uint32_t xs = ring0 + (uint32_t)(kWarps * a.slots) * slot_bytes + (uint32_t)(warp * a.rows * a.xk) * 2u;
+  const uint32_t bars = smem_addr(bars_s) + 8u * (uint32_t)(warp * kFewSlots);
+  auto load_w = [&](int i, int slot) {
+    mbar_expect_tx(bars + 8u * slot, slot_bytes);
+    tma_load_3d(ring + (uint32_t)slot * slot_bytes, &wmap, bars + 8u * slot, 0, tile * a.R, kb0 + i, kEvictFirst);
+  };
+  const int ahead = min(a.slots, nk);
+  if (lane == 0) {
+    prefetch_tensormap(&wmap);
+    for (int s = 0; s < a.slots; ++s) mbar_init(bars + 8u * s, 1);
+    mbar_init_fence();
+    for (int i = 0; i < ahead; ++i) load_w(i, i);
+  }
+  grid_trigger();
+  __syncwarp();
+
+  // ---- everything that does not depend on the rows comes before grid_wait(), the first weights' arrival included ----
+  Share h;
+  h.warp = warp, h.lane = lane, h.lanes = 1 << a.lanes_log2;
+  h.n = lane >> a.lanes_log2, h.first = lane & (h.lanes - 1), h.pieces = nk * 8, h.c0 = kb0 * kKb;
+  h.live = h.n < a.rows, h.xs = xs + (uint32_t)(h.n * a.xk) * 2u;
+  // the tile's rows; SwiGLU: `half` gate channels, then their up channels (the last tile may hold fewer)
+  const int half = OUT == kStreamSwiglu ? min(a.R >> 1, (a.N >> 1) - tile * (a.R >> 1)) : 0;
+  const int mts = MT <= 4 ? MT : OUT == kStreamSwiglu ? half >> 3 : a.R >> 4;
+  // ldmatrix rows of this lane: weights [0, 8) k 0..7, [8, 16) k 0..7, [0, 8) k 8..15, [8, 16) k 8..15; x rows past the
+  // last read row 0 (their columns of the result are not stored)
+  const int row0 = OUT == kStreamSwiglu ? (lane & 7) + ((lane & 8) ? half : 0) : lane & 15;
+  uint32_t x_lane[NT], w_lane[4];
+#pragma unroll
+  for (int t = 0; t < NT; ++t) {
+    const int r = t * 8 + (lane & 7);
+    x_lane[t] = xs + (uint32_t)((r < a.rows ? r : 0) * a.xk + (lane >> 3) * 8) * 2u;
+  }
+#pragma unroll
+  for (int k = 0; k < 4; ++k) w_lane[k] = ring + (uint32_t)row0 * 128u + (uint32_t)(((k * 2 + (lane >> 4)) ^ (lane & 7)) << 4);
+  const int stride = a.R + 4, warp_floats = a.slots * a.R * 32;
+  float* const red0 = reinterpret_cast<float*>(few_smem_raw + (ring0 - smem_addr(few_smem_raw)));
+  float* const red = red0 + warp * warp_floats + (lane & 3) * 2 * stride + (lane >> 2);
+  const int rounds = (h.pieces + h.lanes - 1) >> a.lanes_log2;
+  uint4 g[kNormChunks];
+  if constexpr (NORM == kNormStack || NORM == kNormLm) {
+#pragma unroll
+    for (int j = 0; j < kNormChunks; ++j)
+      if (h.first + j * h.lanes < h.pieces) g[j] = __ldg(reinterpret_cast<const uint4*>(a.norm.gain + h.c0) + h.first + j * h.lanes);
+  }
+  bool fine = true;
+  for (int i = 0; i < ahead; ++i) fine = mbar_wait(bars + 8u * i, 0, a.err) && fine;
+  grid_wait();
+
+  // ---- the rows ----
+  if constexpr (NORM == 0) {
+    if (rounds <= 1) plain_rows<1>(a, h);
+    else plain_rows<4>(a, h);
+  } else {
+    const bool keep = tile == (int)gridDim.x - 1;
+    auto with = [&](auto sums) {
+      constexpr int S = decltype(sums)::value;
+      if (a.rounds <= 1) norm_rows<NORM, S, 1>(a, h, keep, ss_s, g);
+      else if (a.rounds == 2) norm_rows<NORM, S, 2>(a, h, keep, ss_s, g);
+      else if (a.rounds <= 4) norm_rows<NORM, S, 4>(a, h, keep, ss_s, g);
+      else norm_rows<NORM, S, kNormChunks>(a, h, keep, ss_s, g);
+    };
+    if (a.norm.sum.splits == 1) with(std::integral_constant<int, 1>());
+    else if (a.norm.sum.splits == 2) with(std::integral_constant<int, 2>());
+    else with(std::integral_constant<int, 4>());
+  }
+  __syncwarp();
+
+  // ---- w . x^T ----
+  float acc[MT][NT][4];
+#pragma unroll
+  for (int m = 0; m < MT; ++m)
+#pragma unroll
+    for (int t = 0; t < NT; ++t) acc[m][t][0] = acc[m][t][1] = acc[m][t][2] = acc[m][t][3] = 0.f;
+  uint32_t turn = 0, off = 0;  // of the ring; off: bytes to the slot
+#pragma unroll 1
+  for (int i = 0, slot = 0; i < nk; ++i) {
+    if (i >= ahead) fine = mbar_wait(bars + 8u * slot, turn, a.err);
+    if (!fine) {  // nothing may land once the CTA has left
+      for (int j = max(i + 1, ahead); j < min(nk, i + a.slots); ++j) mbar_wait(bars + 8u * (j % a.slots), (uint32_t)(j / a.slots) & 1u, a.err);
+      break;
+    }
+    uint32_t b[2][NT][4];
+#pragma unroll
+    for (int hf = 0; hf < 2; ++hf)
+#pragma unroll
+      for (int t = 0; t < NT; ++t) ldsm4(x_lane[t] + hf * 64, b[hf][t]);
+#pragma unroll
+    for (int t = 0; t < NT; ++t) x_lane[t] += 128u;
+#pragma unroll
+    for (int m = 0; m < MT; ++m) {
+      if (MT <= 4 || m < mts) {
+        uint32_t w[4][4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) ldsm4(w_lane[k] + off + m * (OUT == kStreamSwiglu ? 1024 : 2048), w[k]);
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+#pragma unroll
+          for (int t = 0; t < NT; ++t) mma_16816(acc[m][t], w[k], b[k >> 1][t][(k & 1) * 2], b[k >> 1][t][(k & 1) * 2 + 1]);
+      }
+    }
+    if (ahead < nk) {  // a ring that does not hold the warp's whole share
+      __syncwarp();
+      if (lane == 0 && i + a.slots < nk) load_w(i + a.slots, slot);
+    }
+    off += slot_bytes;
+    if (++slot == a.slots) slot = 0, off = 0, turn ^= 1u;
+  }
+
+  // ---- sum over the warps, through each warp's own (spent) ring: [row of x][weight row], SwiGLU gates then ups ----
+  __syncwarp();
+#pragma unroll
+  for (int m = 0; m < MT; ++m)
+    if (MT <= 4 || m < mts) {
+#pragma unroll
+      for (int t = 0; t < NT; ++t) {
+        float* at = red + t * 8 * stride + m * (OUT == kStreamSwiglu ? 8 : 16);
+        float* at2 = OUT == kStreamSwiglu ? at + (a.R >> 1) : at + 8;
+        at[0] = acc[m][t][0], at[stride] = acc[m][t][1];
+        at2[0] = acc[m][t][2], at2[stride] = acc[m][t][3];
+      }
+    }
+  __syncthreads();
+  auto total = [&](int at) {
+    float f[kWarps];
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w) f[w] = red0[w * warp_floats + at];
+    return ((f[0] + f[1]) + (f[2] + f[3])) + ((f[4] + f[5]) + (f[6] + f[7]));
+  };
+  const int cols = OUT == kStreamSwiglu ? half : min(a.R, a.N - tile * a.R), c0 = tile * (OUT == kStreamSwiglu ? a.R >> 1 : a.R);
+#pragma unroll 1
+  for (int n = warp; n < a.rows; n += kWarps) {  // a row per warp, a column per lane
+#pragma unroll 1
+    for (int c = lane; c < cols; c += 32) {
+      const float v = total(n * stride + c);
+      if constexpr (OUT == kStreamSwiglu) {
+        const float u = bf16_round(total(n * stride + (a.R >> 1) + c)), gate = bf16_round(v);
+        // the fast division is within 2 ulp of an f32 that is rounded to bf16 next
+        a.y[(int64_t)n * a.ldy + c0 + c] = __float2bfloat16(bf16_round(__fdividef(gate, 1.f + __expf(-gate))) * u);
+      } else if constexpr (OUT == kStreamPartials) {
+        a.part[((int64_t)split * a.rows + n) * a.N + c0 + c] = v;
+      } else {
+        float o = bf16_round(v);
+        if (a.kind != kEpiNone) {
+          o = bf16_round(o + __bfloat162float(a.bias[c0 + c]));
+          if (a.kind == kEpiBiasSilu) o = o / (1.f + __expf(-o));
+        }
+        a.y[(int64_t)n * a.ldy + c0 + c] = __float2bfloat16(o);
+      }
+    }
+  }
+}
+
+// More than a third of an SM's shared memory each, so that an SM takes one CTA of this kernel and one of the next, whose
+// weights are then on their way, but not two of the same while another SM is idle; rings stop at half of it.
+constexpr int kFewMinSmem = 76 * 1024, kFewHalf = 112 * 1024, kFewMaxSmem = 148 * 1024;
+
+template <int MT, int NT, typename F>
+cudaError_t few_dispatch_tile(int norm, int out, F&& go) {
+  const bool bf = out == kStreamBf16, swi = out == kStreamSwiglu;
+  if (norm == 0) return bf ? go(few_rows_kernel<MT, NT, 0, kStreamBf16>) : swi ? go(few_rows_kernel<MT, NT, 0, kStreamSwiglu>) : go(few_rows_kernel<MT, NT, 0, kStreamPartials>);
+  if constexpr (NT == 1) {  // kFewNormRows is one tile
+    if (norm == kNormStack && out != kStreamPartials) return bf ? go(few_rows_kernel<MT, 1, kNormStack, kStreamBf16>) : go(few_rows_kernel<MT, 1, kNormStack, kStreamSwiglu>);
+    if (norm == kNormLm && out != kStreamPartials) return bf ? go(few_rows_kernel<MT, 1, kNormLm, kStreamBf16>) : go(few_rows_kernel<MT, 1, kNormLm, kStreamSwiglu>);
+    if (norm == kAddLm && bf) return go(few_rows_kernel<MT, 1, kAddLm, kStreamBf16>);
+  }
+  return cudaErrorInvalidValue;
+}
+
+template <typename F>
+cudaError_t few_dispatch(int mts, int nts, int norm, int out, F&& go) {
+  if (mts == 1) return nts == 1 ? few_dispatch_tile<1, 1>(norm, out, go) : few_dispatch_tile<1, 2>(norm, out, go);
+  if (mts == 2) return nts == 1 ? few_dispatch_tile<2, 1>(norm, out, go) : few_dispatch_tile<2, 2>(norm, out, go);
+  if (mts == 3) return nts == 1 ? few_dispatch_tile<3, 1>(norm, out, go) : few_dispatch_tile<3, 2>(norm, out, go);
+  if (mts == 4) return nts == 1 ? few_dispatch_tile<4, 1>(norm, out, go) : few_dispatch_tile<4, 2>(norm, out, go);
+  return nts == 1 ? few_dispatch_tile<10, 1>(norm, out, go) : cudaErrorInvalidValue;
+}
+
+}  // namespace
+
+void few_configure() {
+  auto set = [](auto kernel) { return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kFewMaxSmem + 1024); };
+  for (int mts : {1, 2, 3, 4, 10})
+    for (int nts : {1, 2})
+      for (int norm : {0, (int)kNormStack, (int)kNormLm, (int)kAddLm})
+        for (int out : {kStreamBf16, kStreamPartials, kStreamSwiglu}) few_dispatch(mts, nts, norm, out, set);
+}
+
+// Lanes per row: the rows of a warp side by side.
+static int few_lanes_log2(int rows) {
+  int log2 = 5;
+  while ((32 >> log2) < rows) --log2;
+  return log2;
+}
+// k-blocks per split and per warp.
+static int few_span(int nkb, int splits) { return (nkb + splits - 1) / splits; }
+static int few_per(int nkb, int splits) { return (few_span(nkb, splits) + kWarps - 1) / kWarps; }
+static int few_rounds(int nkb, int splits, int rows) {
+  const int lanes = 1 << few_lanes_log2(rows);
+  return (few_per(nkb, splits) * 8 + lanes - 1) / lanes;
+}
+
+bool few_norm_fits(int K, int rows) { return rows <= kFewNormRows && K % kKb == 0 && few_rounds(K / kKb, 1, rows) <= kNormChunks; }
+
+int few_plan(FewPlan* plan, const bf16* w, int N, int K, const bf16* x, int rows, int out, bf16* y, int ldy, float* part,
+             Epilogue epi, int sm_count, int granule) {
+  if (rows < 1 || rows > 16 || K % kKb || N < 1) return -2;
+  if (!x && !few_norm_fits(K, rows)) return -2;
+  if (out == kStreamSwiglu && (granule < 8 || granule % 8 || N % 16)) return -2;
+  if ((reinterpret_cast<uintptr_t>(w) & 15) || (reinterpret_cast<uintptr_t>(x) & 15)) return -3;
+  FewPlan& p = *plan;
+  p.N = N, p.K = K, p.rows = rows, p.out = out, p.x = x, p.y = y, p.ldy = ldy, p.part = part, p.epi = epi;
+  const int nkb = K / kKb, most = rows > 8 ? 64 : 160;
+  auto x_bytes = [&](int S) {
+    return kWarps * rows * (few_per(nkb, S) * kKb + 8) * 2;
+  };
+  if (out == kStreamSwiglu) {
+    p.R = 2 * granule, p.splits = 1;
+    if (p.R > most) return -2;
+  } else {
+    // the most even load of weights on the SMs, then the fewest sums for the consumer to add
+    double best = 1e30;
+    for (int R = 16; R <= most; R += 16)
+      for (int S : {1, 2, 4}) {
+        if (S > 1 && (out != kStreamPartials || S * kWarps > nkb)) break;
+        if (x_bytes(S) > 64 * 1024) continue;
+        const double waves = ((N + R - 1) / R * S + sm_count - 1) / sm_count;
+        const double cost = waves * R * 2.0 * K / S / 44e3 + waves * rows * 2.0 * K / S / 150e3 + 0.15 * S + (S > 1 ? 4.0 * S * rows * N / 150e3 : 0.0);
+        if (cost < best) best = cost, p.R = R, p.splits = S;
+      }
+    if (best > 1e29) return -2;
+  }
+  const int xb = x_bytes(p.splits), level = kWarps * p.R * 128;
+  const int per = few_per(nkb, p.splits);
+  if (xb > 64 * 1024) return -2;
+  p.xk = per * kKb + 8;
+  p.slots = std::min(per, kFewSlots);
+  if (1024 + xb + p.slots * level > kFewMaxSmem) p.slots = std::max(1, (kFewHalf - 1024 - xb) / level);
+  if (1024 + xb + p.slots * level > kFewMaxSmem) return -2;
+  p.smem = std::max<size_t>(kFewMinSmem, 1024 + (size_t)xb + (size_t)p.slots * level);
+  const uint64_t wd[3] = {kKb, (uint64_t)N, (uint64_t)nkb}, ws[2] = {(uint64_t)K * 2, kKb * 2};
+  const uint32_t wb[3] = {kKb, (uint32_t)p.R, 1};
+  return tc_encode_bf16(&p.wmap, w, 3, wd, ws, wb) == 0 ? 0 : -4;
+}
+
+cudaError_t few_launch(const FewPlan& p, const FewNorm& norm, uint32_t* err, cudaStream_t stream) {
+  const int sums = norm.sum.splits;
+  if (norm.kind && sums != 1 && sums != 2 && sums != 4) return cudaErrorInvalidValue;
+  FewArgs a;
+  a.x = p.x, a.y = p.y, a.part = p.part, a.bias = p.epi.bias, a.err = err, a.norm = norm, a.kind = p.epi.kind;
+  a.inv_k = 1.f / (float)p.K;
+  a.N = p.N, a.K = p.K, a.rows = p.rows, a.R = p.R, a.slots = p.slots, a.ldy = p.ldy;
+  a.nkb = p.K / kKb, a.span = few_span(a.nkb, p.splits), a.per = few_per(a.nkb, p.splits), a.xk = p.xk;
+  a.lanes_log2 = few_lanes_log2(p.rows), a.rounds = few_rounds(a.nkb, p.splits, p.rows);
+  const dim3 grid((p.N + p.R - 1) / p.R, p.splits);
+  return few_dispatch((p.R + 15) / 16, (p.rows + 7) / 8, norm.kind, p.out, [&](auto kernel) {
+    return launch_pdl(kernel, grid, dim3(kWarps * 32), p.smem, stream, p.wmap, a);
+  });
+}
+
+}  // namespace omni

@@ -70,7 +70,7 @@ struct omni_higgs {
   std::vector<std::unique_ptr<omni_higgs_seq>> seqs;
 
   int max_rows = 0;
-  bf16 *embeds = nullptr, *x = nullptr, *res = nullptr, *qkv = nullptr, *attn = nullptr, *gate_up = nullptr,
+  bf16 *embeds = nullptr, *x = nullptr, *res = nullptr, *res2 = nullptr, *qkv = nullptr, *attn = nullptr, *gate_up = nullptr,
        *act = nullptr, *hidden = nullptr, *logits = nullptr;
   int32_t* codes = nullptr;
 
@@ -89,7 +89,7 @@ struct omni_higgs {
     int seen = 0, nodes = 0;
   };
   std::map<int, StepGraph> step_graphs;
-  std::map<std::tuple<const void*, const void*, const void*, int, int>, StreamGemmPlan> stream_plans;
+  ChainPlans stream_plans;
   int granule = 16, granule_audio = 16;  // channels per group of the gate|up rows (launch_interleave_gate_up)
   Chain chain() { return Chain{stream, err, sm_count, scratch.partials, scratch.partial_floats, &launches, &stream_plans}; }
   bool use_graphs = true;
@@ -223,7 +223,7 @@ int body_forward(omni_higgs* m, const bf16* input, int rows, const RowMap& map, 
   if (rows <= kChainRows && chain_supports(h, I, qd, c.head_dim)) {
     HCUDA(m, chain_pass(m->chain(), m->layers, [&](const Layer& L) { return both ? L.gate_up_audio : L.gate_up; },
                         [&](const Layer& L) { return both ? L.down_audio : L.down; }, h, I, granule, a,
-                        ChainBuffers{m->x, m->res, m->qkv, m->attn, m->act}, rows, map, m->kv, m->pages_total, m->norm, out,
+                        ChainBuffers{m->x, m->res, m->res2, m->qkv, m->attn, m->act}, rows, map, m->kv, m->pages_total, m->norm, out,
                         1, 0, {}, !audio));
     return OMNI_OK;
   }
@@ -428,6 +428,7 @@ int32_t omni_higgs_create(const omni_higgs_config* config, const omni_tensor* te
   HTRY(halloc(m, &m->embeds, R * h));
   HTRY(halloc(m, &m->x, R * h));
   HTRY(halloc(m, &m->res, R * h));
+  HTRY(halloc(m, &m->res2, (size_t)kFewNormRows * h));
   HTRY(halloc(m, &m->qkv, R * (q + 2 * kvw)));
   HTRY(halloc(m, &m->attn, R * q));
   const size_t Iw = c.audio_adapter ? 2 * I : I;  // widest MLP a row goes through

@@ -3,6 +3,7 @@
 
 #include <algorithm>
 
+#include "few_rows.h"
 #include "pdl.cuh"
 #include "sm100.cuh"
 
@@ -235,6 +236,7 @@ constexpr int kMinSmem = 116 * 1024, kMaxSmem = 200 * 1024;
 }  // namespace
 
 void stream_configure() {
+  few_configure();
   cudaFuncSetAttribute(stream_gemm_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
   cudaFuncSetAttribute(stream_gemm_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
   cudaFuncSetAttribute(stream_gemm_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);

@@ -20,23 +20,24 @@ struct Summands {
   int ld = 0;                // elements per row
 };
 
-// Eight columns of row n from column c on: the bf16 values, widened.
+// Eight columns of row n from column c on: the bf16 values, widened. At most MAX splits.
+template <int MAX = 8>
 __device__ __forceinline__ void load_sum8(const Summands& x, int n, int c, float (&v)[8]) {
   if (x.splits == 0) {
     unpack8v(__ldcg(reinterpret_cast<const uint4*>(x.done + (int64_t)n * x.ld + c)), v);
     return;
   }
   const float* p = x.part + (int64_t)n * x.ld + c;
-  float4 f[8][2];
+  float4 f[MAX][2];
 #pragma unroll
-  for (int s = 0; s < 8; ++s)
+  for (int s = 0; s < MAX; ++s)
 #pragma unroll
     for (int h = 0; h < 2; ++h)
       f[s][h] = s < x.splits ? __ldcg(reinterpret_cast<const float4*>(p + s * x.split_stride) + h) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
   for (int k = 0; k < 8; ++k) v[k] = 0.f;
 #pragma unroll
-  for (int s = 0; s < 8; ++s) {  // adding 0 for a missing split leaves the sum unchanged
+  for (int s = 0; s < MAX; ++s) {  // adding 0 for a missing split leaves the sum unchanged
     v[0] += f[s][0].x, v[1] += f[s][0].y, v[2] += f[s][0].z, v[3] += f[s][0].w;
     v[4] += f[s][1].x, v[5] += f[s][1].y, v[6] += f[s][1].z, v[7] += f[s][1].w;
   }

@@ -65,7 +65,7 @@ struct StackW {
 };
 
 struct Scratch {
-  bf16 *x, *res, *qkv, *attn, *gate_up, *act;
+  bf16 *x, *res, *res2, *qkv, *attn, *gate_up, *act;  // res2: the other residual of a few rows' chain
 };
 
 // How the persistent kernel tiles one GEMM: weight rows per tile (the MMA N dimension) and K splits.
@@ -173,7 +173,7 @@ struct omni_talker {
   GemmScratch gemm_scratch;
 
   std::map<std::tuple<const void*, const void*, const void*, int, int>, TcGemmPlan> plans;
-  std::map<std::tuple<const void*, const void*, const void*, int, int>, StreamGemmPlan> stream_plans;
+  ChainPlans stream_plans;
   Chain chain() { return Chain{stream, err, sm_count, gemm_scratch.partials, gemm_scratch.partial_floats, &launches, &stream_plans}; }
   bool use_chain = false;  // programs run as chains of kernels (chain.h) rather than as the persistent kernel
   std::map<std::pair<int, int>, cudaGraphExec_t> graphs;  // (program, bucket)
@@ -344,6 +344,7 @@ int alloc_scratch(omni_talker* m, const StackW& s, int rows, Scratch* out) {
   const omni_stack_config& c = s.cfg;
   TRY(dev_alloc(m, &out->x, (size_t)rows * c.hidden));
   TRY(dev_alloc(m, &out->res, (size_t)rows * c.hidden));
+  TRY(dev_alloc(m, &out->res2, (size_t)kFewNormRows * c.hidden));
   TRY(dev_alloc(m, &out->qkv, (size_t)rows * s.qkv_width()));
   TRY(dev_alloc(m, &out->attn, (size_t)rows * c.q_heads * c.head_dim));
   TRY(dev_alloc(m, &out->gate_up, (size_t)rows * 2 * c.inter));
@@ -392,7 +393,7 @@ int chain_layers(omni_talker* m, const StackW& S, const Scratch& s, int rows, co
                  bool prompt) {
   CUDA_TRY(m, chain_pass(m->chain(), S.layers, [](const StackW::Layer& L) { return L.gate_up; },
                          [](const StackW::Layer& L) { return L.down; }, S.cfg.hidden, S.cfg.inter, S.granule, S.attn(),
-                         ChainBuffers{s.x, s.res, s.qkv, s.attn, s.act}, rows, map, kv, kv_pages, S.norm, keep_out, every,
+                         ChainBuffers{s.x, s.res, s.res2, s.qkv, s.attn, s.act}, rows, map, kv, kv_pages, S.norm, keep_out, every,
                          which, lookup, prompt));
   return OMNI_OK;
 }
