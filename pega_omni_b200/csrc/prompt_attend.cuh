@@ -1,0 +1,206 @@
+// Attention of prompt rows: many rows of a sequence attend to the same keys, so the products are contractions and run on
+// m16n8k16. A CTA takes 32 rows and one kv head: its G query heads of those rows are 32 * G rows of M, sixteen to a warp;
+// keys and values come two pages (32 keys) at a time into shared memory by cp.async, three stages deep, where every warp
+// reads them with ldmatrix. Rows may belong to several sequences: the CTA goes through the runs of rows of one sequence in
+// turn, and rows outside the run (or keys past a row's position) are masked. Value semantics of `attend`
+// (crates/omni-qwen3/kernels/qwen3.cu:123-207): f32 scores, online softmax in f32; a probability enters the second product
+// as the sum of two bf16 (its rounding and the remainder), which keeps 16 bits of it.
+// Bound by shared-memory reads (each warp reads the 16 KB of a stage for its sixteen rows: 512 cycles per 64 x 32 tile at
+// G = 2 against 400 of the MMAs).
+#pragma once
+#include "attend.cuh"
+#include "pdl.cuh"
+
+namespace omni {
+namespace pattn {
+
+constexpr int kRows = 32, kKeys = 32, kStages = 3;
+
+template <int D>
+__host__ __device__ constexpr int stage_bytes() { return kKeys * 2 * D * 2; }  // K and V of 32 tokens
+
+__device__ __forceinline__ void cp16(uint32_t dst, const void* src, bool fetch) {  // zeros where !fetch
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(fetch ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+__device__ __forceinline__ void ldsm4(uint32_t addr, uint32_t (&r)[4]) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(addr)
+               : "memory");
+}
+__device__ __forceinline__ void ldsm4t(uint32_t addr, uint32_t (&r)[4]) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(addr)
+               : "memory");
+}
+__device__ __forceinline__ void mma(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+
+template <int D, int G>
+__global__ void __launch_bounds__(kRows * G * 2, G >= 8 ? 1 : 2)
+    prompt_attend_kernel(const bf16* __restrict__ qkv, const bf16* __restrict__ kv, bf16* __restrict__ out, RowMap map,
+                         int rows, int hq, int hk, float scale) {
+  constexpr int kThreads = kRows * G * 2, C = D / 8;  // C: 16-byte chunks of a row
+  extern __shared__ __align__(128) unsigned char prompt_smem[];
+  __shared__ int seq_s[kRows], pos_s[kRows];
+  grid_trigger();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int n0 = blockIdx.x * kRows, kh = blockIdx.y, count = min(kRows, rows - n0);
+  if (threadIdx.x < kRows) {
+    const bool there = (int)threadIdx.x < count;
+    seq_s[threadIdx.x] = there ? map.seq[n0 + threadIdx.x] : -1;
+    pos_s[threadIdx.x] = there ? map.pos[n0 + threadIdx.x] : -1;
+  }
+  __syncthreads();
+  grid_wait();
+  const uint32_t ring = sm100::smem_addr(prompt_smem);
+
+  // this lane's two rows of M: (row, head of the group); their queries as A fragments
+  int row[2], head[2];
+  uint32_t q[D / 16][4];
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int m = warp * 16 + g + 8 * h;
+    row[h] = m / G, head[h] = m % G;
+    const bf16* src = qkv + ((int64_t)(n0 + min(row[h], count - 1)) * (hq + 2 * hk) + kh * G + head[h]) * D + 2 * t;
+#pragma unroll
+    for (int k = 0; k < D / 16; ++k) {
+      q[k][h] = *reinterpret_cast<const uint32_t*>(src + k * 16);
+      q[k][2 + h] = *reinterpret_cast<const uint32_t*>(src + k * 16 + 8);
+    }
+  }
+  float mx[2] = {-INFINITY, -INFINITY}, sum[2] = {0.f, 0.f}, acc[D / 8][4];
+#pragma unroll
+  for (int i = 0; i < D / 8; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
+  const int warp_r0 = warp * 16 / G, warp_r1 = (warp * 16 + 15) / G;  // rows this warp holds heads of
+
+  for (int r0 = 0; r0 < count;) {
+    // the run of rows of one sequence from r0 on, and its last key
+    const int seq = seq_s[r0];
+    const uint32_t same = __ballot_sync(0xffffffffu, seq_s[lane] == seq) >> r0;
+    const int len = same == 0xffffffffu ? 32 : __ffs(~same) - 1, r1 = r0 + len;
+    const int my_pos = lane >= r0 && lane < r1 ? pos_s[lane] : -1;
+    const int last = __reduce_max_sync(0xffffffffu, my_pos);
+    const int warp_last = __reduce_max_sync(0xffffffffu, lane >= warp_r0 && lane <= warp_r1 ? my_pos : -1);
+    int limit[2];  // keys 0 .. limit count for this lane's rows
+#pragma unroll
+    for (int h = 0; h < 2; ++h) limit[h] = row[h] >= r0 && row[h] < r1 ? pos_s[row[h]] : -1;
+    const int32_t* pages = map.pages + map.indptr[seq];
+    const int tiles = (last + kKeys) / kKeys;
+
+    auto fetch = [&](int tile) {
+      if (tile < tiles) {
+        const uint32_t dst = ring + (uint32_t)(tile % kStages) * stage_bytes<D>();
+        for (int i = threadIdx.x; i < kKeys * 2 * C; i += kThreads) {
+          const int c = i % C, tok = i / C % 16, which = i / (C * 16) & 1, pg = i / (C * 32);
+          const int key = tile * kKeys + pg * 16 + tok;
+          const bool live = key <= last;
+          const int64_t page = live ? pages[key >> 4] : 0;
+          // a stage: K of 32 tokens, V of 32 tokens; chunk c of a token sits at c ^ (token & 7)
+          cp16(dst + (uint32_t)((which * kKeys + pg * 16 + tok) * C + (c ^ (tok & 7))) * 16u, kv + kv_offset<D>(page, hk, kh, which, tok) + c * 8, live);
+        }
+      }
+      cp_commit();
+    };
+    for (int s = 0; s < kStages - 1; ++s) fetch(s);
+    for (int tile = 0; tile < tiles; ++tile) {
+      cp_wait<kStages - 2>();
+      __syncthreads();  // the tile is there for everyone, and everyone is done with the one before
+      fetch(tile + kStages - 1);
+      if (tile * kKeys > warp_last) continue;
+      const uint32_t kb = ring + (uint32_t)(tile % kStages) * stage_bytes<D>(), vb = kb + kKeys * D * 2;
+      float s[4][4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) s[j][0] = s[j][1] = s[j][2] = s[j][3] = 0.f;
+#pragma unroll
+      for (int k = 0; k < D / 16; ++k) {
+#pragma unroll
+        for (int jj = 0; jj < 2; ++jj) {  // 16 keys: matrices (keys 0-7, k 0-7), (keys 0-7, k 8-15), (keys 8-15, ...)
+          const int tok = jj * 16 + (lane & 7) + ((lane >> 4) << 3);
+          uint32_t b[4];
+          ldsm4(kb + (uint32_t)(tok * C + ((k * 2 + ((lane >> 3) & 1)) ^ (tok & 7))) * 16u, b);
+          mma(s[jj * 2], q[k], b[0], b[1]);
+          mma(s[jj * 2 + 1], q[k], b[2], b[3]);
+        }
+      }
+      float corr[2];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        float top = -INFINITY;
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            const int key = tile * kKeys + j * 8 + 2 * t + e;
+            float& x = s[j][2 * h + e];
+            x = key <= limit[h] ? x * scale : -INFINITY;
+            top = fmaxf(top, x);
+          }
+        top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 1));
+        top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 2));
+        const float m2 = fmaxf(mx[h], top), ref = m2 == -INFINITY ? 0.f : m2;
+        corr[h] = __expf(mx[h] - ref);
+        mx[h] = m2;
+        float part = 0.f;
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            float& x = s[j][2 * h + e];
+            x = __expf(x - ref);
+            part += x;
+          }
+        sum[h] = sum[h] * corr[h] + part;  // this lane's keys; the other lanes' are added at the end
+      }
+#pragma unroll
+      for (int i = 0; i < D / 8; ++i) acc[i][0] *= corr[0], acc[i][1] *= corr[0], acc[i][2] *= corr[1], acc[i][3] *= corr[1];
+#pragma unroll
+      for (int kk = 0; kk < 2; ++kk) {  // 16 keys
+        uint32_t hi[4], lo[4];
+#pragma unroll
+        for (int x = 0; x < 4; ++x) {
+          const float a = s[kk * 2 + (x >> 1)][(x & 1) * 2], b = s[kk * 2 + (x >> 1)][(x & 1) * 2 + 1];
+          const __nv_bfloat162 top = __floats2bfloat162_rn(a, b);
+          const float2 f = __bfloat1622float2(top);
+          const __nv_bfloat162 rest = __floats2bfloat162_rn(a - f.x, b - f.y);
+          hi[x] = *reinterpret_cast<const uint32_t*>(&top), lo[x] = *reinterpret_cast<const uint32_t*>(&rest);
+        }
+        const int tok = kk * 16 + (lane & 15);
+#pragma unroll
+        for (int i = 0; i < D / 16; ++i) {  // 16 dims
+          uint32_t b[4];
+          ldsm4t(vb + (uint32_t)(tok * C + ((i * 2 + (lane >> 4)) ^ (tok & 7))) * 16u, b);
+          mma(acc[2 * i], hi, b[0], b[1]);
+          mma(acc[2 * i], lo, b[0], b[1]);
+          mma(acc[2 * i + 1], hi, b[2], b[3]);
+          mma(acc[2 * i + 1], lo, b[2], b[3]);
+        }
+      }
+    }
+    cp_wait<0>();
+    __syncthreads();  // the ring is free for the next run
+    r0 = r1;
+  }
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    sum[h] += __shfl_xor_sync(0xffffffffu, sum[h], 1);
+    sum[h] += __shfl_xor_sync(0xffffffffu, sum[h], 2);
+    if (row[h] >= count) continue;
+    const float inv = 1.f / sum[h];
+    bf16* dst = out + ((int64_t)(n0 + row[h]) * hq + kh * G + head[h]) * D + 2 * t;
+#pragma unroll
+    for (int i = 0; i < D / 8; ++i)
+      *reinterpret_cast<__nv_bfloat162*>(dst + i * 8) = __floats2bfloat162_rn(acc[i][2 * h] * inv, acc[i][2 * h + 1] * inv);
+  }
+}
+
+}  // namespace pattn
+}  // namespace omni

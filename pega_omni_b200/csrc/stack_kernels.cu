@@ -7,6 +7,7 @@
 #include "decode_attend.cuh"
 #include "kernels.h"
 #include "pdl.cuh"
+#include "prompt_attend.cuh"
 #include "rope.cuh"
 #include "sampler.cuh"
 
@@ -181,70 +182,62 @@ __device__ __forceinline__ RowAt locate(const RowMap& m, int n) {
 
 // ---- q/k norm + RoPE + KV write -------------------------------------------------
 
-// One warp per (row, head) over the q, k and v heads of the fused qkv row.
-// Semantics of `rope_kv` (qwen3.cu:66-107): RMSNorm over the head, the
-// normalised value rounded to bf16 before the gain, half-rotation rotary
-// embedding with inv_freq = theta^(-2i/D); q stays in place, k and v go to the
-// row's slot.
+// A CTA per row, a warp per head at a time: a lane's rotation angles depend on the row alone, so they are computed once
+// and serve all the heads the warp takes (a powf and a sincosf per head cost four times the memory traffic:
+// 87 us a layer at 8,700 rows of 32 heads). Semantics of `rope_kv` (qwen3.cu:66-107): RMSNorm over the head, the
+// normalised value rounded to bf16 before the gain, half-rotation rotary embedding with inv_freq = theta^(-2i/D); q stays
+// in place, k and v go to the row's slot.
 template <int D>
 __global__ void __launch_bounds__(256) rope_kv_kernel(bf16* __restrict__ qkv, const bf16* __restrict__ q_norm,
                                                       const bf16* __restrict__ k_norm, bf16* __restrict__ kv,
                                                       RowMap map, int hq, int hk, float eps, float theta,
                                                       int kv_pages, uint32_t* err) {
-  grid_trigger();
-  grid_wait();
   constexpr int E = D / 64;  // elements of each half a lane owns
-  const int n = blockIdx.x;
-  const int head = blockIdx.y * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  const int lane = threadIdx.x & 31;
-  if (head >= hq + 2 * hk) return;
+  grid_trigger();
+  const int n = blockIdx.x, lane = threadIdx.x & 31;
   const RowAt at = locate(map, n);
-  const int64_t page = at.slot >> 4;
-  const int tok = (int)(at.slot & 15);
-  if (page < 0 || page >= kv_pages) {
-    if (lane == 0) raise(err, kErrBadIndex);
-    return;
-  }
-  bf16* row = qkv + ((int64_t)n * (hq + 2 * hk) + head) * D;
-  if (head >= hq + hk) {  // V: a plain copy
-    bf16* dst = kv + kv_offset<D>(page, hk, head - hq - hk, 1, tok);
-    for (int i = lane; i < D; i += 32) dst[i] = row[i];
-    return;
-  }
-  const bool is_q = head < hq;
-  const bf16* w = is_q ? q_norm : k_norm;
-  bf16* dst = is_q ? row : kv + kv_offset<D>(page, hk, head - hq, 0, tok);
-  float lo[E], hi[E], ss = 0.f;
-#pragma unroll
-  for (int e = 0; e < E; ++e) {
-    lo[e] = __bfloat162float(row[lane * E + e]);
-    hi[e] = __bfloat162float(row[D / 2 + lane * E + e]);
-    ss += lo[e] * lo[e] + hi[e] * hi[e];
-  }
-  const float r = rsqrtf(warp_add(ss) / D + eps);
+  float cs[E], sn[E], qlo[E], qhi[E], klo[E], khi[E];
+  rope_angles<D>(lane, at.pos, theta, cs, sn);
 #pragma unroll
   for (int e = 0; e < E; ++e) {
     const int i = lane * E + e;
-    const float a = bf16_round(lo[e] * r) * __bfloat162float(w[i]);
-    const float b = bf16_round(hi[e] * r) * __bfloat162float(w[D / 2 + i]);
-    const float inv_freq = 1.f / powf(theta, (float)(2 * i) / D);
-    float sn, cs;
-    sincosf((float)at.pos * inv_freq, &sn, &cs);
-    dst[i] = __float2bfloat16(a * cs - b * sn);
-    dst[D / 2 + i] = __float2bfloat16(b * cs + a * sn);
+    qlo[e] = __bfloat162float(q_norm[i]), qhi[e] = __bfloat162float(q_norm[D / 2 + i]);
+    klo[e] = __bfloat162float(k_norm[i]), khi[e] = __bfloat162float(k_norm[D / 2 + i]);
+  }
+  grid_wait();
+  const int64_t page = at.slot >> 4;
+  const int tok = (int)(at.slot & 15);
+  if (page < 0 || page >= kv_pages) {
+    if (threadIdx.x == 0) raise(err, kErrBadIndex);
+    return;
+  }
+  for (int head = threadIdx.x >> 5; head < hq + 2 * hk; head += blockDim.x >> 5) {
+    bf16* row = qkv + ((int64_t)n * (hq + 2 * hk) + head) * D;
+    if (head >= hq + hk) {  // V: a plain copy
+      bf16* dst = kv + kv_offset<D>(page, hk, head - hq - hk, 1, tok);
+      if constexpr (E == 2) reinterpret_cast<uint2*>(dst)[lane] = reinterpret_cast<const uint2*>(row)[lane];
+      else reinterpret_cast<uint32_t*>(dst)[lane] = reinterpret_cast<const uint32_t*>(row)[lane];
+      continue;
+    }
+    bf16* dst = head < hq ? row : kv + kv_offset<D>(page, hk, head - hq, 0, tok);
+    float lo[E], hi[E];
+#pragma unroll
+    for (int e = 0; e < E; ++e) lo[e] = __bfloat162float(row[lane * E + e]), hi[e] = __bfloat162float(row[D / 2 + lane * E + e]);
+    if (head < hq) rope_head<D>(lo, hi, qlo, qhi, cs, sn, eps);
+    else rope_head<D>(lo, hi, klo, khi, cs, sn, eps);
+#pragma unroll
+    for (int e = 0; e < E; ++e) dst[lane * E + e] = __float2bfloat16(lo[e]), dst[D / 2 + lane * E + e] = __float2bfloat16(hi[e]);
   }
 }
 
 cudaError_t launch_rope_kv(bf16* qkv, const bf16* q_norm, const bf16* k_norm, bf16* kv, const RowMap& map, int rows,
                            const AttnShape& a, int kv_pages, uint32_t* err, cudaStream_t s) {
-  const int heads = a.q_heads + 2 * a.kv_heads;
-  const dim3 grid(rows, (heads + 7) / 8);
-  if (a.head_dim == 128)
-    return launch_pdl(rope_kv_kernel<128>, grid, dim3(256), 0, s, qkv, q_norm, k_norm, kv, map, a.q_heads, a.kv_heads,
-                      a.rms_eps, a.rope_theta, kv_pages, err);
-  if (a.head_dim == 64)
-    return launch_pdl(rope_kv_kernel<64>, grid, dim3(256), 0, s, qkv, q_norm, k_norm, kv, map, a.q_heads, a.kv_heads,
-                      a.rms_eps, a.rope_theta, kv_pages, err);
+  auto go = [&](auto kernel) {
+    return launch_pdl(kernel, dim3(rows), dim3(256), 0, s, qkv, q_norm, k_norm, kv, map, a.q_heads, a.kv_heads, a.rms_eps,
+                      a.rope_theta, kv_pages, err);
+  };
+  if (a.head_dim == 128) return go(rope_kv_kernel<128>);
+  if (a.head_dim == 64) return go(rope_kv_kernel<64>);
   return cudaErrorInvalidValue;
 }
 
@@ -280,6 +273,13 @@ __global__ void __launch_bounds__(kAttnWarps * 32) attend_kernel(const bf16* __r
 template <int D, int G>
 static cudaError_t launch_attend_dg(const bf16* qkv, const bf16* kv, bf16* out, const RowMap& map, int rows, int hq, int hk,
                                     uint32_t* err, cudaStream_t s) {
+  if (map.seq && map.pages) {  // rows of prompts: sequences with several rows each
+    constexpr int bytes = pattn::kStages * pattn::stage_bytes<D>();
+    const cudaError_t e = cudaFuncSetAttribute(pattn::prompt_attend_kernel<D, G>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e != cudaSuccess) return e;
+    return launch_pdl(pattn::prompt_attend_kernel<D, G>, dim3((rows + pattn::kRows - 1) / pattn::kRows, hk), dim3(pattn::kRows * G * 2),
+                      bytes, s, qkv, kv, out, map, rows, hq, hk, 1.f / sqrtf((float)D));
+  }
   constexpr size_t smem = (size_t)kAttnWarps * kAttnSlots * kv_block_bytes<D>();
   if (smem + sizeof(AttnShared<D, G>) > 40 * 1024) {  // per device and instantiation: above the default limit of dynamic shared memory
     static bool raised[64] = {};

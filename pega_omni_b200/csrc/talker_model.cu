@@ -1217,7 +1217,7 @@ static bool chain_wanted(const omni_talker* m) {
     if (!chain_supports(s->hidden, s->inter, qd, s->head_dim)) return false;
     bytes += 2.0 * s->layers * s->hidden * (2.0 * qd + 2.0 * kvd + 3.0 * s->inter);
   }
-  return bytes > (getenv("CHAIN_ALL") ? 0 : 126e6);
+  return bytes > 126e6;
 }
 
 static int create_impl(omni_talker* m, const omni_tensor* tensors, int32_t n_tensors) {
