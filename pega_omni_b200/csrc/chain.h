@@ -11,6 +11,7 @@
 #include "few_rows.h"
 #include "kernels.h"
 #include "stream_gemm.h"
+#include "wide_gemm.h"
 
 namespace omni {
 
@@ -21,6 +22,8 @@ struct ChainPlan {
   StreamGemmPlan s;
 };
 using ChainPlans = std::map<std::tuple<const void*, const void*, const void*, int, int>, ChainPlan>;
+
+constexpr int kChainRows = 256;  // beyond this the GEMMs are contractions, not streams of weights: wide_gemm.h
 
 struct Chain {
   cudaStream_t stream = nullptr;
@@ -34,6 +37,12 @@ struct Chain {
   // y (bf16 rows, SwiGLU activations) or, for kStreamPartials, *sum
   cudaError_t gemm(const bf16* w, int N, int K, const bf16* x, int rows, int out, bf16* y, int ldy, Summands* sum = nullptr,
                    int granule = 0, Epilogue epi = {}) const {
+    if (rows > kChainRows) {  // prompts: any row count, so the plan (two tensor maps) is made for the call
+      WidePlan wide;
+      if (wide_plan(&wide, w, N, K, x, rows, out, y, ldy, epi, sm_count, granule) != 0) return cudaErrorInvalidValue;
+      ++*launches;
+      return wide_launch(wide, err, stream);
+    }
     ChainPlan* p = plan(w, N, K, x, rows, out, y, ldy, granule, epi);
     return p ? launch(*p, {}, sum) : cudaErrorInvalidValue;
   }
@@ -88,7 +97,6 @@ inline bool chain_supports(int hidden, int inter, int q_width, int head_dim) {
   return hidden % 64 == 0 && hidden / 8 <= 1024 && inter % 64 == 0 && q_width % 64 == 0 && (head_dim == 64 || head_dim == 128);
 }
 
-constexpr int kChainRows = 256;  // beyond this the GEMMs are contractions, not streams of weights
 
 // gate_up(l) and down(l) pick a layer's MLP; `inter` is its width, its gate|up rows lie in groups of `granule`.
 template <typename Layer, typename GateUp, typename Down>

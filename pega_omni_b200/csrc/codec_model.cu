@@ -112,8 +112,6 @@ struct omni_codec {
   float* wav_host = nullptr;
   uint32_t* err = nullptr;
   GemmScratch scratch;
-  std::map<std::tuple<const void*, const void*, const void*, int>, TcGemmPlan> plans;
-  std::map<std::tuple<const void*, const void*, const void*, int>, RmGemmPlan> rm_plans;
   std::map<std::tuple<const void*, const void*, const void*, int, int>, ConvGemmPlan> conv_plans;
   ChainPlans stream_plans;
   Chain chain() { return Chain{stream, err, sm_count, scratch.partials, scratch.partial_floats, &launches, &stream_plans}; }
@@ -451,36 +449,11 @@ size_t elems_per_stream(const omni_codec_config& c) {
 
 // y[rows, N] = x[rows, K] . w[N, K]^T on the library's dense GEMMs (K a multiple of 64).
 int dense(omni_codec* m, const bf16* w, int N, int K, const bf16* x, int rows, bf16* y) {
-  if (rows <= kChainRows && stream_supports(N, K, rows)) {
+  if (stream_supports(N, K, rows)) {
     CCUDA(m, m->chain().gemm(w, N, K, x, rows, kStreamBf16, y, N));
-    return OMNI_OK;
-  }
-  if (rows <= 8 || !tc_supports(N, K, rows)) {
+  } else {
     CLAUNCH(m, gemv_launch(w, N, K, x, rows, y, N, Epilogue{}, m->sm_count, m->stream));
-    return OMNI_OK;
   }
-  const auto key = std::make_tuple((const void*)w, (const void*)x, (const void*)y, rows);
-  if (rm_supports(N, K, rows)) {
-    auto rt = m->rm_plans.find(key);
-    if (rt == m->rm_plans.end()) {
-      RmGemmPlan plan;
-      const int rc = rm_plan(&plan, w, N, K, x, rows, y, N, Epilogue{}, m->sm_count);
-      if (rc != 0) return m->fail(OMNI_ERR_CUDA, "tensor-map encode failed (%d) for N=%d K=%d rows=%d", rc, N, K, rows);
-      rt = m->rm_plans.emplace(key, plan).first;
-    }
-    CLAUNCH(m, rm_launch(rt->second, m->err, m->stream));
-    return OMNI_OK;
-  }
-  auto it = m->plans.find(key);
-  if (it == m->plans.end()) {
-    TcGemmPlan plan;
-    const int rc = tc_plan(&plan, w, N, K, x, rows, y, N, Epilogue{}, m->sm_count);
-    if (rc != 0) return m->fail(OMNI_ERR_CUDA, "tensor-map encode failed (%d) for N=%d K=%d rows=%d", rc, N, K, rows);
-    if (plan.partial_floats() > m->scratch.partial_floats || plan.tiles_n() * plan.row_tiles > m->scratch.counter_slots)
-      return m->fail(OMNI_ERR_UNSUPPORTED, "split-K scratch too small for N=%d K=%d rows=%d", N, K, rows);
-    it = m->plans.emplace(key, plan).first;
-  }
-  CLAUNCH(m, tc_launch(it->second, m->scratch, m->err, m->stream));
   return OMNI_OK;
 }
 
@@ -693,9 +666,7 @@ int create_impl(omni_codec* m, const omni_tensor* tensors, int n_tensors) {
   CCUDA(m, cudaMallocHost(&m->in_host, (size_t)m->cfg.max_batch * (kGroups + 2) * sizeof(int32_t)));
   CCUDA(m, cudaMallocHost(&m->wav_host, (size_t)m->cfg.max_batch * m->spf * sizeof(float)));
   m->scratch.partial_floats = (size_t)32 << 20;
-  m->scratch.counter_slots = 1 << 16;
   CTRY(calloc_dev(m, &m->scratch.partials, m->scratch.partial_floats));
-  CTRY(calloc_dev(m, &m->scratch.counters, (size_t)m->scratch.counter_slots, true));
   CCUDA(m, cudaDeviceSynchronize());
   return OMNI_OK;
 }

@@ -111,8 +111,7 @@ struct omni_duplex {
   bf16 *x = nullptr, *x2 = nullptr, *xn = nullptr,  // x2, dx2: the other residual of a few rows' chain
       *qkv = nullptr, *attn = nullptr, *y = nullptr, *gu = nullptr, *act = nullptr;
   bf16 *text_logits = nullptr, *audio_logits = nullptr;  // [max_sessions, text_vocab], [8][max_sessions][card]
-  bf16 *dproj = nullptr, *dx = nullptr, *dx2 = nullptr, *dxn = nullptr, *dqkv = nullptr, *dattn = nullptr, *dy = nullptr,
-       *dgu = nullptr, *dact = nullptr;
+  bf16 *dproj = nullptr, *dx = nullptr, *dx2 = nullptr, *dxn = nullptr, *dqkv = nullptr, *dattn = nullptr, *dact = nullptr;
   int32_t *rows_buf = nullptr, *drawn = nullptr, *emitted = nullptr;
 
   // staged inputs: one pinned block mirrored on the device
@@ -136,8 +135,6 @@ struct omni_duplex {
   bool use_graphs = true;
 
   GemmScratch scratch;
-  std::map<std::tuple<const void*, const void*, const void*, int>, TcGemmPlan> plans;
-  std::map<std::tuple<const void*, const void*, const void*, int>, RmGemmPlan> rm_plans;
 
   int fail(int code, const char* fmt, ...) {
     char buf[512];
@@ -222,36 +219,11 @@ int weight(omni_duplex* m, const Index& idx, const std::string& name, std::initi
 
 // y[rows, N] = x[rows, K] . w[N, K]^T on the path the row count calls for.
 int gemm(omni_duplex* m, const bf16* w, int N, int K, const bf16* x, int rows, bf16* y, int ldy) {
-  if (rows <= kChainRows && stream_supports(N, K, rows)) {
+  if (stream_supports(N, K, rows)) {
     DCUDA(m, m->chain().gemm(w, N, K, x, rows, kStreamBf16, y, ldy));
-    return OMNI_OK;
-  }
-  if (rows <= 8 || !tc_supports(N, K, rows)) {
+  } else {
     DLAUNCH(m, gemv_launch(w, N, K, x, rows, y, ldy, Epilogue{}, m->sm_count, m->stream));
-    return OMNI_OK;
   }
-  const auto key = std::make_tuple((const void*)w, (const void*)x, (const void*)y, rows);
-  if (rm_supports(N, K, rows)) {  // decode-sized: input rows on the MMA M dimension, no split and no reduction
-    auto rt = m->rm_plans.find(key);
-    if (rt == m->rm_plans.end()) {
-      RmGemmPlan plan;
-      const int rc = rm_plan(&plan, w, N, K, x, rows, y, ldy, Epilogue{}, m->sm_count);
-      if (rc != 0) return m->fail(OMNI_ERR_CUDA, "tensor-map encode failed (%d) for N=%d K=%d rows=%d", rc, N, K, rows);
-      rt = m->rm_plans.emplace(key, plan).first;
-    }
-    DLAUNCH(m, rm_launch(rt->second, m->err, m->stream));
-    return OMNI_OK;
-  }
-  auto it = m->plans.find(key);
-  if (it == m->plans.end()) {
-    TcGemmPlan plan;
-    const int rc = tc_plan(&plan, w, N, K, x, rows, y, ldy, Epilogue{}, m->sm_count);
-    if (rc != 0) return m->fail(OMNI_ERR_CUDA, "tensor-map encode failed (%d) for N=%d K=%d rows=%d", rc, N, K, rows);
-    if (plan.partial_floats() > m->scratch.partial_floats || plan.tiles_n() * plan.row_tiles > m->scratch.counter_slots)
-      return m->fail(OMNI_ERR_UNSUPPORTED, "split-K scratch too small for N=%d K=%d rows=%d", N, K, rows);
-    it = m->plans.emplace(key, plan).first;
-  }
-  DLAUNCH(m, tc_launch(it->second, m->scratch, m->err, m->stream));
   return OMNI_OK;
 }
 
@@ -341,7 +313,7 @@ int helium_forward(omni_duplex* m, int rows, const int32_t* pos, const int32_t* 
     DTRY(projected(L.o, Dl, m->attn, 0, L.norm2));
     if (stream) {
       DTRY(behind_norm(L.norm2, L.gate_up, 2 * Hl, kStreamSwiglu, m->act, Hl, m->granule));
-    } else if (rows <= kChainRows) {
+    } else if (rows <= kChainRows || wide_fuses(2 * Hl, D, m->granule)) {
       DCUDA(m, chain.gemm(L.gate_up, 2 * Hl, D, m->xn, rows, kStreamSwiglu, m->act, Hl, nullptr, m->granule));
     } else {
       DTRY(gemm(m, L.gate_up, 2 * Hl, D, m->xn, rows, m->gu, 2 * Hl));
@@ -535,8 +507,6 @@ int32_t omni_duplex_create(const omni_duplex_config* config, const omni_tensor* 
   DTRY(dalloc(m, &m->dxn, (size_t)S * DD));
   DTRY(dalloc(m, &m->dqkv, (size_t)S * 3 * DD));
   DTRY(dalloc(m, &m->dattn, (size_t)S * DD));
-  DTRY(dalloc(m, &m->dy, (size_t)S * DD));
-  DTRY(dalloc(m, &m->dgu, (size_t)S * 2 * DH));
   DTRY(dalloc(m, &m->dact, (size_t)S * DH));
   DTRY(dalloc(m, &m->rows_buf, (size_t)S * kDuplexStreams, true));
   DTRY(dalloc(m, &m->drawn, (size_t)S * kDuplexDrawn, true));
@@ -551,9 +521,7 @@ int32_t omni_duplex_create(const omni_duplex_config* config, const omni_tensor* 
 
   // split-K scratch of the tensor-core GEMM: the largest plan over the shapes above at max_rows rows
   m->scratch.partial_floats = (size_t)32 << 20;
-  m->scratch.counter_slots = 1 << 16;
   DTRY(dalloc(m, &m->scratch.partials, m->scratch.partial_floats));
-  DTRY(dalloc(m, &m->scratch.counters, (size_t)m->scratch.counter_slots, true));
   return OMNI_OK;
 }
 

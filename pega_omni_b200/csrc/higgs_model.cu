@@ -79,8 +79,6 @@ struct omni_higgs {
   int32_t* out_host = nullptr;
   uint32_t* err = nullptr;
   GemmScratch scratch;
-  std::map<std::tuple<const void*, const void*, const void*, int>, TcGemmPlan> plans;
-  std::map<std::tuple<const void*, const void*, const void*, int>, RmGemmPlan> rm_plans;
   // the padding lease: one page and one state line for the rows between the live sequences and the step's bucket
   int pad_page = 0, pad_line = 0;
   // one CUDA graph of the decode step's kernels per bucket (sequence counts are padded up to 1, 2, 4, ... or max_batch)
@@ -176,36 +174,11 @@ int upload(omni_higgs* m, const Index& idx, const std::string& name, std::initia
 }
 
 int gemm(omni_higgs* m, const bf16* w, int N, int K, const bf16* x, int rows, bf16* y, int ldy) {
-  if (rows <= kChainRows && stream_supports(N, K, rows)) {
+  if (stream_supports(N, K, rows)) {
     HCUDA(m, m->chain().gemm(w, N, K, x, rows, kStreamBf16, y, ldy));
-    return OMNI_OK;
-  }
-  if (rows <= 8 || !tc_supports(N, K, rows)) {
+  } else {
     HLAUNCH(m, gemv_launch(w, N, K, x, rows, y, ldy, Epilogue{}, m->sm_count, m->stream));
-    return OMNI_OK;
   }
-  const auto key = std::make_tuple((const void*)w, (const void*)x, (const void*)y, rows);
-  if (rm_supports(N, K, rows)) {  // decode-sized: input rows on the MMA M dimension, no split and no reduction
-    auto rt = m->rm_plans.find(key);
-    if (rt == m->rm_plans.end()) {
-      RmGemmPlan plan;
-      const int rc = rm_plan(&plan, w, N, K, x, rows, y, ldy, Epilogue{}, m->sm_count);
-      if (rc != 0) return m->fail(OMNI_ERR_CUDA, "tensor-map encode failed (%d) for N=%d K=%d rows=%d", rc, N, K, rows);
-      rt = m->rm_plans.emplace(key, plan).first;
-    }
-    HLAUNCH(m, rm_launch(rt->second, m->err, m->stream));
-    return OMNI_OK;
-  }
-  auto it = m->plans.find(key);
-  if (it == m->plans.end()) {
-    TcGemmPlan plan;
-    const int rc = tc_plan(&plan, w, N, K, x, rows, y, ldy, Epilogue{}, m->sm_count);
-    if (rc != 0) return m->fail(OMNI_ERR_CUDA, "tensor-map encode failed (%d) for N=%d K=%d rows=%d", rc, N, K, rows);
-    if (plan.partial_floats() > m->scratch.partial_floats || plan.tiles_n() * plan.row_tiles > m->scratch.counter_slots)
-      return m->fail(OMNI_ERR_UNSUPPORTED, "split-K scratch too small for N=%d K=%d rows=%d", N, K, rows);
-    it = m->plans.emplace(key, plan).first;
-  }
-  HLAUNCH(m, tc_launch(it->second, m->scratch, m->err, m->stream));
   return OMNI_OK;
 }
 
@@ -234,8 +207,13 @@ int body_forward(omni_higgs* m, const bf16* input, int rows, const RowMap& map, 
     HLAUNCH(m, launch_attend(m->qkv, m->kv[i], m->attn, map, rows, a, m->err, m->stream));
     HTRY(gemm(m, L.o, h, qd, m->attn, rows, m->x, h));
     HLAUNCH(m, launch_add_norm(m->x, m->res, L.ln2, m->x, rows, h, c.rms_eps, 1, 0, m->stream));
-    HTRY(gemm(m, both ? L.gate_up_audio : L.gate_up, 2 * I, h, m->x, rows, m->gate_up, 2 * I));
-    HLAUNCH(m, launch_silu_mul(m->gate_up, m->act, rows, I, granule, m->stream));
+    const bf16* gate_up = both ? L.gate_up_audio : L.gate_up;
+    if (wide_fuses(2 * I, h, granule)) {
+      HCUDA(m, m->chain().gemm(gate_up, 2 * I, h, m->x, rows, kStreamSwiglu, m->act, I, nullptr, granule));
+    } else {
+      HTRY(gemm(m, gate_up, 2 * I, h, m->x, rows, m->gate_up, 2 * I));
+      HLAUNCH(m, launch_silu_mul(m->gate_up, m->act, rows, I, granule, m->stream));
+    }
     HTRY(gemm(m, both ? L.down_audio : L.down, h, I, m->act, rows, m->x, h));
     const bf16* next = i + 1 < c.layers ? m->layers[i + 1].ln1 : m->norm;
     HLAUNCH(m, launch_add_norm(m->x, m->res, next, i + 1 < c.layers ? m->x : out, rows, h, c.rms_eps, 1, 0, m->stream));
@@ -444,9 +422,7 @@ int32_t omni_higgs_create(const omni_higgs_config* config, const omni_tensor* te
   HTRY(halloc(m, &m->in_dev, m->in_bytes));
   HCUDA(m, cudaMallocHost((void**)&m->out_host, ((size_t)c.max_batch * OMNI_HIGGS_CODEBOOKS + 1) * 4));
   m->scratch.partial_floats = (size_t)32 << 20;
-  m->scratch.counter_slots = 1 << 16;
   HTRY(halloc(m, &m->scratch.partials, m->scratch.partial_floats));
-  HTRY(halloc(m, &m->scratch.counters, (size_t)m->scratch.counter_slots, true));
   return OMNI_OK;
 }
 

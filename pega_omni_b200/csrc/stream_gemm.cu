@@ -6,6 +6,7 @@
 #include "few_rows.h"
 #include "pdl.cuh"
 #include "sm100.cuh"
+#include "wide_gemm.h"
 
 namespace omni {
 namespace {
@@ -237,6 +238,7 @@ constexpr int kMinSmem = 116 * 1024, kMaxSmem = 200 * 1024;
 
 void stream_configure() {
   few_configure();
+  wide_configure();
   cudaFuncSetAttribute(stream_gemm_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
   cudaFuncSetAttribute(stream_gemm_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
   cudaFuncSetAttribute(stream_gemm_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);

@@ -363,7 +363,8 @@ int alloc_scratch(omni_talker* m, const StackW& s, int rows, Scratch* out) {
 
 // y[rows, N] = x[rows, K] . w[N, K]^T on the path the row count calls for.
 int gemm(omni_talker* m, const bf16* w, int N, int K, const bf16* x, int rows, bf16* y, int ldy, Epilogue epi = {}) {
-  if (m->use_chain && rows <= kChainRows && stream_supports(N, K, rows)) {
+  // beyond kChainRows rows the chains' GEMM is also the one of the programs that do not run as chains
+  if ((rows <= kChainRows ? m->use_chain : m->cfg.gemm_path == 0) && stream_supports(N, K, rows)) {
     CUDA_TRY(m, m->chain().gemm(w, N, K, x, rows, kStreamBf16, y, ldy, nullptr, 0, epi));
     return OMNI_OK;
   }
@@ -414,8 +415,12 @@ int stack_forward(omni_talker* m, const StackW& S, const Scratch& s, const bf16*
     LAUNCH(m, launch_attend(s.qkv, kv[i], s.attn, map, rows, a, m->err, m->stream));
     TRY(gemm(m, L.o, h, qd, s.attn, rows, s.x, h));
     LAUNCH(m, launch_add_norm(s.x, s.res, L.ln2, s.x, rows, h, c.rms_eps, 1, 0, m->stream));
-    TRY(gemm(m, L.gate_up, 2 * I, h, s.x, rows, s.gate_up, 2 * I));
-    LAUNCH(m, launch_silu_mul(s.gate_up, s.act, rows, I, S.granule, m->stream));
+    if (rows > kChainRows && m->cfg.gemm_path == 0 && wide_fuses(2 * I, h, S.granule)) {
+      CUDA_TRY(m, m->chain().gemm(L.gate_up, 2 * I, h, s.x, rows, kStreamSwiglu, s.act, I, nullptr, S.granule));
+    } else {
+      TRY(gemm(m, L.gate_up, 2 * I, h, s.x, rows, s.gate_up, 2 * I));
+      LAUNCH(m, launch_silu_mul(s.gate_up, s.act, rows, I, S.granule, m->stream));
+    }
     TRY(gemm(m, L.down, h, I, s.act, rows, s.x, h));
     if (i + 1 < c.layers)
       LAUNCH(m, launch_add_norm(s.x, s.res, S.layers[i + 1].ln1, s.x, rows, h, c.rms_eps, 1, 0, m->stream));
