@@ -12,6 +12,7 @@
 #include <algorithm>
 
 #include "codec.h"
+#include "decode_attend.cuh"
 #include "pdl.cuh"
 
 namespace omni {
@@ -91,72 +92,83 @@ __global__ void codec_add_norm_kernel(const bf16* add, int64_t add_stride, bf16*
   }
 }
 
-// A warp per (stream, head): rotary embedding of q and k (a lane holds dims lane and lane + 32, the pair one rotation
-// mixes), k and v into the ring, then q against the last min(p + 1, 72) frames: a lane scores whole frames (its q copy
-// comes from shared memory), the softmax runs across lanes, and for the weighted sum of V a lane owns two dims.
-__global__ void __launch_bounds__(128)
+// A CTA per (stream, head), a warp per sixteen slots of the ring: the order of the frames does not matter to the softmax,
+// so a warp takes its slots as they lie (slots past the stream's first frames are masked) and asks for them before
+// grid_wait(), since only earlier frames wrote them; the frame's own key and value are patched in. The products run on the
+// page step of decode_attend.cuh, whose five partial states are merged at the end. Bound by latency: 15 us a layer when a
+// warp walked all 72 frames with scalar loads and sums, at one stream and 25 us at 64.
+constexpr int kWindowWarps = (kWindow + 15) / 16;
+
+__global__ void __launch_bounds__(kWindowWarps * 32)
     codec_window_attend_kernel(const bf16* __restrict__ qkv, CodecStateRef st, int64_t ring_offset, bf16* __restrict__ out,
                                int heads, float theta) {
   grid_trigger();
-  grid_wait();
-  __shared__ float sq[4][kHeadDim];
-  __shared__ float sp[4][kWindow + 8];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int s = blockIdx.x, head = blockIdx.y * 4 + warp;
-  if (head >= heads) return;
-  const int width = heads * kHeadDim;
-  const bf16* row = qkv + (int64_t)s * 3 * width + head * kHeadDim;
-  bf16* ring = slot_ptr(st, s, ring_offset);
-  const int p = st.pos[s];
-  const int n = min(p + 1, kWindow), first = p - n + 1;
+  __shared__ alignas(16) bf16 sq[kWindowWarps][kHeadDim], sk[kHeadDim], sv[kHeadDim];
+  __shared__ float sm[kWindowWarps], sl[kWindowWarps], so[kWindowWarps][kHeadDim];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int s = blockIdx.x, head = blockIdx.y, width = heads * kHeadDim;
+  const int p = st.pos[s], own = p % kWindow, slots = min(p + 1, kWindow);
+  bf16* ring = slot_ptr(st, s, ring_offset) + head * kHeadDim;
   const int64_t v_ofs = (int64_t)kWindow * width;
+  const int ntok = max(0, min(16, slots - 16 * warp));
+  const bool mine = own >> 4 == warp;
+  dattn::Page<kHeadDim> pg;
+#pragma unroll
+  for (int h = 0; h < 2; ++h)
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+      pg.k[h][j] = *reinterpret_cast<const uint4*>(ring + (int64_t)min(16 * warp + g + 8 * h, kWindow - 1) * width + 8 * t + 32 * j);
+#pragma unroll
+  for (int r = 0; r < 4; ++r)
+    pg.v[r][0] = *reinterpret_cast<const uint4*>(ring + v_ofs + (int64_t)min(16 * warp + 2 * t + (r & 1) + 8 * (r >> 1), kWindow - 1) * width + 8 * g);
   const float inv_freq = 1.f / powf(theta, (float)(2 * lane) / kHeadDim);
   float sn, cs;
   sincosf((float)p * inv_freq, &sn, &cs);
-  const float q_lo = __bfloat162float(row[lane]), q_hi = __bfloat162float(row[lane + 32]);
-  const float k_lo = __bfloat162float(row[width + lane]), k_hi = __bfloat162float(row[width + lane + 32]);
-  const bf16 ka = __float2bfloat16(k_lo * cs - k_hi * sn), kb = __float2bfloat16(k_hi * cs + k_lo * sn);
-  sq[warp][lane] = bf16_round(q_lo * cs - q_hi * sn);
-  sq[warp][lane + 32] = bf16_round(q_hi * cs + q_lo * sn);
-  bf16* at = ring + (int64_t)(p % kWindow) * width + head * kHeadDim;
-  at[lane] = ka;
-  at[lane + 32] = kb;
-  reinterpret_cast<uint32_t*>(at + v_ofs)[lane] = reinterpret_cast<const uint32_t*>(row + 2 * width)[lane];
-  __syncwarp();  // the ring rows of this (stream, head) are written and read by this warp alone
-  float mx = -INFINITY;
-  for (int j = lane; j < n; j += 32) {
-    const uint4* kr = reinterpret_cast<const uint4*>(ring + (int64_t)((first + j) % kWindow) * width + head * kHeadDim);
-    float dot = 0.f;
-#pragma unroll
-    for (int q8 = 0; q8 < 8; ++q8) {
-      float kv[8];
-      unpack8v(kr[q8], kv);
-#pragma unroll
-      for (int e = 0; e < 8; ++e) dot += sq[warp][q8 * 8 + e] * kv[e];
+  const bf16* row = qkv + (int64_t)s * 3 * width + head * kHeadDim;
+  grid_wait();
+  dattn::State<kHeadDim> state;
+  state.reset();
+  if (ntok > 0) {
+    const float q_lo = __bfloat162float(row[lane]), q_hi = __bfloat162float(row[lane + 32]);
+    sq[warp][lane] = __float2bfloat16(q_lo * cs - q_hi * sn);
+    sq[warp][lane + 32] = __float2bfloat16(q_hi * cs + q_lo * sn);
+    if (mine) {  // k and v of the frame: to the ring and into the page
+      const float k_lo = __bfloat162float(row[width + lane]), k_hi = __bfloat162float(row[width + lane + 32]);
+      const uint32_t v2 = reinterpret_cast<const uint32_t*>(row + 2 * width)[lane];
+      const bf16 ka = __float2bfloat16(k_lo * cs - k_hi * sn), kb = __float2bfloat16(k_hi * cs + k_lo * sn);
+      bf16* at = ring + (int64_t)own * width;
+      at[lane] = sk[lane] = ka;
+      at[lane + 32] = sk[lane + 32] = kb;
+      reinterpret_cast<uint32_t*>(at + v_ofs)[lane] = reinterpret_cast<uint32_t*>(sv)[lane] = v2;
     }
-    dot *= 0.125f;  // 1 / sqrt(64)
-    sp[warp][j] = dot;
-    mx = fmaxf(mx, dot);
+    __syncwarp();
+    uint4 q[2];
+#pragma unroll
+    for (int j = 0; j < 2; ++j) q[j] = g == 0 ? *reinterpret_cast<const uint4*>(sq[warp] + 8 * t + 32 * j) : make_uint4(0u, 0u, 0u, 0u);
+    if (mine) pg.patch(own & 15, sk, sv, lane);
+    state.step(pg, q, ntok, 0.125f /* 1 / sqrt(64) */, lane);
+    state.finish();
   }
-  mx = warp_fmax(mx);
-  float l = 0.f;
-  for (int j = lane; j < n; j += 32) {
-    const float e = __expf(sp[warp][j] - mx);
-    sp[warp][j] = e;
-    l += e;
+  if (t == 0) {  // head column 0
+    if (g == 0) sm[warp] = state.m[0], sl[warp] = state.l[0];
+    float v[8];
+    state.dims8(0, 0, v);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) so[warp][8 * g + e] = v[e];
   }
-  l = warp_add(l);
-  __syncwarp();
-  float o0 = 0.f, o1 = 0.f;
-  for (int j = 0; j < n; ++j) {
-    const __nv_bfloat162 v2 = reinterpret_cast<const __nv_bfloat162*>(
-        ring + v_ofs + (int64_t)((first + j) % kWindow) * width + head * kHeadDim)[lane];
-    const float pj = sp[warp][j];
-    o0 += pj * __low2float(v2);
-    o1 += pj * __high2float(v2);
+  __syncthreads();
+  if (threadIdx.x < kHeadDim / 2) {
+    float top = sm[0], o0 = 0.f, o1 = 0.f, l = 0.f;
+#pragma unroll
+    for (int w = 1; w < kWindowWarps; ++w) top = fmaxf(top, sm[w]);
+#pragma unroll
+    for (int w = 0; w < kWindowWarps; ++w) {
+      const float e = __expf(sm[w] - top);  // 0 for a warp without frames
+      const float2 o = *reinterpret_cast<const float2*>(&so[w][2 * threadIdx.x]);
+      o0 += e * o.x, o1 += e * o.y, l += e * sl[w];
+    }
+    reinterpret_cast<__nv_bfloat162*>(out + (int64_t)s * width + head * kHeadDim)[threadIdx.x] = __floats2bfloat162_rn(o0 / l, o1 / l);
   }
-  reinterpret_cast<__nv_bfloat162*>(out + (int64_t)s * width + head * kHeadDim)[lane] =
-      __floats2bfloat162_rn(o0 / l, o1 / l);
 }
 
 __global__ void codec_silu_mul_kernel(const bf16* __restrict__ gate_up, bf16* __restrict__ out, int inter, int64_t total) {
@@ -441,7 +453,7 @@ cudaError_t launch_codec_add_norm(const bf16* add, int64_t add_stride, bf16* res
 
 cudaError_t launch_codec_window_attend(const bf16* qkv, CodecStateRef st, int64_t ring_offset, bf16* out, int n, int heads,
                                        float theta, cudaStream_t stream) {
-  return launch_pdl(codec_window_attend_kernel, dim3(n, (heads + 3) / 4), dim3(128), 0, stream, qkv, st, ring_offset, out, heads, theta);
+  return launch_pdl(codec_window_attend_kernel, dim3(n, heads), dim3(kWindowWarps * 32), 0, stream, qkv, st, ring_offset, out, heads, theta);
 }
 
 cudaError_t launch_codec_silu_mul(const bf16* gate_up, bf16* out, int rows, int inter, cudaStream_t stream) {
