@@ -7,6 +7,7 @@ of the token bookkeeping (crates/omni-personaplex/src/prompt.rs:167-183).
 from __future__ import annotations
 
 import ctypes as C
+import struct
 import zlib
 from dataclasses import dataclass, field
 from typing import Optional, Sequence
@@ -199,6 +200,13 @@ def _contig(t):
     return np.ascontiguousarray(t) if isinstance(t, np.ndarray) else t.contiguous()
 
 
+_STEP = struct.Struct("=%di4xQ" % (DRAWN + 2 * CODEBOOKS))
+
+
+def _padded(values, count):
+    return (list(values) + [0] * count)[:max(len(values), count)]
+
+
 class Model:
     def __init__(self, handle, config: DuplexConfig, max_sessions: int):
         self._h, self.config, self.max_sessions = handle, config, max_sessions
@@ -307,10 +315,13 @@ class Model:
         """rows: [(session, step)]."""
         n = len(rows)
         handles = (C.c_void_p * n)(*[s._h for s, _ in rows])
-        steps = (L.DuplexStep * n)()
+        raw = bytearray(_STEP.size * n)  # omni_duplex_step[n]; ctypes objects row by row take five times as long
         for i, (_, x) in enumerate(rows):
-            steps[i] = L.DuplexStep((C.c_int32 * DRAWN)(*x.force), (C.c_int32 * CODEBOOKS)(*x.force_caller),
-                                    (C.c_int32 * CODEBOOKS)(*x.caller), x.seed & 0xFFFFFFFFFFFFFFFF)
+            force, force_caller, caller = x.force, x.force_caller, x.caller
+            if len(force) != DRAWN or len(force_caller) != CODEBOOKS or len(caller) != CODEBOOKS:
+                force, force_caller, caller = _padded(force, DRAWN), _padded(force_caller, CODEBOOKS), _padded(caller, CODEBOOKS)
+            _STEP.pack_into(raw, i * _STEP.size, *force, *force_caller, *caller, x.seed & 0xFFFFFFFFFFFFFFFF)
+        steps = (L.DuplexStep * n).from_buffer(raw)
         emitted = np.zeros((n, DRAWN), dtype=np.int32)
         self._check(self._lib.omni_duplex_tick(self._h, n, handles, steps,
                                                emitted.ctypes.data_as(C.POINTER(C.c_int32))))

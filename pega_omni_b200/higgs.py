@@ -6,6 +6,7 @@ Names follow crates/omni-higgs-audio/src/delay.rs: ``Delay.forced_from``, ``Dela
 from __future__ import annotations
 
 import ctypes as C
+import struct
 
 import numpy as np
 
@@ -154,6 +155,9 @@ class HiggsSeq:
         return L.load().omni_higgs_seq_rows(self._h)
 
 
+_DRAW, _FREE = struct.Struct("=8f8ii"), (-1,) * CODEBOOKS
+
+
 class HiggsModel:
     def __init__(self, handle, config: HiggsConfig):
         self._h, self.config = handle, config
@@ -201,11 +205,13 @@ class HiggsModel:
 
     @staticmethod
     def _draws(draws):
-        arr = (L.HiggsDraw * len(draws))()
+        raw = bytearray(_DRAW.size * len(draws))  # omni_higgs_draw[n]
         for i, d in enumerate(draws):
-            f = list(d.force) if d.force is not None else [-1] * CODEBOOKS
-            arr[i] = L.HiggsDraw((C.c_float * 8)(*d.uniforms), (C.c_int32 * 8)(*f), int(d.force is not None))
-        return arr
+            u, f = d.uniforms, d.force if d.force is not None else _FREE
+            if len(u) != CODEBOOKS or len(f) != CODEBOOKS:  # missing values are zeros
+                u, f = (list(u) + [0.0] * CODEBOOKS)[:max(len(u), CODEBOOKS)], (list(f) + [0] * CODEBOOKS)[:max(len(f), CODEBOOKS)]
+            _DRAW.pack_into(raw, i * _DRAW.size, *u, *f, d.force is not None)
+        return (L.HiggsDraw * len(draws)).from_buffer(raw)
 
     def _out(self, n):
         return np.zeros((n, CODEBOOKS), dtype=np.int32), np.zeros(n, dtype=np.int32)
