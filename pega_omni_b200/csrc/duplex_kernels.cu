@@ -111,31 +111,33 @@ __global__ void lm_add_norm_kernel(const bf16* __restrict__ y, bf16* __restrict_
 }
 
 // The same over a GEMM's summands: every load of a thread's eight columns is under way at once.
+template <int S>
 __global__ void lm_add_norm_sum_kernel(const Summands y, bf16* __restrict__ x, const bf16* __restrict__ alpha,
                                        bf16* __restrict__ out, int dim, float eps) {
   grid_trigger();
   __shared__ float scratch[32];
-  const int c = threadIdx.x * 8;
+  const int c = threadIdx.x * 8, lane = threadIdx.x & 31;
   const int64_t at = (int64_t)blockIdx.x * dim + c;
-  float v[8], u[8], a[8];
-  if (out) ld8(alpha + c, a);
+  const bool on = c < dim;  // the block is a whole number of warps
+  float v[8], u[8], a[8], ss = 0.f;
+  if (out && on) ld8(alpha + c, a);
   grid_wait();
-  ld8cg(x + at, v);
-  load_sum8(y, blockIdx.x, c, u);
-  float ss = 0.f;
+  if (on) {
+    ld8cg(x + at, v);
+    load_sum8<S>(y, blockIdx.x, c, u);
 #pragma unroll
-  for (int k = 0; k < 8; ++k) {
-    v[k] = bf16_round(v[k] + u[k]);
-    ss += v[k] * v[k];
+    for (int k = 0; k < 8; ++k) {
+      v[k] = bf16_round(v[k] + u[k]);
+      ss += v[k] * v[k];
+    }
+    st8(x + at, v);
   }
-  st8(x + at, v);
   if (!out) return;
   ss = warp_add(ss);
-  if ((threadIdx.x & 31) == 0) scratch[threadIdx.x >> 5] = ss;
+  if (lane == 0) scratch[threadIdx.x >> 5] = ss;
   __syncthreads();
-  float total = 0.f;
-  for (int i = 0; i < (int)(blockDim.x + 31) >> 5; ++i) total += scratch[i];
-  const float r = rsqrtf(total / dim + eps);
+  const float r = rsqrtf(warp_add(lane < (int)blockDim.x >> 5 ? scratch[lane] : 0.f) / dim + eps);
+  if (!on) return;
 #pragma unroll
   for (int k = 0; k < 8; ++k) v[k] = v[k] * (a[k] * r);
   st8(out + at, v);
@@ -827,8 +829,10 @@ cudaError_t launch_lm_add_norm(const bf16* y, bf16* x, const bf16* alpha, bf16* 
 
 cudaError_t launch_lm_add_norm_sum(const Summands& y, bf16* x, const bf16* alpha, bf16* out, int rows, int dim, float eps,
                                    cudaStream_t s) {
-  if (!row_dim_ok(dim) || y.splits > 8) return cudaErrorInvalidValue;
-  return launch_pdl(lm_add_norm_sum_kernel, dim3(rows), dim3(dim / 8), 0, s, y, x, alpha, out, dim, eps);
+  if (!row_dim_ok(dim)) return cudaErrorInvalidValue;
+  return with_summands(y.splits, [&](auto sums) {
+    return launch_pdl(lm_add_norm_sum_kernel<decltype(sums)::value>, dim3(rows), dim3((dim + 255) / 256 * 32), 0, s, y, x, alpha, out, dim, eps);
+  });
 }
 
 cudaError_t launch_lm_tp_add_norm(const bf16* mine, const bf16* peer, bf16* x, const bf16* alpha, bf16* out, int rows,

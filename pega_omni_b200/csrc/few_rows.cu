@@ -20,7 +20,7 @@ namespace omni {
 namespace {
 
 constexpr int kWarps = 8, kKb = 64, kFewSlots = 8;
-constexpr int kNormChunks = 6;  // 8-element pieces of the rows that a lane holds across the norm's sum
+constexpr int kNormChunks = 2;  // 8-element pieces of the rows that a lane holds across the norm's sum
 
 struct FewArgs {
   const bf16* x;
@@ -208,8 +208,6 @@ __global__ void __launch_bounds__(kWarps * 32, 2) few_rows_kernel(const __grid_c
     auto with = [&](auto sums) {
       constexpr int S = decltype(sums)::value;
       if (a.rounds <= 1) norm_rows<NORM, S, 1>(a, h, keep, ss_s, g);
-      else if (a.rounds == 2) norm_rows<NORM, S, 2>(a, h, keep, ss_s, g);
-      else if (a.rounds <= 4) norm_rows<NORM, S, 4>(a, h, keep, ss_s, g);
       else norm_rows<NORM, S, kNormChunks>(a, h, keep, ss_s, g);
     };
     if (a.norm.sum.splits == 1) with(std::integral_constant<int, 1>());

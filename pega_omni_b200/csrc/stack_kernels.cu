@@ -82,32 +82,35 @@ __global__ void silu_mul_kernel(const bf16* __restrict__ gate_up, bf16* __restri
   st8(act + (int64_t)i * 8, g);
 }
 
-// add_norm over a GEMM's summands: a thread owns eight columns, and all its loads - up to eight partial sums, the
-// residual, the gain - are under way together, so the kernel is one L2 round trip and one block reduction long.
+// add_norm over a GEMM's S summands: a thread owns eight columns, and all its loads - the partial sums, the residual, the
+// gain - are under way together, so the kernel is one L2 round trip and one block reduction long. What is left is the
+// number of instructions, executed once: the count of summands is a template argument.
+template <int S>
 __global__ void add_norm_sum_kernel(const Summands x, bf16* __restrict__ res, const bf16* __restrict__ w,
                                     bf16* __restrict__ out, int dim, float eps, int every, int which) {
   grid_trigger();
   __shared__ float scratch[32];
-  const int n = blockIdx.x, c = threadIdx.x * 8;
-  float g[8], v[8], rv[8];
-  ld8(w + c, g);
+  const int n = blockIdx.x, c = threadIdx.x * 8, lane = threadIdx.x & 31;
+  const bool on = c < dim;  // the block is a whole number of warps
+  float g[8], v[8], rv[8], ss = 0.f;
+  if (on) ld8(w + c, g);
   grid_wait();
-  ld8cg(res + (int64_t)n * dim + c, rv);
-  load_sum8(x, n, c, v);
-  float ss = 0.f;
+  if (on) {
+    ld8cg(res + (int64_t)n * dim + c, rv);
+    load_sum8<S>(x, n, c, v);
 #pragma unroll
-  for (int k = 0; k < 8; ++k) {
-    v[k] += rv[k];
-    ss += v[k] * v[k];
+    for (int k = 0; k < 8; ++k) {
+      v[k] += rv[k];
+      ss += v[k] * v[k];
+    }
+    st8(res + (int64_t)n * dim + c, v);
   }
   ss = warp_add(ss);
-  if ((threadIdx.x & 31) == 0) scratch[threadIdx.x >> 5] = ss;
-  st8(res + (int64_t)n * dim + c, v);
+  if (lane == 0) scratch[threadIdx.x >> 5] = ss;
   if (n % every != which) return;
   __syncthreads();
-  float total = 0.f;
-  for (int i = 0; i < (int)(blockDim.x + 31) >> 5; ++i) total += scratch[i];
-  const float r = rsqrtf(total / dim + eps);
+  const float r = rsqrtf(warp_add(lane < (int)blockDim.x >> 5 ? scratch[lane] : 0.f) / dim + eps);
+  if (!on) return;
 #pragma unroll
   for (int k = 0; k < 8; ++k) v[k] = v[k] * r * g[k];
   st8(out + (int64_t)(n / every) * dim + c, v);
@@ -115,8 +118,10 @@ __global__ void add_norm_sum_kernel(const Summands x, bf16* __restrict__ res, co
 
 cudaError_t launch_add_norm_sum(const Summands& x, bf16* res, const bf16* w, bf16* out, int rows, int dim, float eps,
                                 int every, int which, cudaStream_t s) {
-  if (dim % 8 || dim / 8 > 1024 || x.splits > 8) return cudaErrorInvalidValue;
-  return launch_pdl(add_norm_sum_kernel, dim3(rows), dim3(dim / 8), 0, s, x, res, w, out, dim, eps, every, which);
+  if (dim % 8 || dim / 8 > 1024) return cudaErrorInvalidValue;
+  return with_summands(x.splits, [&](auto sums) {
+    return launch_pdl(add_norm_sum_kernel<decltype(sums)::value>, dim3(rows), dim3((dim + 255) / 256 * 32), 0, s, x, res, w, out, dim, eps, every, which);
+  });
 }
 
 __global__ void interleave_gate_up_kernel(const bf16* __restrict__ src, bf16* __restrict__ dst, int inter, int k,

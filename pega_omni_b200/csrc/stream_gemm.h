@@ -5,6 +5,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <type_traits>
+
 #include "gemm.h"
 #include "util.cuh"
 
@@ -20,29 +22,39 @@ struct Summands {
   int ld = 0;                // elements per row
 };
 
-// Eight columns of row n from column c on: the bf16 values, widened. At most MAX splits.
-template <int MAX = 8>
+// Eight columns of row n from column c on, of S summands (0: bf16 rows): the bf16 values, widened.
+template <int S>
 __device__ __forceinline__ void load_sum8(const Summands& x, int n, int c, float (&v)[8]) {
-  if (x.splits == 0) {
+  if constexpr (S == 0) {
     unpack8v(__ldcg(reinterpret_cast<const uint4*>(x.done + (int64_t)n * x.ld + c)), v);
-    return;
+  } else {
+    const float* p = x.part + (int64_t)n * x.ld + c;
+    float4 f[S][2];
+#pragma unroll
+    for (int s = 0; s < S; ++s)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) f[s][h] = __ldcg(reinterpret_cast<const float4*>(p + s * x.split_stride) + h);
+#pragma unroll
+    for (int s = 1; s < S; ++s) {
+      f[0][0].x += f[s][0].x, f[0][0].y += f[s][0].y, f[0][0].z += f[s][0].z, f[0][0].w += f[s][0].w;
+      f[0][1].x += f[s][1].x, f[0][1].y += f[s][1].y, f[0][1].z += f[s][1].z, f[0][1].w += f[s][1].w;
+    }
+    v[0] = bf16_round(f[0][0].x), v[1] = bf16_round(f[0][0].y), v[2] = bf16_round(f[0][0].z), v[3] = bf16_round(f[0][0].w);
+    v[4] = bf16_round(f[0][1].x), v[5] = bf16_round(f[0][1].y), v[6] = bf16_round(f[0][1].z), v[7] = bf16_round(f[0][1].w);
   }
-  const float* p = x.part + (int64_t)n * x.ld + c;
-  float4 f[MAX][2];
-#pragma unroll
-  for (int s = 0; s < MAX; ++s)
-#pragma unroll
-    for (int h = 0; h < 2; ++h)
-      f[s][h] = s < x.splits ? __ldcg(reinterpret_cast<const float4*>(p + s * x.split_stride) + h) : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-  for (int k = 0; k < 8; ++k) v[k] = 0.f;
-#pragma unroll
-  for (int s = 0; s < MAX; ++s) {  // adding 0 for a missing split leaves the sum unchanged
-    v[0] += f[s][0].x, v[1] += f[s][0].y, v[2] += f[s][0].z, v[3] += f[s][0].w;
-    v[4] += f[s][1].x, v[5] += f[s][1].y, v[6] += f[s][1].z, v[7] += f[s][1].w;
+}
+
+// go(std::integral_constant<int, S>) for the summand counts that the plans make.
+template <typename F>
+cudaError_t with_summands(int splits, F&& go) {
+  switch (splits) {
+    case 0: return go(std::integral_constant<int, 0>());
+    case 1: return go(std::integral_constant<int, 1>());
+    case 2: return go(std::integral_constant<int, 2>());
+    case 4: return go(std::integral_constant<int, 4>());
+    case 8: return go(std::integral_constant<int, 8>());
+    default: return cudaErrorInvalidValue;
   }
-#pragma unroll
-  for (int k = 0; k < 8; ++k) v[k] = bf16_round(v[k]);
 }
 
 enum StreamOut : int { kStreamBf16 = 0, kStreamPartials = 1, kStreamSwiglu = 2 };
