@@ -29,11 +29,18 @@ struct Page {
   uint4 k[2][D / 32];
   uint4 v[4][D / 64];
   __device__ __forceinline__ void load(const bf16* block, int lane) {
+    load_k(block, lane);
+    load_v(block, lane);
+  }
+  __device__ __forceinline__ void load_k(const bf16* block, int lane) {
     const int g = lane >> 2, t = lane & 3;
 #pragma unroll
     for (int h = 0; h < 2; ++h)
 #pragma unroll
       for (int j = 0; j < D / 32; ++j) k[h][j] = __ldcg(reinterpret_cast<const uint4*>(block + (g + 8 * h) * D + 8 * t + 32 * j));
+  }
+  __device__ __forceinline__ void load_v(const bf16* block, int lane) {
+    const int g = lane >> 2, t = lane & 3;
 #pragma unroll
     for (int r = 0; r < 4; ++r)
 #pragma unroll
@@ -68,8 +75,10 @@ struct State {
 #pragma unroll
     for (int i = 0; i < D / 16; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
   }
-  // q: row g of [8][D] (heads past G are zero rows), 16 bytes per 32 dims.
-  __device__ __forceinline__ void step(Page<D>& pg, const uint4 (&q)[D / 32], int ntok, float scale, int lane) {
+  // q: row g of [8][D] (heads past G are zero rows), 16 bytes per 32 dims. `next`: the block whose keys are asked for as
+  // soon as this page's have been used, and whose values follow at the end (nullptr: none).
+  __device__ __forceinline__ void step(Page<D>& pg, const uint4 (&q)[D / 32], int ntok, float scale, int lane,
+                                       const bf16* next = nullptr) {
     const int g = lane >> 2, t = lane & 3;
     float s[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
@@ -77,6 +86,7 @@ struct State {
       mma16816(s, pg.k[0][j].x, pg.k[1][j].x, pg.k[0][j].y, pg.k[1][j].y, q[j].x, q[j].y);
       mma16816(s, pg.k[0][j].z, pg.k[1][j].z, pg.k[0][j].w, pg.k[1][j].w, q[j].z, q[j].w);
     }
+    if (next) pg.load_k(next, lane);
     // s[0], s[1]: key g, heads 2t, 2t + 1; s[2], s[3]: key g + 8
 #pragma unroll
     for (int k = 0; k < 4; ++k) s[k] = (g + (k >> 1) * 8) < ntok ? s[k] * scale : -INFINITY;
@@ -129,6 +139,7 @@ struct State {
         mma16816(acc[4 * i + e], a0, a1, a2, a3, bh[0], bh[1]);
         mma16816(acc[4 * i + e], a0, a1, a2, a3, bl[0], bl[1]);
       }
+    if (next) pg.load_v(next, lane);
   }
   // Sums of the lanes' shares: every lane then holds its two heads' sums over all keys of the warp.
   __device__ __forceinline__ void finish() {

@@ -389,18 +389,18 @@ __global__ void __launch_bounds__(W * TEAMS * 32, W == 8 ? 1 : 3)
       if (live && warp == 0 && lane == 0) raise(err, kErrBadIndex);
       own = 0;
     }
-    auto load = [&](int pi) {
+    auto block = [&](int pi) {
       int64_t page = pi == last ? own : pages[pi];
       if (page < 0 || page >= kv_pages) {
         if (lane == 0) raise(err, kErrBadIndex);
         page = 0;
       }
-      pg.load(kv + kv_offset<D>(page, hk, kh, 0, 0), lane);
+      return kv + kv_offset<D>(page, hk, kh, 0, 0);
     };
-    if (paged && live && warp < npages) load(warp);
+    if (paged && live && warp < npages) pg.load(block(warp), lane);
     if (r == 0) grid_wait();
     if (W == 1 && !live) return;  // (a dead team of several warps does not exist: TEAMS is 1 there)
-    if (!paged) load(0);
+    if (!paged) pg.load(block(0), lane);
     const bf16* row = lookup.table ? lookup.table + (int64_t)lookup.codes[n * 16 + lookup.group] * ((hq + 2 * hk) * D)
                                    : qkv + (int64_t)n * ((hq + 2 * hk) * D);
     constexpr int JOBS = (G + 2 + W - 1) / W;
@@ -441,12 +441,11 @@ __global__ void __launch_bounds__(W * TEAMS * 32, W == 8 ? 1 : 3)
     for (int j = 0; j < D / 32; ++j) q[j] = *reinterpret_cast<const uint4*>(sh.q[lane >> 2] + 8 * (lane & 3) + 32 * j);
     st.reset();
     for (int pi = warp; pi < npages; pi += W) {
-      if (pi != warp) load(pi);
       if (pi == last) {
         if (!paged && r > 0) pg.patch(tok - 1, sh.k[(r - 1) & 1], sh.v[(r - 1) & 1], lane);  // (per <= 2)
         pg.patch(tok, sh.k[r & 1], sh.v[r & 1], lane);
       }
-      st.step(pg, q, min(16, pos + 1 - pi * 16), scale, lane);
+      st.step(pg, q, min(16, pos + 1 - pi * 16), scale, lane, pi + W < npages ? block(pi + W) : nullptr);
     }
     st.finish();
     const int g = lane >> 2, t = lane & 3;
@@ -479,18 +478,21 @@ __global__ void __launch_bounds__(W * TEAMS * 32, W == 8 ? 1 : 3)
           }
         }
       __syncthreads();
-      const int used = min(W, npages);  // warps that held a page
-      for (int i = threadIdx.x; i < G * D; i += W * 32) {
-        const int h = i / D, d = i % D;
-        float top = -INFINITY;
-        for (int w = 0; w < used; ++w) top = fmaxf(top, merge.m[w][h]);
-        float num = 0.f, den = 0.f;
-        for (int w = 0; w < used; ++w) {
-          const float e = __expf(merge.m[w][h] - top);
-          num += merge.o[w][h][d] * e;
-          den += merge.l[w][h] * e;
+      // a warp per head and 64 dims at a time; lane w has the weight of warp w's state (0 where it held no page)
+      for (int i = warp; i < G * (D / 64); i += W) {
+        const int h = i / (D / 64), d = i % (D / 64) * 64 + 2 * lane;
+        const float mw = lane < W ? merge.m[lane][h] : -INFINITY;
+        const float e = __expf(mw - warp_fmax(mw));
+        const float den = warp_add(lane < W ? e * merge.l[lane][h] : 0.f);
+        float o0 = 0.f, o1 = 0.f;
+#pragma unroll
+        for (int w = 0; w < W; ++w) {
+          const float ew = __shfl_sync(0xffffffffu, e, w);
+          const float2 o = *reinterpret_cast<const float2*>(&merge.o[w][h][d]);
+          o0 += ew * o.x, o1 += ew * o.y;
         }
-        out[((int64_t)n * hq + kh * G) * D + i] = __float2bfloat16(num / den);
+        const float inv = 1.f / den;
+        *reinterpret_cast<__nv_bfloat162*>(out + ((int64_t)n * hq + kh * G + h) * D + d) = __floats2bfloat162_rn(o0 * inv, o1 * inv);
       }
     }
   }
@@ -508,12 +510,14 @@ static cudaError_t launch_rope_attend_dg(const bf16* qkv, const QkvTable& lookup
                       map, items, a.q_heads, a.kv_heads, a.rms_eps, a.rope_theta, scale, kv_pages, err);
   }
   if (map.seq) return cudaErrorInvalidValue;  // one row per sequence
-  // items that leave SMs idle: eight warps each, so that 128 keys are one round; many: four, four CTAs per SM
-  if (items <= 148)
-    return launch_pdl(rope_attend_kernel<D, G, 8, 1>, dim3(items), dim3(256), 0, s, qkv, lookup, q_norm, k_norm, kv, out, map,
-                      items, a.q_heads, a.kv_heads, a.rms_eps, a.rope_theta, scale, kv_pages, err);
-  return launch_pdl(rope_attend_kernel<D, G, 4, 1>, dim3(items), dim3(128), 0, s, qkv, lookup, q_norm, k_norm, kv, out, map, items,
-                    a.q_heads, a.kv_heads, a.rms_eps, a.rope_theta, scale, kv_pages, err);
+  auto go = [&](auto kernel, int warps) {
+    return launch_pdl(kernel, dim3(items), dim3(warps * 32), 0, s, qkv, lookup, q_norm, k_norm, kv, out, map, items, a.q_heads,
+                      a.kv_heads, a.rms_eps, a.rope_theta, scale, kv_pages, err);
+  };
+  // items that leave SMs idle: eight warps each, so that 128 keys are one round (sixteen would have to spill: 2,282 against
+  // 2,242 us a step of one session, 2,133 against 2,042 us for Higgs at three); more items: four warps, three CTAs an SM
+  // (two warps with more CTAs: 4,485 against 4,024 us at 64 sessions, four CTAs an SM with spills 5,655 against 5,228 at 128)
+  return items <= 148 ? go(rope_attend_kernel<D, G, 8, 1>, 8) : go(rope_attend_kernel<D, G, 4, 1>, 4);
 }
 
 template <int D>
