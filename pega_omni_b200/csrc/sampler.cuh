@@ -54,12 +54,12 @@ __device__ __forceinline__ float philox_uniform(uint64_t seed, uint32_t frame, u
 struct Shared {
   alignas(16) uint32_t hist[4][256];  // one set of digit counters per pass of the k-th key selection
   uint32_t warp_cnt[32];
+  uint32_t warp_max[32], digit_cnt[2][2][32];
   float red[32];
   float wtot[32];
-  float vscan[kVirtualThreads];
   int token, last;
   unsigned long long best;
-  int n_cand;
+  int n_cand, cut;
   alignas(16) int cand_idx[kMaxNucleus];  // 16-byte aligned: the four arrays from here on also stage a row of logits
   float cand_p[kMaxNucleus];
   int sorted_idx[kMaxNucleus];
@@ -80,12 +80,13 @@ struct Params {
   int seen_words;
 };
 
-// Team thread `tid` owns the PER = 4096 / THREADS consecutive logits starting at tid * PER.
-template <int THREADS, typename Sync>
+// Team thread `tid` owns the PER = VOCAB / THREADS consecutive logits starting at tid * PER (VOCAB: the largest vocabulary
+// the team draws from; the virtual threads past it have nothing to add).
+template <int THREADS, typename Sync, int VOCAB = kVocabMax>
 struct Team {
-  static constexpr int PER = kVocabMax / THREADS;
-  static constexpr int VPT = kVirtualThreads / THREADS;  // virtual threads per team thread
-  static_assert(PER % kVirtualPer == 0 && THREADS >= 128 && THREADS <= kVirtualThreads, "team size");
+  static constexpr int PER = VOCAB / THREADS;
+  static constexpr int VPT = PER / kVirtualPer;  // virtual threads per team thread
+  static_assert(PER % kVirtualPer == 0 && VPT >= 1 && THREADS >= 128 && THREADS <= kVirtualThreads, "team size");
   static_assert(32 % PER == 0, "a thread's logits share one word of the seen bitmap");
 
   // The word of the sequence's seen bitmap that covers this thread's logits (0 when nothing is penalised).
@@ -103,6 +104,76 @@ struct Team {
     for (int w = 0; w < THREADS / 32; ++w) m = fmaxf(m, sh.red[w]);
     Sync::sync();
     return m;
+  }
+
+  // From counters of a digit's 256 values: the digit with (keys above it) < left <= (keys at or above it), and in `left`
+  // the rank within that digit. Every warp picks it by itself.
+  static __device__ uint32_t pick_digit(const uint32_t* hist, uint32_t& left, int lane) {
+    uint32_t c[8];
+    *reinterpret_cast<uint4*>(&c[0]) = *reinterpret_cast<const uint4*>(&hist[8 * lane]);
+    *reinterpret_cast<uint4*>(&c[4]) = *reinterpret_cast<const uint4*>(&hist[8 * lane + 4]);
+    uint32_t mine = 0;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) mine += c[j];
+    uint32_t incl = mine;  // keys in this lane's counters and in those of the lanes above it
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t other = __shfl_down_sync(0xffffffffu, incl, o);
+      if (lane + o < 32) incl += other;
+    }
+    uint32_t at_least = incl - mine, digit = 0, new_left = 0;
+    bool found = false;
+#pragma unroll
+    for (int j = 7; j >= 0; --j) {
+      const uint32_t above = at_least;
+      at_least += c[j];
+      if (!found && above < left && at_least >= left) {
+        found = true;
+        digit = 8u * lane + j;
+        new_left = left - above;
+      }
+    }
+    const int src = __ffs(__ballot_sync(0xffffffffu, found)) - 1;  // exactly one lane
+    left = __shfl_sync(0xffffffffu, new_left, src);
+    return __shfl_sync(0xffffffffu, digit, src);
+  }
+
+  // The same for keys of sixteen bits (rows of bf16 logits that no penalty has touched): the upper byte is found by counting
+  // four candidates a round from the largest key's byte down - the bytes of logits a few units wide are two or three - and
+  // the lower byte by one pass over counters, zeroed by the caller before its last barrier.
+  static __device__ uint32_t kth_largest_key16(const uint32_t* key, uint32_t valid, uint32_t k, uint32_t top, int tid, Shared& sh) {
+    const int lane = tid & 31;
+    uint32_t left = k, digit = top >> 8;
+    for (int round = 0;; ++round, digit -= 4) {
+      uint32_t a = 0, b = 0;  // counts of digit, digit - 1 and of digit - 2, digit - 3, sixteen bits each
+#pragma unroll
+      for (int j = 0; j < PER; ++j) {
+        const uint32_t below = valid >> j & 1u ? digit - (key[j] >> 8) : ~0u;
+        a += below == 0u ? 1u : below == 1u ? 0x10000u : 0u;
+        b += below == 2u ? 1u : below == 3u ? 0x10000u : 0u;
+      }
+      a = __reduce_add_sync(0xffffffffu, a), b = __reduce_add_sync(0xffffffffu, b);
+      uint32_t(*cnt)[32] = sh.digit_cnt[round & 1];
+      if (lane == 0) cnt[0][tid >> 5] = a, cnt[1][tid >> 5] = b;
+      Sync::sync();
+      a = __reduce_add_sync(0xffffffffu, lane < THREADS / 32 ? cnt[0][lane] : 0u);
+      b = __reduce_add_sync(0xffffffffu, lane < THREADS / 32 ? cnt[1][lane] : 0u);
+      const uint32_t c[4] = {a & 0xffffu, a >> 16, b & 0xffffu, b >> 16};
+      bool found = false;
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (!found) {
+          if (c[i] >= left) found = true, digit -= i;
+          else left -= c[i];
+        }
+      if (found || round == 64) break;
+    }
+    uint32_t* hist = sh.hist[0];
+#pragma unroll
+    for (int j = 0; j < PER; ++j)
+      if ((valid >> j & 1u) && key[j] >> 8 == digit) atomicAdd(&hist[key[j] & 255u], 1u);
+    Sync::sync();
+    return digit << 8 | pick_digit(hist, left, lane);
   }
 
   // The k-th largest key of the row (ties share it), most significant digit first, eight bits at a time. Logits are
@@ -145,42 +216,15 @@ struct Team {
       for (int j = 0; j < PER; ++j)
         if (tid * PER + j < vocab && ((key[j] ^ prefix) & fixed) == 0) atomicAdd(&hist[(key[j] >> shift) & 255u], 1u);
       Sync::sync();
-      // at_least[d] = keys whose digit is >= d; the digit wanted is the one with at_least - count < left <= at_least
-      uint32_t c[8];
-      *reinterpret_cast<uint4*>(&c[0]) = *reinterpret_cast<const uint4*>(&hist[8 * lane]);
-      *reinterpret_cast<uint4*>(&c[4]) = *reinterpret_cast<const uint4*>(&hist[8 * lane + 4]);
-      uint32_t mine = 0;
-#pragma unroll
-      for (int j = 0; j < 8; ++j) mine += c[j];
-      uint32_t incl = mine;  // keys in this lane's counters and in those of the lanes above it
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t other = __shfl_down_sync(0xffffffffu, incl, o);
-        if (lane + o < 32) incl += other;
-      }
-      uint32_t at_least = incl - mine, digit = 0, new_left = 0;
-      bool found = false;
-#pragma unroll
-      for (int j = 7; j >= 0; --j) {
-        const uint32_t above = at_least;
-        at_least += c[j];
-        if (!found && above < left && at_least >= left) {
-          found = true;
-          digit = 8u * lane + j;
-          new_left = left - above;
-        }
-      }
-      const uint32_t who = __ballot_sync(0xffffffffu, found);  // exactly one lane
-      const int src = __ffs(who) - 1;
-      prefix |= __shfl_sync(0xffffffffu, digit, src) << shift;
-      left = __shfl_sync(0xffffffffu, new_left, src);
+      prefix |= pick_digit(hist, left, lane) << shift;
     }
     return prefix;
   }
 
-  // v: this thread's PER processed logits (-inf beyond the vocabulary).
-  static __device__ int draw(const float* v, int vocab, float temperature, int top_k, float top_p, float u, int tid,
-                             Shared& sh) {
+  // v: this thread's PER processed logits (-inf beyond the vocabulary); `plain`: they are bf16 values as they came. The
+  // caller has a barrier between this call and the next use of `sh`.
+  static __device__ int draw(const float* v, bool plain, int vocab, float temperature, int top_k, float top_p, float u,
+                             int tid, Shared& sh) {
     if (temperature <= 0.f) {  // argmax, lowest index on ties (talker.cu:177-188)
       if (tid == 0) sh.best = 0ull;
       Sync::sync();
@@ -194,21 +238,42 @@ struct Team {
       Sync::sync();
       return token;
     }
-    float x[PER];
-    uint32_t key[PER];
-    float mx = -INFINITY;
-#pragma unroll
-    for (int j = 0; j < PER; ++j) {
-      x[j] = v[j] / temperature;
-      key[j] = order_key(x[j]);
-      mx = fmaxf(mx, x[j]);
-    }
     const int keep = top_k > 0 && top_k < vocab ? top_k : vocab;
-    const float m = team_max(mx, tid, sh);
-    const uint32_t threshold = keep < vocab ? kth_largest_key(key, vocab, (uint32_t)keep, order_key(m) >> 24, tid, sh) : 0u;
     float p[PER];
+    if (plain) {
+      uint32_t key[PER], valid = 0, top = 0;
 #pragma unroll
-    for (int j = 0; j < PER; ++j) p[j] = tid * PER + j < vocab && key[j] >= threshold ? __expf(x[j] - m) : 0.f;
+      for (int j = 0; j < PER; ++j) {
+        key[j] = order_key(v[j]) >> 16;
+        if (tid * PER + j < vocab) valid |= 1u << j, top = max(top, key[j]);
+      }
+      for (int i = tid; i < 256; i += THREADS) sh.hist[0][i] = 0;
+      top = __reduce_max_sync(0xffffffffu, top);
+      if ((tid & 31) == 0) sh.warp_max[tid >> 5] = top;
+      Sync::sync();
+      top = __reduce_max_sync(0xffffffffu, (tid & 31) < THREADS / 32 ? sh.warp_max[tid & 31] : 0u);
+      const float m = __uint_as_float((top & 0x8000u ? top & 0x7fffu : ~top & 0xffffu) << 16) / temperature;
+      const uint32_t threshold = keep < vocab ? kth_largest_key16(key, valid, (uint32_t)keep, top, tid, sh) : 0u;
+#pragma unroll
+      for (int j = 0; j < PER; ++j) {
+        p[j] = 0.f;
+        if ((valid >> j & 1u) && key[j] >= threshold) p[j] = __expf(v[j] / temperature - m);
+      }
+    } else {
+      float x[PER];
+      uint32_t key[PER];
+      float mx = -INFINITY;
+#pragma unroll
+      for (int j = 0; j < PER; ++j) {
+        x[j] = v[j] / temperature;
+        key[j] = order_key(x[j]);
+        mx = fmaxf(mx, x[j]);
+      }
+      const float m = team_max(mx, tid, sh);
+      const uint32_t threshold = keep < vocab ? kth_largest_key(key, vocab, (uint32_t)keep, order_key(m) >> 24, tid, sh) : 0u;
+#pragma unroll
+      for (int j = 0; j < PER; ++j) p[j] = tid * PER + j < vocab && key[j] >= threshold ? __expf(x[j] - m) : 0.f;
+    }
 
     if (top_p < 1.f) {
       // compact the survivors, rank them by (probability desc, index asc), walk the ranking once
@@ -238,20 +303,31 @@ struct Team {
         sh.sorted_idx[rank] = ia;
         sh.sorted_p[rank] = pa;
       }
+      for (int r = nc + tid; r < ((nc + 7) & ~7); r += THREADS) sh.sorted_p[r] = 0.f;
       Sync::sync();
-      if (tid == 0) {
+      if (tid == 0) {  // the masses are added one by one in rank order; only the sums depend on one another
         float tot = 0.f;
-        for (int r = 0; r < nc; ++r) tot += sh.sorted_p[r];
-        float before = 0.f;
-        for (int r = 0; r < nc; ++r) {
-          const float mine = sh.sorted_p[r];
-          if (r > 0 && before >= top_p * tot) {
-            const int idx = sh.sorted_idx[r];
-            sh.drop[idx >> 5] |= 1u << (idx & 31);
-          }
-          before += mine;
+        for (int r = 0; r < nc; r += 8) {
+          const float4 f = *reinterpret_cast<const float4*>(&sh.sorted_p[r]), g = *reinterpret_cast<const float4*>(&sh.sorted_p[r + 4]);
+          tot += f.x, tot += f.y, tot += f.z, tot += f.w, tot += g.x, tot += g.y, tot += g.z, tot += g.w;
         }
+        const float bound = top_p * tot;
+        float before = 0.f;
+        int cut = nc;  // the first rank after the top whose preceding mass reaches the bound; so do all behind it
+        for (int r = 0; r < nc && cut == nc; r += 8) {
+          float f[8];
+          *reinterpret_cast<float4*>(&f[0]) = *reinterpret_cast<const float4*>(&sh.sorted_p[r]);
+          *reinterpret_cast<float4*>(&f[4]) = *reinterpret_cast<const float4*>(&sh.sorted_p[r + 4]);
+#pragma unroll
+          for (int e = 0; e < 8; ++e) {
+            if (cut == nc && r + e > 0 && before >= bound) cut = min(r + e, nc);
+            before += f[e];
+          }
+        }
+        sh.cut = cut;
       }
+      Sync::sync();
+      for (int r = sh.cut + tid; r < nc; r += THREADS) atomicOr(&sh.drop[sh.sorted_idx[r] >> 5], 1u << (sh.sorted_idx[r] & 31));
       Sync::sync();
 #pragma unroll
       for (int j = 0; j < PER; ++j) {
@@ -293,24 +369,23 @@ struct Team {
       for (int q = 0; q < VPT; ++q)
         if (((tid * VPT + q) & 31) >= o) incl[q] += up[q];
     }
-    if (((tid * VPT + VPT - 1) & 31) == 31) sh.vscan[tid * VPT + VPT - 1] = incl[VPT - 1];  // a virtual warp's total
+    const int lane = tid & 31, vw = tid * VPT >> 5;  // a thread's virtual lanes share their virtual warp
+    if (((tid * VPT + VPT - 1) & 31) == 31) sh.wtot[vw] = incl[VPT - 1];
     Sync::sync();
-    if (tid < 32) {  // the same scan over the 32 group totals
-      float wsum = sh.vscan[tid * 32 + 31];
+    // the same scan over the group totals (32 of them; those past VOCAB are empty), by every warp for itself
+    float wsum = lane < THREADS * VPT / 32 ? sh.wtot[lane] : 0.f;
 #pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const float up = __shfl_up_sync(0xffffffffu, wsum, o);
-        if (tid >= o) wsum += up;
-      }
-      sh.wtot[tid] = wsum;
+    for (int o = 1; o < 32; o <<= 1) {
+      const float up = __shfl_up_sync(0xffffffffu, wsum, o);
+      if (lane >= o) wsum += up;
     }
-    Sync::sync();
-    const float total = sh.wtot[31];
+    const float total = __shfl_sync(0xffffffffu, wsum, 31);
+    const float before_me = __shfl_sync(0xffffffffu, wsum, max(vw - 1, 0));
     const float target = u * total;
 #pragma unroll
     for (int q = 0; q < VPT; ++q) {
-      const int vt = tid * VPT + q, vw = vt >> 5;
-      const float before = vw > 0 ? sh.wtot[vw - 1] : 0.f;
+      const int vt = tid * VPT + q;
+      const float before = vw > 0 ? before_me : 0.f;
       float run = before + incl[q] - own[q];
 #pragma unroll
       for (int e = 0; e < kVirtualPer; ++e) {
@@ -324,9 +399,7 @@ struct Team {
       }
     }
     Sync::sync();
-    const int token = sh.token >= 0 ? sh.token : sh.last;
-    Sync::sync();
-    return token;
+    return sh.token >= 0 ? sh.token : sh.last;
   }
 
   // `talker_sample` (talker.cu:259-293) for one row. `load(i, j)` returns logit i = tid * PER + j as f32 (already rounded
@@ -358,7 +431,7 @@ struct Team {
         const uint64_t seed = *reinterpret_cast<const uint64_t*>(seen + prm.seen_words + (prm.seen_words & 1));
         u = philox_uniform(seed, (uint32_t)frame, (uint32_t)prm.group);
       }
-      token = min(max(draw(v, prm.vocab, prm.temperature, prm.top_k, prm.top_p, u, tid, sh), 0), prm.vocab - 1);
+      token = min(max(draw(v, !prm.penalize, prm.vocab, prm.temperature, prm.top_k, prm.top_p, u, tid, sh), 0), prm.vocab - 1);
     }
     Sync::sync();  // every thread has read the bitmap before it changes
     if (tid == 0) {
