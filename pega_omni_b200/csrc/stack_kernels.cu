@@ -3,6 +3,8 @@
 // over the paged KV. Rounding points follow the reference's kernels
 // (crates/omni-qwen3/kernels/qwen3.cu, crates/omni-kern/kernels/common.cuh):
 // every tensor that crosses HBM is bf16, arithmetic is f32.
+#include <type_traits>
+
 #include "attend.cuh"
 #include "decode_attend.cuh"
 #include "kernels.h"
@@ -185,11 +187,22 @@ __device__ __forceinline__ RowAt locate(const RowMap& m, int n) {
   return r;
 }
 
+// A lane's E elements of each half of a head, E = D / 64.
+template <int D>
+__device__ __forceinline__ void st_half(bf16* dst, int lane, const float (&lo)[D / 64], const float (&hi)[D / 64]) {
+  if constexpr (D == 128) {
+    reinterpret_cast<__nv_bfloat162*>(dst)[lane] = __floats2bfloat162_rn(lo[0], lo[1]);
+    reinterpret_cast<__nv_bfloat162*>(dst)[32 + lane] = __floats2bfloat162_rn(hi[0], hi[1]);
+  } else {
+    dst[lane] = __float2bfloat16(lo[0]), dst[32 + lane] = __float2bfloat16(hi[0]);
+  }
+}
+
 // ---- q/k norm + RoPE + KV write -------------------------------------------------
 
 // A CTA per row, a warp per head at a time: a lane's rotation angles depend on the row alone, so they are computed once
 // and serve all the heads the warp takes (a powf and a sincosf per head cost four times the memory traffic:
-// 87 us a layer at 8,700 rows of 32 heads). Semantics of `rope_kv` (qwen3.cu:66-107): RMSNorm over the head, the
+// 87 us a layer at 8,700 rows of 32 heads; 57 us with one head's loads at a time). Semantics of `rope_kv` (qwen3.cu:66-107): RMSNorm over the head, the
 // normalised value rounded to bf16 before the gain, half-rotation rotary embedding with inv_freq = theta^(-2i/D); q stays
 // in place, k and v go to the row's slot.
 template <int D>
@@ -216,22 +229,33 @@ __global__ void __launch_bounds__(256) rope_kv_kernel(bf16* __restrict__ qkv, co
     if (threadIdx.x == 0) raise(err, kErrBadIndex);
     return;
   }
-  for (int head = threadIdx.x >> 5; head < hq + 2 * hk; head += blockDim.x >> 5) {
-    bf16* row = qkv + ((int64_t)n * (hq + 2 * hk) + head) * D;
-    if (head >= hq + hk) {  // V: a plain copy
-      bf16* dst = kv + kv_offset<D>(page, hk, head - hq - hk, 1, tok);
-      if constexpr (E == 2) reinterpret_cast<uint2*>(dst)[lane] = reinterpret_cast<const uint2*>(row)[lane];
-      else reinterpret_cast<uint32_t*>(dst)[lane] = reinterpret_cast<const uint32_t*>(row)[lane];
-      continue;
+  // four heads of a warp at a time: their loads are all under way before the first is used
+  constexpr int B = 4;
+  const int heads = hq + 2 * hk, warps = blockDim.x >> 5;
+  bf16* const row = qkv + (int64_t)n * heads * D;
+  using Half = std::conditional_t<E == 2, uint32_t, uint16_t>;  // a lane's elements of half a head
+  for (int h0 = threadIdx.x >> 5; h0 < heads; h0 += B * warps) {
+    Half raw[B][2];
+#pragma unroll
+    for (int b = 0; b < B; ++b) {
+      const int head = h0 + b * warps;
+      if (head < heads) {
+        const Half* src = reinterpret_cast<const Half*>(row + head * D);
+        raw[b][0] = __ldcg(src + lane), raw[b][1] = __ldcg(src + 32 + lane);
+      }
     }
-    bf16* dst = head < hq ? row : kv + kv_offset<D>(page, hk, head - hq, 0, tok);
-    float lo[E], hi[E];
 #pragma unroll
-    for (int e = 0; e < E; ++e) lo[e] = __bfloat162float(row[lane * E + e]), hi[e] = __bfloat162float(row[D / 2 + lane * E + e]);
-    if (head < hq) rope_head<D>(lo, hi, qlo, qhi, cs, sn, eps);
-    else rope_head<D>(lo, hi, klo, khi, cs, sn, eps);
-#pragma unroll
-    for (int e = 0; e < E; ++e) dst[lane * E + e] = __float2bfloat16(lo[e]), dst[D / 2 + lane * E + e] = __float2bfloat16(hi[e]);
+    for (int b = 0; b < B; ++b) {
+      const int head = h0 + b * warps;
+      if (head >= heads) break;
+      float lo[E], hi[E];
+      lo[0] = __uint_as_float((uint32_t)raw[b][0] << 16), hi[0] = __uint_as_float((uint32_t)raw[b][1] << 16);
+      if constexpr (E == 2) lo[1] = __uint_as_float(raw[b][0] & 0xffff0000u), hi[1] = __uint_as_float(raw[b][1] & 0xffff0000u);
+      if (head < hq) rope_head<D>(lo, hi, qlo, qhi, cs, sn, eps);
+      else if (head < hq + hk) rope_head<D>(lo, hi, klo, khi, cs, sn, eps);
+      bf16* dst = head < hq ? row + head * D : kv + kv_offset<D>(page, hk, (head - hq) % hk, head >= hq + hk, tok);
+      st_half<D>(dst, lane, lo, hi);
+    }
   }
 }
 
@@ -428,12 +452,8 @@ __global__ void __launch_bounds__(W * TEAMS * 32, W == 8 ? 1 : 3)
       else if (job == G) rope_head<D>(lo, hi, kwl, kwh, cs, sn, eps);
       bf16* dst = job < G ? sh.q[job] : job == G ? sh.k[r & 1] : sh.v[r & 1];
       bf16* page = job < G ? nullptr : kv + kv_offset<D>(own, hk, kh, job - G, tok);
-#pragma unroll
-      for (int e = 0; e < E; ++e) {
-        const bf16 a = __float2bfloat16(lo[e]), b = __float2bfloat16(hi[e]);
-        dst[lane * E + e] = a, dst[D / 2 + lane * E + e] = b;
-        if (page) page[lane * E + e] = a, page[D / 2 + lane * E + e] = b;
-      }
+      st_half<D>(dst, lane, lo, hi);
+      if (page) st_half<D>(page, lane, lo, hi);
     }
     team_sync();
     uint4 q[D / 32];
