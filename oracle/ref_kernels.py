@@ -39,8 +39,8 @@ def available() -> bool:
 
 
 def build(force: bool = False) -> bool:
-    """Compiles the cubins if the reference is here; returns whether they exist afterwards."""
-    if not REFERENCE.exists():
+    """Compiles the cubins if the reference's sources are here; returns whether they exist afterwards."""
+    if not all((REFERENCE / rel).exists() for rel in SOURCES.values()):
         return available()
     OUT.mkdir(exist_ok=True)
     for name, rel in SOURCES.items():
