@@ -62,6 +62,27 @@ int32_t omni_op_rope_attend(omni_ops* ctx, void* qkv, const void* q_norm, const 
                             const int32_t* indptr, const int32_t* pages, int32_t rows, int32_t q_heads,
                             int32_t kv_heads, int32_t head_dim, float eps, float theta, void* out);
 
+/* The same for one row per sequence (decode): normed and rotated, written to
+ * the row's slot and attended to in one kernel; qkv is not changed. */
+int32_t omni_op_decode_attend(omni_ops* ctx, const void* qkv, const void* q_norm, const void* k_norm, void* kv,
+                              int32_t kv_pages, const int32_t* pos, const int32_t* slot, const int32_t* indptr,
+                              const int32_t* pages, int32_t rows, int32_t q_heads, int32_t kv_heads, int32_t head_dim,
+                              float eps, float theta, void* out);
+
+/* The GEMM of the kernel chains, which picks its kernel by the row count:
+ * y[rows, N] = x[rows, K] . w[N, K]^T with an optional bias epilogue, or, with
+ * `swiglu`, y[rows, N / 2] = bf16(silu(x . gate^T)) * (x . up^T) for
+ * w = [gate; up] (regrouped by the call). K a multiple of 64. */
+int32_t omni_op_chain_gemm(omni_ops* ctx, const void* w, int32_t N, int32_t K, const void* x, int32_t rows, void* y,
+                           int32_t ldy, const void* bias, int32_t epilogue, int32_t swiglu);
+
+/* A projection, the add + norm behind it and the next projection as the chains
+ * run them (up to 256 rows): s = x . w1^T [rows, D]; res += s (bf16), h =
+ * norm(res) * gain over the unrounded sum (`qwen3_add_norm`, qwen3.cu:37-57);
+ * y[rows, N] = h . w2^T. K and D multiples of 64. */
+int32_t omni_op_chain_norm_gemm(omni_ops* ctx, const void* w1, int32_t D, int32_t K, const void* x, int32_t rows,
+                                void* res, const void* gain, float eps, const void* w2, int32_t N, void* y);
+
 /* `talker_sample` (crates/omni-qwen3-tts/kernels/talker.cu:259-293). state:
  * per-sequence slots of `stride` bytes, each i32 last_frame[16], u32
  * seen[ceil(vocab/32)], then (8-byte aligned) the u64 Philox seed. */
@@ -103,6 +124,11 @@ int32_t omni_op_lm_embed(omni_ops* ctx, const int32_t* ids, const void* text_emb
 int32_t omni_op_lm_rope_attend(omni_ops* ctx, void* qkv, void* kv, int32_t kv_pages, const int32_t* pos,
                                const int32_t* slot, const int32_t* seq, const int32_t* indptr, const int32_t* pages,
                                int32_t rows, int32_t heads, float coef, float scale, int32_t context, void* out);
+
+/* The same for one row per session (decode) in one kernel; qkv is not changed. */
+int32_t omni_op_lm_decode_attend(omni_ops* ctx, const void* qkv, void* kv, int32_t kv_pages, const int32_t* pos,
+                                 const int32_t* slot, const int32_t* indptr, const int32_t* pages, int32_t rows,
+                                 int32_t heads, float coef, float scale, int32_t context, void* out);
 
 /* `lm_dep_embed_norm` (lm.cu:301-313) then `lm_dep_kv_attend` is a separate call below.
  * x = bf16(projected[s][k] + table[drawn[s][k]]), xn = norm(x). */

@@ -7,6 +7,7 @@
 
 #include "../../include/omni_b200.h"
 #include "../../include/omni_b200_ops.h"
+#include "chain.h"
 #include "codec.h"
 #include "gemm.h"
 #include "duplex.h"
@@ -55,6 +56,7 @@ int32_t omni_ops_create(int32_t device, omni_ops** out) {
   OPS_CUDA(c, cudaEventCreate(&c->ev[1]));
   if (tc_init() != 0) return c->fail(OMNI_ERR_CUDA, "cuTensorMapEncodeTiled entry point not found");
   tc_configure();
+  stream_configure();
   c->scratch.partial_floats = (size_t)64 << 20;  // 256 MB of f32 partials: any test shape
   c->scratch.counter_slots = 1 << 16;
   OPS_CUDA(c, cudaMalloc((void**)&c->scratch.partials, c->scratch.partial_floats * 4));
@@ -173,6 +175,74 @@ int32_t omni_op_rope_attend(omni_ops* c, void* qkv, const void* q_norm, const vo
   return OMNI_OK;
 }
 
+int32_t omni_op_decode_attend(omni_ops* c, const void* qkv, const void* q_norm, const void* k_norm, void* kv,
+                              int32_t kv_pages, const int32_t* pos, const int32_t* slot, const int32_t* indptr,
+                              const int32_t* pages, int32_t rows, int32_t q_heads, int32_t kv_heads, int32_t head_dim,
+                              float eps, float theta, void* out) {
+  if (!c || !pos || !slot || !indptr || !pages || rows < 1) return OMNI_ERR_INVALID;
+  RowMap map;
+  map.pos = pos, map.slot = slot, map.indptr = indptr, map.pages = pages;
+  const AttnShape a{q_heads, kv_heads, head_dim, eps, theta};
+  OPS_CUDA(c, launch_rope_attend((const bf16*)qkv, {}, (const bf16*)q_norm, (const bf16*)k_norm, (bf16*)kv, (bf16*)out, map, rows,
+                                 a, kv_pages, c->err, c->stream));
+  return OMNI_OK;
+}
+
+int32_t omni_op_chain_gemm(omni_ops* c, const void* w, int32_t N, int32_t K, const void* x, int32_t rows, void* y,
+                           int32_t ldy, const void* bias, int32_t epilogue, int32_t swiglu) {
+  if (!c || !w || !x || !y || N < 1 || rows < 1 || !stream_supports(N, K, rows)) return OMNI_ERR_INVALID;
+  if (epilogue != OMNI_EPI_NONE && (!bias || swiglu)) return c->fail(OMNI_ERR_INVALID, "epilogue %d needs a bias and no swiglu", epilogue);
+  int launches = 0;
+  ChainPlans plans;
+  const Chain chain{c->stream, c->err, c->sm_count, c->scratch.partials, c->scratch.partial_floats, &launches, &plans};
+  if (!swiglu) {
+    Epilogue epi;
+    epi.bias = static_cast<const bf16*>(bias), epi.kind = epilogue;
+    OPS_CUDA(c, chain.gemm((const bf16*)w, N, K, (const bf16*)x, rows, kStreamBf16, (bf16*)y, ldy, nullptr, 0, epi));
+    return OMNI_OK;
+  }
+  const int granule = stream_granule(N / 2, c->sm_count);
+  if (rows > kChainRows && !wide_fuses(N, K, granule)) return c->fail(OMNI_ERR_UNSUPPORTED, "groups of %d channels do not fill tiles", granule);
+  bf16* grouped = nullptr;
+  OPS_CUDA(c, cudaMalloc((void**)&grouped, (size_t)N * K * sizeof(bf16)));
+  cudaError_t e = launch_interleave_gate_up((const bf16*)w, grouped, N / 2, K, granule, c->stream);
+  if (e == cudaSuccess) e = chain.gemm(grouped, N, K, (const bf16*)x, rows, kStreamSwiglu, (bf16*)y, ldy, nullptr, granule);
+  const cudaError_t done = cudaStreamSynchronize(c->stream);
+  cudaFree(grouped);
+  OPS_CUDA(c, e);
+  OPS_CUDA(c, done);
+  return OMNI_OK;
+}
+
+int32_t omni_op_chain_norm_gemm(omni_ops* c, const void* w1, int32_t D, int32_t K, const void* x, int32_t rows,
+                                void* res, const void* gain, float eps, const void* w2, int32_t N, void* y) {
+  if (!c || !w1 || !x || !res || !gain || !w2 || !y || rows < 1 || rows > kChainRows || !stream_supports(D, K, rows) || D % 64)
+    return OMNI_ERR_INVALID;
+  int launches = 0;
+  ChainPlans plans;
+  const Chain chain{c->stream, c->err, c->sm_count, c->scratch.partials, c->scratch.partial_floats, &launches, &plans};
+  bf16* tmp = nullptr;  // the rows of a norm of its own, the other residual of a folded one
+  const size_t row_bytes = (size_t)rows * D * sizeof(bf16);
+  OPS_CUDA(c, cudaMalloc((void**)&tmp, 2 * row_bytes));
+  bf16 *in = (bf16*)res, *spare = tmp + (size_t)rows * D;
+  Summands sum;
+  FewNorm norm;
+  cudaError_t e = chain.gemm((const bf16*)w1, D, K, (const bf16*)x, rows, kStreamPartials, nullptr, D, &sum);
+  norm.kind = kNormStack, norm.sum = sum, norm.gain = (const bf16*)gain, norm.eps = eps;
+  if (e == cudaSuccess)
+    e = chain.norm_gemm(norm, &in, &spare,
+                        [&](const Summands& from, bf16* r) {
+                          return launch_add_norm_sum(from, r, (const bf16*)gain, tmp, rows, D, eps, 1, 0, c->stream);
+                        },
+                        (const bf16*)w2, N, D, tmp, rows, kStreamBf16, (bf16*)y, N);
+  if (e == cudaSuccess && in != (bf16*)res) e = cudaMemcpyAsync(res, in, row_bytes, cudaMemcpyDeviceToDevice, c->stream);
+  const cudaError_t done = cudaStreamSynchronize(c->stream);
+  cudaFree(tmp);
+  OPS_CUDA(c, e);
+  OPS_CUDA(c, done);
+  return OMNI_OK;
+}
+
 int32_t omni_op_sample(omni_ops* c, const void* logits, int32_t vocab, float temperature, int32_t top_k, float top_p,
                        float penalty, int32_t suppress_lo, int32_t suppress_hi, int32_t exempt, int32_t min_frames,
                        const int32_t* frames, const float* uniforms, const int32_t* force, void* state,
@@ -236,6 +306,15 @@ int32_t omni_op_lm_rope_attend(omni_ops* c, void* qkv, void* kv, int32_t kv_page
   OPS_CUDA(c, launch_lm_rope_kv((bf16*)qkv, pos, slot, kv, rows, heads, coef, kv_pages, c->err, c->stream));
   OPS_CUDA(c, launch_lm_attend((const bf16*)qkv, kv, pos, seq, indptr, pages, (bf16*)out, rows, heads, scale, context,
                                kv_pages, c->err, c->stream));
+  return OMNI_OK;
+}
+
+int32_t omni_op_lm_decode_attend(omni_ops* c, const void* qkv, void* kv, int32_t kv_pages, const int32_t* pos,
+                                 const int32_t* slot, const int32_t* indptr, const int32_t* pages, int32_t rows,
+                                 int32_t heads, float coef, float scale, int32_t context, void* out) {
+  if (!c || !qkv || !kv || !pos || !slot || !indptr || !pages || !out || rows < 1) return OMNI_ERR_INVALID;
+  OPS_CUDA(c, launch_lm_rope_attend((const bf16*)qkv, kv, pos, slot, indptr, pages, (bf16*)out, rows, heads, coef, scale, context,
+                                    kv_pages, c->err, c->stream));
   return OMNI_OK;
 }
 

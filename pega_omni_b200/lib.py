@@ -124,6 +124,9 @@ SYMBOLS = {
     "omni_op_silu_mul": (I32, [VP, VP, VP, I32, I32]),
     "omni_op_rope_attend": (I32, [VP, VP, VP, VP, VP, I32, VP, VP, VP, VP, VP, I32, I32, I32, I32, C.c_float,
                                   C.c_float, VP]),
+    "omni_op_decode_attend": (I32, [VP, VP, VP, VP, VP, I32, VP, VP, VP, VP, I32, I32, I32, I32, C.c_float, C.c_float, VP]),
+    "omni_op_chain_gemm": (I32, [VP, VP, I32, I32, VP, I32, VP, I32, VP, I32, I32]),
+    "omni_op_chain_norm_gemm": (I32, [VP, VP, I32, I32, VP, I32, VP, VP, C.c_float, VP, I32, VP]),
     "omni_op_sample": (I32, [VP, VP, I32, C.c_float, I32, C.c_float, C.c_float, I32, I32, I32, I32, VP, VP, VP, VP,
                              VP, C.c_int64, I32, I32, VP, I32, I32]),
     "omni_op_gemm_noalloc": (I32, [VP, I32, I32, VP, I32, VP, I32, I32, VP, I32, VP, C.c_char_p, C.c_size_t]),
@@ -131,6 +134,7 @@ SYMBOLS = {
     "omni_op_lm_tp_add_norm": (I32, [VP, VP, VP, VP, VP, VP, I32, I32, C.c_float, VP]),
     "omni_op_lm_embed": (I32, [VP, VP, VP, I32, VP, I32, VP, I32, I32]),
     "omni_op_lm_rope_attend": (I32, [VP, VP, VP, I32, VP, VP, VP, VP, VP, I32, I32, C.c_float, C.c_float, I32, VP]),
+    "omni_op_lm_decode_attend": (I32, [VP, VP, VP, I32, VP, VP, VP, VP, I32, I32, C.c_float, C.c_float, I32, VP]),
     "omni_op_lm_dep_embed_norm": (I32, [VP, VP, I32, VP, I32, VP, VP, VP, VP, I32, I32, C.c_float]),
     "omni_op_lm_dep_kv_attend": (I32, [VP, VP, VP, I32, VP, I32, I32, C.c_float]),
     "omni_op_lm_sample": (I32, [VP, VP, I32, C.c_int64, C.c_float, I32, VP, VP, I32, VP, I32]),

@@ -74,6 +74,20 @@ class Ops:
                                                   _p(slot), _p(seq), _p(indptr), _p(pages), qkv.shape[0], hq, hk, d,
                                                   eps, theta, _p(out)))
 
+    def decode_attend(self, qkv, q_norm, k_norm, kv, kv_pages, pos, slot, indptr, pages, hq, hk, d, eps, theta, out):
+        self._check(self._lib.omni_op_decode_attend(self._h, _p(qkv), _p(q_norm), _p(k_norm), _p(kv), kv_pages, _p(pos),
+                                                    _p(slot), _p(indptr), _p(pages), qkv.shape[0], hq, hk, d, eps, theta,
+                                                    _p(out)))
+
+    def chain_gemm(self, w, x, y, bias=None, epilogue=0, swiglu=False):
+        n, k = w.shape
+        self._check(self._lib.omni_op_chain_gemm(self._h, _p(w), n, k, _p(x), x.shape[0], _p(y), y.stride(0), _p(bias),
+                                                 epilogue, int(swiglu)))
+
+    def chain_norm_gemm(self, w1, x, res, gain, eps, w2, y):
+        self._check(self._lib.omni_op_chain_norm_gemm(self._h, _p(w1), w1.shape[0], w1.shape[1], _p(x), x.shape[0],
+                                                      _p(res), _p(gain), eps, _p(w2), w2.shape[0], _p(y)))
+
     def sample(self, logits, temperature, top_k, top_p, penalty, suppress_lo, suppress_hi, exempt, min_frames, frames,
                uniforms, force, state, lines, stride, penalize, philox, codes, group):
         rows, vocab = logits.shape
@@ -102,6 +116,10 @@ class Ops:
         self._check(self._lib.omni_op_lm_rope_attend(self._h, _p(qkv), _p(kv), kv_pages, _p(pos), _p(slot), _p(seq),
                                                      _p(indptr), _p(pages), qkv.shape[0], heads, coef, scale, context,
                                                      _p(out)))
+
+    def lm_decode_attend(self, qkv, kv, kv_pages, pos, slot, indptr, pages, heads, coef, scale, context, out):
+        self._check(self._lib.omni_op_lm_decode_attend(self._h, _p(qkv), _p(kv), kv_pages, _p(pos), _p(slot), _p(indptr),
+                                                       _p(pages), qkv.shape[0], heads, coef, scale, context, _p(out)))
 
     def lm_dep_embed_norm(self, projected, k, table, drawn, alpha, x, xn, eps):
         rows, dim = x.shape

@@ -1,0 +1,223 @@
+"""The kernels of the decode chains and of the prompts, at the sizes where they can go wrong: the row counts at which
+another kernel takes over, ragged tiles and K splits, the smallest and largest team of an attention item. Products are
+checked against fp32 torch, attention in one kernel against the separate rotation and attention kernels."""
+import dataclasses
+
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ops(built_lib):
+    from pega_omni_b200.ops import Ops
+    o = Ops(0)
+    yield o
+    o.close()
+
+
+def rand(shape, seed, scale=1.0):
+    g = torch.Generator(device="cuda")
+    g.manual_seed(seed)
+    return (torch.randn(shape, generator=g, device="cuda") * scale).to(torch.bfloat16)
+
+
+def close(got, want, steps=2.0, floor=0.05):
+    """Within `steps` bf16 steps of the fp32 value; `floor`: the size of what was rounded on the way, where sums cancel."""
+    g, w = got.float(), want.float()
+    bad = (g - w).abs() > steps * 2.0 ** -7 * w.abs().clamp_min(floor)
+    assert not bad.any(), (int(bad.sum()), float((g - w).abs().max()))
+
+
+def product(x, w):
+    return x.float() @ w.float().T
+
+
+def i32(v):
+    return torch.tensor(v, dtype=torch.int32, device="cuda")
+
+
+# rows: one and two 8-row tiles of the warp-level kernel, then tcgen05 with M = 64, 128, two row tiles, SM pairs
+@pytest.mark.parametrize("rows", [1, 7, 8, 9, 16, 17, 64, 65, 128, 129, 256, 257, 300])
+@pytest.mark.parametrize("n,k,epilogue", [(200, 128, 0), (1000, 1088, 1), (4096, 64, 2), (24, 6144, 0)])
+def test_chain_gemm(ops, rows, n, k, epilogue):
+    w, x, bias = rand((n, k), 1, k ** -0.5), rand((rows, k), 2), rand((n,), 3)
+    y = torch.full((rows + 1, n), 7.0, dtype=torch.bfloat16, device="cuda")
+    torch.cuda.synchronize()
+    ops.chain_gemm(w, x, y[:rows], bias=bias if epilogue else None, epilogue=epilogue)
+    ops.sync()
+    want = product(x, w).bfloat16().float()
+    if epilogue:
+        want = (want + bias.float()).bfloat16().float()
+    if epilogue == 2:
+        want = torch.nn.functional.silu(want)
+    close(y[:rows], want, floor=4.0 if epilogue else 0.05)
+    assert (y[rows] == 7.0).all()  # nothing past the last row
+
+
+@pytest.mark.parametrize("rows", [1, 9, 17, 128, 129, 257])
+@pytest.mark.parametrize("inter,k", [(256, 64), (3072, 1024), (4096, 576)])
+def test_chain_swiglu(ops, rows, inter, k):
+    """The last group of gate and up rows may be smaller than the others."""
+    w, x = rand((2 * inter, k), 4, k ** -0.5), rand((rows, k), 5)
+    y = torch.zeros((rows, inter), dtype=torch.bfloat16, device="cuda")
+    torch.cuda.synchronize()
+    ops.chain_gemm(w, x, y, swiglu=True)
+    ops.sync()
+    gate, up = product(x, w[:inter]).bfloat16().float(), product(x, w[inter:]).bfloat16().float()
+    close(y, torch.nn.functional.silu(gate).bfloat16().float() * up, steps=3.0)
+
+
+@pytest.mark.parametrize("rows", [1, 2, 4, 5, 8, 9, 17, 130, 256])
+@pytest.mark.parametrize("d,k,n", [(1024, 3072, 512), (2560, 64, 200), (64, 2048, 96), (4096, 128, 64)])
+def test_chain_norm_gemm(ops, rows, d, k, n):
+    """Split sums, the add + norm over them (folded into the next product or on its own) and that product."""
+    w1, x, res, gain = rand((d, k), 6, k ** -0.5), rand((rows, k), 7), rand((rows, d), 8), rand((d,), 9, 0.2) + 1
+    w2, y = rand((n, d), 10, d ** -0.5), torch.zeros((rows, n), dtype=torch.bfloat16, device="cuda")
+    v = product(x, w1).bfloat16().float() + res.float()
+    h = (v * torch.rsqrt((v * v).mean(1, keepdim=True) + 1e-6) * gain.float()).bfloat16()
+    torch.cuda.synchronize()
+    ops.chain_norm_gemm(w1, x, res, gain, 1e-6, w2, y)
+    ops.sync()
+    close(res, v, floor=4.0)
+    close(y, product(h, w2), floor=4.0)
+
+
+def paged(lens, seed, spare=3):
+    """Shuffled pages of sequences that hold lens[s] tokens: (pos, slot, indptr, pages, page count)."""
+    rng = np.random.default_rng(seed)
+    count = sum((n + 15) // 16 for n in lens) + spare
+    perm, at = rng.permutation(count), 0
+    pos, slot, indptr, pages = [], [], [0], []
+    for n in lens:
+        mine = [int(p) for p in perm[at:at + (n + 15) // 16]]
+        at += len(mine)
+        pages += mine
+        indptr.append(len(pages))
+        pos.append(n - 1)
+        slot.append(mine[(n - 1) // 16] * 16 + (n - 1) % 16)
+    return i32(pos), i32(slot), i32(indptr), i32(pages), count
+
+
+# up to 148 (sequence, kv head) items a team has eight warps, beyond that four
+@pytest.mark.parametrize("hq,hk,d", [(16, 8, 128), (4, 4, 64), (5, 1, 128), (8, 2, 64), (8, 1, 128)])
+@pytest.mark.parametrize("sessions", [1, 40, 160])
+def test_decode_attention_in_one_kernel(ops, hq, hk, d, sessions):
+    lens = [[1, 16, 17, 129, 300][s % 5] for s in range(sessions)]
+    pos, slot, indptr, pages, count = paged(lens, sessions)
+    qkv, qn, kn = rand((sessions, (hq + 2 * hk) * d), 11), rand((d,), 12, 0.2) + 1, rand((d,), 13, 0.2) + 1
+    kv = rand((count, hk, 2, 16, d), 14)
+    a, b = (torch.zeros((sessions, hq * d), dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    kv_b, qkv_b = kv.clone(), qkv.clone()
+    torch.cuda.synchronize()
+    ops.decode_attend(qkv, qn, kn, kv, count, pos, slot, indptr, pages, hq, hk, d, 1e-6, 1e6, a)
+    ops.rope_attend(qkv_b, qn, kn, kv_b, count, pos, slot, None, indptr, pages, hq, hk, d, 1e-6, 1e6, b)
+    ops.sync()
+    assert torch.equal(kv, kv_b)
+    close(a, b, steps=1.5, floor=0.25)
+
+
+@pytest.mark.parametrize("heads,sessions", [(4, 1), (4, 37), (32, 5), (16, 16)])
+def test_fp8_ring_attention_in_one_kernel(ops, heads, sessions):
+    """Positions before, at and past the end of a ring of 40 tokens."""
+    context, per = 40, 3
+    rng = np.random.default_rng(heads + sessions)
+    pages = rng.permutation(sessions * per)
+    at = [[0, 15, 16, 39, 40, 55, 131][s % 7] for s in range(sessions)]
+    slot = [int(pages[s * per + (p % context) // 16]) * 16 + p % context % 16 for s, p in enumerate(at)]
+    block = heads * (2 * 16 * 128 + 2 * 16 * 4)
+    kv = torch.zeros(sessions * per, block, dtype=torch.uint8, device="cuda")
+    coef, scale = float(np.float32(-np.log(10000.0) * 2.0 / 128)), 128 ** -0.5
+    indptr, table = i32([s * per for s in range(sessions + 1)]), i32(pages.tolist())
+    for p in range(context):  # fills the rings through the separate kernels
+        qkv = rand((sessions, 3 * heads * 128), 100 + p)
+        where = i32([int(pages[s * per + p // 16]) * 16 + p % 16 for s in range(sessions)])
+        out = torch.zeros((sessions, heads * 128), dtype=torch.bfloat16, device="cuda")
+        torch.cuda.synchronize()
+        ops.lm_rope_attend(qkv, kv, sessions * per, i32([p] * sessions), where, None, indptr, table, heads, coef, scale, context, out)
+        ops.sync()
+    qkv = rand((sessions, 3 * heads * 128), 99)
+    qkv_b, kv_b = qkv.clone(), kv.clone()
+    a, b = (torch.zeros((sessions, heads * 128), dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    torch.cuda.synchronize()
+    ops.lm_decode_attend(qkv, kv, sessions * per, i32(at), i32(slot), indptr, table, heads, coef, scale, context, a)
+    ops.lm_rope_attend(qkv_b, kv_b, sessions * per, i32(at), i32(slot), None, indptr, table, heads, coef, scale, context, b)
+    ops.sync()
+    assert torch.equal(kv, kv_b)
+    close(a, b, steps=1.5, floor=0.25)
+
+
+@pytest.mark.parametrize("vocab", [1, 2047, 2048, 2049, 32768, 40001])
+def test_duplex_sampler_takes_the_largest(ops, vocab):
+    """top_k = 1 leaves the largest logit whatever the noise, at both ends of each register budget."""
+    rows = 5
+    logits = rand((rows, vocab), vocab, 3.0)
+    top = torch.randint(0, vocab, (rows,), generator=torch.Generator().manual_seed(vocab))
+    logits[torch.arange(rows), top.cuda()] = 40.0
+    force = torch.full((rows, 9), -1, dtype=torch.int32, device="cuda")
+    force[2, 3] = 0
+    drawn = torch.full((rows, 9), -7, dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    ops.lm_sample(logits, 0.8, 1, force, i32([[r, 7] for r in range(rows)]), 3, drawn)
+    ops.sync()
+    want = top.clone()
+    want[2] = 0
+    assert drawn[:, 3].cpu().tolist() == want.tolist()
+
+
+# 96 channels take zero-filled boxes; one stream leaves most of a 128-row tile empty; 70 streams fill several tiles
+@pytest.mark.parametrize("n", [1, 3, 70])
+@pytest.mark.parametrize("T,C,N,taps,dil,kind", [(4, 4096, 64, 1, 1, 1), (32, 128, 256, 7, 9, 2), (160, 192, 200, 7, 3, 0),
+                                                 (128, 96, 96, 7, 1, 2), (2, 64, 24, 1, 1, 0), (64, 96, 96, 1, 1, 1)])
+def test_codec_conv(ops, n, T, C, N, taps, dil, kind):
+    P = (taps - 1) * dil + T
+    w, x, bias = rand((N, taps * C), 20, (taps * C) ** -0.5), rand((n, P, C), 21), rand((N,), 22)
+    y = rand((n * T, N), 23)
+    alpha, inv_b = torch.rand(N, device="cuda") + 0.5, torch.rand(N, device="cuda") + 0.5
+    cols = torch.stack([x[:, j * dil:j * dil + T] for j in range(taps)], 2).reshape(n * T, taps * C)
+    want = product(cols, w)
+    if kind == 1:
+        want = want + y.float()
+    if kind == 2:
+        want = want.bfloat16().float() + bias.float()
+        want = want + inv_b * torch.sin(alpha * want) ** 2
+    torch.cuda.synchronize()
+    ops.codec_conv(w, C, taps, dil, x, T, n, y, epilogue=kind, bias=bias, alpha=alpha, inv_b=inv_b)
+    ops.sync()
+    close(y, want, floor=4.0)
+
+
+@pytest.mark.parametrize("sessions", [1, 5, 20])
+def test_talker_as_a_chain_agrees_with_per_op_kernels(built_lib, sessions):
+    """Stacks too large for the L2 run as chains: forced frames give the logits of the per-op kernels."""
+    from pega_omni_b200.config import presets
+    from pega_omni_b200.model import Draw, Limits, Model, Prompt
+    from pega_omni_b200.synthetic import random_checkpoint
+    base = presets["mid"]()
+    cfg = dataclasses.replace(base, talker=dataclasses.replace(base.talker, hidden_size=1024, intermediate_size=3072,
+                                                               num_hidden_layers=6, num_attention_heads=16,
+                                                               num_key_value_heads=8, head_dim=128))
+    ck = random_checkpoint(cfg, seed=3, device="cuda")
+    rng = np.random.default_rng(sessions)
+    lens = [9 + (31 * s) % 90 for s in range(sessions)]
+    prompts = [Prompt(list(rng.integers(0, cfg.text_vocab_size, n)), [-1] * n) for n in lens]
+    hi = min(cfg.talker.vocab_size - cfg.control_tokens, cfg.predictor.vocab_size)
+    forced = rng.integers(0, hi, (4, sessions, 16)).astype(np.int32)
+    forced[:, :, cfg.num_code_groups:] = 0
+    got = []
+    for tick_kernel in (True, False):
+        m = Model.load(0, ck, cfg, Limits(max_batch=max(sessions, 8), max_tokens=2048, kv_gib=0.5), tick_kernel=tick_kernel)
+        seqs, rows = [m.open(n, 8) for n in lens], []
+        for t in range(4):
+            draws = [Draw([0.5] * 16, list(forced[t, s])) for s in range(sessions)]
+            out = m.start(list(zip(seqs, prompts, draws))) if t == 0 else m.step(list(zip(seqs, draws)))
+            assert (out.codes == forced[t]).all()
+            rows.append(np.stack([np.concatenate([m.talker_logits(s), m.predictor_logits(s).ravel()]) for s in range(sessions)]))
+        assert m.stats().last_call_launches > 1
+        got.append(np.stack(rows))
+        m.close()
+    a, b = got
+    step = np.exp2(np.floor(np.log2(np.maximum(np.abs(b), 2.0))) - 7)
+    assert float((np.abs(a - b) / step).max()) <= 2.0
