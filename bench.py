@@ -819,7 +819,8 @@ def main():
     if rank == 0:
         peak, peak_kind = measured_peaks()
         mean_len = float(np.mean(lens)) + 1
-        weight_bytes = cfg.tick_weight_bytes() - (cfg.tick_folded_bytes(n) if launches_per_tick <= 2 else 0)
+        folded = launches_per_tick <= 2 or not args.per_op  # the persistent kernel and the chains read the folded tables
+        weight_bytes = cfg.tick_weight_bytes() - (cfg.tick_folded_bytes(n) if folded else 0)
         tick_bytes = weight_bytes + cfg.talker.kv_bytes_per_token() * n * (mean_len + 1)
         tick_s = elapsed / K
         # two more readings of the same time: against the nominal 8 TB/s, and counting the predictor's weights once per tick
@@ -827,9 +828,10 @@ def main():
         p_cfg, t_cfg = cfg.predictor, cfg.talker
         per_pass = p_cfg.num_hidden_layers * p_cfg.layer_weight_bytes() + 2 * p_cfg.hidden_size * t_cfg.hidden_size
         once_bytes = tick_bytes - (cfg.num_code_groups - 2) * per_pass
-        # the dominant kernel IS the tick: one persistent cooperative launch per step (or, with --per-op, the graph)
+        # the unit is the tick: one graph of a kernel chain, one persistent launch, or, with --per-op, the per-op graph
         roof = {"bound": "hbm", "kernel": ("tick_kernel (one launch = one decode tick)" if launches_per_tick == 1 else
-                           "tick_kernel + pred_kernel" if launches_per_tick == 2 else "per-op graph"),
+                           "tick_kernel + pred_kernel" if launches_per_tick == 2 else
+                           "per-op graph" if args.per_op else "kernel chain (one graph = one decode tick)"),
                 "achieved": tick_bytes / tick_s / 1e9, "peak": peak, "unit": "GB/s",
                 "frac": tick_bytes / tick_s / 1e9 / peak, "peak_source": f"of {peak_kind}",
                 "frac_nominal": tick_bytes / tick_s / 1e9 / 8000.0, "peak_nominal": 8000.0,
@@ -851,7 +853,7 @@ def main():
                        "step": "one decode tick = 64 frames per GPU", "positions": [lens[0], lens[-1]],
                        "parallelism": f"{world} replica(s), sessions round-robin, no collective",
                        "l2": "each tick streams 5.3 GB of weights, far larger than the 126 MB L2",
-                       "engine": "persistent tick kernel" if launches_per_tick == 1 else "persistent talker kernel + cluster predictor kernel" if launches_per_tick == 2 else "per-op CUDA graph"},
+                       "engine": "persistent tick kernel" if launches_per_tick == 1 else "persistent talker kernel + cluster predictor kernel" if launches_per_tick == 2 else "per-op CUDA graph" if args.per_op else "kernel chain"},
             "tick_p99_ms": float(t_p99.item()), "tick_p50_ms": float(np.percentile(tick_ms, 50)),
             "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": int(h2d), "d2h_bytes_per_step": int(d2h),
                     "timing": "wall clock around K steps through the C ABI, each staging its draws from host memory and reading its frame back; "

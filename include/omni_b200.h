@@ -90,8 +90,10 @@ typedef struct omni_talker_config {
   double kv_gib;          /* Limits::kv_gib: talker KV pool size */
   int32_t use_graphs;     /* 1: one CUDA graph per batch bucket per program; 0: eager launches */
   int32_t gemm_path;      /* 0: auto (vector GEMV for few rows, tcgen05 tiles otherwise); 1: GEMV only */
-  int32_t tick_kernel;    /* 1: run each graph program as ONE persistent cooperative kernel (phase list with grid
-                             barriers, weights streamed across phase boundaries) when the shapes allow it;
+  int32_t tick_kernel;    /* 1: run each graph program as a chain of kernels under programmatic dependent launch where
+                             the two stacks hold more than the 126 MB of L2, else as ONE persistent cooperative kernel
+                             (phase list with grid barriers, weights streamed across phase boundaries) when the shapes
+                             allow it;
                              3: the same for the talker step, then ONE launch of thread-block clusters for the code
                              predictor's sub-steps (sessions dealt to clusters of 16 CTAs that never talk to one
                              another; measured slower than 1 on B200 at every session count, kept as an option);

@@ -6,8 +6,10 @@
 // needs to itself: its eighth of K, its own ring of weight blocks, its rows of x, so that only the final sum over the
 // eight warps crosses a barrier. One m16n8k16 takes 2 cycles of the SM's pipe, which is ten times the rate at which DRAM
 // delivers weights, and up to sixteen rows there is nothing for a larger tile to reuse.
-// The add + norm before a projection is made by every CTA from the summands (L2 broadcast reads, 16 KB to 100 KB), which
-// takes about 1 us where a kernel of its own takes 2.7.
+// The add + norm before a projection is made by every CTA from the summands (L2 broadcast reads, 16 KB to 100 KB) while
+// two pieces a lane suffice; a kernel of its own takes 2.7 us and beyond two pieces is faster. Measured as nodes of a chain
+// at one row: 1,024 x 3,072 2.5 us, 6,144 x 1,024 with norm and SwiGLU 4.7 us, 4,096 x 1,024 with norm 4.3 us (4.5 to
+// 5.3 us and 2.7 us for the norm with the tcgen05 kernel of stream_gemm.cu).
 #include "few_rows.h"
 
 #include <algorithm>

@@ -5,9 +5,10 @@
 // turn, and rows outside the run (or keys past a row's position) are masked. Value semantics of `attend`
 // (crates/omni-qwen3/kernels/qwen3.cu:123-207): f32 scores, online softmax in f32; a probability enters the second product
 // as the sum of two bf16 (its rounding and the remainder), which keeps 16 bits of it.
-// Measured at 8,700 rows of 28 ragged prompts, D = 128, G = 2: 146 us a layer, before page numbers were read a tile ahead (scalar multiply-adds, each row reading its
-// keys for itself: 1,184 us). Three CTAs an SM with fewer registers are no faster. Bound by shared-memory reads (each warp reads the 16 KB of a stage for its sixteen rows: 512 cycles per 64 x 32 tile at
-// G = 2 against 400 of the MMAs).
+// Measured at 8,700 rows of 28 ragged prompts, D = 128, G = 2: 146 us a layer, before page numbers were read a tile ahead
+// (scalar multiply-adds, each row reading its keys for itself: 1,184 us). Three CTAs an SM with fewer registers are no
+// faster. Bound by shared-memory reads (each warp reads the 16 KB of a stage for its sixteen rows: 512 cycles per 64 x 32
+// tile at G = 2 against 400 of the MMAs).
 #pragma once
 #include "attend.cuh"
 #include "pdl.cuh"
