@@ -13,6 +13,7 @@
 #include "few_rows.h"
 
 #include <algorithm>
+#include <cmath>
 #include <type_traits>
 
 #include "pdl.cuh"
@@ -354,6 +355,42 @@ static int few_rounds(int nkb, int splits, int rows) {
 
 bool few_norm_fits(int K, int rows) { return rows <= kFewNormRows && K % kKb == 0 && few_rounds(K / kKb, 1, rows) <= kNormChunks; }
 
+// R weight rows a CTA, K in `splits`: what fits into shared memory and what it would cost (us behind the rows' arrival).
+struct FewShape {
+  int R, splits, slots;
+  size_t smem;
+  double cost, even;  // even: by the busiest SM's weights and rows alone
+  bool early;         // most of every warp's share is under way before the rows are there
+};
+
+// Fitted to a sweep of R and the splits over nine shapes from 2,048 x 2,048 to 4,096 x 11,264 at one to sixteen rows. The
+// terms: DRAM, less what the rings hold before the rows are there and more where CTAs are fewer than SMs; an SM's copies at
+// 0.1 us each; a warp's chain of blocks, a round trip each unless the ring is deeper (one slot also adds to DRAM, as
+// nothing is under way while a warp works); the rows' bytes. Against the most even load alone: 12,288 x 4,096 19.7 ->
+// 14.7 us, 4,096 x 4,096 9.1 -> 6.8, 2,560 x 9,728 10.4 -> 8.4.
+static FewShape few_shape(int N, int K, int rows, int R, int splits, int sm_count) {
+  FewShape f{R, splits, 0, 0, 1e30, 1e30, false};
+  const int nkb = K / kKb, per = few_per(nkb, splits), level = kWarps * R * kKb * 2;
+  const int x_bytes = kWarps * rows * (per * kKb + 8) * 2;
+  if (x_bytes > 72 * 1024) return f;
+  f.slots = std::min(per, kFewSlots);
+  if (1024 + x_bytes + f.slots * level > kFewMaxSmem) f.slots = std::max(1, (kFewHalf - 1024 - x_bytes) / level);
+  if (1024 + x_bytes + f.slots * level > kFewMaxSmem) return f;
+  f.smem = std::max<size_t>(kFewMinSmem, 1024 + (size_t)x_bytes + (size_t)f.slots * level);
+  const double ctas = (N + R - 1) / R * splits, sms = sm_count, resident = f.smem <= kFewHalf ? 2 : 1;
+  const double dram = 2.0 * N * K / 6.8e6 * std::max(1.0, sms / ctas) * (per <= f.slots ? 0.5 : 1.0);
+  const double copies = ctas * kWarps * per / sms * 0.1;
+  const double chain = per <= f.slots ? 0.2 * per : per * (0.55 + 0.0088 * R) / f.slots;
+  const double x = rows * 2.0 * K / splits / 31e3 * std::ceil(std::min(ctas, resident * sms) / sms);
+  // where the norm behind the product is folded into the next one, all of its CTAs read every sum
+  const double sums = 0.15 * splits + (splits > 1 && few_norm_fits(N, rows) ? 4.0 * splits * rows * N / 150e3 : 0.0);
+  f.cost = std::max({dram, copies, chain}) + (f.slots == 1 && per > 1 ? 0.35 * std::min(dram, chain) : 0.0);
+  f.cost = f.cost * (ctas > resident * sms ? 1.1 : 1.0) + x + sums + 0.02 * copies;
+  f.even = std::ceil(ctas / sms) * (R * 2.0 * K / splits / 44e3 + rows * 2.0 * K / splits / 31e3) + sums;
+  f.early = 2 * per <= 3 * f.slots;
+  return f;
+}
+
 int few_plan(FewPlan* plan, const bf16* w, int N, int K, const bf16* x, int rows, int out, bf16* y, int ldy, float* part,
              Epilogue epi, int sm_count, int granule) {
   if (rows < 1 || rows > 16 || K % kKb || N < 1) return -2;
@@ -362,34 +399,30 @@ int few_plan(FewPlan* plan, const bf16* w, int N, int K, const bf16* x, int rows
   if ((reinterpret_cast<uintptr_t>(w) & 15) || (reinterpret_cast<uintptr_t>(x) & 15)) return -3;
   FewPlan& p = *plan;
   p.N = N, p.K = K, p.rows = rows, p.out = out, p.x = x, p.y = y, p.ldy = ldy, p.part = part, p.epi = epi;
-  const int nkb = K / kKb, most = rows > 8 ? 64 : 160;
-  auto x_bytes = [&](int S) {
-    return kWarps * rows * (few_per(nkb, S) * kKb + 8) * 2;
-  };
+  const int most = rows > 8 ? 64 : 160;
+  FewShape best{};
+  best.cost = 1e30;
   if (out == kStreamSwiglu) {
-    p.R = 2 * granule, p.splits = 1;
-    if (p.R > most) return -2;
+    if (2 * granule > most) return -2;
+    best = few_shape(N, K, rows, 2 * granule, 1, sm_count);
   } else {
-    // the most even load of weights on the SMs, then the fewest sums for the consumer to add
-    double best = 1e30;
+    // The most even load of weights and rows, whose tiles are narrow and leave little to do behind the wait, where it has
+    // most of every warp's share in its ring by then; otherwise by cost.
+    FewShape even = best;
+    even.even = 1e30;
     for (int R = 16; R <= most; R += 16)
       for (int S : {1, 2, 4}) {
-        if (S > 1 && (out != kStreamPartials || S * kWarps > nkb)) break;
-        if (x_bytes(S) > 64 * 1024) continue;
-        const double waves = ((N + R - 1) / R * S + sm_count - 1) / sm_count;
-        const double cost = waves * R * 2.0 * K / S / 44e3 + waves * rows * 2.0 * K / S / 150e3 + 0.15 * S + (S > 1 ? 4.0 * S * rows * N / 150e3 : 0.0);
-        if (cost < best) best = cost, p.R = R, p.splits = S;
+        if (S > 1 && (out != kStreamPartials || S * kWarps > K / kKb)) break;
+        const FewShape shape = few_shape(N, K, rows, R, S, sm_count);
+        if (shape.cost < best.cost) best = shape;
+        if (shape.even < even.even) even = shape;
       }
-    if (best > 1e29) return -2;
+    if (even.early) best = even;
   }
-  const int xb = x_bytes(p.splits), level = kWarps * p.R * 128;
-  const int per = few_per(nkb, p.splits);
-  if (xb > 64 * 1024) return -2;
-  p.xk = per * kKb + 8;
-  p.slots = std::min(per, kFewSlots);
-  if (1024 + xb + p.slots * level > kFewMaxSmem) p.slots = std::max(1, (kFewHalf - 1024 - xb) / level);
-  if (1024 + xb + p.slots * level > kFewMaxSmem) return -2;
-  p.smem = std::max<size_t>(kFewMinSmem, 1024 + (size_t)xb + (size_t)p.slots * level);
+  if (best.cost > 1e29) return -2;
+  p.R = best.R, p.splits = best.splits, p.slots = best.slots, p.smem = best.smem;
+  p.xk = few_per(K / kKb, p.splits) * kKb + 8;
+  const int nkb = K / kKb;
   const uint64_t wd[3] = {kKb, (uint64_t)N, (uint64_t)nkb}, ws[2] = {(uint64_t)K * 2, kKb * 2};
   const uint32_t wb[3] = {kKb, (uint32_t)p.R, 1};
   return tc_encode_bf16(&p.wmap, w, 3, wd, ws, wb) == 0 ? 0 : -4;
