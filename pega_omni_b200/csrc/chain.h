@@ -36,14 +36,14 @@ struct Chain {
 
   // y (bf16 rows, SwiGLU activations) or, for kStreamPartials, *sum
   cudaError_t gemm(const bf16* w, int N, int K, const bf16* x, int rows, int out, bf16* y, int ldy, Summands* sum = nullptr,
-                   int granule = 0, Epilogue epi = {}) const {
+                   int granule = kGateGroup, Epilogue epi = {}) const {
     if (rows > kChainRows) {  // prompts: any row count, so the plan (two tensor maps) is made for the call
       WidePlan wide;
       if (wide_plan(&wide, w, N, K, x, rows, out, y, ldy, epi, sm_count, granule) != 0) return cudaErrorInvalidValue;
       ++*launches;
       return wide_launch(wide, err, stream);
     }
-    ChainPlan* p = plan(w, N, K, x, rows, out, y, ldy, granule, epi);
+    ChainPlan* p = plan(w, N, K, x, rows, out, y, ldy, epi);
     return p ? launch(*p, {}, sum) : cudaErrorInvalidValue;
   }
 
@@ -51,9 +51,9 @@ struct Chain {
   // kernel where few_rows.h takes the shape, otherwise by `apart`, which updates *res in place and writes x.
   template <typename Apart>
   cudaError_t norm_gemm(FewNorm norm, bf16** res, bf16** spare, const Apart& apart, const bf16* w, int N, int K, const bf16* x,
-                        int rows, int out, bf16* y, int ldy, int granule = 0) const {
+                        int rows, int out, bf16* y, int ldy) const {
     if (few_norm_fits(K, rows) && norm.sum.splits >= 1 && norm.sum.splits <= 4) {
-      if (ChainPlan* p = plan(w, N, K, nullptr, rows, out, y, ldy, granule, {})) {
+      if (ChainPlan* p = plan(w, N, K, nullptr, rows, out, y, ldy, {})) {
         norm.res_in = *res, norm.res_out = *spare;
         std::swap(*res, *spare);
         return launch(*p, norm, nullptr);
@@ -61,17 +61,17 @@ struct Chain {
     }
     ++*launches;
     const cudaError_t e = apart(norm.sum, *res);
-    return e != cudaSuccess ? e : gemm(w, N, K, x, rows, out, y, ldy, nullptr, granule);
+    return e != cudaSuccess ? e : gemm(w, N, K, x, rows, out, y, ldy);
   }
 
  private:
-  ChainPlan* plan(const bf16* w, int N, int K, const bf16* x, int rows, int out, bf16* y, int ldy, int granule, Epilogue epi) const {
+  ChainPlan* plan(const bf16* w, int N, int K, const bf16* x, int rows, int out, bf16* y, int ldy, Epilogue epi) const {
     const auto key = std::make_tuple((const void*)w, (const void*)x, (const void*)y, rows, out);
     auto it = plans->find(key);
     if (it != plans->end()) return &it->second;
     ChainPlan p;
-    p.few = few_plan(&p.f, w, N, K, x, rows, out, y, ldy, partials, epi, sm_count, granule) == 0;
-    if (!p.few && (!x || stream_plan(&p.s, w, N, K, x, rows, out, y, ldy, partials, epi, sm_count, granule) != 0)) return nullptr;
+    p.few = few_plan(&p.f, w, N, K, x, rows, out, y, ldy, partials, epi, sm_count) == 0;
+    if (!p.few && (!x || stream_plan(&p.s, w, N, K, x, rows, out, y, ldy, partials, epi, sm_count) != 0)) return nullptr;
     if (out == kStreamPartials && (p.few ? p.f.partial_floats() : p.s.partial_floats()) > partial_floats) return nullptr;
     return &plans->emplace(key, p).first->second;
   }
@@ -98,10 +98,10 @@ inline bool chain_supports(int hidden, int inter, int q_width, int head_dim) {
 }
 
 
-// gate_up(l) and down(l) pick a layer's MLP; `inter` is its width, its gate|up rows lie in groups of `granule`.
+// gate_up(l) and down(l) pick a layer's MLP; `inter` is its width, its gate|up rows lie in groups of kGateGroup.
 template <typename Layer, typename GateUp, typename Down>
 cudaError_t chain_pass(const Chain& c, const std::vector<Layer>& layers, const GateUp& gate_up, const Down& down, int hidden,
-                       int inter, int granule, const AttnShape& a, ChainBuffers b, int rows, const RowMap& map,
+                       int inter, const AttnShape& a, ChainBuffers b, int rows, const RowMap& map,
                        const std::vector<bf16*>& kv, int kv_pages, const bf16* final_gain, bf16* keep_out, int every,
                        int which, const QkvTable& lookup = {}, bool prompt = false) {
   const int qd = a.q_heads * a.head_dim, qw = (a.q_heads + 2 * a.kv_heads) * a.head_dim;
@@ -109,18 +109,18 @@ cudaError_t chain_pass(const Chain& c, const std::vector<Layer>& layers, const G
   FewNorm norm;
   norm.kind = kNormStack, norm.eps = a.rms_eps;
   // the add + norm of `sum` by layer gain `gain`, and the GEMM of the rows it makes
-  auto norm_gemm = [&](const bf16* gain, const bf16* w, int N, int out, bf16* y, int ldy, int g) {
+  auto norm_gemm = [&](const bf16* gain, const bf16* w, int N, int out, bf16* y, int ldy) {
     norm.sum = sum, norm.gain = gain;
     return c.norm_gemm(norm, &b.res, &b.spare,
                        [&](const Summands& from, bf16* res) {
                          return launch_add_norm_sum(from, res, gain, b.x, rows, hidden, a.rms_eps, 1, 0, c.stream);
                        },
-                       w, N, hidden, b.x, rows, out, y, ldy, g);
+                       w, N, hidden, b.x, rows, out, y, ldy);
   };
   for (size_t i = 0; i < layers.size(); ++i) {
     const Layer& L = layers[i];
     const QkvTable& from = i == 0 ? lookup : QkvTable{};
-    if (i > 0) OMNI_CHAIN(norm_gemm(L.ln1, L.qkv, qw, kStreamBf16, b.qkv, qw, 0));
+    if (i > 0) OMNI_CHAIN(norm_gemm(L.ln1, L.qkv, qw, kStreamBf16, b.qkv, qw));
     else if (!from.table) OMNI_CHAIN(c.gemm(L.qkv, qw, hidden, b.x, rows, kStreamBf16, b.qkv, qw));
     if (prompt) {  // rows of one sequence attend to one another: every key is written before the first is read
       *c.launches += 2;
@@ -131,7 +131,7 @@ cudaError_t chain_pass(const Chain& c, const std::vector<Layer>& layers, const G
       OMNI_CHAIN(launch_rope_attend(b.qkv, from, L.q_norm, L.k_norm, kv[i], b.attn, map, rows, a, kv_pages, c.err, c.stream));
     }
     OMNI_CHAIN(c.gemm(L.o, hidden, qd, b.attn, rows, kStreamPartials, nullptr, hidden, &sum));
-    OMNI_CHAIN(norm_gemm(L.ln2, gate_up(L), 2 * inter, kStreamSwiglu, b.act, inter, granule));
+    OMNI_CHAIN(norm_gemm(L.ln2, gate_up(L), 2 * inter, kStreamSwiglu, b.act, inter));
     OMNI_CHAIN(c.gemm(down(L), hidden, inter, b.act, rows, kStreamPartials, nullptr, hidden, &sum));
   }
   ++*c.launches;

@@ -130,7 +130,6 @@ struct omni_duplex {
   };
   std::map<int, TickGraph> tick_graphs;
   ChainPlans stream_plans;
-  int granule = 16, d_granule = 16;  // channels per group of the gate|up rows (launch_interleave_gate_up)
   Chain chain() { return Chain{stream, err, sm_count, scratch.partials, scratch.partial_floats, &launches, &stream_plans}; }
   bool use_graphs = true;
 
@@ -252,15 +251,14 @@ float rope_coef(const omni_duplex_config& c) {  // helium.rs:79-81
 
 // A projection behind Helium's add + norm (kAddLm: the add alone, whose rows are then the residual itself).
 static cudaError_t lm_norm_gemm(const Chain& c, int kind, const Summands& sum, bf16** res, bf16** spare, const bf16* gain,
-                                float eps, bf16* xn, const bf16* w, int N, int K, int rows, int out, bf16* y, int ldy,
-                                int granule) {
+                                float eps, bf16* xn, const bf16* w, int N, int K, int rows, int out, bf16* y, int ldy) {
   FewNorm norm;
   norm.kind = kind, norm.sum = sum, norm.gain = gain, norm.eps = eps;
   return c.norm_gemm(norm, res, spare,
                      [&](const Summands& from, bf16* x) {
                        return launch_lm_add_norm_sum(from, x, gain, kind == kAddLm ? nullptr : xn, rows, K, eps, c.stream);
                      },
-                     w, N, K, kind == kAddLm ? *res : xn, rows, out, y, ldy, granule);
+                     w, N, K, kind == kAddLm ? *res : xn, rows, out, y, ldy);
 }
 
 // Every Helium layer over `rows` rows of m->x; the output norm's rows end in m->xn (helium.rs:225-284). In a
@@ -293,14 +291,14 @@ int helium_forward(omni_duplex* m, int rows, const int32_t* pos, const int32_t* 
     }
     return OMNI_OK;
   };
-  auto behind_norm = [&](const bf16* gain, const bf16* w, int N, int out, bf16* to, int ld, int granule) -> int {
-    DCUDA(m, lm_norm_gemm(chain, kNormLm, y, &res, &spare, gain, c.norm_eps, m->xn, w, N, D, rows, out, to, ld, granule));
+  auto behind_norm = [&](const bf16* gain, const bf16* w, int N, int out, bf16* to, int ld) -> int {
+    DCUDA(m, lm_norm_gemm(chain, kNormLm, y, &res, &spare, gain, c.norm_eps, m->xn, w, N, D, rows, out, to, ld));
     return OMNI_OK;
   };
   DLAUNCH(m, launch_lm_norm(m->x, m->h[0].norm1, m->xn, rows, D, c.norm_eps, m->stream));
   for (int i = 0; i < c.layers; ++i) {
     const HeliumLayer& L = m->h[i];
-    if (stream && i > 0) DTRY(behind_norm(L.norm1, L.qkv, 3 * Dl, kStreamBf16, m->qkv, 3 * Dl, 0));
+    if (stream && i > 0) DTRY(behind_norm(L.norm1, L.qkv, 3 * Dl, kStreamBf16, m->qkv, 3 * Dl));
     else DTRY(gemm(m, L.qkv, 3 * Dl, D, m->xn, rows, m->qkv, 3 * Dl));
     if (!seq) {
       DLAUNCH(m, launch_lm_rope_attend(m->qkv, m->kv[i], pos, slot, indptr, pages, m->attn, rows, m->local_heads(),
@@ -312,12 +310,12 @@ int helium_forward(omni_duplex* m, int rows, const int32_t* pos, const int32_t* 
     }
     DTRY(projected(L.o, Dl, m->attn, 0, L.norm2));
     if (stream) {
-      DTRY(behind_norm(L.norm2, L.gate_up, 2 * Hl, kStreamSwiglu, m->act, Hl, m->granule));
-    } else if (rows <= kChainRows || wide_fuses(2 * Hl, D, m->granule)) {
-      DCUDA(m, chain.gemm(L.gate_up, 2 * Hl, D, m->xn, rows, kStreamSwiglu, m->act, Hl, nullptr, m->granule));
+      DTRY(behind_norm(L.norm2, L.gate_up, 2 * Hl, kStreamSwiglu, m->act, Hl));
+    } else if (rows <= kChainRows || wide_fuses(2 * Hl, D, kGateGroup)) {
+      DCUDA(m, chain.gemm(L.gate_up, 2 * Hl, D, m->xn, rows, kStreamSwiglu, m->act, Hl));
     } else {
       DTRY(gemm(m, L.gate_up, 2 * Hl, D, m->xn, rows, m->gu, 2 * Hl));
-      DLAUNCH(m, launch_silu_mul(m->gu, m->act, rows, Hl, m->granule, m->stream));
+      DLAUNCH(m, launch_silu_mul(m->gu, m->act, rows, Hl, kGateGroup, m->stream));
     }
     DTRY(projected(L.down, Hl, m->act, 1, i + 1 < c.layers ? m->h[i + 1].norm1 : m->out_norm));
   }
@@ -339,22 +337,22 @@ int depformer_step(omni_duplex* m, int n, const int32_t* force, const int32_t* s
                                         c.norm_eps, m->err, m->stream));
     bf16 *res = m->dx, *spare = m->dx2;
     Summands y;
-    auto behind_norm = [&](int kind, const bf16* gain, const bf16* w, int N, int out, bf16* to, int granule) -> int {
-      DCUDA(m, lm_norm_gemm(chain, kind, y, &res, &spare, gain, c.norm_eps, m->dxn, w, N, D, n, out, to, out == kStreamSwiglu ? N / 2 : N, granule));
+    auto behind_norm = [&](int kind, const bf16* gain, const bf16* w, int N, int out, bf16* to) -> int {
+      DCUDA(m, lm_norm_gemm(chain, kind, y, &res, &spare, gain, c.norm_eps, m->dxn, w, N, D, n, out, to, out == kStreamSwiglu ? N / 2 : N));
       return OMNI_OK;
     };
     for (int i = 0; i < c.dep_layers; ++i) {
       const DepLayer& L = m->d[i];
       const bf16* qkv = L.qkv + (size_t)k * 3 * D * D;
-      if (i > 0) DTRY(behind_norm(kNormLm, L.norm1, qkv, 3 * D, kStreamBf16, m->dqkv, 0));
+      if (i > 0) DTRY(behind_norm(kNormLm, L.norm1, qkv, 3 * D, kStreamBf16, m->dqkv));
       else DTRY(gemm(m, qkv, 3 * D, D, m->dxn, n, m->dqkv, 3 * D));
       DLAUNCH(m, launch_lm_dep_kv_attend(m->dqkv, m->dkv[i], k, m->dattn, n, c.dep_heads, scale, m->stream));
       DCUDA(m, chain.gemm(L.out + (size_t)k * D * D, D, D, m->dattn, n, kStreamPartials, nullptr, D, &y));
-      DTRY(behind_norm(kNormLm, L.norm2, L.gate_in + (size_t)k * 2 * H * D, 2 * H, kStreamSwiglu, m->dact, m->d_granule));
+      DTRY(behind_norm(kNormLm, L.norm2, L.gate_in + (size_t)k * 2 * H * D, 2 * H, kStreamSwiglu, m->dact));
       DCUDA(m, chain.gemm(L.gate_out + (size_t)k * D * H, D, H, m->dact, n, kStreamPartials, nullptr, D, &y));
     }
     bf16* logits = m->audio_logits + (size_t)k * S * c.card;
-    DTRY(behind_norm(kAddLm, nullptr, m->d_heads + (size_t)k * c.card * D, c.card, kStreamBf16, logits, 0));
+    DTRY(behind_norm(kAddLm, nullptr, m->d_heads + (size_t)k * c.card * D, c.card, kStreamBf16, logits));
     DLAUNCH(m, launch_lm_sample(logits, c.card, c.card, c.audio_temperature, c.audio_top_k, force, seeds, 1 + k,
                                 m->drawn, n, m->stream));
   }
@@ -453,19 +451,17 @@ int32_t omni_duplex_create(const omni_duplex_config* config, const omni_tensor* 
   }
 
   {  // gate|up rows regrouped for the fused SwiGLU
-    m->granule = stream_granule((int)Hl, m->sm_count);
-    m->d_granule = stream_granule((int)DH, m->sm_count);
     bf16* tmp = nullptr;
     DCUDA(m, cudaDeviceSynchronize());  // the weights were copied on the default stream
     DCUDA(m, cudaMalloc((void**)&tmp, (size_t)2 * std::max(Hl * D, DH * DD) * sizeof(bf16)));
-    auto regroup = [&](bf16* rows, int64_t inter, int64_t k, int granule) -> int {
+    auto regroup = [&](bf16* rows, int64_t inter, int64_t k) -> int {
       DCUDA(m, cudaMemcpyAsync(tmp, rows, (size_t)2 * inter * k * sizeof(bf16), cudaMemcpyDeviceToDevice, m->stream));
-      DCUDA(m, launch_interleave_gate_up(tmp, rows, (int)inter, (int)k, granule, m->stream));
+      DCUDA(m, launch_interleave_gate_up(tmp, rows, (int)inter, (int)k, kGateGroup, m->stream));
       return OMNI_OK;
     };
-    for (const HeliumLayer& L : m->h) DTRY(regroup(L.gate_up, Hl, D, m->granule));
+    for (const HeliumLayer& L : m->h) DTRY(regroup(L.gate_up, Hl, D));
     for (const DepLayer& L : m->d)
-      for (int k = 0; k < kDepSteps; ++k) DTRY(regroup(L.gate_in + (size_t)k * 2 * DH * DD, DH, DD, m->d_granule));
+      for (int k = 0; k < kDepSteps; ++k) DTRY(regroup(L.gate_in + (size_t)k * 2 * DH * DD, DH, DD));
     DCUDA(m, cudaStreamSynchronize(m->stream));
     DCUDA(m, cudaFree(tmp));
   }

@@ -174,12 +174,9 @@ __global__ void __launch_bounds__(kWarps * 32, 2) few_rows_kernel(const __grid_c
   h.warp = warp, h.lane = lane, h.lanes = 1 << a.lanes_log2;
   h.n = lane >> a.lanes_log2, h.first = lane & (h.lanes - 1), h.pieces = nk * 8, h.c0 = kb0 * kKb;
   h.live = h.n < a.rows, h.xs = xs + (uint32_t)(h.n * a.xk) * 2u;
-  // the tile's rows; SwiGLU: `half` gate channels, then their up channels (the last tile may hold fewer)
-  const int half = OUT == kStreamSwiglu ? min(a.R >> 1, (a.N >> 1) - tile * (a.R >> 1)) : 0;
-  const int mts = MT <= 4 ? MT : OUT == kStreamSwiglu ? half >> 3 : a.R >> 4;
+  const int mts = MT <= 4 ? MT : a.R >> 4;
   // ldmatrix rows of this lane: weights [0, 8) k 0..7, [8, 16) k 0..7, [0, 8) k 8..15, [8, 16) k 8..15; x rows past the
   // last read row 0 (their columns of the result are not stored)
-  const int row0 = OUT == kStreamSwiglu ? (lane & 7) + ((lane & 8) ? half : 0) : lane & 15;
   uint32_t x_lane[NT], w_lane[4];
 #pragma unroll
   for (int t = 0; t < NT; ++t) {
@@ -187,7 +184,7 @@ __global__ void __launch_bounds__(kWarps * 32, 2) few_rows_kernel(const __grid_c
     x_lane[t] = xs + (uint32_t)((r < a.rows ? r : 0) * a.xk + (lane >> 3) * 8) * 2u;
   }
 #pragma unroll
-  for (int k = 0; k < 4; ++k) w_lane[k] = ring + (uint32_t)row0 * 128u + (uint32_t)(((k * 2 + (lane >> 4)) ^ (lane & 7)) << 4);
+  for (int k = 0; k < 4; ++k) w_lane[k] = ring + (uint32_t)(lane & 15) * 128u + (uint32_t)(((k * 2 + (lane >> 4)) ^ (lane & 7)) << 4);
   const int stride = a.R + 4, warp_floats = a.slots * a.R * 32;
   float* const red0 = reinterpret_cast<float*>(few_smem_raw + (ring0 - smem_addr(few_smem_raw)));
   float* const red = red0 + warp * warp_floats + (lane & 3) * 2 * stride + (lane >> 2);
@@ -245,7 +242,7 @@ __global__ void __launch_bounds__(kWarps * 32, 2) few_rows_kernel(const __grid_c
       if (MT <= 4 || m < mts) {
         uint32_t w[4][4];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) ldsm4(w_lane[k] + off + m * (OUT == kStreamSwiglu ? 1024 : 2048), w[k]);
+        for (int k = 0; k < 4; ++k) ldsm4(w_lane[k] + off + m * 2048, w[k]);
 #pragma unroll
         for (int k = 0; k < 4; ++k)
 #pragma unroll
@@ -260,7 +257,8 @@ __global__ void __launch_bounds__(kWarps * 32, 2) few_rows_kernel(const __grid_c
     if (++slot == a.slots) slot = 0, off = 0, turn ^= 1u;
   }
 
-  // ---- sum over the warps, through each warp's own (spent) ring: [row of x][weight row], SwiGLU gates then ups ----
+  // ---- sum over the warps, through each warp's own (spent) ring: [row of x][weight row]; SwiGLU, whose 16-row tiles are
+  // eight gates and their ups, all gates then all ups ----
   __syncwarp();
 #pragma unroll
   for (int m = 0; m < MT; ++m)
@@ -280,7 +278,7 @@ __global__ void __launch_bounds__(kWarps * 32, 2) few_rows_kernel(const __grid_c
     for (int w = 0; w < kWarps; ++w) f[w] = red0[w * warp_floats + at];
     return ((f[0] + f[1]) + (f[2] + f[3])) + ((f[4] + f[5]) + (f[6] + f[7]));
   };
-  const int cols = OUT == kStreamSwiglu ? half : min(a.R, a.N - tile * a.R), c0 = tile * (OUT == kStreamSwiglu ? a.R >> 1 : a.R);
+  const int halves = OUT == kStreamSwiglu ? 1 : 0, cols = min(a.R, a.N - tile * a.R) >> halves, c0 = (tile * a.R) >> halves;
 #pragma unroll 1
   for (int n = warp; n < a.rows; n += kWarps) {  // a row per warp, a column per lane
 #pragma unroll 1
@@ -392,33 +390,28 @@ static FewShape few_shape(int N, int K, int rows, int R, int splits, int sm_coun
 }
 
 int few_plan(FewPlan* plan, const bf16* w, int N, int K, const bf16* x, int rows, int out, bf16* y, int ldy, float* part,
-             Epilogue epi, int sm_count, int granule) {
+             Epilogue epi, int sm_count) {
   if (rows < 1 || rows > 16 || K % kKb || N < 1) return -2;
   if (!x && !few_norm_fits(K, rows)) return -2;
-  if (out == kStreamSwiglu && (granule < 8 || granule % 8 || N % 16)) return -2;
+  if (out == kStreamSwiglu && N % (2 * kGateGroup)) return -2;
   if ((reinterpret_cast<uintptr_t>(w) & 15) || (reinterpret_cast<uintptr_t>(x) & 15)) return -3;
   FewPlan& p = *plan;
   p.N = N, p.K = K, p.rows = rows, p.out = out, p.x = x, p.y = y, p.ldy = ldy, p.part = part, p.epi = epi;
   const int most = rows > 8 ? 64 : 160;
   FewShape best{};
   best.cost = 1e30;
-  if (out == kStreamSwiglu) {
-    if (2 * granule > most) return -2;
-    best = few_shape(N, K, rows, 2 * granule, 1, sm_count);
-  } else {
-    // The most even load of weights and rows, whose tiles are narrow and leave little to do behind the wait, where it has
-    // most of every warp's share in its ring by then; otherwise by cost.
-    FewShape even = best;
-    even.even = 1e30;
-    for (int R = 16; R <= most; R += 16)
-      for (int S : {1, 2, 4}) {
-        if (S > 1 && (out != kStreamPartials || S * kWarps > K / kKb)) break;
-        const FewShape shape = few_shape(N, K, rows, R, S, sm_count);
-        if (shape.cost < best.cost) best = shape;
-        if (shape.even < even.even) even = shape;
-      }
-    if (even.early) best = even;
-  }
+  // The most even load of weights and rows, whose tiles are narrow and leave little to do behind the wait, where it has
+  // most of every warp's share in its ring by then; otherwise by cost.
+  FewShape even = best;
+  even.even = 1e30;
+  for (int R = 16; R <= most; R += 16)
+    for (int S : {1, 2, 4}) {
+      if (S > 1 && (out != kStreamPartials || S * kWarps > K / kKb)) break;
+      const FewShape shape = few_shape(N, K, rows, R, S, sm_count);
+      if (shape.cost < best.cost) best = shape;
+      if (shape.even < even.even) even = shape;
+    }
+  if (even.early) best = even;
   if (best.cost > 1e29) return -2;
   p.R = best.R, p.splits = best.splits, p.slots = best.slots, p.smem = best.smem;
   p.xk = few_per(K / kKb, p.splits) * kKb + 8;

@@ -88,7 +88,6 @@ struct omni_higgs {
   };
   std::map<int, StepGraph> step_graphs;
   ChainPlans stream_plans;
-  int granule = 16, granule_audio = 16;  // channels per group of the gate|up rows (launch_interleave_gate_up)
   Chain chain() { return Chain{stream, err, sm_count, scratch.partials, scratch.partial_floats, &launches, &stream_plans}; }
   bool use_graphs = true;
 
@@ -191,11 +190,10 @@ int body_forward(omni_higgs* m, const bf16* input, int rows, const RowMap& map, 
   const bool both = audio && m->cfg.audio_adapter != 0;
   const int h = c.hidden, I = both ? 2 * c.inter : c.inter, qd = c.q_heads * c.head_dim, qw = m->qkv_width();
   const AttnShape a{c.q_heads, c.kv_heads, c.head_dim, c.rms_eps, c.rope_theta};
-  const int granule = both ? m->granule_audio : m->granule;
   HLAUNCH(m, launch_norm_copy(input, m->layers[0].ln1, m->x, m->res, rows, h, c.rms_eps, m->stream));
   if (rows <= kChainRows && chain_supports(h, I, qd, c.head_dim)) {
     HCUDA(m, chain_pass(m->chain(), m->layers, [&](const Layer& L) { return both ? L.gate_up_audio : L.gate_up; },
-                        [&](const Layer& L) { return both ? L.down_audio : L.down; }, h, I, granule, a,
+                        [&](const Layer& L) { return both ? L.down_audio : L.down; }, h, I, a,
                         ChainBuffers{m->x, m->res, m->res2, m->qkv, m->attn, m->act}, rows, map, m->kv, m->pages_total, m->norm, out,
                         1, 0, {}, !audio));
     return OMNI_OK;
@@ -208,11 +206,11 @@ int body_forward(omni_higgs* m, const bf16* input, int rows, const RowMap& map, 
     HTRY(gemm(m, L.o, h, qd, m->attn, rows, m->x, h));
     HLAUNCH(m, launch_add_norm(m->x, m->res, L.ln2, m->x, rows, h, c.rms_eps, 1, 0, m->stream));
     const bf16* gate_up = both ? L.gate_up_audio : L.gate_up;
-    if (wide_fuses(2 * I, h, granule)) {
-      HCUDA(m, m->chain().gemm(gate_up, 2 * I, h, m->x, rows, kStreamSwiglu, m->act, I, nullptr, granule));
+    if (wide_fuses(2 * I, h, kGateGroup)) {
+      HCUDA(m, m->chain().gemm(gate_up, 2 * I, h, m->x, rows, kStreamSwiglu, m->act, I));
     } else {
       HTRY(gemm(m, gate_up, 2 * I, h, m->x, rows, m->gate_up, 2 * I));
-      HLAUNCH(m, launch_silu_mul(m->gate_up, m->act, rows, I, granule, m->stream));
+      HLAUNCH(m, launch_silu_mul(m->gate_up, m->act, rows, I, kGateGroup, m->stream));
     }
     HTRY(gemm(m, both ? L.down_audio : L.down, h, I, m->act, rows, m->x, h));
     const bf16* next = i + 1 < c.layers ? m->layers[i + 1].ln1 : m->norm;
@@ -330,14 +328,12 @@ int32_t omni_higgs_create(const omni_higgs_config* config, const omni_tensor* te
     if (tensors[i].name) idx[tensors[i].name] = &tensors[i];
   const int64_t h = b.hidden, d = b.head_dim, q = (int64_t)b.q_heads * d, kvw = (int64_t)b.kv_heads * d, I = b.inter;
   m->layers.resize(b.layers);
-  m->granule = stream_granule((int)I, m->sm_count);
-  m->granule_audio = stream_granule((int)(2 * I), m->sm_count);
   bf16* regroup_tmp = nullptr;  // [gate; up] rows on their way into groups; freed below
   const size_t gate_up_bytes = (size_t)(c.audio_adapter ? 4 : 2) * I * h * 2;
   HCUDA(m, cudaMalloc((void**)&regroup_tmp, gate_up_bytes));
-  auto regroup = [&](bf16* rows, int inter, int granule) -> int {
+  auto regroup = [&](bf16* rows, int inter) -> int {
     HCUDA(m, cudaMemcpyAsync(regroup_tmp, rows, (size_t)2 * inter * h * 2, cudaMemcpyDeviceToDevice, m->stream));
-    HCUDA(m, launch_interleave_gate_up(regroup_tmp, rows, inter, (int)h, granule, m->stream));
+    HCUDA(m, launch_interleave_gate_up(regroup_tmp, rows, inter, (int)h, kGateGroup, m->stream));
     return OMNI_OK;
   };
   bf16* adapter_tmp = nullptr;  // staging for the audio branch's down projection (stays allocated with the model)
@@ -376,8 +372,8 @@ int32_t omni_higgs_create(const omni_higgs_config* config, const omni_tensor* te
       HCUDA(m, cudaMemcpy2D(L.down_audio + I, 2 * I * 2, adapter_tmp, I * 2, I * 2, h, cudaMemcpyDeviceToDevice));
     }
     HCUDA(m, cudaDeviceSynchronize());  // the copies above ran on the default stream
-    HTRY(regroup(L.gate_up, (int)I, m->granule));
-    if (c.audio_adapter) HTRY(regroup(L.gate_up_audio, (int)(2 * I), m->granule_audio));
+    HTRY(regroup(L.gate_up, (int)I));
+    if (c.audio_adapter) HTRY(regroup(L.gate_up_audio, (int)(2 * I)));
   }
   HCUDA(m, cudaStreamSynchronize(m->stream));
   HCUDA(m, cudaFree(regroup_tmp));

@@ -201,12 +201,11 @@ int32_t omni_op_chain_gemm(omni_ops* c, const void* w, int32_t N, int32_t K, con
     OPS_CUDA(c, chain.gemm((const bf16*)w, N, K, (const bf16*)x, rows, kStreamBf16, (bf16*)y, ldy, nullptr, 0, epi));
     return OMNI_OK;
   }
-  const int granule = stream_granule(N / 2, c->sm_count);
-  if (rows > kChainRows && !wide_fuses(N, K, granule)) return c->fail(OMNI_ERR_UNSUPPORTED, "groups of %d channels do not fill tiles", granule);
+  if (!wide_fuses(N, K, kGateGroup)) return c->fail(OMNI_ERR_UNSUPPORTED, "gate and up rows are no groups of %d", kGateGroup);
   bf16* grouped = nullptr;
   OPS_CUDA(c, cudaMalloc((void**)&grouped, (size_t)N * K * sizeof(bf16)));
-  cudaError_t e = launch_interleave_gate_up((const bf16*)w, grouped, N / 2, K, granule, c->stream);
-  if (e == cudaSuccess) e = chain.gemm(grouped, N, K, (const bf16*)x, rows, kStreamSwiglu, (bf16*)y, ldy, nullptr, granule);
+  cudaError_t e = launch_interleave_gate_up((const bf16*)w, grouped, N / 2, K, kGateGroup, c->stream);
+  if (e == cudaSuccess) e = chain.gemm(grouped, N, K, (const bf16*)x, rows, kStreamSwiglu, (bf16*)y, ldy);
   const cudaError_t done = cudaStreamSynchronize(c->stream);
   cudaFree(grouped);
   OPS_CUDA(c, e);

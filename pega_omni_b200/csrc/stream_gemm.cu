@@ -188,12 +188,12 @@ __global__ void __launch_bounds__(kThreads, 1)
     const bool warp_live = m0 + (a.M == 128 ? quad * 32 : quad * 16) < a.rows;
     if (ok && warp_live) {
       if constexpr (OUT == kStreamSwiglu) {
-        // the tile's rows are `half` gate channels, then their up channels (the last tile may hold fewer)
+        // the tile's rows are groups of gates and their ups
         const int ch0 = tile * (a.tn >> 1), half = min(a.tn >> 1, (a.N >> 1) - ch0);
-        for (int c = 0; c < half; c += 8) {
+        for (int c = 0; c < half; c += kGateGroup) {
           float g[8], u[8];
-          acc_cols8(lane_addr, c, a, g);
-          acc_cols8(lane_addr, half + c, a, u);
+          acc_cols8(lane_addr, 2 * c, a, g);
+          acc_cols8(lane_addr, 2 * c + kGateGroup, a, u);
           if (!row_live) continue;
           float o[8];
 #pragma unroll
@@ -253,13 +253,6 @@ void stream_configure() {
 
 bool stream_supports(int N, int K, int rows) { return K % kKb == 0 && K >= kKb && N >= 1 && rows >= 1; }
 
-int stream_granule(int inter, int sm_count) {
-  int waves = 1;
-  auto width = [&](int w) { return (2 * inter + sm_count * w - 1) / (sm_count * w); };
-  while (width(waves) > 256) ++waves;
-  return std::max(16, (width(waves) + 15) / 16 * 16) / 2;
-}
-
 // Weight rows per tile (tn) and K splits: the shape with the shortest estimated time after the inputs are there. A CTA
 // pulls its tile's inputs at about 170 GB/s whatever the number of CTAs (they all read the same rows), the tensor pipe
 // takes (M + tn) / 4 cycles per 16 elements of K, stores leave an SM at 57 GB/s, and weights only count where a shape
@@ -270,34 +263,30 @@ static double stream_cost(int N, int K, int rows, int M, int bn, int tn, int S, 
   const double t_x = kc * 2 * bn * per_sm / 170e3;
   const double t_w = kc * 2 * tn * per_sm / std::min(170e3, 6.5e6 / std::min(ctas, sms));
   const double t_mma = kc / 16 * std::max(0.25 * (M + tn), tn > 128 ? 40.0 : 20.0) * per_sm / 1900;
-  const double t_out = std::min(rows, 128) * tn * (out == kStreamPartials ? 4.0 : 2.0) * per_sm / 57e3;
+  const double t_out = std::min(rows, 128) * tn * (out == kStreamPartials ? 4.0 : out == kStreamSwiglu ? 1.0 : 2.0) * per_sm / 57e3;
   return std::max({t_x + 0.3 * t_mma, t_mma, 0.5 * t_x + t_w}) + t_out + 0.1 * S;
 }
 
 int stream_plan(StreamGemmPlan* plan, const bf16* w, int N, int K, const bf16* x, int rows, int out, bf16* y, int ldy,
-                float* part, Epilogue epi, int sm_count, int granule, int force_splits) {
+                float* part, Epilogue epi, int sm_count, int force_splits) {
   if (!stream_supports(N, K, rows)) return -2;
   if (out == kStreamPartials && N % 8) return -2;
-  if (out == kStreamSwiglu && (granule < 8 || granule % 8 || granule > 128 || N % 16 || ldy % 8)) return -2;
+  if (out == kStreamSwiglu && (N % (2 * kGateGroup) || ldy % 8)) return -2;
   if ((reinterpret_cast<uintptr_t>(w) & 15) || (reinterpret_cast<uintptr_t>(x) & 15)) return -3;
   StreamGemmPlan& p = *plan;
   p.N = N, p.K = K, p.rows = rows, p.out = out, p.y = y, p.ldy = ldy, p.part = part, p.epi = epi;
   p.M = rows <= 64 ? 64 : 128;
   p.bn = std::min(128, (rows + 7) / 8 * 8);
   const int nkb = K / kKb, row_tiles = (rows + 127) / 128;
-  if (out == kStreamSwiglu) {
-    p.tn = 2 * granule, p.splits = 1;
-  } else {
-    double best = 1e30;
-    for (int tn = 16; tn <= 256; tn += 16)
-      for (int S : {1, 2, 4, 8}) {
-        if (S > 1 && (out != kStreamPartials || S * 2 > nkb)) break;
-        if (force_splits > 0 && S != force_splits) continue;
-        const double cost = stream_cost(N, K, rows, p.M, p.bn, tn, S, out, sm_count, row_tiles);
-        if (cost < best - 1e-9) best = cost, p.tn = tn, p.splits = S;
-      }
-    if (best > 1e29) return -2;
-  }
+  double best = 1e30;
+  for (int tn = 16; tn <= 256; tn += 16)
+    for (int S : {1, 2, 4, 8}) {
+      if (S > 1 && (out != kStreamPartials || S * 2 > nkb)) break;
+      if (force_splits > 0 && S != force_splits) continue;
+      const double cost = stream_cost(N, K, rows, p.M, p.bn, tn, S, out, sm_count, row_tiles);
+      if (cost < best - 1e-9) best = cost, p.tn = tn, p.splits = S;
+    }
+  if (best > 1e29) return -2;
   // k-blocks per stage: as many (up to four) as leave three stages in the ring; a copy costs its thread about 0.16 us
   const int kb_bytes = (p.bn + p.tn) * 128, room = kMaxSmem - 1024 - (p.M - p.bn) * 128;
   p.kbs = 1;

@@ -299,7 +299,7 @@ int load_stack(omni_talker* m, const TensorIndex& idx, const std::string& prefix
   // gate and up channels are interleaved in groups of half the tile the persistent kernel will use for this GEMM
   out->granule = choose_tiling(2 * c.inter, c.hidden, std::max(1, m->tick_ctas > 0 ? m->tick_ctas : 148), true).tile_n / 2;
   if (c.inter % out->granule) out->granule = 64;
-  if (m->use_chain) out->granule = stream_granule(c.inter, m->sm_count);
+  if (m->use_chain) out->granule = kGateGroup;
   const int64_t h = c.hidden, d = c.head_dim, q = (int64_t)c.q_heads * d, kv = (int64_t)c.kv_heads * d, I = c.inter;
   out->layers.resize(c.layers);
   for (int i = 0; i < c.layers; ++i) {
@@ -393,7 +393,7 @@ int chain_layers(omni_talker* m, const StackW& S, const Scratch& s, int rows, co
                  const std::vector<bf16*>& kv, int kv_pages, bf16* keep_out, int every, int which, const QkvTable& lookup,
                  bool prompt) {
   CUDA_TRY(m, chain_pass(m->chain(), S.layers, [](const StackW::Layer& L) { return L.gate_up; },
-                         [](const StackW::Layer& L) { return L.down; }, S.cfg.hidden, S.cfg.inter, S.granule, S.attn(),
+                         [](const StackW::Layer& L) { return L.down; }, S.cfg.hidden, S.cfg.inter, S.attn(),
                          ChainBuffers{s.x, s.res, s.res2, s.qkv, s.attn, s.act}, rows, map, kv, kv_pages, S.norm, keep_out, every,
                          which, lookup, prompt));
   return OMNI_OK;

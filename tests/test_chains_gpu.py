@@ -60,7 +60,7 @@ def test_chain_gemm(ops, rows, n, k, epilogue):
 @pytest.mark.parametrize("rows", [1, 9, 17, 128, 129, 257])
 @pytest.mark.parametrize("inter,k", [(256, 64), (3072, 1024), (4096, 576)])
 def test_chain_swiglu(ops, rows, inter, k):
-    """The last group of gate and up rows may be smaller than the others."""
+    """The last tile may hold fewer channels than the others."""
     w, x = rand((2 * inter, k), 4, k ** -0.5), rand((rows, k), 5)
     y = torch.zeros((rows, inter), dtype=torch.bfloat16, device="cuda")
     torch.cuda.synchronize()
