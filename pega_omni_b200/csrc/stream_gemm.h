@@ -79,8 +79,9 @@ struct StreamGemmPlan {
 void stream_configure();
 bool stream_supports(int N, int K, int rows);
 // Channels per group of the gate|up weight layout the fused SwiGLU wants ([8 gate rows; their 8 up rows; next group ...]): a
-// tile of any multiple of sixteen rows holds whole channels, and an epilogue's piece of eight columns is one group's gates. Groups as wide as half a tile fixed
-// the tile: 12,288 x 2,048 at one row kept one ring slot a warp (12.6 us), free tiles take a step 2,176 -> 2,091 us.
+// tile of any multiple of sixteen rows holds whole channels, and an epilogue's piece of eight columns is one group's gates.
+// Groups as wide as half a tile would fix the tile for every row count: at one row 12,288 x 2,048 then kept one ring slot a
+// warp, and a talker step took 2,176 us instead of 2,091.
 constexpr int kGateGroup = 8;
 int stream_plan(StreamGemmPlan* plan, const bf16* w, int N, int K, const bf16* x, int rows, int out, bf16* y, int ldy,
                 float* part, Epilogue epi, int sm_count, int force_splits = 0);
