@@ -484,7 +484,7 @@ int32_t omni_duplex_create(const omni_duplex_config* config, const omni_tensor* 
   m->max_rows = std::max(c.max_prefill, S);
   const size_t R = m->max_rows;
   DTRY(dalloc(m, &m->x, R * D));
-  DTRY(dalloc(m, &m->x2, (size_t)kFewNormRows * D));
+  DTRY(dalloc(m, &m->x2, (size_t)kFewRows * D));
   DTRY(dalloc(m, &m->xn, R * D));
   DTRY(dalloc(m, &m->qkv, R * 3 * D));
   DTRY(dalloc(m, &m->attn, R * D));
@@ -499,7 +499,7 @@ int32_t omni_duplex_create(const omni_duplex_config* config, const omni_tensor* 
   DTRY(dalloc(m, &m->audio_logits, (size_t)kDepSteps * S * c.card, true));
   DTRY(dalloc(m, &m->dproj, (size_t)S * kDepSteps * DD));
   DTRY(dalloc(m, &m->dx, (size_t)S * DD));
-  DTRY(dalloc(m, &m->dx2, (size_t)kFewNormRows * DD));
+  DTRY(dalloc(m, &m->dx2, (size_t)kFewRows * DD));
   DTRY(dalloc(m, &m->dxn, (size_t)S * DD));
   DTRY(dalloc(m, &m->dqkv, (size_t)S * 3 * DD));
   DTRY(dalloc(m, &m->dattn, (size_t)S * DD));

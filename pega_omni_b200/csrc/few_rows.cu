@@ -1,11 +1,13 @@
-// The GEMM of the kernel chains for up to sixteen rows (see few_rows.h).
+// The GEMM of the kernel chains for up to eight rows (see few_rows.h).
 //
 // A decode node of a few rows is latency: its weights were asked for before its inputs existed, so what counts is the
 // path from the inputs' arrival to the outputs' stores. tcgen05 puts four hand-overs on it (rows to shared memory by TMA,
 // MMA issue, commit, TMEM load); here the weights are M of m16n8k16 and the rows its N, and a warp keeps everything it
 // needs to itself: its eighth of K, its own ring of weight blocks, its rows of x, so that only the final sum over the
 // eight warps crosses a barrier. One m16n8k16 takes 2 cycles of the SM's pipe, which is ten times the rate at which DRAM
-// delivers weights, and up to sixteen rows there is nothing for a larger tile to reuse.
+// delivers weights, and up to eight rows there is nothing for a larger tile to reuse. Two 8-row tiles of x a warp double the
+// rows' arrival and the shared memory they take from the rings: at 16 rows a talker step took 3,526 us against 3,361 with the
+// tcgen05 kernel, a Higgs step 2,375 against 2,326, a duplex tick 4,604 against 4,548.
 // The add + norm before a projection is made by every CTA from the summands (L2 broadcast reads, 16 KB to 100 KB) while
 // two pieces a lane suffice; a kernel of its own takes 2.7 us and beyond two pieces is faster. Measured as nodes of a chain
 // at one row: 1,024 x 3,072 2.5 us, 6,144 x 1,024 with norm and SwiGLU 4.7 us, 4,096 x 1,024 with norm 4.3 us (4.5 to
@@ -134,11 +136,11 @@ __device__ __forceinline__ void plain_rows(const FewArgs& a, const Share& h) {
   }
 }
 
-// MT: 16-row tiles of weights per CTA (10: up to ten); NT: 8-row tiles of x.
+// MT: 16-row tiles of weights per CTA (10: up to ten).
 // Every instruction behind grid_wait() is on the chain's critical path and is executed once: what costs is how many a
 // warp goes through (about 5 cycles each, more when its line has to come from L2), hence the index arithmetic in front of
 // the wait, loops that run as often as there is work and bodies chosen by the number of pieces and sums.
-template <int MT, int NT, int NORM, int OUT>
+template <int MT, int NORM, int OUT>
 __global__ void __launch_bounds__(kWarps * 32, 2) few_rows_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ FewArgs a) {
   using namespace sm100;
   extern __shared__ unsigned char few_smem_raw[];
@@ -177,12 +179,7 @@ __global__ void __launch_bounds__(kWarps * 32, 2) few_rows_kernel(const __grid_c
   const int mts = MT <= 4 ? MT : a.R >> 4;
   // ldmatrix rows of this lane: weights [0, 8) k 0..7, [8, 16) k 0..7, [0, 8) k 8..15, [8, 16) k 8..15; x rows past the
   // last read row 0 (their columns of the result are not stored)
-  uint32_t x_lane[NT], w_lane[4];
-#pragma unroll
-  for (int t = 0; t < NT; ++t) {
-    const int r = t * 8 + (lane & 7);
-    x_lane[t] = xs + (uint32_t)((r < a.rows ? r : 0) * a.xk + (lane >> 3) * 8) * 2u;
-  }
+  uint32_t x_lane = xs + (uint32_t)(((lane & 7) < a.rows ? lane & 7 : 0) * a.xk + (lane >> 3) * 8) * 2u, w_lane[4];
 #pragma unroll
   for (int k = 0; k < 4; ++k) w_lane[k] = ring + (uint32_t)(lane & 15) * 128u + (uint32_t)(((k * 2 + (lane >> 4)) ^ (lane & 7)) << 4);
   const int stride = a.R + 4, warp_floats = a.slots * a.R * 32;
@@ -217,11 +214,9 @@ __global__ void __launch_bounds__(kWarps * 32, 2) few_rows_kernel(const __grid_c
   __syncwarp();
 
   // ---- w . x^T ----
-  float acc[MT][NT][4];
+  float acc[MT][4];
 #pragma unroll
-  for (int m = 0; m < MT; ++m)
-#pragma unroll
-    for (int t = 0; t < NT; ++t) acc[m][t][0] = acc[m][t][1] = acc[m][t][2] = acc[m][t][3] = 0.f;
+  for (int m = 0; m < MT; ++m) acc[m][0] = acc[m][1] = acc[m][2] = acc[m][3] = 0.f;
   uint32_t turn = 0, off = 0;  // of the ring; off: bytes to the slot
 #pragma unroll 1
   for (int i = 0, slot = 0; i < nk; ++i) {
@@ -230,13 +225,9 @@ __global__ void __launch_bounds__(kWarps * 32, 2) few_rows_kernel(const __grid_c
       for (int j = max(i + 1, ahead); j < min(nk, i + a.slots); ++j) mbar_wait(bars + 8u * (j % a.slots), (uint32_t)(j / a.slots) & 1u, a.err);
       break;
     }
-    uint32_t b[2][NT][4];
-#pragma unroll
-    for (int hf = 0; hf < 2; ++hf)
-#pragma unroll
-      for (int t = 0; t < NT; ++t) ldsm4(x_lane[t] + hf * 64, b[hf][t]);
-#pragma unroll
-    for (int t = 0; t < NT; ++t) x_lane[t] += 128u;
+    uint32_t b[2][4];
+    ldsm4(x_lane, b[0]), ldsm4(x_lane + 64, b[1]);
+    x_lane += 128u;
 #pragma unroll
     for (int m = 0; m < MT; ++m) {
       if (MT <= 4 || m < mts) {
@@ -244,9 +235,7 @@ __global__ void __launch_bounds__(kWarps * 32, 2) few_rows_kernel(const __grid_c
 #pragma unroll
         for (int k = 0; k < 4; ++k) ldsm4(w_lane[k] + off + m * 2048, w[k]);
 #pragma unroll
-        for (int k = 0; k < 4; ++k)
-#pragma unroll
-          for (int t = 0; t < NT; ++t) mma_16816(acc[m][t], w[k], b[k >> 1][t][(k & 1) * 2], b[k >> 1][t][(k & 1) * 2 + 1]);
+        for (int k = 0; k < 4; ++k) mma_16816(acc[m], w[k], b[k >> 1][(k & 1) * 2], b[k >> 1][(k & 1) * 2 + 1]);
       }
     }
     if (ahead < nk) {  // a ring that does not hold the warp's whole share
@@ -263,13 +252,10 @@ __global__ void __launch_bounds__(kWarps * 32, 2) few_rows_kernel(const __grid_c
 #pragma unroll
   for (int m = 0; m < MT; ++m)
     if (MT <= 4 || m < mts) {
-#pragma unroll
-      for (int t = 0; t < NT; ++t) {
-        float* at = red + t * 8 * stride + m * (OUT == kStreamSwiglu ? 8 : 16);
-        float* at2 = OUT == kStreamSwiglu ? at + (a.R >> 1) : at + 8;
-        at[0] = acc[m][t][0], at[stride] = acc[m][t][1];
-        at2[0] = acc[m][t][2], at2[stride] = acc[m][t][3];
-      }
+      float* at = red + m * (OUT == kStreamSwiglu ? 8 : 16);
+      float* at2 = OUT == kStreamSwiglu ? at + (a.R >> 1) : at + 8;
+      at[0] = acc[m][0], at[stride] = acc[m][1];
+      at2[0] = acc[m][2], at2[stride] = acc[m][3];
     }
   __syncthreads();
   auto total = [&](int at) {
@@ -306,25 +292,23 @@ __global__ void __launch_bounds__(kWarps * 32, 2) few_rows_kernel(const __grid_c
 // weights are then on their way, but not two of the same while another SM is idle; rings stop at half of it.
 constexpr int kFewMinSmem = 76 * 1024, kFewHalf = 112 * 1024, kFewMaxSmem = 148 * 1024;
 
-template <int MT, int NT, typename F>
+template <int MT, typename F>
 cudaError_t few_dispatch_tile(int norm, int out, F&& go) {
   const bool bf = out == kStreamBf16, swi = out == kStreamSwiglu;
-  if (norm == 0) return bf ? go(few_rows_kernel<MT, NT, 0, kStreamBf16>) : swi ? go(few_rows_kernel<MT, NT, 0, kStreamSwiglu>) : go(few_rows_kernel<MT, NT, 0, kStreamPartials>);
-  if constexpr (NT == 1) {  // kFewNormRows is one tile
-    if (norm == kNormStack && out != kStreamPartials) return bf ? go(few_rows_kernel<MT, 1, kNormStack, kStreamBf16>) : go(few_rows_kernel<MT, 1, kNormStack, kStreamSwiglu>);
-    if (norm == kNormLm && out != kStreamPartials) return bf ? go(few_rows_kernel<MT, 1, kNormLm, kStreamBf16>) : go(few_rows_kernel<MT, 1, kNormLm, kStreamSwiglu>);
-    if (norm == kAddLm && bf) return go(few_rows_kernel<MT, 1, kAddLm, kStreamBf16>);
-  }
+  if (norm == 0) return bf ? go(few_rows_kernel<MT, 0, kStreamBf16>) : swi ? go(few_rows_kernel<MT, 0, kStreamSwiglu>) : go(few_rows_kernel<MT, 0, kStreamPartials>);
+  if (norm == kNormStack && out != kStreamPartials) return bf ? go(few_rows_kernel<MT, kNormStack, kStreamBf16>) : go(few_rows_kernel<MT, kNormStack, kStreamSwiglu>);
+  if (norm == kNormLm && out != kStreamPartials) return bf ? go(few_rows_kernel<MT, kNormLm, kStreamBf16>) : go(few_rows_kernel<MT, kNormLm, kStreamSwiglu>);
+  if (norm == kAddLm && bf) return go(few_rows_kernel<MT, kAddLm, kStreamBf16>);
   return cudaErrorInvalidValue;
 }
 
 template <typename F>
-cudaError_t few_dispatch(int mts, int nts, int norm, int out, F&& go) {
-  if (mts == 1) return nts == 1 ? few_dispatch_tile<1, 1>(norm, out, go) : few_dispatch_tile<1, 2>(norm, out, go);
-  if (mts == 2) return nts == 1 ? few_dispatch_tile<2, 1>(norm, out, go) : few_dispatch_tile<2, 2>(norm, out, go);
-  if (mts == 3) return nts == 1 ? few_dispatch_tile<3, 1>(norm, out, go) : few_dispatch_tile<3, 2>(norm, out, go);
-  if (mts == 4) return nts == 1 ? few_dispatch_tile<4, 1>(norm, out, go) : few_dispatch_tile<4, 2>(norm, out, go);
-  return nts == 1 ? few_dispatch_tile<10, 1>(norm, out, go) : cudaErrorInvalidValue;
+cudaError_t few_dispatch(int mts, int norm, int out, F&& go) {
+  if (mts == 1) return few_dispatch_tile<1>(norm, out, go);
+  if (mts == 2) return few_dispatch_tile<2>(norm, out, go);
+  if (mts == 3) return few_dispatch_tile<3>(norm, out, go);
+  if (mts == 4) return few_dispatch_tile<4>(norm, out, go);
+  return few_dispatch_tile<10>(norm, out, go);
 }
 
 }  // namespace
@@ -332,9 +316,8 @@ cudaError_t few_dispatch(int mts, int nts, int norm, int out, F&& go) {
 void few_configure() {
   auto set = [](auto kernel) { return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kFewMaxSmem + 1024); };
   for (int mts : {1, 2, 3, 4, 10})
-    for (int nts : {1, 2})
-      for (int norm : {0, (int)kNormStack, (int)kNormLm, (int)kAddLm})
-        for (int out : {kStreamBf16, kStreamPartials, kStreamSwiglu}) few_dispatch(mts, nts, norm, out, set);
+    for (int norm : {0, (int)kNormStack, (int)kNormLm, (int)kAddLm})
+      for (int out : {kStreamBf16, kStreamPartials, kStreamSwiglu}) few_dispatch(mts, norm, out, set);
 }
 
 // Lanes per row: the rows of a warp side by side.
@@ -351,7 +334,7 @@ static int few_rounds(int nkb, int splits, int rows) {
   return (few_per(nkb, splits) * 8 + lanes - 1) / lanes;
 }
 
-bool few_norm_fits(int K, int rows) { return rows <= kFewNormRows && K % kKb == 0 && few_rounds(K / kKb, 1, rows) <= kNormChunks; }
+bool few_norm_fits(int K, int rows) { return rows <= kFewRows && K % kKb == 0 && few_rounds(K / kKb, 1, rows) <= kNormChunks; }
 
 // R weight rows a CTA, K in `splits`: what fits into shared memory and what it would cost (us behind the rows' arrival).
 struct FewShape {
@@ -361,7 +344,7 @@ struct FewShape {
   bool early;         // most of every warp's share is under way before the rows are there
 };
 
-// Fitted to a sweep of R and the splits over nine shapes from 2,048 x 2,048 to 4,096 x 11,264 at one to sixteen rows. The
+// Fitted to a sweep of R and the splits over nine shapes from 2,048 x 2,048 to 4,096 x 11,264 at one to eight rows. The
 // terms: DRAM, less what the rings hold before the rows are there and more where CTAs are fewer than SMs; an SM's copies at
 // 0.1 us each; a warp's chain of blocks, a round trip each unless the ring is deeper (one slot also adds to DRAM, as
 // nothing is under way while a warp works); the rows' bytes. Against the most even load alone: 12,288 x 4,096 19.7 ->
@@ -391,20 +374,19 @@ static FewShape few_shape(int N, int K, int rows, int R, int splits, int sm_coun
 
 int few_plan(FewPlan* plan, const bf16* w, int N, int K, const bf16* x, int rows, int out, bf16* y, int ldy, float* part,
              Epilogue epi, int sm_count) {
-  if (rows < 1 || rows > 16 || K % kKb || N < 1) return -2;
+  if (rows < 1 || rows > kFewRows || K % kKb || N < 1) return -2;
   if (!x && !few_norm_fits(K, rows)) return -2;
   if (out == kStreamSwiglu && N % (2 * kGateGroup)) return -2;
   if ((reinterpret_cast<uintptr_t>(w) & 15) || (reinterpret_cast<uintptr_t>(x) & 15)) return -3;
   FewPlan& p = *plan;
   p.N = N, p.K = K, p.rows = rows, p.out = out, p.x = x, p.y = y, p.ldy = ldy, p.part = part, p.epi = epi;
-  const int most = rows > 8 ? 64 : 160;
   FewShape best{};
   best.cost = 1e30;
   // The most even load of weights and rows, whose tiles are narrow and leave little to do behind the wait, where it has
   // most of every warp's share in its ring by then; otherwise by cost.
   FewShape even = best;
   even.even = 1e30;
-  for (int R = 16; R <= most; R += 16)
+  for (int R = 16; R <= 160; R += 16)
     for (int S : {1, 2, 4}) {
       if (S > 1 && (out != kStreamPartials || S * kWarps > K / kKb)) break;
       const FewShape shape = few_shape(N, K, rows, R, S, sm_count);
@@ -431,7 +413,7 @@ cudaError_t few_launch(const FewPlan& p, const FewNorm& norm, uint32_t* err, cud
   a.nkb = p.K / kKb, a.span = few_span(a.nkb, p.splits), a.per = few_per(a.nkb, p.splits), a.xk = p.xk;
   a.lanes_log2 = few_lanes_log2(p.rows), a.rounds = few_rounds(a.nkb, p.splits, p.rows);
   const dim3 grid((p.N + p.R - 1) / p.R, p.splits);
-  return few_dispatch((p.R + 15) / 16, (p.rows + 7) / 8, norm.kind, p.out, [&](auto kernel) {
+  return few_dispatch(p.R / 16, norm.kind, p.out, [&](auto kernel) {
     return launch_pdl(kernel, grid, dim3(kWarps * 32), p.smem, stream, p.wmap, a);
   });
 }

@@ -1,4 +1,4 @@
-// y[rows, N] = f(x)[rows, K] . w[N, K]^T for up to sixteen rows, where f is the identity or the add + norm that a decoder
+// y[rows, N] = f(x)[rows, K] . w[N, K]^T for up to eight rows, where f is the identity or the add + norm that a decoder
 // stack puts in front of its projections. Launched with programmatic dependent launch, like the GEMM of stream_gemm.h.
 #pragma once
 #include "stream_gemm.h"
@@ -39,7 +39,7 @@ struct FewPlan {
   }
 };
 
-constexpr int kFewNormRows = 8;  // most rows whose norm the projection's CTAs make for themselves
+constexpr int kFewRows = 8;  // one tile of m16n8k16; beyond, the tcgen05 kernel of stream_gemm.h is the faster one
 
 void few_configure();
 // Whether the norm of `rows` rows of K elements can be made by every CTA of the projection.

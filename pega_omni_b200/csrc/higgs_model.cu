@@ -402,7 +402,7 @@ int32_t omni_higgs_create(const omni_higgs_config* config, const omni_tensor* te
   HTRY(halloc(m, &m->embeds, R * h));
   HTRY(halloc(m, &m->x, R * h));
   HTRY(halloc(m, &m->res, R * h));
-  HTRY(halloc(m, &m->res2, (size_t)kFewNormRows * h));
+  HTRY(halloc(m, &m->res2, (size_t)kFewRows * h));
   HTRY(halloc(m, &m->qkv, R * (q + 2 * kvw)));
   HTRY(halloc(m, &m->attn, R * q));
   const size_t Iw = c.audio_adapter ? 2 * I : I;  // widest MLP a row goes through

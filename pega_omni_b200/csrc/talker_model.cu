@@ -344,7 +344,7 @@ int alloc_scratch(omni_talker* m, const StackW& s, int rows, Scratch* out) {
   const omni_stack_config& c = s.cfg;
   TRY(dev_alloc(m, &out->x, (size_t)rows * c.hidden));
   TRY(dev_alloc(m, &out->res, (size_t)rows * c.hidden));
-  TRY(dev_alloc(m, &out->res2, (size_t)kFewNormRows * c.hidden));
+  TRY(dev_alloc(m, &out->res2, (size_t)kFewRows * c.hidden));
   TRY(dev_alloc(m, &out->qkv, (size_t)rows * s.qkv_width()));
   TRY(dev_alloc(m, &out->attn, (size_t)rows * c.q_heads * c.head_dim));
   TRY(dev_alloc(m, &out->gate_up, (size_t)rows * 2 * c.inter));
