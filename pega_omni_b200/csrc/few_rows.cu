@@ -199,7 +199,8 @@ __global__ void __launch_bounds__(kWarps * 32, 2) few_rows_kernel(const __grid_c
   // ---- the rows ----
   if constexpr (NORM == 0) {
     if (rounds <= 1) plain_rows<1>(a, h);
-    else plain_rows<4>(a, h);
+    else if (((rounds + 3) >> 2) & 1) plain_rows<4>(a, h);
+    else plain_rows<8>(a, h);  // a whole number of eights: half the round trips (a duplex tick of 8 4,535 -> 4,485 us)
   } else {
     const bool keep = tile == (int)gridDim.x - 1;
     auto with = [&](auto sums) {
