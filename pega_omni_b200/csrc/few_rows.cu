@@ -9,7 +9,7 @@
 // rows' arrival and the shared memory they take from the rings: at 16 rows a talker step took 3,526 us against 3,361 with the
 // tcgen05 kernel, a Higgs step 2,375 against 2,326, a duplex tick 4,604 against 4,548.
 // The add + norm before a projection is made by every CTA from the summands (L2 broadcast reads, 16 KB to 100 KB) while
-// two pieces a lane suffice; a kernel of its own takes 2.7 us and beyond two pieces is faster. Measured as nodes of a chain
+// one or two pieces a lane suffice (few_norm_fits); a kernel of its own takes 2.7 us and beyond that is faster. Measured as nodes of a chain
 // at one row: 1,024 x 3,072 2.5 us, 6,144 x 1,024 with norm and SwiGLU 4.7 us, 4,096 x 1,024 with norm 4.3 us (4.5 to
 // 5.3 us and 2.7 us for the norm with the tcgen05 kernel of stream_gemm.cu).
 #include "few_rows.h"
@@ -335,7 +335,12 @@ static int few_rounds(int nkb, int splits, int rows) {
   return (few_per(nkb, splits) * 8 + lanes - 1) / lanes;
 }
 
-bool few_norm_fits(int K, int rows) { return rows <= kFewRows && K % kKb == 0 && few_rounds(K / kKb, 1, rows) <= kNormChunks; }
+// Two pieces a lane only for rows of up to 2,048: longer ones (one row, that is) are in front of products long enough to hide
+// the norm's own kernel, a Higgs step of one (2,560) 1,716 us folded and 1,598 apart, a duplex tick (4,096) 3,261 and 3,230;
+// four rows of 1,024 the other way round, a talker step of four 2,431 us and 2,540.
+bool few_norm_fits(int K, int rows) {
+  return rows <= kFewRows && K % kKb == 0 && few_rounds(K / kKb, 1, rows) <= (K <= 2048 ? kNormChunks : 1);
+}
 
 // R weight rows a CTA, K in `splits`: what fits into shared memory and what it would cost (us behind the rows' arrival).
 struct FewShape {
