@@ -111,7 +111,7 @@ struct omni_duplex {
   bf16 *x = nullptr, *x2 = nullptr, *xn = nullptr,  // x2, dx2: the other residual of a few rows' chain
       *qkv = nullptr, *attn = nullptr, *y = nullptr, *gu = nullptr, *act = nullptr;
   bf16 *text_logits = nullptr, *audio_logits = nullptr;  // [max_sessions, text_vocab], [8][max_sessions][card]
-  bf16 *dproj = nullptr, *dx = nullptr, *dx2 = nullptr, *dxn = nullptr, *dqkv = nullptr, *dattn = nullptr, *dact = nullptr;
+  bf16 *dproj = nullptr, *dx = nullptr, *dx2 = nullptr, *dxn = nullptr, *dqkv = nullptr, *dattn = nullptr, *dact = nullptr, *dy = nullptr;
   int32_t *rows_buf = nullptr, *drawn = nullptr, *emitted = nullptr;
 
   // staged inputs: one pinned block mirrored on the device
@@ -329,6 +329,18 @@ int depformer_step(omni_duplex* m, int n, const int32_t* force, const int32_t* s
   const int D = c.dep_dim, H = c.dep_hidden, S = c.max_sessions;
   const float scale = 1.f / std::sqrt((float)kDepHeadDim);
   const Chain chain = m->chain();
+  // the out projections' rows, which the add + norm behind them takes: partial sums up to kChainRows sessions, finished
+  // rows beyond (the GEMM of that size makes no partial sums)
+  Summands y;
+  auto projected = [&](const bf16* w, int K, const bf16* x) -> int {
+    if (n <= kChainRows) {
+      DCUDA(m, chain.gemm(w, D, K, x, n, kStreamPartials, nullptr, D, &y));
+    } else {
+      DCUDA(m, chain.gemm(w, D, K, x, n, kStreamBf16, m->dy, D));
+      y.done = m->dy, y.splits = 0, y.ld = D;
+    }
+    return OMNI_OK;
+  };
   DTRY(gemm(m, m->d_input, kDepSteps * D, c.dim, m->xn, n, m->dproj, kDepSteps * D));
   for (int k = 0; k < kDepSteps; ++k) {
     const bf16* table = k == 0 ? m->d_text_emb : m->d_emb + (size_t)(k - 1) * (c.card + 1) * D;
@@ -336,7 +348,6 @@ int depformer_step(omni_duplex* m, int n, const int32_t* force, const int32_t* s
     DLAUNCH(m, launch_lm_dep_embed_norm(m->dproj, k, table, table_rows, m->drawn, m->d[0].norm1, m->dx, m->dxn, n, D,
                                         c.norm_eps, m->err, m->stream));
     bf16 *res = m->dx, *spare = m->dx2;
-    Summands y;
     auto behind_norm = [&](int kind, const bf16* gain, const bf16* w, int N, int out, bf16* to) -> int {
       DCUDA(m, lm_norm_gemm(chain, kind, y, &res, &spare, gain, c.norm_eps, m->dxn, w, N, D, n, out, to, out == kStreamSwiglu ? N / 2 : N));
       return OMNI_OK;
@@ -347,9 +358,9 @@ int depformer_step(omni_duplex* m, int n, const int32_t* force, const int32_t* s
       if (i > 0) DTRY(behind_norm(kNormLm, L.norm1, qkv, 3 * D, kStreamBf16, m->dqkv));
       else DTRY(gemm(m, qkv, 3 * D, D, m->dxn, n, m->dqkv, 3 * D));
       DLAUNCH(m, launch_lm_dep_kv_attend(m->dqkv, m->dkv[i], k, m->dattn, n, c.dep_heads, scale, m->stream));
-      DCUDA(m, chain.gemm(L.out + (size_t)k * D * D, D, D, m->dattn, n, kStreamPartials, nullptr, D, &y));
+      DTRY(projected(L.out + (size_t)k * D * D, D, m->dattn));
       DTRY(behind_norm(kNormLm, L.norm2, L.gate_in + (size_t)k * 2 * H * D, 2 * H, kStreamSwiglu, m->dact));
-      DCUDA(m, chain.gemm(L.gate_out + (size_t)k * D * H, D, H, m->dact, n, kStreamPartials, nullptr, D, &y));
+      DTRY(projected(L.gate_out + (size_t)k * D * H, H, m->dact));
     }
     bf16* logits = m->audio_logits + (size_t)k * S * c.card;
     DTRY(behind_norm(kAddLm, nullptr, m->d_heads + (size_t)k * c.card * D, c.card, kStreamBf16, logits));
@@ -504,6 +515,7 @@ int32_t omni_duplex_create(const omni_duplex_config* config, const omni_tensor* 
   DTRY(dalloc(m, &m->dqkv, (size_t)S * 3 * DD));
   DTRY(dalloc(m, &m->dattn, (size_t)S * DD));
   DTRY(dalloc(m, &m->dact, (size_t)S * DH));
+  if (S > kChainRows) DTRY(dalloc(m, &m->dy, (size_t)S * DD));
   DTRY(dalloc(m, &m->rows_buf, (size_t)S * kDuplexStreams, true));
   DTRY(dalloc(m, &m->drawn, (size_t)S * kDuplexDrawn, true));
   DTRY(dalloc(m, &m->emitted, (size_t)S * kDuplexDrawn, true));

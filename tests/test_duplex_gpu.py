@@ -303,3 +303,37 @@ def test_warmup_takes_graph_capture_out_of_live_ticks(built_lib):
     assert all(n == first_launches for _, n in steady), (first_launches, steady)
     assert first_ms <= 1.25 * float(np.median([ms for ms, _ in steady])), (first_ms, steady)
     m.close()
+
+
+def test_ticks_of_more_than_256_sessions_agree_with_small_ones(built_lib):
+    """Beyond 256 rows every projection takes another GEMM: the logits are those of the same sessions, twenty a tick."""
+    from pega_omni_b200.duplex import PRESETS, Model, random_checkpoint
+    c = PRESETS["duplex-tiny"]
+    ck = random_checkpoint(c, seed=8, head_std=0.15)
+    rng = np.random.default_rng(11)
+    n, ticks, some = 280, 3, list(range(0, 280, 14))
+    prompts = [make_prompt(c, rng, 2 + i % 3) for i in range(n)]
+    steps = [[forced_step(c, rng, seed=i) for i in range(n)] for _ in range(ticks)]
+
+    def run(model, which):
+        sessions = [model.open() for _ in which]
+        model.start([(s, prompts[i]) for s, i in zip(sessions, which)])
+        rows = []
+        for t in range(ticks):
+            out = model.tick([(s, steps[t][i]) for s, i in zip(sessions, which)]).emitted
+            at = [which.index(i) for i in some]
+            rows.append([(out[k], model.text_logits(k), model.audio_logits(k)) for k in at])
+        return rows
+
+    big = Model.load(0, ck, c, max_sessions=300, max_prefill=2048)
+    big.warmup()  # runs the largest bucket
+    got = run(big, list(range(n)))
+    big.close()
+    small = Model.load(0, ck, c, max_sessions=32, max_prefill=256)
+    want = run(small, some)
+    small.close()
+    for a, b in zip((r for t in got for r in t), (r for t in want for r in t)):
+        assert np.array_equal(a[0], b[0])
+        for x, y in zip(a[1:], b[1:]):  # two bf16 steps, as against the oracle above
+            step = np.exp2(np.floor(np.log2(np.maximum(np.abs(y), 2.0))) - 7)
+            assert float((np.abs(x - y) / step).max()) <= 2.0
