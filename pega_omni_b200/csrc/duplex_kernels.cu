@@ -247,10 +247,10 @@ __global__ void __launch_bounds__(kRopeWarps * 32)
     const float freq = expf((float)threadIdx.x * coef);
     sincosf(freq * (float)pos[n], &sn[threadIdx.x], &cs[threadIdx.x]);
   }
-  int64_t slot = slots[n];
-  if (slot < 0 || (slot >> 4) >= kv_pages) {
+  const int64_t slot = slots[n];
+  if (slot < 0 || (slot >> 4) >= kv_pages) {  // nothing is stored: page 0 is some session's
     if (threadIdx.x == 0) raise(err, kErrBadIndex);
-    slot = 0;
+    return;
   }
   const int tok = (int)(slot & 15);
   __syncthreads();
@@ -441,7 +441,8 @@ __global__ void __launch_bounds__(W * 32)
   const int at = pos[n], len = min(at + 1, context), npages = (len + 15) >> 4, own = (at % context) >> 4;
   const int32_t* my_pages = pages + indptr[n];
   int64_t slot_id = slots[n];
-  if (slot_id < 0 || (slot_id >> 4) >= kv_pages) {
+  const bool owned = slot_id >= 0 && (slot_id >> 4) < kv_pages;  // otherwise the row stores nothing: page 0 is some session's
+  if (!owned) {
     if (threadIdx.x == 0) raise(err, kErrBadIndex);
     slot_id = 0;
   }
@@ -487,7 +488,7 @@ __global__ void __launch_bounds__(W * 32)
     if (warp == 0) {
 #pragma unroll
       for (int k = 0; k < 4; ++k) q[lane * 4 + k] = bf16_round(v[k]);
-    } else {
+    } else if (owned) {
       const float amax = warp_fmax(fmaxf(fmaxf(fabsf(v[0]), fabsf(v[1])), fmaxf(fabsf(v[2]), fabsf(v[3]))));
       const float sc = e4m3_scale(amax), inv = 1.f / sc;
       uint8_t* block = page_head(kv, slot_id >> 4, heads, h);

@@ -409,7 +409,8 @@ __global__ void __launch_bounds__(W * TEAMS * 32, W == 8 ? 1 : 3)
     const int64_t slot = paged ? map.slot[n] : (int64_t)seq * 16 + pos;
     int64_t own = slot >> 4;
     const int tok = (int)(slot & 15);
-    if (own < 0 || own >= kv_pages) {
+    const bool owned = own >= 0 && own < kv_pages;  // otherwise the row stores nothing: page 0 is somebody's
+    if (!owned) {
       if (live && warp == 0 && lane == 0) raise(err, kErrBadIndex);
       own = 0;
     }
@@ -451,7 +452,7 @@ __global__ void __launch_bounds__(W * TEAMS * 32, W == 8 ? 1 : 3)
       if (job < G) rope_head<D>(lo, hi, qwl, qwh, cs, sn, eps);
       else if (job == G) rope_head<D>(lo, hi, kwl, kwh, cs, sn, eps);
       bf16* dst = job < G ? sh.q[job] : job == G ? sh.k[r & 1] : sh.v[r & 1];
-      bf16* page = job < G ? nullptr : kv + kv_offset<D>(own, hk, kh, job - G, tok);
+      bf16* page = job < G || !owned ? nullptr : kv + kv_offset<D>(own, hk, kh, job - G, tok);
       st_half<D>(dst, lane, lo, hi);
       if (page) st_half<D>(page, lane, lo, hi);
     }

@@ -221,3 +221,46 @@ def test_talker_as_a_chain_agrees_with_per_op_kernels(built_lib, sessions):
     a, b = got
     step = np.exp2(np.floor(np.log2(np.maximum(np.abs(b), 2.0))) - 7)
     assert float((np.abs(a - b) / step).max()) <= 2.0
+
+
+@pytest.mark.parametrize("bad", [-16, 1 << 20])
+def test_a_row_without_a_page_stores_nothing(ops, bad):
+    """A slot outside the pool is reported; the pages, page 0 among them, keep what the other rows need."""
+    from pega_omni_b200.ops import OpsError
+    hq, hk, d, lens, lost = 4, 2, 128, [17, 5, 33], 1
+    pos, slot, indptr, pages, count = paged(lens, 3)
+    wrong = slot.clone()
+    wrong[lost] = bad
+    qkv, qn, kn = rand((3, (hq + 2 * hk) * d), 31), rand((d,), 32, 0.2) + 1, rand((d,), 33, 0.2) + 1
+    kv = rand((count, hk, 2, 16, d), 34)
+    own = (int(slot[lost]) // 16, slice(None), slice(None), int(slot[lost]) % 16)
+    want, before = kv.clone(), kv[own].clone()
+    out = torch.zeros((3, hq * d), dtype=torch.bfloat16, device="cuda")
+    torch.cuda.synchronize()
+    ops.decode_attend(qkv, qn, kn, want, count, pos, slot, indptr, pages, hq, hk, d, 1e-6, 1e6, out)
+    ops.sync()
+    want[own] = before
+    torch.cuda.synchronize()
+    ops.decode_attend(qkv, qn, kn, kv, count, pos, wrong, indptr, pages, hq, hk, d, 1e-6, 1e6, out)
+    with pytest.raises(OpsError):
+        ops.sync()
+    assert torch.equal(kv, want)
+
+
+@pytest.mark.parametrize("in_one", [True, False])
+def test_a_ring_row_without_a_page_stores_nothing(ops, in_one):
+    from pega_omni_b200.ops import OpsError
+    heads, context, sessions = 2, 32, 3
+    table, indptr = i32([4, 1, 0, 2, 5, 3]), i32([0, 2, 4, 6])
+    at, slot = i32([3, 20, 9]), i32([4 * 16 + 3, 2 * 16 + 4, 1 << 20])
+    qkv = rand((sessions, 3 * heads * 128), 41)
+    kv = torch.zeros(6, heads, 2 * 16 * 128 + 2 * 16 * 4, dtype=torch.uint8, device="cuda")
+    out = torch.zeros((sessions, heads * 128), dtype=torch.bfloat16, device="cuda")
+    torch.cuda.synchronize()
+    if in_one:
+        ops.lm_decode_attend(qkv, kv, 6, at, slot, indptr, table, heads, -0.14, 0.1, context, out)
+    else:
+        ops.lm_rope_attend(qkv, kv, 6, at, slot, None, indptr, table, heads, -0.14, 0.1, context, out)
+    with pytest.raises(OpsError):
+        ops.sync()
+    assert not kv[[0, 1, 3, 5]].any() and kv[4].any() and kv[2].any()
