@@ -18,13 +18,14 @@
 #include <cmath>
 #include <type_traits>
 
+#include "few_share.h"
 #include "pdl.cuh"
 #include "sm100.cuh"
 
 namespace omni {
 namespace {
 
-constexpr int kWarps = 8, kKb = 64, kFewSlots = 8;
+constexpr int kWarps = kFewWarps, kKb = kFewKb, kFewSlots = 8;
 constexpr int kNormChunks = 2;  // 8-element pieces of the rows that a lane holds across the norm's sum
 
 struct FewArgs {
@@ -55,17 +56,16 @@ __device__ __forceinline__ void st_shared16(uint32_t addr, const uint4& v) {
   asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
 }
 
-// Where a lane's pieces of the rows lie: piece first + j * lanes of this warp's share of row n, 16 bytes each.
-struct Share {
-  int warp, lane, n, first, lanes, pieces, c0;  // c0: first column of the warp's share
-  bool live;
+// Where a lane's pieces of the rows lie (few_share.h), and where they go.
+struct Share : FewShare {
+  int warp;
   uint32_t xs;  // row n's share in shared memory
 };
 
 // The add + norm's rows, RD pieces a lane, from S partial sums; `keep`: this CTA stores the residual.
 template <int NORM, int S, int RD>
 __device__ __forceinline__ void norm_rows(const FewArgs& a, const Share& h, bool keep, float (*ss_s)[kWarps], const uint4* gain) {
-  const int64_t at = (int64_t)(h.live ? h.n : 0) * a.K + h.c0 + h.first * 8;
+  const int64_t at = few_at(h, a.K);
   const float* part = a.norm.sum.part + at;
   constexpr int B = S >= 4 ? 2 : RD < 4 ? RD : RD == 4 && S == 1 ? 4 : 2;  // pieces under way at a time
   float v[RD][8], ss = 0.f;
@@ -75,7 +75,7 @@ __device__ __forceinline__ void norm_rows(const FewArgs& a, const Share& h, bool
     float4 f[B][S][2];
 #pragma unroll
     for (int j = 0; j < B; ++j) {
-      const int o = h.first + (j0 + j) * h.lanes < h.pieces ? (j0 + j) * h.lanes * 8 : 0;
+      const int o = few_step(h, j0 + j);
       r[j] = __ldcg(reinterpret_cast<const uint4*>(a.norm.res_in + at + o));
 #pragma unroll
       for (int s = 0; s < S; ++s) {
@@ -149,8 +149,7 @@ __global__ void __launch_bounds__(kWarps * 32, 2) few_rows_kernel(const __grid_c
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int tile = blockIdx.x, split = blockIdx.y;
   // k-blocks: `span` per split, `per` per warp, the last of each fewer
-  const int kb0 = split * a.span + warp * a.per;
-  const int nk = max(0, min(min(a.per, a.span - warp * a.per), a.nkb - kb0));
+  const int kb0 = few_first(warp, split, a.span, a.per), nk = few_count(warp, split, a.span, a.per, a.nkb);
   const uint32_t slot_bytes = (uint32_t)a.R * 128u;
   const uint32_t ring0 = (smem_addr(few_smem_raw) + 1023u) & ~1023u;
   const uint32_t ring = ring0 + (uint32_t)(warp * a.slots) * slot_bytes;
@@ -173,9 +172,8 @@ __global__ void __launch_bounds__(kWarps * 32, 2) few_rows_kernel(const __grid_c
 
   // ---- everything that does not depend on the rows comes before grid_wait(), the first weights' arrival included ----
   Share h;
-  h.warp = warp, h.lane = lane, h.lanes = 1 << a.lanes_log2;
-  h.n = lane >> a.lanes_log2, h.first = lane & (h.lanes - 1), h.pieces = nk * 8, h.c0 = kb0 * kKb;
-  h.live = h.n < a.rows, h.xs = xs + (uint32_t)(h.n * a.xk) * 2u;
+  static_cast<FewShare&>(h) = few_share(lane, kb0, nk, a.lanes_log2, a.rows);
+  h.warp = warp, h.xs = xs + (uint32_t)(h.n * a.xk) * 2u;
   const int mts = MT <= 4 ? MT : a.R >> 4;
   // ldmatrix rows of this lane: weights [0, 8) k 0..7, [8, 16) k 0..7, [0, 8) k 8..15, [8, 16) k 8..15; x rows past the
   // last read row 0 (their columns of the result are not stored)
@@ -321,15 +319,6 @@ void few_configure() {
       for (int out : {kStreamBf16, kStreamPartials, kStreamSwiglu}) few_dispatch(mts, norm, out, set);
 }
 
-// Lanes per row: the rows of a warp side by side.
-static int few_lanes_log2(int rows) {
-  int log2 = 5;
-  while ((32 >> log2) < rows) --log2;
-  return log2;
-}
-// k-blocks per split and per warp.
-static int few_span(int nkb, int splits) { return (nkb + splits - 1) / splits; }
-static int few_per(int nkb, int splits) { return (few_span(nkb, splits) + kWarps - 1) / kWarps; }
 static int few_rounds(int nkb, int splits, int rows) {
   const int lanes = 1 << few_lanes_log2(rows);
   return (few_per(nkb, splits) * 8 + lanes - 1) / lanes;
