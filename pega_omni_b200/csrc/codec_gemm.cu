@@ -134,7 +134,7 @@ __global__ void __launch_bounds__(kConvThreads, 1)
   if (warp < 2) {
     if (lane == 0) {
       const bool is_w = warp == 0;
-      if (!is_w) asm volatile("fence.proxy.async.global;" ::: "memory");  // rows written by ordinary stores, read by TMA
+      if (!is_w) fence_async_global();  // rows written by ordinary stores, read by TMA
       int stage = 0, done = 0;
       uint32_t phase = 0;
       bool alive = true;

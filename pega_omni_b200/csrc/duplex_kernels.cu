@@ -375,6 +375,7 @@ __global__ void __launch_bounds__(kAttendWarps * 32)
   __syncthreads();
 
   unsigned char* mine = slots + (size_t)warp * 2 * kAttendSlotBytes;
+  sm100::fence_async_global();  // keys and values written by ordinary stores, read by bulk copies
   auto fetch = [&](int pi, int slot) {  // lane 0: one bulk copy of page pi's block for this head
     int64_t page = my_pages[pi];
     if (page < 0 || page >= kv_pages) {
@@ -497,7 +498,7 @@ __global__ void __launch_bounds__(W * 32)
       const uint32_t hi = __nv_cvt_float2_to_fp8x2(make_float2(v[2] * inv, v[3] * inv), __NV_SATFINITE, __NV_E4M3);
       *reinterpret_cast<uint32_t*>(block + (is_v * 16 + tok) * kHeliumHeadDim + lane * 4) = lo | hi << 16;
       if (lane == 0) reinterpret_cast<float*>(block + 2 * 16 * kHeliumHeadDim + is_v * 64)[tok] = sc;
-      asm volatile("fence.proxy.async.global;" ::: "memory");
+      sm100::fence_async_global();
     }
   }
   __syncthreads();

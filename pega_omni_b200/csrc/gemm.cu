@@ -225,6 +225,7 @@ __global__ void __launch_bounds__(128, 1)
   bool ok = true;
   if (warp == 0) {
     if (lane == 0) {
+      fence_async_global();  // rows written by ordinary stores, read by TMA
       int stage = 0;
       uint32_t phase = 0;
       for (int kb = kb_begin; kb < kb_end; kb += kbs) {
@@ -432,6 +433,7 @@ __global__ void __launch_bounds__(128, 1)
 
   if (warp == 0) {
     if (lane == 0) {
+      fence_async_global();  // rows written by ordinary stores, read by TMA
       int stage = 0;
       uint32_t phase = 0;
       for (int kb = 0; kb < nkb; kb += kbs) {

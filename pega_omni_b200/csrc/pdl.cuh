@@ -1,13 +1,17 @@
 // Programmatic dependent launch. A kernel started with launch_pdl() may begin while the kernel before it in the stream
 // (or graph) is still running: everything it does before grid_wait() overlaps that kernel's tail - barrier and TMEM
 // set-up, descriptor and weight fetches - and grid_wait() returns once the kernel before it has completed and its writes
-// are visible. The rules every kernel launched this way keeps:
-//   - before grid_wait() it reads only what no kernel of the same stream writes (weights, tables, staged inputs), and
+// are visible.
+// The rules every kernel launched this way keeps:
+//   - before grid_wait() it reads only what no kernel of the same call writes - weights, tables, staged inputs, and what
+//     earlier calls left (a call starts behind a copy in its stream, which is ordered behind everything before it) - and
 //     writes nothing to global memory;
-//   - every CTA passes grid_wait() in at least one thread before it ends, on every path, so that a kernel's completion
-//     implies that of all kernels before it;
-//   - grid_trigger() comes first: it lets the next kernel be scheduled as soon as all CTAs of this one have started
-//     (what the next kernel reads is ordered by its own grid_wait(), not by the trigger).
+//   - behind grid_wait(), TMA and bulk copies of what an earlier kernel of the call wrote come behind fence_async_global()
+//     in the thread that issues them (sm100.cuh);
+//   - at least one thread of it passes grid_wait() on every path, so that its completion implies that of all kernels
+//     before it;
+//   - grid_trigger() comes first, or as soon as the CTA holds its TMEM columns: it lets the next kernel be scheduled once
+//     all CTAs of this one have started (what the next kernel reads is ordered by its own grid_wait(), not by the trigger).
 #pragma once
 #include <cuda_runtime.h>
 

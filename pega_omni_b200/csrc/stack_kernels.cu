@@ -294,6 +294,7 @@ __global__ void __launch_bounds__(kAttnWarps * 32) attend_kernel(const bf16* __r
   for (int i = threadIdx.x; i < G * D; i += blockDim.x) sh.qs[i / D][i % D] = __bfloat162float(q[i]);
   __syncthreads();
   const int warp = threadIdx.x >> 5;
+  sm100::fence_async_global();  // keys and values written by ordinary stores, read by bulk copies
   PageStage<kAttnSlots> stage{attend_slots + (size_t)warp * kAttnSlots * kv_block_bytes<D>(), bars + warp * kAttnSlots, 0u, err};
   attend_pages<D, G, kAttnWarps>(sh, kv, at.pages, at.seq, at.pos + 1, hk, kh, scale, out + ((int64_t)n * hq + kh * G) * D,
                                  threadIdx.x, sampler::CtaSync(), &stage);

@@ -132,7 +132,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   } else if (warp == 1) {
     if (lane == 0) {
       grid_wait();
-      asm volatile("fence.proxy.async.global;" ::: "memory");  // rows written by ordinary stores, read by TMA
+      fence_async_global();  // rows written by ordinary stores, read by TMA
       int slot = 0;
       uint32_t phase = 0;
       for (int i = 0; i < n_st; ++i) {

@@ -134,7 +134,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kWideThreads, 1)
 
   if (warp == 0) {
     if (lane == 0) {
-      asm volatile("fence.proxy.async.global;" ::: "memory");  // rows written by ordinary stores, read by TMA
+      fence_async_global();  // rows written by ordinary stores, read by TMA
       int slot = 0;
       uint32_t phase = 1;
       bool alive = true;
