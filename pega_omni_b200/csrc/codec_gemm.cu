@@ -242,7 +242,7 @@ __global__ void __launch_bounds__(kConvThreads, 1)
         if (a.kind == kConvAccumulate && c0 + 8 * chunk < a.tn && nn + 8 <= a.N) {
 #pragma unroll
           for (int i = 0; i < 4; ++i)
-            if (stream_of[i] < live_streams) old[i] = *reinterpret_cast<const uint4*>(tile_y + row_at[i] + nn);
+            if (stream_of[i] < live_streams) old[i] = __ldcg(reinterpret_cast<const uint4*>(tile_y + row_at[i] + nn));
         }
       };
       load_old(32 * turn);

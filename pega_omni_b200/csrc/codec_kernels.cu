@@ -53,7 +53,7 @@ __global__ void codec_rvq_kernel(const int32_t* __restrict__ codes, const bf16* 
 }
 
 // A warp per row, dim a multiple of 256 up to 1024.
-__global__ void codec_add_norm_kernel(const bf16* add, int64_t add_stride, bf16* __restrict__ res,
+__global__ void codec_add_norm_kernel(const bf16* add, int64_t add_stride, bf16* res,
                                       const bf16* __restrict__ w, bf16* out, int rows, int dim, float eps) {
   grid_trigger();
   grid_wait();  // out may be add
@@ -68,8 +68,8 @@ __global__ void codec_add_norm_kernel(const bf16* add, int64_t add_stride, bf16*
     const int c = (k * 32 + lane) * 8;
     if (c < dim) {
       float x[8];
-      ld8v(a + c, x);
-      ld8v(rr + c, v[k]);
+      ld8cg(a + c, x);
+      ld8cg(rr + c, v[k]);
 #pragma unroll
       for (int e = 0; e < 8; ++e) {
         v[k][e] += x[e];
@@ -100,7 +100,7 @@ __global__ void codec_add_norm_kernel(const bf16* add, int64_t add_stride, bf16*
 constexpr int kWindowWarps = (kWindow + 15) / 16;
 
 __global__ void __launch_bounds__(kWindowWarps * 32)
-    codec_window_attend_kernel(const bf16* __restrict__ qkv, CodecStateRef st, int64_t ring_offset, bf16* __restrict__ out,
+    codec_window_attend_kernel(const bf16* qkv, CodecStateRef st, int64_t ring_offset, bf16* __restrict__ out,
                                int heads, float theta) {
   grid_trigger();
   __shared__ alignas(16) bf16 sq[kWindowWarps][kHeadDim], sk[kHeadDim], sv[kHeadDim];
@@ -129,12 +129,12 @@ __global__ void __launch_bounds__(kWindowWarps * 32)
   dattn::State<kHeadDim> state;
   state.reset();
   if (ntok > 0) {
-    const float q_lo = __bfloat162float(row[lane]), q_hi = __bfloat162float(row[lane + 32]);
+    const float q_lo = __bfloat162float(__ldcg(row + lane)), q_hi = __bfloat162float(__ldcg(row + lane + 32));
     sq[warp][lane] = __float2bfloat16(q_lo * cs - q_hi * sn);
     sq[warp][lane + 32] = __float2bfloat16(q_hi * cs + q_lo * sn);
     if (mine) {  // k and v of the frame: to the ring and into the page
-      const float k_lo = __bfloat162float(row[width + lane]), k_hi = __bfloat162float(row[width + lane + 32]);
-      const uint32_t v2 = reinterpret_cast<const uint32_t*>(row + 2 * width)[lane];
+      const float k_lo = __bfloat162float(__ldcg(row + width + lane)), k_hi = __bfloat162float(__ldcg(row + width + lane + 32));
+      const uint32_t v2 = __ldcg(reinterpret_cast<const uint32_t*>(row + 2 * width) + lane);
       const bf16 ka = __float2bfloat16(k_lo * cs - k_hi * sn), kb = __float2bfloat16(k_hi * cs + k_lo * sn);
       bf16* at = ring + (int64_t)own * width;
       at[lane] = sk[lane] = ka;
@@ -171,7 +171,7 @@ __global__ void __launch_bounds__(kWindowWarps * 32)
   }
 }
 
-__global__ void codec_silu_mul_kernel(const bf16* __restrict__ gate_up, bf16* __restrict__ out, int inter, int64_t total) {
+__global__ void codec_silu_mul_kernel(const bf16* gate_up, bf16* __restrict__ out, int inter, int64_t total) {
   grid_trigger();
   grid_wait();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -179,20 +179,20 @@ __global__ void codec_silu_mul_kernel(const bf16* __restrict__ gate_up, bf16* __
   const int per = inter / 8;
   const int64_t r = i / per, c = i % per * 8;
   float g[8], u[8];
-  ld8v(gate_up + r * 2 * inter + c, g);
-  ld8v(gate_up + r * 2 * inter + inter + c, u);
+  ld8cg(gate_up + r * 2 * inter + c, g);
+  ld8cg(gate_up + r * 2 * inter + inter + c, u);
 #pragma unroll
   for (int k = 0; k < 8; ++k) g[k] = bf16_round(g[k] / (1.f + __expf(-g[k]))) * u[k];
   st8v(out + i * 8, g);
 }
 
-__global__ void codec_bias_gelu_kernel(bf16* __restrict__ x, const bf16* __restrict__ bias, int cols, int64_t total) {
+__global__ void codec_bias_gelu_kernel(bf16* x, const bf16* __restrict__ bias, int cols, int64_t total) {
   grid_trigger();
   grid_wait();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= total) return;
   float v[8], b[8];
-  ld8v(x + i * 8, v);
+  ld8cg(x + i * 8, v);
   ld8v(bias + i % (cols / 8) * 8, b);
 #pragma unroll
   for (int k = 0; k < 8; ++k) {
@@ -211,7 +211,7 @@ __device__ __forceinline__ void bias_snake8(float* v, const bf16* bias, const fl
   for (int k = 0; k < 8; ++k) v[k] = snake_beta(v[k] + b[k], al[k], ib[k]);
 }
 
-__global__ void codec_bias_snake_kernel(const bf16* __restrict__ x, const bf16* __restrict__ bias,
+__global__ void codec_bias_snake_kernel(const bf16* x, const bf16* __restrict__ bias,
                                         const float* __restrict__ alpha, const float* __restrict__ inv_b,
                                         bf16* __restrict__ out, int cols, int64_t total) {
   grid_trigger();
@@ -219,14 +219,14 @@ __global__ void codec_bias_snake_kernel(const bf16* __restrict__ x, const bf16* 
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= total) return;
   float v[8];
-  ld8v(x + i * 8, v);
+  ld8cg(x + i * 8, v);
   bias_snake8(v, bias, alpha, inv_b, (int)(i % (cols / 8)) * 8);
   st8v(out + i * 8, v);
 }
 
 // One thread per eight channels of a padded row: rows below H come from the history, the rest are the transformed
 // frame; whatever lands in the last H rows is also the next frame's history.
-__global__ void codec_stage_kernel(const bf16* __restrict__ x, const bf16* __restrict__ bias, const float* __restrict__ alpha,
+__global__ void codec_stage_kernel(const bf16* x, const bf16* __restrict__ bias, const float* __restrict__ alpha,
                                    const float* __restrict__ inv_b, CodecStateRef st, int64_t hist_offset,
                                    bf16* __restrict__ padded, int T, int C, int H, int64_t total) {
   grid_trigger();
@@ -245,7 +245,7 @@ __global__ void codec_stage_kernel(const bf16* __restrict__ x, const bf16* __res
     u = *reinterpret_cast<const uint4*>(hist + (p & 1) * half + (int64_t)r * C + c);
   } else {
     float v[8];
-    ld8v(x + ((int64_t)s * T + r - H) * C + c, v);
+    ld8cg(x + ((int64_t)s * T + r - H) * C + c, v);
     if (alpha != nullptr) {
       bias_snake8(v, bias, alpha, inv_b, c);
     } else {
@@ -260,7 +260,7 @@ __global__ void codec_stage_kernel(const bf16* __restrict__ x, const bf16* __res
   if (r >= T) *reinterpret_cast<uint4*>(hist + ((p + 1) & 1) * half + (int64_t)(r - T) * C + c) = u;
 }
 
-__global__ void codec_gather_taps_kernel(const bf16* __restrict__ padded, bf16* __restrict__ col, int T, int C, int taps,
+__global__ void codec_gather_taps_kernel(const bf16* padded, bf16* __restrict__ col, int T, int C, int taps,
                                          int dil, int64_t total) {
   grid_trigger();
   grid_wait();
@@ -273,10 +273,10 @@ __global__ void codec_gather_taps_kernel(const bf16* __restrict__ padded, bf16* 
   g /= taps;
   const int t = (int)(g % T), s = (int)(g / T);
   *reinterpret_cast<uint4*>(col + (((int64_t)s * T + t) * taps + j) * C + c) =
-      *reinterpret_cast<const uint4*>(padded + ((int64_t)s * P + t + j * dil) * C + c);
+      __ldcg(reinterpret_cast<const uint4*>(padded + ((int64_t)s * P + t + j * dil) * C + c));
 }
 
-__global__ void codec_overlap_add_kernel(const bf16* __restrict__ z, const bf16* __restrict__ bias, CodecStateRef st,
+__global__ void codec_overlap_add_kernel(const bf16* z, const bf16* __restrict__ bias, CodecStateRef st,
                                          int64_t prev_offset, bf16* __restrict__ out, int L, int r, int C, int64_t total) {
   grid_trigger();
   grid_wait();
@@ -291,15 +291,15 @@ __global__ void codec_overlap_add_kernel(const bf16* __restrict__ z, const bf16*
   const bf16* zs = z + (int64_t)s * L * w;
   float v[8], y[8];
   ld8v(bias + c, v);
-  ld8v(zs + l * w + (int64_t)j * C + c, y);
+  ld8cg(zs + l * w + (int64_t)j * C + c, y);
 #pragma unroll
   for (int k = 0; k < 8; ++k) v[k] += y[k];
   if (l > 0) {
-    ld8v(zs + (l - 1) * w + (int64_t)(j + r) * C + c, y);
+    ld8cg(zs + (l - 1) * w + (int64_t)(j + r) * C + c, y);
   } else {  // the row before the frame's first: kept from the last call; this thread alone touches the entry
     bf16* prev = slot_ptr(st, s, prev_offset) + (int64_t)j * C + c;
     ld8v(prev, y);
-    *reinterpret_cast<uint4*>(prev) = *reinterpret_cast<const uint4*>(zs + (L - 1) * w + (int64_t)(j + r) * C + c);
+    *reinterpret_cast<uint4*>(prev) = __ldcg(reinterpret_cast<const uint4*>(zs + (L - 1) * w + (int64_t)(j + r) * C + c));
   }
 #pragma unroll
   for (int k = 0; k < 8; ++k) v[k] += y[k];
@@ -308,7 +308,7 @@ __global__ void codec_overlap_add_kernel(const bf16* __restrict__ z, const bf16*
 
 // One block per row, eight channels per thread; the block is a whole number of warps, threads past the last channel
 // only take part in the two block-wide sums.
-__global__ void codec_dwconv_ln_kernel(const bf16* __restrict__ z, const bf16* __restrict__ zb, const bf16* __restrict__ w,
+__global__ void codec_dwconv_ln_kernel(const bf16* z, const bf16* __restrict__ zb, const bf16* __restrict__ w,
                                        const bf16* __restrict__ b, const bf16* __restrict__ ln_w,
                                        const bf16* __restrict__ ln_b, CodecStateRef st, int64_t hist_offset,
                                        bf16* __restrict__ xin, bf16* __restrict__ out, int T, int r, int C, float eps) {
@@ -332,7 +332,7 @@ __global__ void codec_dwconv_ln_kernel(const bf16* __restrict__ z, const bf16* _
       float v[8], wt[8];
       if (src >= 0) {
         float bias[8];
-        ld8v(z + ((int64_t)s * T + src) * C + c, v);
+        ld8cg(z + ((int64_t)s * T + src) * C + c, v);
         ld8v(zb + (int64_t)(src % r) * C + c, bias);
 #pragma unroll
         for (int k = 0; k < 8; ++k) v[k] = bf16_round(v[k] + bias[k]);
@@ -382,7 +382,7 @@ constexpr int kOutTile = 64;  // output samples per block
 // channel it reads ten rows and seven weights for 28 multiply-adds, and sixteen lanes reduce. Rows are C + 4 floats
 // apart, so the two row groups a warp reads (four rows apart) fall into opposite halves of the banks.
 __global__ void __launch_bounds__(256)
-    codec_out_conv_kernel(const bf16* __restrict__ x, const bf16* __restrict__ bias, const float* __restrict__ alpha,
+    codec_out_conv_kernel(const bf16* x, const bf16* __restrict__ bias, const float* __restrict__ alpha,
                           const float* __restrict__ inv_b, const bf16* __restrict__ w, const bf16* __restrict__ wb,
                           CodecStateRef st, int64_t hist_offset, float* __restrict__ wav, int T, int C) {
   grid_trigger();
@@ -404,7 +404,7 @@ __global__ void __launch_bounds__(256)
     if (src < 0) {
       ld8v(old + (int64_t)(H + src) * C + c, v);
     } else {
-      ld8v(x + ((int64_t)s * T + src) * C + c, v);
+      ld8cg(x + ((int64_t)s * T + src) * C + c, v);
       bias_snake8(v, bias, alpha, inv_b, c);
 #pragma unroll
       for (int k = 0; k < 8; ++k) v[k] = bf16_round(v[k]);

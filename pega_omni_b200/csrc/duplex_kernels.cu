@@ -83,27 +83,27 @@ __device__ __forceinline__ void norm_row(const float* v, const bf16* alpha, bf16
   st8(out + threadIdx.x * 8, y);
 }
 
-__global__ void lm_norm_kernel(const bf16* __restrict__ x, const bf16* __restrict__ alpha, bf16* __restrict__ out,
+__global__ void lm_norm_kernel(const bf16* x, const bf16* __restrict__ alpha, bf16* __restrict__ out,
                                int dim, float eps) {
   grid_trigger();
   grid_wait();
   __shared__ float scratch[32];
   const int64_t at = (int64_t)blockIdx.x * dim;
   float v[8];
-  ld8(x + at + threadIdx.x * 8, v);
+  ld8cg(x + at + threadIdx.x * 8, v);
   norm_row(v, alpha, out + at, dim, eps, scratch);
 }
 
 // x = bf16(x + y), out = norm(x) over the rounded sum (lm.cu:95-106; out == nullptr: `lm_add`, lm.cu:109-120)
-__global__ void lm_add_norm_kernel(const bf16* __restrict__ y, bf16* __restrict__ x, const bf16* __restrict__ alpha,
+__global__ void lm_add_norm_kernel(const bf16* y, bf16* x, const bf16* __restrict__ alpha,
                                    bf16* __restrict__ out, int dim, float eps) {
   grid_trigger();
   grid_wait();
   __shared__ float scratch[32];
   const int64_t at = (int64_t)blockIdx.x * dim + threadIdx.x * 8;
   float v[8], u[8];
-  ld8(x + at, v);
-  ld8(y + at, u);
+  ld8cg(x + at, v);
+  ld8cg(y + at, u);
 #pragma unroll
   for (int k = 0; k < 8; ++k) v[k] = bf16_round(v[k] + u[k]);
   st8(x + at, v);
@@ -237,7 +237,7 @@ __device__ __forceinline__ float e4m3_scale(float amax) { return fmaxf(amax * (1
 constexpr int kRopeWarps = 8, kRopeParts = 4;
 
 __global__ void __launch_bounds__(kRopeWarps * 32)
-    lm_rope_kv_kernel(bf16* __restrict__ qkv, const int32_t* __restrict__ pos, const int32_t* __restrict__ slots, void* kv,
+    lm_rope_kv_kernel(bf16* qkv, const int32_t* __restrict__ pos, const int32_t* __restrict__ slots, void* kv,
                       int heads, float coef, int kv_pages, uint32_t* err) {
   grid_trigger();
   grid_wait();
@@ -256,7 +256,7 @@ __global__ void __launch_bounds__(kRopeWarps * 32)
   __syncthreads();
   for (int head = blockIdx.y * kRopeWarps + warp; head < 3 * heads; head += kRopeWarps * kRopeParts) {
     bf16* src = qkv + ((int64_t)n * 3 * heads + head) * kHeliumHeadDim + lane * 4;
-    const uint2 raw = *reinterpret_cast<const uint2*>(src);
+    const uint2 raw = __ldcg(reinterpret_cast<const uint2*>(src));
     const float2 p0 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.x));
     const float2 p1 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.y));
     float v[4] = {p0.x, p0.y, p1.x, p1.y};
@@ -352,7 +352,7 @@ struct AttendShared {
 };
 
 __global__ void __launch_bounds__(kAttendWarps * 32)
-    lm_attend_kernel(const bf16* __restrict__ qkv, const void* kv, const int32_t* __restrict__ pos,
+    lm_attend_kernel(const bf16* qkv, const void* kv, const int32_t* __restrict__ pos,
                      const int32_t* __restrict__ seq, const int32_t* __restrict__ indptr,
                      const int32_t* __restrict__ pages, bf16* __restrict__ out, int heads, float scale, int context,
                      int kv_pages, uint32_t* err) {
@@ -366,7 +366,7 @@ __global__ void __launch_bounds__(kAttendWarps * 32)
   const int len = min(pos[n] + 1, context), npages = (len + 15) >> 4;
   const int32_t* my_pages = pages + indptr[s];
   if (threadIdx.x < kHeliumHeadDim)
-    sh.q[threadIdx.x] = __bfloat162float(qkv[((int64_t)n * 3 * heads + h) * kHeliumHeadDim + threadIdx.x]);
+    sh.q[threadIdx.x] = __bfloat162float(__ldcg(qkv + ((int64_t)n * 3 * heads + h) * kHeliumHeadDim + threadIdx.x));
   if (lane == 0) {
     sm100::mbar_init(sm100::smem_addr(&sh.bar[warp][0]), 1);
     sm100::mbar_init(sm100::smem_addr(&sh.bar[warp][1]), 1);
@@ -430,7 +430,7 @@ __global__ void __launch_bounds__(kAttendWarps * 32)
 // the row is written to comes last: its writers' stores are fenced for the bulk copy that reads them back.
 template <int W>
 __global__ void __launch_bounds__(W * 32)
-    lm_rope_attend_kernel(const bf16* __restrict__ qkv, void* kv, const int32_t* __restrict__ pos,
+    lm_rope_attend_kernel(const bf16* qkv, void* kv, const int32_t* __restrict__ pos,
                           const int32_t* __restrict__ slots, const int32_t* __restrict__ indptr,
                           const int32_t* __restrict__ pages, bf16* __restrict__ out, int heads, float coef, float scale,
                           int context, int kv_pages, uint32_t* err) {
@@ -539,21 +539,21 @@ __global__ void __launch_bounds__(W * 32)
 }
 
 // `lm_dep_embed_norm` (lm.cu:301-313)
-__global__ void lm_dep_embed_norm_kernel(const bf16* __restrict__ projected, int k, const bf16* __restrict__ table,
-                                         int table_rows, const int32_t* __restrict__ drawn,
+__global__ void lm_dep_embed_norm_kernel(const bf16* projected, int k, const bf16* __restrict__ table, int table_rows,
+                                         const int32_t* drawn,
                                          const bf16* __restrict__ alpha, bf16* __restrict__ x, bf16* __restrict__ xn,
                                          int dim, float eps, uint32_t* err) {
   grid_trigger();
   grid_wait();
   __shared__ float scratch[32];
   const int s = blockIdx.x, c = threadIdx.x * 8;
-  int64_t id = drawn[s * kDuplexDrawn + k];
+  int64_t id = __ldcg(drawn + s * kDuplexDrawn + k);
   if (id < 0 || id >= table_rows) {
     if (threadIdx.x == 0) raise(err, kErrBadIndex);
     id = 0;
   }
   float v[8], e[8];
-  ld8(projected + ((int64_t)s * kDepSteps + k) * dim + c, v);
+  ld8cg(projected + ((int64_t)s * kDepSteps + k) * dim + c, v);
   ld8(table + id * dim + c, e);
 #pragma unroll
   for (int j = 0; j < 8; ++j) v[j] = bf16_round(v[j] + e[j]);
@@ -563,7 +563,7 @@ __global__ void lm_dep_embed_norm_kernel(const bf16* __restrict__ projected, int
 
 // `lm_dep_kv_attend` (lm.cu:319-366): a warp per (session, head), a lane owns two of the 64 dims; the step's own K
 // and V stay in registers.
-__global__ void lm_dep_kv_attend_kernel(const bf16* __restrict__ qkv, bf16* __restrict__ ws, int step,
+__global__ void lm_dep_kv_attend_kernel(const bf16* qkv, bf16* ws, int step,
                                         bf16* __restrict__ out, int heads, float scale) {
   grid_trigger();
   grid_wait();
@@ -572,9 +572,9 @@ __global__ void lm_dep_kv_attend_kernel(const bf16* __restrict__ qkv, bf16* __re
   const int width = heads * kDepHeadDim;
   const bf16* row = qkv + (int64_t)s * 3 * width;
   const int at = h * kDepHeadDim + lane * 2;
-  const __nv_bfloat162 q2 = *reinterpret_cast<const __nv_bfloat162*>(row + at);
-  const __nv_bfloat162 k2 = *reinterpret_cast<const __nv_bfloat162*>(row + width + at);
-  const __nv_bfloat162 v2 = *reinterpret_cast<const __nv_bfloat162*>(row + 2 * width + at);
+  const __nv_bfloat162 q2 = __ldcg(reinterpret_cast<const __nv_bfloat162*>(row + at));
+  const __nv_bfloat162 k2 = __ldcg(reinterpret_cast<const __nv_bfloat162*>(row + width + at));
+  const __nv_bfloat162 v2 = __ldcg(reinterpret_cast<const __nv_bfloat162*>(row + 2 * width + at));
   bf16* base = ws + (int64_t)s * kDepSteps * 2 * width;
   *reinterpret_cast<__nv_bfloat162*>(base + (int64_t)step * 2 * width + at) = k2;
   *reinterpret_cast<__nv_bfloat162*>(base + (int64_t)step * 2 * width + width + at) = v2;
@@ -583,8 +583,8 @@ __global__ void lm_dep_kv_attend_kernel(const bf16* __restrict__ qkv, bf16* __re
   for (int t = 0; t <= step; ++t) {
     __nv_bfloat162 kt = k2, vt = v2;
     if (t < step) {
-      kt = *reinterpret_cast<const __nv_bfloat162*>(base + (int64_t)t * 2 * width + at);
-      vt = *reinterpret_cast<const __nv_bfloat162*>(base + (int64_t)t * 2 * width + width + at);
+      kt = __ldcg(reinterpret_cast<const __nv_bfloat162*>(base + (int64_t)t * 2 * width + at));
+      vt = __ldcg(reinterpret_cast<const __nv_bfloat162*>(base + (int64_t)t * 2 * width + width + at));
     }
     const float sc = warp_add(q0 * __bfloat162float(kt.x) + q1 * __bfloat162float(kt.y)) * scale;
     const float m2 = fmaxf(m, sc);
@@ -632,7 +632,7 @@ __device__ __forceinline__ uint32_t mix32(uint32_t x) {
 
 template <int THREADS, int R>
 __global__ void __launch_bounds__(THREADS)
-    lm_sample_kernel(const bf16* __restrict__ logits, int vocab, int64_t ld, float temperature, int top_k,
+    lm_sample_kernel(const bf16* logits, int vocab, int64_t ld, float temperature, int top_k,
                      const int32_t* __restrict__ force, const int32_t* __restrict__ seeds, int col,
                      int32_t* __restrict__ drawn) {
   constexpr int WARPS = THREADS / 32;
@@ -739,7 +739,7 @@ __global__ void __launch_bounds__(THREADS)
 
 // `lm_advance` (lm.cu:546-573): one thread per session.
 __global__ void lm_advance_kernel(void* state, const int32_t* __restrict__ lines, int64_t stride,
-                                  const int32_t* __restrict__ drawn, const int32_t* __restrict__ caller,
+                                  const int32_t* drawn, const int32_t* __restrict__ caller,
                                   const int32_t* __restrict__ force_caller, int32_t* __restrict__ emitted, int seqs) {
   grid_trigger();
   grid_wait();
@@ -747,8 +747,9 @@ __global__ void lm_advance_kernel(void* state, const int32_t* __restrict__ lines
   if (s >= seqs) return;
   int32_t* row = const_cast<int32_t*>(state_row(state, lines, s, stride));
   int32_t* pending = row + kDuplexStreams;
-  const int32_t* d = drawn + s * kDuplexDrawn;
-  int32_t heard[kDuplexBooks];
+  int32_t d[kDuplexDrawn], heard[kDuplexBooks];
+#pragma unroll
+  for (int k = 0; k < kDuplexDrawn; ++k) d[k] = __ldcg(drawn + s * kDuplexDrawn + k);
 #pragma unroll
   for (int k = 0; k < kDuplexBooks; ++k) {
     const int f = force_caller[s * kDuplexBooks + k];

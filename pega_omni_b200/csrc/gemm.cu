@@ -30,7 +30,7 @@ constexpr int kGemvWarps = 8;
 
 template <int R>
 __global__ void __launch_bounds__(kGemvWarps * 32) gemv_kernel(const bf16* __restrict__ w, int N, int K,
-                                                                const bf16* __restrict__ x, int rows,
+                                                                const bf16* x, int rows,
                                                                 bf16* __restrict__ y, int ldy, const bf16* bias,
                                                                 int kind, int cols_per_warp) {
   grid_trigger();
@@ -44,7 +44,7 @@ __global__ void __launch_bounds__(kGemvWarps * 32) gemv_kernel(const bf16* __res
     for (int i = threadIdx.x; i < R * K / 8; i += blockDim.x) {
       const int r = i / (K / 8), c = i % (K / 8) * 8;
       *reinterpret_cast<uint4*>(xs + r * K + c) =
-          r0 + r < rows ? *reinterpret_cast<const uint4*>(x + (int64_t)(r0 + r) * K + c) : make_uint4(0u, 0u, 0u, 0u);
+          r0 + r < rows ? __ldcg(reinterpret_cast<const uint4*>(x + (int64_t)(r0 + r) * K + c)) : make_uint4(0u, 0u, 0u, 0u);
     }
     __syncthreads();
     for (int j = 0; j < cols_per_warp; ++j) {

@@ -37,7 +37,7 @@ __global__ void higgs_frame_embed_kernel(SlotState st, const bf16* __restrict__ 
 // `higgs_sample` (higgs.cu:186-208): a block per (sequence, codebook) over logits[s][b][vocab]; the code goes to
 // codes[s][b] and to word b of the sequence's slot.
 __global__ void __launch_bounds__(1024)
-    higgs_sample_kernel(const bf16* __restrict__ logits, int vocab, float temperature, int top_k,
+    higgs_sample_kernel(const bf16* logits, int vocab, float temperature, int top_k,
                         const float* __restrict__ uniforms, const int32_t* __restrict__ force, SlotState st,
                         int32_t* __restrict__ codes) {
   grid_trigger();
@@ -55,7 +55,7 @@ __global__ void __launch_bounds__(1024)
   prm.penalty = 1.f;
   prm.exempt = -1;
   prm.group = b;
-  Team::sample_row([&](int i, int) { return __bfloat162float(l[i]); }, prm, 0, uniforms[s * kHiggsBooks + b],
+  Team::sample_row([&](int i, int) { return __bfloat162float(__ldcg(l + i)); }, prm, 0, uniforms[s * kHiggsBooks + b],
                    force[s * kHiggsBooks + b], own, 0u, codes + s * kHiggsBooks + b, threadIdx.x, sh);
 }
 

@@ -6,6 +6,8 @@
 //   - before grid_wait() it reads only what no kernel of the same call writes - weights, tables, staged inputs, and what
 //     earlier calls left (a call starts behind a copy in its stream, which is ordered behind everything before it) - and
 //     writes nothing to global memory;
+//   - behind grid_wait(), what an earlier kernel of the call wrote is read past L1 (__ldcg, ld8cg) and through no pointer
+//     declared const __restrict__: that tells the compiler that nothing writes the data while the kernel lives, which it does;
 //   - behind grid_wait(), TMA and bulk copies of what an earlier kernel of the call wrote come behind fence_async_global()
 //     in the thread that issues them (sm100.cuh);
 //   - at least one thread of it passes grid_wait() on every path, so that its completion implies that of all kernels

@@ -48,7 +48,7 @@ __device__ __forceinline__ void mma(float (&d)[4], const uint32_t (&a)[4], uint3
 
 template <int D, int G>
 __global__ void __launch_bounds__(kRows * G * 2, G >= 4 ? 1 : 2)
-    prompt_attend_kernel(const bf16* __restrict__ qkv, const bf16* __restrict__ kv, bf16* __restrict__ out, RowMap map,
+    prompt_attend_kernel(const bf16* qkv, const bf16* kv, bf16* __restrict__ out, RowMap map,
                          int rows, int hq, int hk, float scale) {
   constexpr int kThreads = kRows * G * 2, C = D / 8;  // C: 16-byte chunks of a row
   extern __shared__ __align__(128) unsigned char prompt_smem[];

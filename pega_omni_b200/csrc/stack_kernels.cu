@@ -19,14 +19,14 @@ namespace omni {
 
 // One block of dim/8 threads per row. Semantics of `qwen3_norm_copy`
 // (qwen3.cu:18-31).
-__global__ void norm_copy_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, bf16* __restrict__ out,
+__global__ void norm_copy_kernel(const bf16* x, const bf16* __restrict__ w, bf16* __restrict__ out,
                                  bf16* __restrict__ res, int dim, float eps) {
   grid_trigger();
   grid_wait();
   __shared__ float scratch[32];
   const int64_t at = (int64_t)blockIdx.x * dim + threadIdx.x * 8;
   float v[8], g[8];
-  ld8(x + at, v);
+  ld8cg(x + at, v);
   float ss = 0.f;
 #pragma unroll
   for (int k = 0; k < 8; ++k) ss += v[k] * v[k];
@@ -40,16 +40,15 @@ __global__ void norm_copy_kernel(const bf16* __restrict__ x, const bf16* __restr
 
 // Semantics of `qwen3_add_norm` (qwen3.cu:37-57): the residual is stored
 // rounded, the norm is taken over the unrounded sum.
-__global__ void add_norm_kernel(const bf16* __restrict__ x, bf16* __restrict__ res, const bf16* __restrict__ w,
-                                bf16* __restrict__ out, int dim, float eps, int every, int which) {
+__global__ void add_norm_kernel(const bf16* x, bf16* res, const bf16* __restrict__ w, bf16* out, int dim, float eps, int every, int which) {
   grid_trigger();
   grid_wait();
   __shared__ float scratch[32];
   const int n = blockIdx.x;
   const int64_t at = (int64_t)n * dim + threadIdx.x * 8;
   float v[8], rv[8], g[8];
-  ld8(x + at, v);
-  ld8(res + at, rv);
+  ld8cg(x + at, v);  // (out may be x)
+  ld8cg(res + at, rv);
   float ss = 0.f;
 #pragma unroll
   for (int k = 0; k < 8; ++k) {
@@ -67,7 +66,7 @@ __global__ void add_norm_kernel(const bf16* __restrict__ x, bf16* __restrict__ r
 
 // `silu_mul` (common.cuh:66-76). With `interleaved` = g > 0, the fused row alternates g gate channels and the matching
 // g up channels (the weight layout the tensor-core SwiGLU epilogue wants) instead of [all gate | all up].
-__global__ void silu_mul_kernel(const bf16* __restrict__ gate_up, bf16* __restrict__ act, int inter, int total,
+__global__ void silu_mul_kernel(const bf16* gate_up, bf16* __restrict__ act, int inter, int total,
                                 int interleaved) {
   grid_trigger();
   grid_wait();
@@ -77,8 +76,8 @@ __global__ void silu_mul_kernel(const bf16* __restrict__ gate_up, bf16* __restri
   float g[8], u[8];
   const int64_t g_at = interleaved ? (c / interleaved) * 2 * interleaved + c % interleaved : c;
   const int64_t u_at = interleaved ? g_at + min((int64_t)interleaved, inter - c / interleaved * interleaved) : inter + c;
-  ld8(gate_up + n * 2 * inter + g_at, g);
-  ld8(gate_up + n * 2 * inter + u_at, u);
+  ld8cg(gate_up + n * 2 * inter + g_at, g);
+  ld8cg(gate_up + n * 2 * inter + u_at, u);
 #pragma unroll
   for (int k = 0; k < 8; ++k) g[k] = bf16_round(g[k] / (1.f + __expf(-g[k]))) * u[k];
   st8(act + (int64_t)i * 8, g);
@@ -278,8 +277,7 @@ cudaError_t launch_rope_kv(bf16* qkv, const bf16* q_norm, const bf16* k_norm, bf
 constexpr int kAttnSlots = 1;
 
 template <int D, int G>
-__global__ void __launch_bounds__(kAttnWarps * 32) attend_kernel(const bf16* __restrict__ qkv,
-                                                                 const bf16* __restrict__ kv, bf16* __restrict__ out,
+__global__ void __launch_bounds__(kAttnWarps * 32) attend_kernel(const bf16* qkv, const bf16* kv, bf16* __restrict__ out,
                                                                  RowMap map, int hq, int hk, float scale, uint32_t* err) {
   grid_trigger();
   grid_wait();
@@ -291,7 +289,7 @@ __global__ void __launch_bounds__(kAttnWarps * 32) attend_kernel(const bf16* __r
   const bf16* q = qkv + ((int64_t)n * (hq + 2 * hk) + kh * G) * D;
   if (threadIdx.x < kAttnWarps * kAttnSlots) sm100::mbar_init(sm100::smem_addr(&bars[threadIdx.x]), 1);
   if (threadIdx.x == 0) sm100::mbar_init_fence();
-  for (int i = threadIdx.x; i < G * D; i += blockDim.x) sh.qs[i / D][i % D] = __bfloat162float(q[i]);
+  for (int i = threadIdx.x; i < G * D; i += blockDim.x) sh.qs[i / D][i % D] = __bfloat162float(__ldcg(q + i));
   __syncthreads();
   const int warp = threadIdx.x >> 5;
   sm100::fence_async_global();  // keys and values written by ordinary stores, read by bulk copies
@@ -372,7 +370,7 @@ struct MergeShared<D, G, 1> {};
 
 template <int D, int G, int W, int TEAMS>
 __global__ void __launch_bounds__(W * TEAMS * 32, W == 8 ? 1 : 3)
-    rope_attend_kernel(const bf16* __restrict__ qkv, const QkvTable lookup, const bf16* __restrict__ q_norm,
+    rope_attend_kernel(const bf16* qkv, const QkvTable lookup, const bf16* __restrict__ q_norm,
                        const bf16* __restrict__ k_norm, bf16* kv, bf16* __restrict__ out, RowMap map, int items, int hq,
                        int hk, float eps, float theta, float scale, int kv_pages, uint32_t* err) {
   static_assert(W == 1 || TEAMS == 1, "a team of several warps is a CTA");
@@ -427,7 +425,7 @@ __global__ void __launch_bounds__(W * TEAMS * 32, W == 8 ? 1 : 3)
     if (r == 0) grid_wait();
     if (W == 1 && !live) return;  // (a dead team of several warps does not exist: TEAMS is 1 there)
     if (!paged) pg.load(block(0), lane);
-    const bf16* row = lookup.table ? lookup.table + (int64_t)lookup.codes[n * 16 + lookup.group] * ((hq + 2 * hk) * D)
+    const bf16* row = lookup.table ? lookup.table + (int64_t)__ldcg(lookup.codes + n * 16 + lookup.group) * ((hq + 2 * hk) * D)
                                    : qkv + (int64_t)n * ((hq + 2 * hk) * D);
     constexpr int JOBS = (G + 2 + W - 1) / W;
     uint32_t raw[JOBS][2];

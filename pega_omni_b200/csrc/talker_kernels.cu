@@ -10,22 +10,21 @@ namespace omni {
 
 constexpr int kGroups = 16;
 
-__global__ void gather_kernel(const int32_t* __restrict__ ids, int stride, const bf16* __restrict__ table,
-                              int table_rows, bf16* __restrict__ out, int dim, uint32_t* err) {
+__global__ void gather_kernel(const int32_t* ids, int stride, const bf16* table, int table_rows, bf16* __restrict__ out, int dim, uint32_t* err) {
   grid_trigger();
   grid_wait();
   const int c = threadIdx.x * 8;
-  int64_t id = ids[(int64_t)blockIdx.x * stride];
+  int64_t id = __ldcg(ids + (int64_t)blockIdx.x * stride);  // ids and table may be an earlier kernel's output
   if (id < 0 || id >= table_rows) {
     if (threadIdx.x == 0) raise(err, kErrBadIndex);
     id = 0;
   }
   *reinterpret_cast<uint4*>(out + (int64_t)blockIdx.x * dim + c) =
-      *reinterpret_cast<const uint4*>(table + id * dim + c);
+      __ldcg(reinterpret_cast<const uint4*>(table + id * dim + c));
 }
 
 // `talker_prompt_codec` (talker.cu:55-71): x + bias (+ codec embedding), one rounding.
-__global__ void prompt_codec_kernel(bf16* __restrict__ x, const bf16* __restrict__ bias,
+__global__ void prompt_codec_kernel(bf16* x, const bf16* __restrict__ bias,
                                     const bf16* __restrict__ table, int table_rows, const int32_t* __restrict__ ids,
                                     int dim, uint32_t* err) {
   grid_trigger();
@@ -38,7 +37,7 @@ __global__ void prompt_codec_kernel(bf16* __restrict__ x, const bf16* __restrict
     id = -1;
   }
   float v[8], b[8], e[8];
-  ld8(row, v);
+  ld8cg(row, v);
   ld8(bias + c, b);
 #pragma unroll
   for (int k = 0; k < 8; ++k) v[k] += b[k];
@@ -117,8 +116,8 @@ __global__ void frame_embed_norm_kernel(SlotState st, const bf16* __restrict__ p
 }
 
 // `talker_pred_input` (talker.cu:100-106).
-__global__ void pred_input_kernel(const bf16* __restrict__ hidden, const bf16* __restrict__ codec_emb, int vocab,
-                                  const int32_t* __restrict__ codes, bf16* __restrict__ out, int dim, uint32_t* err) {
+__global__ void pred_input_kernel(const bf16* hidden, const bf16* codec_emb, int vocab, const int32_t* codes,
+                                  bf16* __restrict__ out, int dim, uint32_t* err) {
   grid_trigger();
   grid_wait();
   const int s = blockIdx.x, c = threadIdx.x * 8;
@@ -126,14 +125,14 @@ __global__ void pred_input_kernel(const bf16* __restrict__ hidden, const bf16* _
   if (blockIdx.y == 0) {
     src = hidden + (int64_t)s * dim;
   } else {
-    int id = codes[s * kGroups];
+    int id = __ldcg(codes + s * kGroups);
     if (id < 0 || id >= vocab) {
       if (threadIdx.x == 0) raise(err, kErrBadIndex);
       id = 0;
     }
     src = codec_emb + (int64_t)id * dim;
   }
-  *reinterpret_cast<uint4*>(out + ((int64_t)2 * s + blockIdx.y) * dim + c) = *reinterpret_cast<const uint4*>(src + c);
+  *reinterpret_cast<uint4*>(out + ((int64_t)2 * s + blockIdx.y) * dim + c) = __ldcg(reinterpret_cast<const uint4*>(src + c));
 }
 
 cudaError_t launch_gather(const int32_t* ids, int stride, const bf16* table, int table_rows, bf16* out, int rows,
@@ -171,7 +170,7 @@ cudaError_t launch_pred_input(const bf16* hidden, const bf16* codec_emb, int voc
 
 template <int THREADS, int VOCAB>
 __global__ void __launch_bounds__(THREADS)
-    sample_kernel(const bf16* __restrict__ logits, sampler::Params prm, const int32_t* __restrict__ frames,
+    sample_kernel(const bf16* logits, sampler::Params prm, const int32_t* __restrict__ frames,
                   const float* __restrict__ uniforms, const int32_t* __restrict__ force, SlotState st,
                   int32_t* __restrict__ codes, NextRow next) {
   using Team = sampler::Team<THREADS, sampler::CtaSync, VOCAB>;
@@ -195,7 +194,7 @@ __global__ void __launch_bounds__(THREADS)
     }
   } else {
     for (int j = 0; j < Team::PER; ++j)
-      mine[j] = tid * Team::PER + j < prm.vocab ? __bfloat162float(l[tid * Team::PER + j]) : 0.f;
+      mine[j] = tid * Team::PER + j < prm.vocab ? __bfloat162float(__ldcg(l + tid * Team::PER + j)) : 0.f;
   }
   const int token = Team::sample_row([&](int, int j) { return mine[j]; }, prm, frame, uniform, forced, slot,
                                      Team::seen_word(slot, prm, tid), codes + s * kGroups + prm.group, tid, sh);
