@@ -33,6 +33,15 @@ struct omni_ops {
   }
 };
 
+// Nothing of the next launch starts before everything in front of it in the stream has ended. Attention kernels ask for their
+// pages, GEMMs for their weights before they wait for the kernel in front of them, because no other kernel of a model's call
+// writes those; calls made one by one here may.
+__global__ void order_kernel() {}
+static cudaError_t order(cudaStream_t s) {
+  order_kernel<<<1, 1, 0, s>>>();
+  return cudaGetLastError();
+}
+
 #define OPS_CUDA(ctx, expr)                                                                       \
   do {                                                                                            \
     cudaError_t e_ = (expr);                                                                      \
@@ -183,6 +192,7 @@ int32_t omni_op_decode_attend(omni_ops* c, const void* qkv, const void* q_norm, 
   RowMap map;
   map.pos = pos, map.slot = slot, map.indptr = indptr, map.pages = pages;
   const AttnShape a{q_heads, kv_heads, head_dim, eps, theta};
+  OPS_CUDA(c, order(c->stream));
   OPS_CUDA(c, launch_rope_attend((const bf16*)qkv, {}, (const bf16*)q_norm, (const bf16*)k_norm, (bf16*)kv, (bf16*)out, map, rows,
                                  a, kv_pages, c->err, c->stream));
   return OMNI_OK;
@@ -205,6 +215,7 @@ int32_t omni_op_chain_gemm(omni_ops* c, const void* w, int32_t N, int32_t K, con
   bf16* grouped = nullptr;
   OPS_CUDA(c, cudaMalloc((void**)&grouped, (size_t)N * K * sizeof(bf16)));
   cudaError_t e = launch_interleave_gate_up((const bf16*)w, grouped, N / 2, K, kGateGroup, c->stream);
+  if (e == cudaSuccess) e = order(c->stream);  // the GEMM asks for its weights before it waits
   if (e == cudaSuccess) e = chain.gemm(grouped, N, K, (const bf16*)x, rows, kStreamSwiglu, (bf16*)y, ldy);
   const cudaError_t done = cudaStreamSynchronize(c->stream);
   cudaFree(grouped);
@@ -312,6 +323,7 @@ int32_t omni_op_lm_decode_attend(omni_ops* c, const void* qkv, void* kv, int32_t
                                  const int32_t* slot, const int32_t* indptr, const int32_t* pages, int32_t rows,
                                  int32_t heads, float coef, float scale, int32_t context, void* out) {
   if (!c || !qkv || !kv || !pos || !slot || !indptr || !pages || !out || rows < 1) return OMNI_ERR_INVALID;
+  OPS_CUDA(c, order(c->stream));
   OPS_CUDA(c, launch_lm_rope_attend((const bf16*)qkv, kv, pos, slot, indptr, pages, (bf16*)out, rows, heads, coef, scale, context,
                                     kv_pages, c->err, c->stream));
   return OMNI_OK;
@@ -417,6 +429,7 @@ int32_t omni_op_codec_add_norm(omni_ops* c, const void* add, int64_t add_stride,
 int32_t omni_op_codec_window_attend(omni_ops* c, const void* qkv, void* state, const int32_t* lines, const int32_t* pos,
                                     int64_t stride, int64_t ring_offset, void* out, int32_t n, int32_t heads, float theta) {
   if (!c || !qkv || !state || !lines || !pos || !out) return OMNI_ERR_INVALID;
+  OPS_CUDA(c, order(c->stream));
   OPS_CUDA(c, launch_codec_window_attend((const bf16*)qkv, CodecStateRef{(char*)state, lines, pos, stride}, ring_offset,
                                          (bf16*)out, n, heads, theta, c->stream));
   return OMNI_OK;

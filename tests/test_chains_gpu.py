@@ -264,3 +264,23 @@ def test_a_ring_row_without_a_page_stores_nothing(ops, in_one):
     with pytest.raises(OpsError):
         ops.sync()
     assert not kv[[0, 1, 3, 5]].any() and kv[4].any() and kv[2].any()
+
+
+def test_decode_attention_calls_one_behind_the_other(ops):
+    """A call's own token is a key of the next call, made without waiting for it."""
+    hq, hk, d, n = 4, 2, 128, 40
+    qkv = [rand((1, (hq + 2 * hk) * d), 50 + t) for t in range(n)]
+    qn, kn, pages = rand((d,), 48, 0.2) + 1, rand((d,), 49, 0.2) + 1, i32([2, 0, 1])
+    at = [(i32([t]), i32([int(pages[t // 16]) * 16 + t % 16]), i32([0, 3])) for t in range(n)]
+    outs = []
+    for wait in (True, False):
+        kv = torch.zeros((3, hk, 2, 16, d), dtype=torch.bfloat16, device="cuda")
+        out = torch.zeros((n, hq * d), dtype=torch.bfloat16, device="cuda")
+        torch.cuda.synchronize()
+        for t, (pos, slot, indptr) in enumerate(at):
+            ops.decode_attend(qkv[t], qn, kn, kv, 3, pos, slot, indptr, pages, hq, hk, d, 1e-6, 1e6, out[t:t + 1])
+            if wait:
+                ops.sync()
+        ops.sync()
+        outs.append(out)
+    assert torch.equal(outs[0], outs[1])
