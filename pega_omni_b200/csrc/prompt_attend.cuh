@@ -4,7 +4,9 @@
 // reads them with ldmatrix. Rows may belong to several sequences: the CTA goes through the runs of rows of one sequence in
 // turn, and rows outside the run (or keys past a row's position) are masked. Value semantics of `attend`
 // (crates/omni-qwen3/kernels/qwen3.cu:123-207): f32 scores, online softmax in f32; a probability enters the second product
-// as the sum of two bf16 (its rounding and the remainder), which keeps 16 bits of it.
+// as the sum of three bf16, which is all of it, and sums are kept out of long chains of matrix instructions (decode_attend.cuh):
+// 0.01 to 0.02 % of the outputs of prompts of 77 to 512 rows are not the bf16 nearest to float64's (scalar kernel 0.01 to
+// 0.02 %, two bf16 a probability 0.17 to 0.22 %).
 // Measured at 8,700 rows of 28 ragged prompts, D = 128, G = 2: 146 us a layer, before page numbers were read a tile ahead
 // (scalar multiply-adds, each row reading its keys for itself: 1,184 us). Three CTAs an SM with fewer registers are no
 // faster. Bound by shared-memory reads (each warp reads the 16 KB of a stage for its sixteen rows: 512 cycles per 64 x 32
@@ -135,9 +137,7 @@ __global__ void __launch_bounds__(kRows * G * 2, G >= 4 ? 1 : 2)
       fetch(tile + kStages - 1);
       if (tile * kKeys > warp_last) continue;
       const uint32_t kb = ring + (uint32_t)(tile % kStages) * stage_bytes<D>(), vb = kb + kKeys * D * 2;
-      float s[4][4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) s[j][0] = s[j][1] = s[j][2] = s[j][3] = 0.f;
+      float s[4][4] = {}, s2[4][4] = {};
 #pragma unroll
       for (int k = 0; k < D / 16; ++k) {
 #pragma unroll
@@ -145,10 +145,14 @@ __global__ void __launch_bounds__(kRows * G * 2, G >= 4 ? 1 : 2)
           const int tok = jj * 16 + (lane & 7) + ((lane >> 4) << 3);
           uint32_t b[4];
           ldsm4(kb + (uint32_t)(tok * C + ((k * 2 + ((lane >> 3) & 1)) ^ (tok & 7))) * 16u, b);
-          mma(s[jj * 2], q[k], b[0], b[1]);
-          mma(s[jj * 2 + 1], q[k], b[2], b[3]);
+          mma(k & 1 ? s2[jj * 2] : s[jj * 2], q[k], b[0], b[1]);
+          mma(k & 1 ? s2[jj * 2 + 1] : s[jj * 2 + 1], q[k], b[2], b[3]);
         }
       }
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) s[j][e] += s2[j][e];
       float corr[2];
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
@@ -185,29 +189,33 @@ __global__ void __launch_bounds__(kRows * G * 2, G >= 4 ? 1 : 2)
           }
         sum[h] = sum[h] * corr[h] + part;  // this lane's keys; the other lanes' are added at the end
       }
+      uint32_t p[2][3][4];  // 16 keys each
 #pragma unroll
-      for (int i = 0; i < D / 8; ++i) acc[i][0] *= corr[0], acc[i][1] *= corr[0], acc[i][2] *= corr[1], acc[i][3] *= corr[1];
-#pragma unroll
-      for (int kk = 0; kk < 2; ++kk) {  // 16 keys
-        uint32_t hi[4], lo[4];
+      for (int kk = 0; kk < 2; ++kk)
 #pragma unroll
         for (int x = 0; x < 4; ++x) {
-          const float a = s[kk * 2 + (x >> 1)][(x & 1) * 2], b = s[kk * 2 + (x >> 1)][(x & 1) * 2 + 1];
-          const __nv_bfloat162 top = __floats2bfloat162_rn(a, b);
-          const float2 f = __bfloat1622float2(top);
-          const __nv_bfloat162 rest = __floats2bfloat162_rn(a - f.x, b - f.y);
-          hi[x] = *reinterpret_cast<const uint32_t*>(&top), lo[x] = *reinterpret_cast<const uint32_t*>(&rest);
+          uint32_t part[3];
+          split3(s[kk * 2 + (x >> 1)][(x & 1) * 2], s[kk * 2 + (x >> 1)][(x & 1) * 2 + 1], part);
+          p[kk][0][x] = part[0], p[kk][1][x] = part[1], p[kk][2][x] = part[2];
         }
-        const int tok = kk * 16 + (lane & 15);
 #pragma unroll
-        for (int i = 0; i < D / 16; ++i) {  // 16 dims
+      for (int i = 0; i < D / 16; ++i) {  // 16 dims
+        float o[2][4] = {};
+#pragma unroll
+        for (int kk = 0; kk < 2; ++kk) {
+          const int tok = kk * 16 + (lane & 15);
           uint32_t b[4];
           ldsm4t(vb + (uint32_t)(tok * C + ((i * 2 + (lane >> 4)) ^ (tok & 7))) * 16u, b);
-          mma(acc[2 * i], hi, b[0], b[1]);
-          mma(acc[2 * i], lo, b[0], b[1]);
-          mma(acc[2 * i + 1], hi, b[2], b[3]);
-          mma(acc[2 * i + 1], lo, b[2], b[3]);
+#pragma unroll
+          for (int x = 2; x >= 0; --x) {
+            mma(o[0], p[kk][x], b[0], b[1]);
+            mma(o[1], p[kk][x], b[2], b[3]);
+          }
         }
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) acc[2 * i + u][e] = fmaf(acc[2 * i + u][e], corr[e >> 1], o[u][e]);
       }
     }
     cp_wait<0>();

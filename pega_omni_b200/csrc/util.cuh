@@ -80,6 +80,18 @@ __device__ __forceinline__ void st8(bf16* dst, const float* v) { st8v(dst, v); }
 // The same past L1, for rows that another SM wrote while this kernel had already started.
 __device__ __forceinline__ void ld8cg(const bf16* src, float* v) { unpack8v(__ldcg(reinterpret_cast<const uint4*>(src)), v); }
 
+// Two f32 values as the sum of three bf16 each (value, rest of it, rest of that), packed: 24 bits of a value, its whole
+// mantissa. A matrix instruction on bf16 then multiplies it as f32 would.
+__device__ __forceinline__ void split3(float a, float b, uint32_t (&part)[3]) {
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    const __nv_bfloat162 t = __floats2bfloat162_rn(a, b);
+    part[i] = *reinterpret_cast<const uint32_t*>(&t);
+    const float2 f = __bfloat1622float2(t);
+    a -= f.x, b -= f.y;
+  }
+}
+
 __device__ __forceinline__ float warp_add(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);

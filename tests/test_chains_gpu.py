@@ -284,3 +284,44 @@ def test_decode_attention_calls_one_behind_the_other(ops):
         ops.sync()
         outs.append(out)
     assert torch.equal(outs[0], outs[1])
+
+
+def attention64(q, kv, pages, length, hq, hk, d):
+    """One row in float64 from the bf16 queries, keys and values the kernels read."""
+    block = kv[pages.long()].double()
+    k, v = (block[:, :, i].permute(1, 0, 2, 3).reshape(hk, -1, d)[:, :length] for i in range(2))
+    p = torch.softmax(torch.einsum("hgd,hld->hgl", q.double().reshape(hk, hq // hk, d), k) / d ** 0.5, -1)
+    return torch.einsum("hgl,hld->hgd", p, v).reshape(hq * d)
+
+
+# Outputs that are not the bf16 nearest to float64's: an error of a few f32 ulp (2^-22) moves a value over a rounding boundary
+# (2^-8 apart) in one of 2^13 cases, four times that where values cancel - 0.05 %. Sixteen-bit probabilities (2^-17): 0.2 %.
+NOT_NEAREST = 5e-4
+
+
+@pytest.mark.parametrize("hq,hk,d", [(16, 8, 128), (20, 4, 128), (8, 8, 64)])
+@pytest.mark.parametrize("prompt", [False, True])
+def test_attention_keeps_f32_probabilities(ops, hq, hk, d, prompt):
+    n, length = (256, 256) if prompt else (96, 200)
+    per = (length + 15) // 16
+    rng = np.random.default_rng(d)
+    table = rng.permutation(per if prompt else n * per).reshape(-1, per)
+    at = list(range(n)) if prompt else [length - 1 - s % 9 for s in range(n)]
+    page = [table[0] if prompt else table[s] for s in range(n)]
+    pos, slot = i32(at), i32([int(page[s][at[s] // 16]) * 16 + at[s] % 16 for s in range(n)])
+    qkv, qn, kn = rand((n, (hq + 2 * hk) * d), 61), rand((d,), 62, 0.2) + 1, rand((d,), 63, 0.2) + 1
+    kv = rand((table.size, hk, 2, 16, d), 64)
+    out, scalar = (torch.zeros((n, hq * d), dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    q, kv2 = qkv.clone(), kv.clone()
+    each, lists = i32([s * per for s in range(n + 1)]), i32(np.concatenate(page).tolist())
+    torch.cuda.synchronize()
+    ops.rope_attend(q, qn, kn, kv2, table.size, pos, slot, None, each, lists, hq, hk, d, 1e-6, 1e6, scalar)
+    if prompt:
+        ops.rope_attend(qkv, qn, kn, kv, table.size, pos, slot, i32([0] * n), i32([0, per]), i32(page[0].tolist()), hq, hk, d, 1e-6, 1e6, out)
+    else:
+        ops.decode_attend(qkv, qn, kn, kv, table.size, pos, slot, each, lists, hq, hk, d, 1e-6, 1e6, out)
+    ops.sync()
+    assert torch.equal(kv, kv2)
+    want = torch.stack([attention64(q[s, :hq * d].reshape(hq, d), kv2, torch.tensor(page[s], device="cuda"), at[s] + 1, hq, hk, d) for s in range(n)])
+    for got in (scalar, out):
+        assert float((got != want.to(torch.bfloat16)).double().mean()) <= NOT_NEAREST
