@@ -59,13 +59,14 @@ __device__ __forceinline__ void st_shared16(uint32_t addr, const uint4& v) {
 // Where a lane's pieces of the rows lie (few_share.h), and where they go.
 struct Share : FewShare {
   int warp;
+  int64_t at;   // the lane's first piece (few_at)
   uint32_t xs;  // row n's share in shared memory
 };
 
 // The add + norm's rows, RD pieces a lane, from S partial sums; `keep`: this CTA stores the residual.
 template <int NORM, int S, int RD>
 __device__ __forceinline__ void norm_rows(const FewArgs& a, const Share& h, bool keep, float (*ss_s)[kWarps], const uint4* gain) {
-  const int64_t at = few_at(h, a.K);
+  const int64_t at = h.at;
   const float* part = a.norm.sum.part + at;
   constexpr int B = S >= 4 ? 2 : RD < 4 ? RD : RD == 4 && S == 1 ? 4 : 2;  // pieces under way at a time
   float v[RD][8], ss = 0.f;
@@ -173,7 +174,7 @@ __global__ void __launch_bounds__(kWarps * 32, 2) few_rows_kernel(const __grid_c
   // ---- everything that does not depend on the rows comes before grid_wait(), the first weights' arrival included ----
   Share h;
   static_cast<FewShare&>(h) = few_share(lane, kb0, nk, a.lanes_log2, a.rows);
-  h.warp = warp, h.xs = xs + (uint32_t)(h.n * a.xk) * 2u;
+  h.warp = warp, h.at = few_at(h, a.K), h.xs = xs + (uint32_t)(h.n * a.xk) * 2u;
   const int mts = MT <= 4 ? MT : a.R >> 4;
   // ldmatrix rows of this lane: weights [0, 8) k 0..7, [8, 16) k 0..7, [0, 8) k 8..15, [8, 16) k 8..15; x rows past the
   // last read row 0 (their columns of the result are not stored)
