@@ -272,8 +272,7 @@ __global__ void __launch_bounds__(kWarps * 32, 2) few_rows_kernel(const __grid_c
       const float v = total(n * stride + c);
       if constexpr (OUT == kStreamSwiglu) {
         const float u = bf16_round(total(n * stride + (a.R >> 1) + c)), gate = bf16_round(v);
-        // the fast division is within 2 ulp of an f32 that is rounded to bf16 next
-        a.y[(int64_t)n * a.ldy + c0 + c] = __float2bfloat16(bf16_round(__fdividef(gate, 1.f + __expf(-gate))) * u);
+        a.y[(int64_t)n * a.ldy + c0 + c] = __float2bfloat16(silu_bf16(gate) * u);
       } else if constexpr (OUT == kStreamPartials) {
         a.part[((int64_t)split * a.rows + n) * a.N + c0 + c] = v;
       } else {

@@ -198,9 +198,7 @@ __global__ void __launch_bounds__(kThreads, 1)
           float o[8];
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
-            const float gg = bf16_round(g[j]);
-            // the fast division is within 2 ulp of an f32 that is rounded to bf16 next
-            o[j] = bf16_round(__fdividef(gg, 1.f + __expf(-gg))) * bf16_round(u[j]);
+            o[j] = silu_bf16(bf16_round(g[j])) * bf16_round(u[j]);
           }
           st8(a.y + (size_t)m * a.ldy + ch0 + c, o);
         }

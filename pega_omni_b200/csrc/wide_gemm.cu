@@ -220,9 +220,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kWideThreads, 1)
               float o[8];
 #pragma unroll
               for (int j = 0; j < 8; ++j) {
-                const float g = bf16_round(__uint_as_float(r[0][j]));
-                // the fast division is within 2 ulp of an f32 that is rounded to bf16 next
-                o[j] = bf16_round(__fdividef(g, 1.f + __expf(-g))) * bf16_round(__uint_as_float(r[1][j]));
+                o[j] = silu_bf16(bf16_round(__uint_as_float(r[0][j]))) * bf16_round(__uint_as_float(r[1][j]));
               }
               if (live) st8(a.y + (size_t)row * a.ldy + ch0 + c, o);
             }

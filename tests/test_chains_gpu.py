@@ -325,3 +325,23 @@ def test_attention_keeps_f32_probabilities(ops, hq, hk, d, prompt):
     want = torch.stack([attention64(q[s, :hq * d].reshape(hq, d), kv2, torch.tensor(page[s], device="cuda"), at[s] + 1, hq, hk, d) for s in range(n)])
     for got in (scalar, out):
         assert float((got != want.to(torch.bfloat16)).double().mean()) <= NOT_NEAREST
+
+
+@pytest.mark.parametrize("rows", [1, 40, 300])
+def test_swiglu_of_every_gate(ops, rows):
+    """Each finite bf16 as the gate, the up channel 1: the result nearest to float64's, the last f32 bit apart at a tie."""
+    v = torch.arange(0, 65536, dtype=torch.int32).to(torch.int16).view(torch.bfloat16)
+    v = v[torch.isfinite(v.float())].cuda()
+    w = torch.zeros((2 * len(v), 64), dtype=torch.bfloat16, device="cuda")
+    w[:len(v), 0], w[len(v):, 1] = v, 1
+    x = torch.zeros((rows, 64), dtype=torch.bfloat16, device="cuda")
+    x[:, :2] = 1
+    y = torch.zeros((rows, len(v)), dtype=torch.bfloat16, device="cuda")
+    torch.cuda.synchronize()
+    ops.chain_gemm(w, x, y, swiglu=True)
+    ops.sync()
+    want = v.double() * torch.sigmoid(v.double())
+    assert (y == y[0]).all()
+    assert int((y[0] != want.to(torch.bfloat16)).sum()) <= 1
+    # half a bf16 step of the value and 2^-22 of it for the f32 arithmetic; below the smallest normal f32 a step is fixed
+    assert ((y[0].double() - want).abs() <= want.abs() * (2.0 ** -8 + 2.0 ** -22) + 2.0 ** -134).all()
