@@ -74,9 +74,6 @@ __global__ void __launch_bounds__(kRows * G * 2, G >= 4 ? 1 : 2)
     row[h] = m / G, head[h] = m % G;
   }
   uint32_t q[D / 16][4];  // their queries as A fragments
-  float mx[2] = {-INFINITY, -INFINITY}, sum[2] = {0.f, 0.f}, acc[D / 8][4];
-#pragma unroll
-  for (int i = 0; i < D / 8; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
   const int warp_r0 = warp * 16 / G, warp_r1 = (warp * 16 + 15) / G;  // rows this warp holds heads of
 
   for (int r0 = 0; r0 < count;) {
@@ -120,6 +117,9 @@ __global__ void __launch_bounds__(kRows * G * 2, G >= 4 ? 1 : 2)
     look(0);
     if (r0 == 0) grid_wait();
     for (int s = 0; s < kStages - 1; ++s) fetch(s);
+    // every run starts from nothing and stores its own rows: what it leaves in the other rows' sums (0 times another
+    // sequence's values, which is no 0 where those are infinite) is never used
+    float mx[2] = {-INFINITY, -INFINITY}, sum[2] = {0.f, 0.f}, acc[D / 8][4] = {};
     if (r0 == 0) {
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
@@ -218,20 +218,20 @@ __global__ void __launch_bounds__(kRows * G * 2, G >= 4 ? 1 : 2)
           for (int e = 0; e < 4; ++e) acc[2 * i + u][e] = fmaf(acc[2 * i + u][e], corr[e >> 1], o[u][e]);
       }
     }
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      sum[h] += __shfl_xor_sync(0xffffffffu, sum[h], 1);
+      sum[h] += __shfl_xor_sync(0xffffffffu, sum[h], 2);
+      if (limit[h] < 0) continue;  // not a row of this run
+      const float inv = 1.f / sum[h];
+      bf16* dst = out + ((int64_t)(n0 + row[h]) * hq + kh * G + head[h]) * D + 2 * t;
+#pragma unroll
+      for (int i = 0; i < D / 8; ++i)
+        *reinterpret_cast<__nv_bfloat162*>(dst + i * 8) = __floats2bfloat162_rn(acc[i][2 * h] * inv, acc[i][2 * h + 1] * inv);
+    }
     cp_wait<0>();
     __syncthreads();  // the ring is free for the next run
     r0 = r1;
-  }
-#pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    sum[h] += __shfl_xor_sync(0xffffffffu, sum[h], 1);
-    sum[h] += __shfl_xor_sync(0xffffffffu, sum[h], 2);
-    if (row[h] >= count) continue;
-    const float inv = 1.f / sum[h];
-    bf16* dst = out + ((int64_t)(n0 + row[h]) * hq + kh * G + head[h]) * D + 2 * t;
-#pragma unroll
-    for (int i = 0; i < D / 8; ++i)
-      *reinterpret_cast<__nv_bfloat162*>(dst + i * 8) = __floats2bfloat162_rn(acc[i][2 * h] * inv, acc[i][2 * h + 1] * inv);
   }
 }
 

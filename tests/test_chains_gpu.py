@@ -345,3 +345,29 @@ def test_swiglu_of_every_gate(ops, rows):
     assert int((y[0] != want.to(torch.bfloat16)).sum()) <= 1
     # half a bf16 step of the value and 2^-22 of it for the f32 arithmetic; below the smallest normal f32 a step is fixed
     assert ((y[0].double() - want).abs() <= want.abs() * (2.0 ** -8 + 2.0 ** -22) + 2.0 ** -134).all()
+
+
+@pytest.mark.parametrize("lens,broken", [([10, 9], 0), ([10, 9], 1), ([33, 5, 40], 1), ([3, 3, 3, 3], 2)])
+def test_prompts_of_a_tile_do_not_touch_one_another(ops, lens, broken):
+    """One sequence's values are infinite: the others, in the same tiles of rows, give what they give beside a sound one."""
+    hq, hk, d, n = 4, 2, 128, sum(lens)
+    per = [(x + 15) // 16 for x in lens]
+    first = np.cumsum([0] + per)
+    table = np.random.default_rng(n).permutation(int(first[-1]))
+    where = [(s, t) for s, x in enumerate(lens) for t in range(x)]
+    pos, seq = i32([t for _, t in where]), i32([s for s, _ in where])
+    slot = i32([int(table[first[s] + t // 16]) * 16 + t % 16 for s, t in where])
+    qkv, qn, kn = rand((n, (hq + 2 * hk) * d), 71), rand((d,), 72, 0.2) + 1, rand((d,), 73, 0.2) + 1
+    outs = []
+    for bad in (False, True):
+        x = qkv.clone()
+        if bad:
+            x[seq == broken, (hq + hk) * d:] = float("inf")
+        kv = torch.zeros((len(table), hk, 2, 16, d), dtype=torch.bfloat16, device="cuda")
+        out = torch.zeros((n, hq * d), dtype=torch.bfloat16, device="cuda")
+        torch.cuda.synchronize()
+        ops.rope_attend(x, qn, kn, kv, len(table), pos, slot, seq, i32(first.tolist()), i32(table.tolist()), hq, hk, d, 1e-6, 1e6, out)
+        ops.sync()
+        outs.append(out)
+    others = seq != broken
+    assert torch.equal(outs[0][others], outs[1][others])
