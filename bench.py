@@ -637,7 +637,7 @@ def main():
     ap.add_argument("--no-codec", action="store_true", help="talker: skip the tick + codec decoder arm (with_codec)")
     ap.add_argument("--e2e-waited", action="store_true", help="talker: the end-to-end arm waits on every step (Model.step) "
                     "instead of keeping two steps under way (step_begin / step_end)")
-    ap.add_argument("--trace", default=None, help="talker: write the tick kernel's per-phase device timestamps here")
+    ap.add_argument("--trace", default=None, help="talker: write the last tick's device timestamps here, per phase or per kernel")
     args = ap.parse_args()
 
     rank = int(os.environ.get("RANK", "0"))

@@ -23,6 +23,22 @@ struct ChainPlan {
 };
 using ChainPlans = std::map<std::tuple<const void*, const void*, const void*, int, int>, ChainPlan>;
 
+// Stands behind every kernel of a traced program: a stamp of the device's clock, and the kernel's name and shape.
+struct ChainTrace {
+  struct Line {
+    const char* what;
+    int N, K, rows;
+  };
+  unsigned long long* stamps = nullptr;  // device, one per line
+  size_t capacity = 0;
+  std::vector<Line>* lines = nullptr;    // those of the program being enqueued
+  cudaError_t mark(const char* what, int N, int K, int rows, cudaStream_t stream) const {
+    if (!lines || lines->size() >= capacity) return cudaSuccess;
+    lines->push_back(Line{what, N, K, rows});
+    return launch_stamp(stamps + lines->size() - 1, stream);
+  }
+};
+
 constexpr int kChainRows = 256;  // beyond this the GEMMs are contractions, not streams of weights: wide_gemm.h
 
 struct Chain {
@@ -33,6 +49,13 @@ struct Chain {
   size_t partial_floats = 0;
   int* launches = nullptr;
   ChainPlans* plans = nullptr;
+  const ChainTrace* trace = nullptr;
+
+  // Behind every launch: counted, and stamped where the program is traced.
+  cudaError_t done(cudaError_t launched, const char* what, int N, int K, int rows) const {
+    ++*launches;
+    return launched == cudaSuccess && trace ? trace->mark(what, N, K, rows, stream) : launched;
+  }
 
   // y (bf16 rows, SwiGLU activations) or, for kStreamPartials, *sum
   cudaError_t gemm(const bf16* w, int N, int K, const bf16* x, int rows, int out, bf16* y, int ldy, Summands* sum = nullptr,
@@ -40,8 +63,7 @@ struct Chain {
     if (rows > kChainRows) {  // prompts: any row count, so the plan (two tensor maps) is made for the call
       WidePlan wide;
       if (wide_plan(&wide, w, N, K, x, rows, out, y, ldy, epi, sm_count, granule) != 0) return cudaErrorInvalidValue;
-      ++*launches;
-      return wide_launch(wide, err, stream);
+      return done(wide_launch(wide, err, stream), out == kStreamSwiglu ? "gemm_swiglu" : "gemm", N, K, rows);
     }
     ChainPlan* p = plan(w, N, K, x, rows, out, y, ldy, epi);
     return p ? launch(*p, {}, sum) : cudaErrorInvalidValue;
@@ -59,8 +81,7 @@ struct Chain {
         return launch(*p, norm, nullptr);
       }
     }
-    ++*launches;
-    const cudaError_t e = apart(norm.sum, *res);
+    const cudaError_t e = done(apart(norm.sum, *res), "add_norm", 0, K, rows);
     return e != cudaSuccess ? e : gemm(w, N, K, x, rows, out, y, ldy);
   }
 
@@ -77,8 +98,10 @@ struct Chain {
   }
   cudaError_t launch(const ChainPlan& p, const FewNorm& norm, Summands* sum) const {
     if (sum) *sum = p.few ? p.f.summands() : p.s.summands();
-    ++*launches;
-    return p.few ? few_launch(p.f, norm, err, stream) : stream_launch(p.s, err, stream);
+    const int out = p.few ? p.f.out : p.s.out;
+    const char* what = norm.kind ? (out == kStreamSwiglu ? "norm_gemm_swiglu" : "norm_gemm") : out == kStreamSwiglu ? "gemm_swiglu" : "gemm";
+    return p.few ? done(few_launch(p.f, norm, err, stream), what, p.f.N, p.f.K, p.f.rows)
+                 : done(stream_launch(p.s, err, stream), what, p.s.N, p.s.K, p.s.rows);
   }
 };
 
@@ -123,19 +146,18 @@ cudaError_t chain_pass(const Chain& c, const std::vector<Layer>& layers, const G
     if (i > 0) OMNI_CHAIN(norm_gemm(L.ln1, L.qkv, qw, kStreamBf16, b.qkv, qw));
     else if (!from.table) OMNI_CHAIN(c.gemm(L.qkv, qw, hidden, b.x, rows, kStreamBf16, b.qkv, qw));
     if (prompt) {  // rows of one sequence attend to one another: every key is written before the first is read
-      *c.launches += 2;
-      OMNI_CHAIN(launch_rope_kv(b.qkv, L.q_norm, L.k_norm, kv[i], map, rows, a, kv_pages, c.err, c.stream));
-      OMNI_CHAIN(launch_attend(b.qkv, kv[i], b.attn, map, rows, a, c.err, c.stream));
+      OMNI_CHAIN(c.done(launch_rope_kv(b.qkv, L.q_norm, L.k_norm, kv[i], map, rows, a, kv_pages, c.err, c.stream), "rope_kv", 0, 0, rows));
+      OMNI_CHAIN(c.done(launch_attend(b.qkv, kv[i], b.attn, map, rows, a, c.err, c.stream), "attend", 0, 0, rows));
     } else {
-      ++*c.launches;
-      OMNI_CHAIN(launch_rope_attend(b.qkv, from, L.q_norm, L.k_norm, kv[i], b.attn, map, rows, a, kv_pages, c.err, c.stream));
+      OMNI_CHAIN(c.done(launch_rope_attend(b.qkv, from, L.q_norm, L.k_norm, kv[i], b.attn, map, rows, a, kv_pages, c.err, c.stream),
+                        "rope_attend", 0, 0, rows));
     }
     OMNI_CHAIN(c.gemm(L.o, hidden, qd, b.attn, rows, kStreamPartials, nullptr, hidden, &sum));
     OMNI_CHAIN(norm_gemm(L.ln2, gate_up(L), 2 * inter, kStreamSwiglu, b.act, inter));
     OMNI_CHAIN(c.gemm(down(L), hidden, inter, b.act, rows, kStreamPartials, nullptr, hidden, &sum));
   }
-  ++*c.launches;
-  return launch_add_norm_sum(sum, b.res, final_gain, keep_out, rows, hidden, a.rms_eps, every, which, c.stream);
+  return c.done(launch_add_norm_sum(sum, b.res, final_gain, keep_out, rows, hidden, a.rms_eps, every, which, c.stream), "add_norm",
+                0, hidden, rows);
 }
 
 }  // namespace omni

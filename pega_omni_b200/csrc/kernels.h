@@ -68,6 +68,9 @@ cudaError_t launch_rope_attend(const bf16* qkv, const QkvTable& lookup, const bf
 cudaError_t launch_attend(const bf16* qkv, const bf16* kv, bf16* out, const RowMap& map, int rows, const AttnShape& a,
                           uint32_t* err, cudaStream_t s);
 
+// *at = the device's clock in ns once every kernel before it in the stream has ended; what follows may be launched early.
+cudaError_t launch_stamp(unsigned long long* at, cudaStream_t s);
+
 // out[r] = table[ids[r * stride]]
 cudaError_t launch_gather(const int32_t* ids, int stride, const bf16* table, int table_rows, bf16* out, int rows,
                           int dim, uint32_t* err, cudaStream_t s);

@@ -5,6 +5,7 @@
 #include "kernels.h"
 #include "sampler.cuh"
 #include "pdl.cuh"
+#include "sm100.cuh"
 
 namespace omni {
 
@@ -133,6 +134,16 @@ __global__ void pred_input_kernel(const bf16* hidden, const bf16* codec_emb, int
     src = codec_emb + (int64_t)id * dim;
   }
   *reinterpret_cast<uint4*>(out + ((int64_t)2 * s + blockIdx.y) * dim + c) = __ldcg(reinterpret_cast<const uint4*>(src + c));
+}
+
+__global__ void stamp_kernel(unsigned long long* at) {
+  grid_trigger();
+  grid_wait();
+  *at = sm100::global_timer_ns();
+}
+
+cudaError_t launch_stamp(unsigned long long* at, cudaStream_t s) {
+  return launch_pdl(stamp_kernel, dim3(1), dim3(1), 0, s, at);
 }
 
 cudaError_t launch_gather(const int32_t* ids, int stride, const bf16* table, int table_rows, bf16* out, int rows,

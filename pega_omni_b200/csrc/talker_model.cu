@@ -117,7 +117,7 @@ struct omni_seq {
   omni_codec_stream* audio = nullptr;  // the sequence's slot in the attached codec decoder
 };
 
-constexpr int kTraceMaxPhases = 1024;
+constexpr int kTraceMaxPhases = 1024, kTraceMaxKernels = 4096;
 
 struct omni_talker {
   omni_talker_config cfg;
@@ -174,7 +174,10 @@ struct omni_talker {
 
   std::map<std::tuple<const void*, const void*, const void*, int, int>, TcGemmPlan> plans;
   ChainPlans stream_plans;
-  Chain chain() { return Chain{stream, err, sm_count, gemm_scratch.partials, gemm_scratch.partial_floats, &launches, &stream_plans}; }
+  Chain chain() {
+    return Chain{stream, err, sm_count, gemm_scratch.partials, gemm_scratch.partial_floats, &launches, &stream_plans,
+                 chain_trace.lines ? &chain_trace : nullptr};
+  }
   bool use_chain = false;  // programs run as chains of kernels (chain.h) rather than as the persistent kernel
   std::map<std::pair<int, int>, cudaGraphExec_t> graphs;  // (program, bucket)
   std::map<std::pair<int, int>, int> graph_nodes;           // kernel nodes of each captured graph
@@ -195,6 +198,9 @@ struct omni_talker {
   std::string trace_path;  // omni_talker_trace: where the per-phase device timestamps of a tick are written
   unsigned long long* trace = nullptr;
   const TickProgram* trace_program = nullptr;
+  ChainTrace chain_trace;  // of programs that run as kernels; `lines` is set while one is enqueued
+  std::map<std::pair<int, int>, std::vector<ChainTrace::Line>> trace_lines;  // (program, bucket)
+  const std::vector<ChainTrace::Line>* traced = nullptr;                     // the latest traced program's
   omni_stats stats{};
   int last_n = 0;
   // omni_talker_step_begin / _end: up to two decode steps under way, each with its own pinned staging and read-back
@@ -358,6 +364,7 @@ int alloc_scratch(omni_talker* m, const StackW& s, int rows, Scratch* out) {
   do {                                                                                         \
     cudaError_t e_ = (expr);                                                                   \
     ++(m)->launches;                                                                           \
+    if (e_ == cudaSuccess && (m)->chain_trace.lines) e_ = (m)->chain_trace.mark(#expr, 0, 0, 0, (m)->stream); \
     if (e_ != cudaSuccess) return (m)->fail(OMNI_ERR_CUDA, "%s: %s", #expr, cudaGetErrorString(e_)); \
   } while (0)
 
@@ -539,11 +546,22 @@ int enqueue_tail(omni_talker* m, int b) {
   return OMNI_OK;
 }
 
-enum Program { kFirst = 0, kDecode = 1 };
+enum Program { kFirst = 0, kDecode = 1, kTraced = 2 };  // kTraced: added to either
+
+int enqueue_kernels(omni_talker* m, int program, int b) {
+  if ((program & kDecode) != 0) TRY(enqueue_advance(m, b));
+  return enqueue_tail(m, b);
+}
 
 int enqueue_program(omni_talker* m, int program, int b) {
-  if (program == kDecode) TRY(enqueue_advance(m, b));
-  return enqueue_tail(m, b);
+  if ((program & kTraced) == 0) return enqueue_kernels(m, program, b);
+  auto& lines = m->trace_lines[std::make_pair(program, b)];
+  lines.clear();
+  m->chain_trace.lines = &lines;
+  const cudaError_t e = m->chain_trace.mark("start", 0, 0, b, m->stream);
+  const int rc = e != cudaSuccess ? m->fail(OMNI_ERR_CUDA, "trace: %s", cudaGetErrorString(e)) : enqueue_kernels(m, program, b);
+  m->chain_trace.lines = nullptr;
+  return rc;
 }
 
 
@@ -974,7 +992,16 @@ int run_tick_program(omni_talker* m, int program, int b) {
 // as a replay of their captured graph (or eager launches).
 int run_program(omni_talker* m, int program, int b) {
   m->launches = 0;
+  m->traced = nullptr;
   if (!m->use_chain && m->cfg.tick_kernel && tick_usable(m, b)) return run_tick_program(m, program, b);
+  if (!m->trace_path.empty()) {  // a program of its own: the untraced one has no stamps between its kernels
+    program |= kTraced;
+    if (!m->chain_trace.stamps) {
+      TRY(dev_alloc(m, &m->chain_trace.stamps, kTraceMaxKernels, true));
+      m->chain_trace.capacity = kTraceMaxKernels;
+    }
+    m->traced = &m->trace_lines[std::make_pair(program, b)];
+  }
   if (!m->cfg.use_graphs) return enqueue_program(m, program, b);
   auto key = std::make_pair(program, b);
   auto it = m->graphs.find(key);
@@ -1082,7 +1109,7 @@ size_t stage_graph_inputs(omni_talker* m, char* host, const std::vector<FrameRow
 }
 
 
-// Writes one line per phase of the last traced tick: its shape, then (ns, relative to the median time at which the
+// Writes one line per kernel of the last traced tick (see omni_talker_trace), or per phase of the persistent kernel: its shape, then (ns, relative to the median time at which the
 // CTAs saw the previous barrier complete) the median and the latest over CTAs of: first activation tile in shared
 // memory, first accumulator complete, own share done, barrier seen complete.
 void dump_trace(omni_talker* m) {
@@ -1100,6 +1127,21 @@ void dump_trace(omni_talker* m) {
         fclose(f);
       }
     }
+  }
+  if (m->traced && !m->trace_path.empty()) {
+    std::vector<unsigned long long> t(m->traced->size());
+    if (cudaMemcpy(t.data(), m->chain_trace.stamps, t.size() * 8, cudaMemcpyDeviceToHost) != cudaSuccess) return;
+    FILE* f = fopen(m->trace_path.c_str(), "w");
+    if (!f) return;
+    fprintf(f, "kernel what N K rows dur end\n");
+    for (size_t i = 1; i < t.size(); ++i) {
+      const ChainTrace::Line& l = (*m->traced)[i];
+      const char* open = strchr(l.what, '(');  // a launch as it stands in the source: its name
+      fprintf(f, "%zu %.*s %d %d %d %lld %lld\n", i, open ? (int)(open - l.what) : (int)strlen(l.what), l.what, l.N, l.K, l.rows,
+              (long long)(t[i] - t[i - 1]), (long long)(t[i] - t[0]));
+    }
+    fclose(f);
+    return;
   }
   if (!m->trace || !m->trace_program || m->trace_path.empty()) return;
   const TickProgram& prog = *m->trace_program;
