@@ -120,6 +120,7 @@ struct NextRow {
   int dim = 0;
   float eps = 0.f;
 };
+constexpr int kNextRowMax = 4096;  // elements: eight a thread of the draw
 // launch_sample followed by that row.
 cudaError_t launch_sample_next(const bf16* logits, const SampleParams& p, const int32_t* frames, const float* uniforms,
                                const int32_t* force, SlotState st, int32_t* codes, const NextRow& next, int rows,

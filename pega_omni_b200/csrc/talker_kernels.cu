@@ -240,7 +240,7 @@ cudaError_t launch_sample_next(const bf16* logits, const SampleParams& p, const 
   if (p.top_p < 1.f && (p.top_k <= 0 || p.top_k > sampler::kMaxNucleus)) return cudaErrorInvalidValue;
   sampler::Params prm{p.vocab,  p.temperature, p.top_k,    p.top_p, p.penalty, p.suppress_lo, p.suppress_hi,
                       p.exempt, p.min_frames,  p.penalize, p.group, p.philox,  p.seen_words};
-  if (next.table && next.dim > 8 * 512) return cudaErrorInvalidValue;
+  if (next.table && next.dim > kNextRowMax) return cudaErrorInvalidValue;
   auto go = [&](auto kernel) {
     return launch_pdl(kernel, dim3(rows), dim3(512), 0, s, logits, prm, frames, uniforms, force, st, codes, next);
   };

@@ -521,7 +521,7 @@ int enqueue_tail(omni_talker* m, int b) {
   bias.kind = kEpiBias;
   // From the second predictor pass on a pass's one input row per sequence is a function of the code just drawn: its
   // projection and the first layer's q | k | v of it are rows of tables computed at load (p_emb_proj, p_qkv0)
-  const bool folded = m->use_chain && m->p_emb_proj && m->p_qkv0 && 2 * b <= kChainRows;
+  const bool folded = m->use_chain && m->p_emb_proj && m->p_qkv0 && 2 * b <= kChainRows && p <= kNextRowMax;
   const int qw = m->pred.qkv_width();
   for (int g = 1; g < c.groups; ++g) {
     const int per = g == 1 ? 2 : 1, rows = b * per;

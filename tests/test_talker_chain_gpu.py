@@ -18,11 +18,11 @@ def chain_config(**generation):
     return cfg.with_generation(**generation)
 
 
-def make(cfg=None, seed=3, max_batch=16, **kw):
+def make(cfg=None, seed=3, max_batch=16, std=0.02, **kw):
     from pega_omni_b200.model import Limits, Model
     from pega_omni_b200.synthetic import random_checkpoint
     cfg = cfg or chain_config()
-    ck = random_checkpoint(cfg, seed=seed, device="cuda")
+    ck = random_checkpoint(cfg, seed=seed, std=std, device="cuda")
     return cfg, ck, Model.load(0, ck, cfg, Limits(max_batch=max_batch, max_tokens=2048, kv_gib=0.5), **kw)
 
 
@@ -58,3 +58,27 @@ def test_trace_writes_a_line_per_kernel(built_lib, tmp_path):
     m.run_ticks(seqs, [draws_for(rng, 3) for _ in range(2)])
     assert not path.exists() and m.stats().last_call_launches // 2 == kernels
     m.close()
+
+
+def test_predictor_wider_than_a_draw_holds(built_lib):
+    """A predictor of 4,352 channels: its rows do not come out of the draw, and its logits are those of the per-op kernels."""
+    from pega_omni_b200.model import Draw
+    base = chain_config()
+    cfg = dataclasses.replace(base, predictor=dataclasses.replace(base.predictor, hidden_size=4352, num_hidden_layers=1))
+    rng = np.random.default_rng(2)
+    forced = rng.integers(0, 64, (3, 3, 16)).astype(np.int32)
+    forced[:, :, cfg.num_code_groups:] = 0
+    got = []
+    for tick_kernel in (True, False):
+        _, _, m = make(cfg, max_batch=4, std=0.01, tick_kernel=tick_kernel)
+        seqs, prompts, rows = [m.open(7, 8) for _ in range(3)], prompts_for(cfg, [7] * 3), []
+        for t in range(3):
+            draws = [Draw([0.5] * 16, list(forced[t, s])) for s in range(3)]
+            out = m.start(list(zip(seqs, prompts, draws))) if t == 0 else m.step(list(zip(seqs, draws)))
+            assert (out.codes == forced[t]).all()
+            rows.append(np.stack([np.concatenate([m.talker_logits(s), m.predictor_logits(s).ravel()]) for s in range(3)]))
+        got.append(np.stack(rows))
+        m.close()
+    a, b = got
+    step = np.exp2(np.floor(np.log2(np.maximum(np.abs(b), 2.0))) - 7)
+    assert float((np.abs(a - b) / step).max()) <= 2.0
