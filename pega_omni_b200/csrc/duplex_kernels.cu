@@ -70,12 +70,13 @@ __global__ void lm_embed_state_kernel(const void* state, const int32_t* __restri
   embed_row(row, t, out + (int64_t)s * dim, dim, err);
 }
 
-// y = x * (alpha * rsqrt(eps + mean(x^2))) (lm.cu:74-84)
+// y = x * (alpha * rsqrt(eps + mean(x^2))) (lm.cu:74-84); v is 0 in threads past the row
 __device__ __forceinline__ void norm_row(const float* v, const bf16* alpha, bf16* out, int dim, float eps, float* scratch) {
   float ss = 0.f;
 #pragma unroll
   for (int k = 0; k < 8; ++k) ss += v[k] * v[k];
   const float r = rsqrtf(block_add(ss, scratch) / dim + eps);
+  if (threadIdx.x * 8 >= dim) return;
   float a[8], y[8];
   ld8(alpha + threadIdx.x * 8, a);
 #pragma unroll
@@ -89,8 +90,8 @@ __global__ void lm_norm_kernel(const bf16* x, const bf16* __restrict__ alpha, bf
   grid_wait();
   __shared__ float scratch[32];
   const int64_t at = (int64_t)blockIdx.x * dim;
-  float v[8];
-  ld8cg(x + at + threadIdx.x * 8, v);
+  float v[8] = {};
+  if (threadIdx.x * 8 < dim) ld8cg(x + at + threadIdx.x * 8, v);
   norm_row(v, alpha, out + at, dim, eps, scratch);
 }
 
@@ -101,12 +102,14 @@ __global__ void lm_add_norm_kernel(const bf16* y, bf16* x, const bf16* __restric
   grid_wait();
   __shared__ float scratch[32];
   const int64_t at = (int64_t)blockIdx.x * dim + threadIdx.x * 8;
-  float v[8], u[8];
-  ld8cg(x + at, v);
-  ld8cg(y + at, u);
+  float v[8] = {}, u[8];
+  if (threadIdx.x * 8 < dim) {
+    ld8cg(x + at, v);
+    ld8cg(y + at, u);
 #pragma unroll
-  for (int k = 0; k < 8; ++k) v[k] = bf16_round(v[k] + u[k]);
-  st8(x + at, v);
+    for (int k = 0; k < 8; ++k) v[k] = bf16_round(v[k] + u[k]);
+    st8(x + at, v);
+  }
   if (out) norm_row(v, alpha, out + (int64_t)blockIdx.x * dim, dim, eps, scratch);
 }
 
@@ -192,24 +195,23 @@ __global__ void lm_tp_add_norm_kernel(const bf16* __restrict__ mine, const bf16*
   }
   __syncthreads();
   const int64_t at = (int64_t)blockIdx.x * dim + threadIdx.x * 8;
-  float v[8], a[8], b[8];
-  ld8(x + at, v);
-  ld8(mine + at, a);
-  if (peer_ready) {
-    Pack8 raw;
-    uint32_t* w = reinterpret_cast<uint32_t*>(&raw);
-    asm volatile("ld.relaxed.sys.global.v4.u32 {%0, %1, %2, %3}, [%4];"
-                 : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3])
-                 : "l"(peer + at)
-                 : "memory");
-    unpack8(raw, b);
-  } else {
+  float v[8] = {}, a[8], b[8] = {};
+  if (threadIdx.x * 8 < dim) {
+    ld8(x + at, v);
+    ld8(mine + at, a);
+    if (peer_ready) {
+      Pack8 raw;
+      uint32_t* w = reinterpret_cast<uint32_t*>(&raw);
+      asm volatile("ld.relaxed.sys.global.v4.u32 {%0, %1, %2, %3}, [%4];"
+                   : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3])
+                   : "l"(peer + at)
+                   : "memory");
+      unpack8(raw, b);
+    }
 #pragma unroll
-    for (int k = 0; k < 8; ++k) b[k] = 0.f;
+    for (int k = 0; k < 8; ++k) v[k] = bf16_round(v[k] + bf16_round(a[k] + b[k]));
+    st8(x + at, v);
   }
-#pragma unroll
-  for (int k = 0; k < 8; ++k) v[k] = bf16_round(v[k] + bf16_round(a[k] + b[k]));
-  st8(x + at, v);
   if (out) norm_row(v, alpha, out + (int64_t)blockIdx.x * dim, dim, eps, scratch);
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -552,12 +554,14 @@ __global__ void lm_dep_embed_norm_kernel(const bf16* projected, int k, const bf1
     if (threadIdx.x == 0) raise(err, kErrBadIndex);
     id = 0;
   }
-  float v[8], e[8];
-  ld8cg(projected + ((int64_t)s * kDepSteps + k) * dim + c, v);
-  ld8(table + id * dim + c, e);
+  float v[8] = {}, e[8];
+  if (c < dim) {
+    ld8cg(projected + ((int64_t)s * kDepSteps + k) * dim + c, v);
+    ld8(table + id * dim + c, e);
 #pragma unroll
-  for (int j = 0; j < 8; ++j) v[j] = bf16_round(v[j] + e[j]);
-  st8(x + (int64_t)s * dim + c, v);
+    for (int j = 0; j < 8; ++j) v[j] = bf16_round(v[j] + e[j]);
+    st8(x + (int64_t)s * dim + c, v);
+  }
   norm_row(v, alpha, xn + (int64_t)s * dim, dim, eps, scratch);
 }
 
@@ -821,27 +825,27 @@ cudaError_t launch_lm_embed_state(const void* state, const int32_t* lines, int64
 
 cudaError_t launch_lm_norm(const bf16* x, const bf16* alpha, bf16* out, int rows, int dim, float eps, cudaStream_t s) {
   if (!row_dim_ok(dim)) return cudaErrorInvalidValue;
-  return launch_pdl(lm_norm_kernel, dim3(rows), dim3(dim / 8), 0, s, x, alpha, out, dim, eps);
+  return launch_pdl(lm_norm_kernel, dim3(rows), dim3(row_threads(dim)), 0, s, x, alpha, out, dim, eps);
 }
 
 cudaError_t launch_lm_add_norm(const bf16* y, bf16* x, const bf16* alpha, bf16* out, int rows, int dim, float eps,
                                cudaStream_t s) {
   if (!row_dim_ok(dim)) return cudaErrorInvalidValue;
-  return launch_pdl(lm_add_norm_kernel, dim3(rows), dim3(dim / 8), 0, s, y, x, alpha, out, dim, eps);
+  return launch_pdl(lm_add_norm_kernel, dim3(rows), dim3(row_threads(dim)), 0, s, y, x, alpha, out, dim, eps);
 }
 
 cudaError_t launch_lm_add_norm_sum(const Summands& y, bf16* x, const bf16* alpha, bf16* out, int rows, int dim, float eps,
                                    cudaStream_t s) {
   if (!row_dim_ok(dim)) return cudaErrorInvalidValue;
   return with_summands(y.splits, [&](auto sums) {
-    return launch_pdl(lm_add_norm_sum_kernel<decltype(sums)::value>, dim3(rows), dim3((dim + 255) / 256 * 32), 0, s, y, x, alpha, out, dim, eps);
+    return launch_pdl(lm_add_norm_sum_kernel<decltype(sums)::value>, dim3(rows), dim3(row_threads(dim)), 0, s, y, x, alpha, out, dim, eps);
   });
 }
 
 cudaError_t launch_lm_tp_add_norm(const bf16* mine, const bf16* peer, bf16* x, const bf16* alpha, bf16* out, int rows,
                                   int dim, float eps, const TpLink& link, uint32_t* err, cudaStream_t s) {
   if (!row_dim_ok(dim) || !peer || !link.my_flag || !link.peer_flag) return cudaErrorInvalidValue;
-  lm_tp_add_norm_kernel<<<rows, dim / 8, 0, s>>>(mine, peer, x, alpha, out, dim, eps, link.my_flag, link.peer_flag,
+  lm_tp_add_norm_kernel<<<rows, row_threads(dim), 0, s>>>(mine, peer, x, alpha, out, dim, eps, link.my_flag, link.peer_flag,
                                                  link.counter, link.finished, err);
   return cudaGetLastError();
 }
@@ -897,7 +901,7 @@ cudaError_t launch_lm_dep_embed_norm(const bf16* projected, int k, const bf16* t
                                      const int32_t* drawn, const bf16* alpha, bf16* x, bf16* xn, int rows, int dim,
                                      float eps, uint32_t* err, cudaStream_t s) {
   if (!row_dim_ok(dim)) return cudaErrorInvalidValue;
-  return launch_pdl(lm_dep_embed_norm_kernel, dim3(rows), dim3(dim / 8), 0, s, projected, k, table, table_rows, drawn, alpha, x, xn, dim, eps, err);
+  return launch_pdl(lm_dep_embed_norm_kernel, dim3(rows), dim3(row_threads(dim)), 0, s, projected, k, table, table_rows, drawn, alpha, x, xn, dim, eps, err);
 }
 
 cudaError_t launch_lm_dep_kv_attend(const bf16* qkv, bf16* ws, int step, bf16* out, int rows, int heads, float scale,

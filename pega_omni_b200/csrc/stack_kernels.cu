@@ -17,7 +17,7 @@ namespace omni {
 
 // ---- RMSNorm + residual ------------------------------------------------------
 
-// One block of dim/8 threads per row. Semantics of `qwen3_norm_copy`
+// One block per row, eight elements a thread. Semantics of `qwen3_norm_copy`
 // (qwen3.cu:18-31).
 __global__ void norm_copy_kernel(const bf16* x, const bf16* __restrict__ w, bf16* __restrict__ out,
                                  bf16* __restrict__ res, int dim, float eps) {
@@ -25,12 +25,14 @@ __global__ void norm_copy_kernel(const bf16* x, const bf16* __restrict__ w, bf16
   grid_wait();
   __shared__ float scratch[32];
   const int64_t at = (int64_t)blockIdx.x * dim + threadIdx.x * 8;
-  float v[8], g[8];
-  ld8cg(x + at, v);
+  const bool on = threadIdx.x * 8 < dim;
+  float v[8] = {}, g[8];
+  if (on) ld8cg(x + at, v);
   float ss = 0.f;
 #pragma unroll
   for (int k = 0; k < 8; ++k) ss += v[k] * v[k];
   const float r = rsqrtf(block_add(ss, scratch) / dim + eps);
+  if (!on) return;
   st8(res + at, v);
   ld8(w + threadIdx.x * 8, g);
 #pragma unroll
@@ -46,9 +48,12 @@ __global__ void add_norm_kernel(const bf16* x, bf16* res, const bf16* __restrict
   __shared__ float scratch[32];
   const int n = blockIdx.x;
   const int64_t at = (int64_t)n * dim + threadIdx.x * 8;
-  float v[8], rv[8], g[8];
-  ld8cg(x + at, v);  // (out may be x)
-  ld8cg(res + at, rv);
+  const bool on = threadIdx.x * 8 < dim;
+  float v[8] = {}, rv[8] = {}, g[8];
+  if (on) {
+    ld8cg(x + at, v);  // (out may be x)
+    ld8cg(res + at, rv);
+  }
   float ss = 0.f;
 #pragma unroll
   for (int k = 0; k < 8; ++k) {
@@ -56,6 +61,7 @@ __global__ void add_norm_kernel(const bf16* x, bf16* res, const bf16* __restrict
     ss += v[k] * v[k];
   }
   const float r = rsqrtf(block_add(ss, scratch) / dim + eps);
+  if (!on) return;
   st8(res + at, v);
   if (n % every != which) return;
   ld8(w + threadIdx.x * 8, g);
@@ -121,7 +127,7 @@ cudaError_t launch_add_norm_sum(const Summands& x, bf16* res, const bf16* w, bf1
                                 int every, int which, cudaStream_t s) {
   if (dim % 8 || dim / 8 > 1024) return cudaErrorInvalidValue;
   return with_summands(x.splits, [&](auto sums) {
-    return launch_pdl(add_norm_sum_kernel<decltype(sums)::value>, dim3(rows), dim3((dim + 255) / 256 * 32), 0, s, x, res, w, out, dim, eps, every, which);
+    return launch_pdl(add_norm_sum_kernel<decltype(sums)::value>, dim3(rows), dim3(row_threads(dim)), 0, s, x, res, w, out, dim, eps, every, which);
   });
 }
 
@@ -147,13 +153,13 @@ cudaError_t launch_interleave_gate_up(const bf16* src, bf16* dst, int inter, int
 cudaError_t launch_norm_copy(const bf16* x, const bf16* w, bf16* out, bf16* res, int rows, int dim, float eps,
                              cudaStream_t s) {
   if (dim % 8 || dim / 8 > 1024) return cudaErrorInvalidValue;
-  return launch_pdl(norm_copy_kernel, dim3(rows), dim3(dim / 8), 0, s, x, w, out, res, dim, eps);
+  return launch_pdl(norm_copy_kernel, dim3(rows), dim3(row_threads(dim)), 0, s, x, w, out, res, dim, eps);
 }
 
 cudaError_t launch_add_norm(const bf16* x, bf16* res, const bf16* w, bf16* out, int rows, int dim, float eps,
                             int every, int which, cudaStream_t s) {
   if (dim % 8 || dim / 8 > 1024) return cudaErrorInvalidValue;
-  return launch_pdl(add_norm_kernel, dim3(rows), dim3(dim / 8), 0, s, x, res, w, out, dim, eps, every, which);
+  return launch_pdl(add_norm_kernel, dim3(rows), dim3(row_threads(dim)), 0, s, x, res, w, out, dim, eps, every, which);
 }
 
 cudaError_t launch_silu_mul(const bf16* gate_up, bf16* act, int rows, int inter, int interleaved, cudaStream_t s) {

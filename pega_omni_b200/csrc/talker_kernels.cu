@@ -103,13 +103,15 @@ __global__ void frame_embed_norm_kernel(SlotState st, const bf16* __restrict__ p
   grid_trigger();
   __shared__ float scratch[32];
   const int64_t at = (int64_t)blockIdx.x * dim + threadIdx.x * 8;
-  float v[8], g[8], ss = 0.f;
-  ld8(gain + threadIdx.x * 8, g);
+  const bool on = threadIdx.x * 8 < dim;
+  float v[8] = {}, g[8], ss = 0.f;
+  if (on) ld8(gain + threadIdx.x * 8, g);
   grid_wait();
-  frame_embed_row(st, pad, codec_emb, vocab, p_emb, p_vocab, groups, dim, err, v);
+  if (on) frame_embed_row(st, pad, codec_emb, vocab, p_emb, p_vocab, groups, dim, err, v);
 #pragma unroll
   for (int k = 0; k < 8; ++k) v[k] = bf16_round(v[k]), ss += v[k] * v[k];
   const float r = rsqrtf(block_add(ss, scratch) / dim + eps);
+  if (!on) return;
   st8(res + at, v);
 #pragma unroll
   for (int k = 0; k < 8; ++k) v[k] = v[k] * r * g[k];
@@ -164,7 +166,7 @@ cudaError_t launch_frame_embed(SlotState st, const bf16* pad, const bf16* codec_
 cudaError_t launch_frame_embed_norm(SlotState st, const bf16* pad, const bf16* codec_emb, int vocab, const bf16* p_emb,
                                     int p_vocab, int groups, const bf16* gain, bf16* res, bf16* x, int rows, int dim,
                                     float eps, uint32_t* err, cudaStream_t s) {
-  return launch_pdl(frame_embed_norm_kernel, dim3(rows), dim3(dim / 8), 0, s, st, pad, codec_emb, vocab, p_emb, p_vocab, groups,
+  return launch_pdl(frame_embed_norm_kernel, dim3(rows), dim3(row_threads(dim)), 0, s, st, pad, codec_emb, vocab, p_emb, p_vocab, groups,
                     gain, res, x, dim, eps, err);
 }
 

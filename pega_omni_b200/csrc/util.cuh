@@ -112,10 +112,10 @@ __device__ __forceinline__ float warp_fmax(float v) {
   return v;
 }
 
-// Sum over the block; `scratch` is 32 floats of shared memory. Ends with a
+// Sum over the block, a whole number of warps; `scratch` is 32 floats of shared memory. Ends with a
 // barrier so `scratch` can be reused at once.
 __device__ __forceinline__ float block_add(float v, float* scratch) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = (blockDim.x + 31) >> 5;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   v = warp_add(v);
   if (lane == 0) scratch[warp] = v;
   __syncthreads();
@@ -125,15 +125,8 @@ __device__ __forceinline__ float block_add(float v, float* scratch) {
   return v;
 }
 
-__device__ __forceinline__ float block_fmax(float v, float* scratch) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = (blockDim.x + 31) >> 5;
-  v = warp_fmax(v);
-  if (lane == 0) scratch[warp] = v;
-  __syncthreads();
-  v = lane < nwarps ? scratch[lane] : -INFINITY;
-  v = warp_fmax(v);
-  __syncthreads();
-  return v;
-}
+// Threads of a block that works on a row of `dim` elements, eight a thread: whole warps, since in a part of one block_add
+// would add up as many warps as it has lanes.
+inline int row_threads(int dim) { return (dim + 255) / 256 * 32; }
 
 }  // namespace omni

@@ -371,3 +371,27 @@ def test_prompts_of_a_tile_do_not_touch_one_another(ops, lens, broken):
         outs.append(out)
     others = seq != broken
     assert torch.equal(outs[0][others], outs[1][others])
+
+
+@pytest.mark.parametrize("dim", [128, 320, 2112, 4160, 8192])
+def test_norms_of_rows_that_end_inside_a_warp(ops, dim):
+    x, y, gain = rand((3, dim), 81), rand((3, dim), 82), rand((dim,), 83, 0.2) + 1
+    out, res, out2 = (torch.zeros((3, dim), dtype=torch.bfloat16, device="cuda") for _ in range(3))
+    res2 = y.clone()
+    torch.cuda.synchronize()
+    ops.norm_copy(x, gain, out, res, 1e-6)
+    ops.add_norm(x, res2, gain, out2, 1e-6)
+    ops.sync()
+
+    def norm(v):
+        return v * torch.rsqrt((v * v).mean(1, keepdim=True) + 1e-6) * gain.float()
+    close(out, norm(x.float()), steps=1.0)
+    close(out2, norm(x.float() + y.float()), steps=1.0)
+    if dim >= 256:
+        z = y.clone()
+        torch.cuda.synchronize()
+        ops.lm_norm(x, gain, out, 1e-6)
+        ops.lm_norm(z, gain, out2, 1e-6, y=x)
+        ops.sync()
+        close(out, norm(x.float()), steps=1.0)
+        close(out2, norm((x.float() + y.float()).bfloat16().float()), steps=1.0)
