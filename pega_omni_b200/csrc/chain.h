@@ -149,7 +149,8 @@ cudaError_t chain_pass(const Chain& c, const std::vector<Layer>& layers, const G
       OMNI_CHAIN(c.done(launch_rope_kv(b.qkv, L.q_norm, L.k_norm, kv[i], map, rows, a, kv_pages, c.err, c.stream), "rope_kv", 0, 0, rows));
       OMNI_CHAIN(c.done(launch_attend(b.qkv, kv[i], b.attn, map, rows, a, c.err, c.stream), "attend", 0, 0, rows));
     } else {
-      OMNI_CHAIN(c.done(launch_rope_attend(b.qkv, from, L.q_norm, L.k_norm, kv[i], b.attn, map, rows, a, kv_pages, c.err, c.stream),
+      OMNI_CHAIN(c.done(launch_rope_attend(b.qkv, from, L.q_norm, L.k_norm, kv[i], b.attn, map, rows, a, kv_pages, c.sm_count, c.err,
+                                       c.stream),
                         "rope_attend", 0, 0, rows));
     }
     OMNI_CHAIN(c.gemm(L.o, hidden, qd, b.attn, rows, kStreamPartials, nullptr, hidden, &sum));

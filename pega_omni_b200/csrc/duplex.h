@@ -63,7 +63,7 @@ cudaError_t launch_lm_attend(const bf16* qkv, const void* kv, const int32_t* pos
 // launch_lm_rope_kv and launch_lm_attend of one row per session in one kernel.
 cudaError_t launch_lm_rope_attend(const bf16* qkv, void* kv, const int32_t* pos, const int32_t* slots,
                                   const int32_t* indptr, const int32_t* pages, bf16* out, int rows, int heads, float coef,
-                                  float scale, int context, int kv_pages, uint32_t* err, cudaStream_t s);
+                                  float scale, int context, int kv_pages, int sm_count, uint32_t* err, cudaStream_t s);
 // Depformer step k: x = bf16(projected[s][k] + table[drawn[s][k]]); xn = norm(x).
 cudaError_t launch_lm_dep_embed_norm(const bf16* projected, int k, const bf16* table, int table_rows,
                                      const int32_t* drawn, const bf16* alpha, bf16* x, bf16* xn, int rows, int dim,

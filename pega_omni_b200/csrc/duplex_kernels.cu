@@ -891,8 +891,8 @@ static cudaError_t launch_lm_rope_attend_w(const bf16* qkv, void* kv, const int3
 
 cudaError_t launch_lm_rope_attend(const bf16* qkv, void* kv, const int32_t* pos, const int32_t* slots,
                                   const int32_t* indptr, const int32_t* pages, bf16* out, int rows, int heads, float coef,
-                                  float scale, int context, int kv_pages, uint32_t* err, cudaStream_t s) {
-  if (rows * heads <= 148)  // one CTA per SM at most: more warps of it
+                                  float scale, int context, int kv_pages, int sm_count, uint32_t* err, cudaStream_t s) {
+  if (rows * heads <= sm_count)  // one CTA per SM at most: more warps of it
     return launch_lm_rope_attend_w<16>(qkv, kv, pos, slots, indptr, pages, out, rows, heads, coef, scale, context, kv_pages, err, s);
   return launch_lm_rope_attend_w<4>(qkv, kv, pos, slots, indptr, pages, out, rows, heads, coef, scale, context, kv_pages, err, s);
 }

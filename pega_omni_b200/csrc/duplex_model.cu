@@ -302,7 +302,7 @@ int helium_forward(omni_duplex* m, int rows, const int32_t* pos, const int32_t* 
     else DTRY(gemm(m, L.qkv, 3 * Dl, D, m->xn, rows, m->qkv, 3 * Dl));
     if (!seq) {
       DLAUNCH(m, launch_lm_rope_attend(m->qkv, m->kv[i], pos, slot, indptr, pages, m->attn, rows, m->local_heads(),
-                                       rope_coef(c), scale, c.context, m->kv_pages, m->err, m->stream));
+                                       rope_coef(c), scale, c.context, m->kv_pages, m->sm_count, m->err, m->stream));
     } else {
       DLAUNCH(m, launch_lm_rope_kv(m->qkv, pos, slot, m->kv[i], rows, m->local_heads(), rope_coef(c), m->kv_pages, m->err, m->stream));
       DLAUNCH(m, launch_lm_attend(m->qkv, m->kv[i], pos, seq, indptr, pages, m->attn, rows, m->local_heads(), scale, c.context,

@@ -62,8 +62,8 @@ struct QkvTable {
   int group = 0;
 };
 cudaError_t launch_rope_attend(const bf16* qkv, const QkvTable& lookup, const bf16* q_norm, const bf16* k_norm, bf16* kv,
-                               bf16* out, const RowMap& map, int rows, const AttnShape& a, int kv_pages, uint32_t* err,
-                               cudaStream_t s);
+                               bf16* out, const RowMap& map, int rows, const AttnShape& a, int kv_pages, int sm_count,
+                               uint32_t* err, cudaStream_t s);
 // Decode/prefill attention of every row over positions 0..pos of its sequence.
 cudaError_t launch_attend(const bf16* qkv, const bf16* kv, bf16* out, const RowMap& map, int rows, const AttnShape& a,
                           uint32_t* err, cudaStream_t s);

@@ -194,7 +194,7 @@ int32_t omni_op_decode_attend(omni_ops* c, const void* qkv, const void* q_norm, 
   const AttnShape a{q_heads, kv_heads, head_dim, eps, theta};
   OPS_CUDA(c, order(c->stream));
   OPS_CUDA(c, launch_rope_attend((const bf16*)qkv, {}, (const bf16*)q_norm, (const bf16*)k_norm, (bf16*)kv, (bf16*)out, map, rows,
-                                 a, kv_pages, c->err, c->stream));
+                                 a, kv_pages, c->sm_count, c->err, c->stream));
   return OMNI_OK;
 }
 
@@ -325,7 +325,7 @@ int32_t omni_op_lm_decode_attend(omni_ops* c, const void* qkv, void* kv, int32_t
   if (!c || !qkv || !kv || !pos || !slot || !indptr || !pages || !out || rows < 1) return OMNI_ERR_INVALID;
   OPS_CUDA(c, order(c->stream));
   OPS_CUDA(c, launch_lm_rope_attend((const bf16*)qkv, kv, pos, slot, indptr, pages, (bf16*)out, rows, heads, coef, scale, context,
-                                    kv_pages, c->err, c->stream));
+                                    kv_pages, c->sm_count, c->err, c->stream));
   return OMNI_OK;
 }
 

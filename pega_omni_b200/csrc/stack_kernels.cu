@@ -380,7 +380,7 @@ __global__ void __launch_bounds__(W * TEAMS * 32, W == 8 ? 1 : 3)
                        const bf16* __restrict__ k_norm, bf16* kv, bf16* __restrict__ out, RowMap map, int items, int hq,
                        int hk, float eps, float theta, float scale, int kv_pages, uint32_t* err) {
   static_assert(W == 1 || TEAMS == 1, "a team of several warps is a CTA");
-  constexpr int E = D / 64, VE = D / 32;
+  constexpr int E = D / 64;
   grid_trigger();
   __shared__ RopeShared<D, G> shared[TEAMS];
   __shared__ MergeShared<D, G, W> merge;
@@ -527,7 +527,7 @@ __global__ void __launch_bounds__(W * TEAMS * 32, W == 8 ? 1 : 3)
 template <int D, int G>
 static cudaError_t launch_rope_attend_dg(const bf16* qkv, const QkvTable& lookup, const bf16* q_norm, const bf16* k_norm,
                                          bf16* kv, bf16* out, const RowMap& map, int rows, const AttnShape& a,
-                                         int kv_pages, uint32_t* err, cudaStream_t s) {
+                                         int kv_pages, int sm_count, uint32_t* err, cudaStream_t s) {
   const int items = (map.pages ? rows : rows / map.per) * a.kv_heads;
   const float scale = 1.f / sqrtf((float)D);
   if (!map.pages) {
@@ -543,29 +543,29 @@ static cudaError_t launch_rope_attend_dg(const bf16* qkv, const QkvTable& lookup
   // items that leave SMs idle: eight warps each, so that 128 keys are one round (sixteen would have to spill: 2,282 against
   // 2,242 us a step of one session, 2,133 against 2,042 us for Higgs at three); more items: four warps, three CTAs an SM
   // (two warps with more CTAs: 4,485 against 4,024 us at 64 sessions, four CTAs an SM with spills 5,655 against 5,228 at 128)
-  return items <= 148 ? go(rope_attend_kernel<D, G, 8, 1>, 8) : go(rope_attend_kernel<D, G, 4, 1>, 4);
+  return items <= sm_count ? go(rope_attend_kernel<D, G, 8, 1>, 8) : go(rope_attend_kernel<D, G, 4, 1>, 4);
 }
 
 template <int D>
 static cudaError_t launch_rope_attend_d(const bf16* qkv, const QkvTable& lookup, const bf16* q_norm, const bf16* k_norm,
                                         bf16* kv, bf16* out, const RowMap& map, int rows, const AttnShape& a,
-                                        int kv_pages, uint32_t* err, cudaStream_t s) {
+                                        int kv_pages, int sm_count, uint32_t* err, cudaStream_t s) {
   switch (a.q_heads / a.kv_heads) {
-    case 1: return launch_rope_attend_dg<D, 1>(qkv, lookup, q_norm, k_norm, kv, out, map, rows, a, kv_pages, err, s);
-    case 2: return launch_rope_attend_dg<D, 2>(qkv, lookup, q_norm, k_norm, kv, out, map, rows, a, kv_pages, err, s);
-    case 4: return launch_rope_attend_dg<D, 4>(qkv, lookup, q_norm, k_norm, kv, out, map, rows, a, kv_pages, err, s);
-    case 5: return launch_rope_attend_dg<D, 5>(qkv, lookup, q_norm, k_norm, kv, out, map, rows, a, kv_pages, err, s);
-    case 8: return launch_rope_attend_dg<D, 8>(qkv, lookup, q_norm, k_norm, kv, out, map, rows, a, kv_pages, err, s);
+    case 1: return launch_rope_attend_dg<D, 1>(qkv, lookup, q_norm, k_norm, kv, out, map, rows, a, kv_pages, sm_count, err, s);
+    case 2: return launch_rope_attend_dg<D, 2>(qkv, lookup, q_norm, k_norm, kv, out, map, rows, a, kv_pages, sm_count, err, s);
+    case 4: return launch_rope_attend_dg<D, 4>(qkv, lookup, q_norm, k_norm, kv, out, map, rows, a, kv_pages, sm_count, err, s);
+    case 5: return launch_rope_attend_dg<D, 5>(qkv, lookup, q_norm, k_norm, kv, out, map, rows, a, kv_pages, sm_count, err, s);
+    case 8: return launch_rope_attend_dg<D, 8>(qkv, lookup, q_norm, k_norm, kv, out, map, rows, a, kv_pages, sm_count, err, s);
     default: return cudaErrorInvalidValue;
   }
 }
 
 cudaError_t launch_rope_attend(const bf16* qkv, const QkvTable& lookup, const bf16* q_norm, const bf16* k_norm, bf16* kv,
-                               bf16* out, const RowMap& map, int rows, const AttnShape& a, int kv_pages, uint32_t* err,
-                               cudaStream_t s) {
+                               bf16* out, const RowMap& map, int rows, const AttnShape& a, int kv_pages, int sm_count,
+                               uint32_t* err, cudaStream_t s) {
   if (a.q_heads % a.kv_heads) return cudaErrorInvalidValue;
-  if (a.head_dim == 128) return launch_rope_attend_d<128>(qkv, lookup, q_norm, k_norm, kv, out, map, rows, a, kv_pages, err, s);
-  if (a.head_dim == 64) return launch_rope_attend_d<64>(qkv, lookup, q_norm, k_norm, kv, out, map, rows, a, kv_pages, err, s);
+  if (a.head_dim == 128) return launch_rope_attend_d<128>(qkv, lookup, q_norm, k_norm, kv, out, map, rows, a, kv_pages, sm_count, err, s);
+  if (a.head_dim == 64) return launch_rope_attend_d<64>(qkv, lookup, q_norm, k_norm, kv, out, map, rows, a, kv_pages, sm_count, err, s);
   return cudaErrorInvalidValue;
 }
 
