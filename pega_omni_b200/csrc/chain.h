@@ -15,13 +15,14 @@
 
 namespace omni {
 
-// A GEMM of a chain is planned once per (weights, inputs, outputs, rows) and kept by the model.
+// A GEMM of a chain is planned once per everything its plan holds - operands, shape, output, epilogue - and kept by the model.
 struct ChainPlan {
   bool few = false;
   FewPlan f;
   StreamGemmPlan s;
 };
-using ChainPlans = std::map<std::tuple<const void*, const void*, const void*, int, int>, ChainPlan>;
+using ChainKey = std::tuple<const void*, const void*, const void*, const void*, int, int, int, int, int, int>;
+using ChainPlans = std::map<ChainKey, ChainPlan>;
 
 // Stands behind every kernel of a traced program: a stamp of the device's clock, and the kernel's name and shape.
 struct ChainTrace {
@@ -87,7 +88,7 @@ struct Chain {
 
  private:
   ChainPlan* plan(const bf16* w, int N, int K, const bf16* x, int rows, int out, bf16* y, int ldy, Epilogue epi) const {
-    const auto key = std::make_tuple((const void*)w, (const void*)x, (const void*)y, rows, out);
+    const ChainKey key(w, x, y, epi.bias, N, K, rows, out, ldy, epi.kind);
     auto it = plans->find(key);
     if (it != plans->end()) return &it->second;
     ChainPlan p;
