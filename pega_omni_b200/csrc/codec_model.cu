@@ -449,11 +449,7 @@ size_t elems_per_stream(const omni_codec_config& c) {
 
 // y[rows, N] = x[rows, K] . w[N, K]^T on the library's dense GEMMs (K a multiple of 64).
 int dense(omni_codec* m, const bf16* w, int N, int K, const bf16* x, int rows, bf16* y) {
-  if (stream_supports(N, K, rows)) {
-    CCUDA(m, m->chain().gemm(w, N, K, x, rows, kStreamBf16, y, N));
-  } else {
-    CLAUNCH(m, gemv_launch(w, N, K, x, rows, y, N, Epilogue{}, m->sm_count, m->stream));
-  }
+  CCUDA(m, m->chain().gemm(w, N, K, x, rows, kStreamBf16, y, N));
   return OMNI_OK;
 }
 

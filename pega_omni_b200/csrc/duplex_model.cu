@@ -109,7 +109,7 @@ struct omni_duplex {
   // activations (max_rows = max(max_prefill, max_sessions))
   int max_rows = 0;
   bf16 *x = nullptr, *x2 = nullptr, *xn = nullptr,  // x2, dx2: the other residual of a few rows' chain
-      *qkv = nullptr, *attn = nullptr, *y = nullptr, *gu = nullptr, *act = nullptr;
+      *qkv = nullptr, *attn = nullptr, *y = nullptr, *act = nullptr;
   bf16 *text_logits = nullptr, *audio_logits = nullptr;  // [max_sessions, text_vocab], [8][max_sessions][card]
   bf16 *dproj = nullptr, *dx = nullptr, *dx2 = nullptr, *dxn = nullptr, *dqkv = nullptr, *dattn = nullptr, *dact = nullptr, *dy = nullptr;
   int32_t *rows_buf = nullptr, *drawn = nullptr, *emitted = nullptr;
@@ -216,13 +216,9 @@ int weight(omni_duplex* m, const Index& idx, const std::string& name, std::initi
   return OMNI_OK;
 }
 
-// y[rows, N] = x[rows, K] . w[N, K]^T on the path the row count calls for.
+// y[rows, N] = x[rows, K] . w[N, K]^T (valid_config: every K a multiple of 64).
 int gemm(omni_duplex* m, const bf16* w, int N, int K, const bf16* x, int rows, bf16* y, int ldy) {
-  if (stream_supports(N, K, rows)) {
-    DCUDA(m, m->chain().gemm(w, N, K, x, rows, kStreamBf16, y, ldy));
-  } else {
-    DLAUNCH(m, gemv_launch(w, N, K, x, rows, y, ldy, Epilogue{}, m->sm_count, m->stream));
-  }
+  DCUDA(m, m->chain().gemm(w, N, K, x, rows, kStreamBf16, y, ldy));
   return OMNI_OK;
 }
 
@@ -309,14 +305,8 @@ int helium_forward(omni_duplex* m, int rows, const int32_t* pos, const int32_t* 
                                   m->kv_pages, m->err, m->stream));
     }
     DTRY(projected(L.o, Dl, m->attn, 0, L.norm2));
-    if (stream) {
-      DTRY(behind_norm(L.norm2, L.gate_up, 2 * Hl, kStreamSwiglu, m->act, Hl));
-    } else if (rows <= kChainRows || wide_fuses(2 * Hl, D, kGateGroup)) {
-      DCUDA(m, chain.gemm(L.gate_up, 2 * Hl, D, m->xn, rows, kStreamSwiglu, m->act, Hl));
-    } else {
-      DTRY(gemm(m, L.gate_up, 2 * Hl, D, m->xn, rows, m->gu, 2 * Hl));
-      DLAUNCH(m, launch_silu_mul(m->gu, m->act, rows, Hl, kGateGroup, m->stream));
-    }
+    if (stream) DTRY(behind_norm(L.norm2, L.gate_up, 2 * Hl, kStreamSwiglu, m->act, Hl));
+    else DCUDA(m, chain.gemm(L.gate_up, 2 * Hl, D, m->xn, rows, kStreamSwiglu, m->act, Hl));
     DTRY(projected(L.down, Hl, m->act, 1, i + 1 < c.layers ? m->h[i + 1].norm1 : m->out_norm));
   }
   if (stream) DLAUNCH(m, launch_lm_add_norm_sum(y, res, m->out_norm, m->xn, rows, D, c.norm_eps, m->stream));
@@ -504,7 +494,6 @@ int32_t omni_duplex_create(const omni_duplex_config* config, const omni_tensor* 
     m->tp_buf_bytes = (R * D * sizeof(bf16) + 255) & ~(size_t)255;
     DTRY(dalloc(m, &m->tp_region, 256 + 2 * m->tp_buf_bytes, true));
   }
-  DTRY(dalloc(m, &m->gu, R * 2 * H));
   DTRY(dalloc(m, &m->act, R * H));
   DTRY(dalloc(m, &m->text_logits, (size_t)S * c.text_vocab, true));
   DTRY(dalloc(m, &m->audio_logits, (size_t)kDepSteps * S * c.card, true));

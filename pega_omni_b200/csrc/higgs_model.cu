@@ -70,7 +70,7 @@ struct omni_higgs {
   std::vector<std::unique_ptr<omni_higgs_seq>> seqs;
 
   int max_rows = 0;
-  bf16 *embeds = nullptr, *x = nullptr, *res = nullptr, *res2 = nullptr, *qkv = nullptr, *attn = nullptr, *gate_up = nullptr,
+  bf16 *embeds = nullptr, *x = nullptr, *res = nullptr, *res2 = nullptr, *qkv = nullptr, *attn = nullptr,
        *act = nullptr, *hidden = nullptr, *logits = nullptr;
   int32_t* codes = nullptr;
 
@@ -173,11 +173,7 @@ int upload(omni_higgs* m, const Index& idx, const std::string& name, std::initia
 }
 
 int gemm(omni_higgs* m, const bf16* w, int N, int K, const bf16* x, int rows, bf16* y, int ldy) {
-  if (stream_supports(N, K, rows)) {
-    HCUDA(m, m->chain().gemm(w, N, K, x, rows, kStreamBf16, y, ldy));
-  } else {
-    HLAUNCH(m, gemv_launch(w, N, K, x, rows, y, ldy, Epilogue{}, m->sm_count, m->stream));
-  }
+  HCUDA(m, m->chain().gemm(w, N, K, x, rows, kStreamBf16, y, ldy));
   return OMNI_OK;
 }
 
@@ -191,7 +187,7 @@ int body_forward(omni_higgs* m, const bf16* input, int rows, const RowMap& map, 
   const int h = c.hidden, I = both ? 2 * c.inter : c.inter, qd = c.q_heads * c.head_dim, qw = m->qkv_width();
   const AttnShape a{c.q_heads, c.kv_heads, c.head_dim, c.rms_eps, c.rope_theta};
   HLAUNCH(m, launch_norm_copy(input, m->layers[0].ln1, m->x, m->res, rows, h, c.rms_eps, m->stream));
-  if (rows <= kChainRows && chain_supports(h, I, qd, c.head_dim)) {
+  if (rows <= kChainRows) {
     HCUDA(m, chain_pass(m->chain(), m->layers, [&](const Layer& L) { return both ? L.gate_up_audio : L.gate_up; },
                         [&](const Layer& L) { return both ? L.down_audio : L.down; }, h, I, a,
                         ChainBuffers{m->x, m->res, m->res2, m->qkv, m->attn, m->act}, rows, map, m->kv, m->pages_total, m->norm, out,
@@ -206,12 +202,7 @@ int body_forward(omni_higgs* m, const bf16* input, int rows, const RowMap& map, 
     HTRY(gemm(m, L.o, h, qd, m->attn, rows, m->x, h));
     HLAUNCH(m, launch_add_norm(m->x, m->res, L.ln2, m->x, rows, h, c.rms_eps, 1, 0, m->stream));
     const bf16* gate_up = both ? L.gate_up_audio : L.gate_up;
-    if (wide_fuses(2 * I, h, kGateGroup)) {
-      HCUDA(m, m->chain().gemm(gate_up, 2 * I, h, m->x, rows, kStreamSwiglu, m->act, I));
-    } else {
-      HTRY(gemm(m, gate_up, 2 * I, h, m->x, rows, m->gate_up, 2 * I));
-      HLAUNCH(m, launch_silu_mul(m->gate_up, m->act, rows, I, kGateGroup, m->stream));
-    }
+    HCUDA(m, m->chain().gemm(gate_up, 2 * I, h, m->x, rows, kStreamSwiglu, m->act, I));
     HTRY(gemm(m, both ? L.down_audio : L.down, h, I, m->act, rows, m->x, h));
     const bf16* next = i + 1 < c.layers ? m->layers[i + 1].ln1 : m->norm;
     HLAUNCH(m, launch_add_norm(m->x, m->res, next, i + 1 < c.layers ? m->x : out, rows, h, c.rms_eps, 1, 0, m->stream));
@@ -406,7 +397,6 @@ int32_t omni_higgs_create(const omni_higgs_config* config, const omni_tensor* te
   HTRY(halloc(m, &m->qkv, R * (q + 2 * kvw)));
   HTRY(halloc(m, &m->attn, R * q));
   const size_t Iw = c.audio_adapter ? 2 * I : I;  // widest MLP a row goes through
-  HTRY(halloc(m, &m->gate_up, R * 2 * Iw));
   HTRY(halloc(m, &m->act, R * Iw));
   HTRY(halloc(m, &m->hidden, (size_t)c.max_batch * h, true));
   HTRY(halloc(m, &m->logits, (size_t)c.max_batch * head, true));
