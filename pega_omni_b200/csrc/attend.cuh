@@ -195,7 +195,8 @@ __device__ __forceinline__ void attend_pages(AttnShared<D, G, W>& sh, const bf16
     KvBlock<D> blk;
     if constexpr (S > 0) {
       const int s = turn % S;
-      sm100::mbar_wait(sm100::smem_addr(stage->bars + s), stage->par >> s & 1u, stage->err);
+      static_assert(S == 1, "with more slots an abort would have to wait for the other copies");
+      if (!sm100::mbar_wait(sm100::smem_addr(stage->bars + s), stage->par >> s & 1u, stage->err)) break;
       stage->par ^= 1u << s;
       blk.load(reinterpret_cast<const bf16*>(stage->slots + s * kv_block_bytes<D>()), lane);
       __syncwarp();  // the block is in registers: its slot takes the block S turns ahead

@@ -86,6 +86,7 @@ __global__ void __launch_bounds__(kConvThreads, 1)
   extern __shared__ unsigned char conv_smem_raw[];
   __shared__ __align__(8) uint64_t bars_s[2 * kConvMaxStages + 4];
   __shared__ uint32_t tmem_slot_s;
+  __shared__ int gave_up_s, issued_s[2];  // a wait ran out; stages the producers had filled by then (-1: all)
   const uint32_t raw = smem_addr(conv_smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
   unsigned char* base_ptr = conv_smem_raw + (base - raw);
@@ -106,6 +107,7 @@ __global__ void __launch_bounds__(kConvThreads, 1)
   };
 
   if (threadIdx.x == 0) {
+    gave_up_s = 0, issued_s[0] = issued_s[1] = -1;
     prefetch_tensormap(&wmap);
     for (int s = 0; s < a.stages; ++s) {
       mbar_init(full_bar(s), 2);  // the two producers
@@ -160,10 +162,7 @@ __global__ void __launch_bounds__(kConvThreads, 1)
           if (++stage == a.stages) stage = 0, phase ^= 1u;
         }
       }
-      if (!alive) {  // no copy may land once the CTA has left: time for those under way, whose barriers may lack the other half
-        const uint64_t start = global_timer_ns();
-        while (global_timer_ns() - start < 2000000ull) {}
-      }
+      if (!alive) gave_up_s = 1, issued_s[warp] = done;
     }
     __syncwarp();
   } else if (warp < 2 + kConvIssuers) {
@@ -207,6 +206,7 @@ __global__ void __launch_bounds__(kConvThreads, 1)
         if (alive && elect_one()) mma_commit(acc_full(buf));
         __syncwarp();
       }
+      if (!alive && lane == 0) gave_up_s = 1;
     }
   } else {
     // Epilogue. A warp reaches the 32 TMEM lanes of quadrant warp % 4, one output row per thread, and takes the tile 32
@@ -321,6 +321,14 @@ __global__ void __launch_bounds__(kConvThreads, 1)
   }
   tc_fence_before_sync();
   __syncthreads();
+  if (gave_up_s && threadIdx.x == 0) {
+    // no copy may land once the CTA has left: a stage that only one producer filled gets the other's arrival from here,
+    // so that its barrier, too, tells when the copy is there
+    const int all = ((a.tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x) * steps;
+    const int w = issued_s[0] < 0 ? all : issued_s[0], x = issued_s[1] < 0 ? all : issued_s[1];
+    for (int i = min(w, x); i < max(w, x); ++i) mbar_arrive(full_bar(i % a.stages));
+    drain_ring(full_bar(0), a.stages, max(w, x), a.err);
+  }
   if (warp == 2) tmem_dealloc(tmem_base, a.tmem_cols);
 }
 

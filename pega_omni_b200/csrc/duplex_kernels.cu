@@ -396,7 +396,10 @@ __global__ void __launch_bounds__(kAttendWarps * 32)
   int slot = 0;
   for (int pi = warp; pi < npages; pi += kAttendWarps, slot ^= 1) {
     if (pi + kAttendWarps < npages && lane == 0) fetch(pi + kAttendWarps, slot ^ 1);  // (that slot was read a round ago)
-    if (!sm100::mbar_wait(sm100::smem_addr(&sh.bar[warp][slot]), parity[slot], err)) break;
+    if (!sm100::mbar_wait(sm100::smem_addr(&sh.bar[warp][slot]), parity[slot], err)) {
+      if (pi + kAttendWarps < npages) sm100::mbar_wait(sm100::smem_addr(&sh.bar[warp][slot ^ 1]), parity[slot ^ 1], err);  // nothing may land later
+      break;
+    }
     parity[slot] ^= 1u;
     const unsigned char* blk = mine + (size_t)slot * kAttendSlotBytes;
     const int ntok = min(16, len - pi * 16);
@@ -513,7 +516,10 @@ __global__ void __launch_bounds__(W * 32)
   uint32_t parity[2] = {0, 0};
   int slot = 0;
   for (int vi = warp; vi < npages; vi += W, slot ^= 1) {
-    if (!sm100::mbar_wait(sm100::smem_addr(&bars[warp][slot]), parity[slot], err)) break;
+    if (!sm100::mbar_wait(sm100::smem_addr(&bars[warp][slot]), parity[slot], err)) {
+      if (vi + W < npages) sm100::mbar_wait(sm100::smem_addr(&bars[warp][slot ^ 1]), parity[slot ^ 1], err);  // nothing may land later
+      break;
+    }
     parity[slot] ^= 1u;
     const unsigned char* blk = mine + (size_t)slot * kAttendSlotBytes;
     const int ntok = min(16, len - page_of(vi) * 16);

@@ -229,7 +229,10 @@ __global__ void __launch_bounds__(128, 1)
       int stage = 0;
       uint32_t phase = 0;
       for (int kb = kb_begin; kb < kb_end; kb += kbs) {
-        if (!mbar_wait(empty_bar(stage), phase ^ 1u, err)) break;
+        if (!mbar_wait(empty_bar(stage), phase ^ 1u, err)) {
+          drain_ring(full_bar(0), n_stages, (kb - kb_begin) / kbs, err);
+          break;
+        }
         const uint32_t a_dst = base + stage * stage_bytes, b_dst = a_dst + x_base;
         mbar_expect_tx(full_bar(stage), stage_bytes);
         if (kbs == 1) {
@@ -437,7 +440,10 @@ __global__ void __launch_bounds__(128, 1)
       int stage = 0;
       uint32_t phase = 0;
       for (int kb = 0; kb < nkb; kb += kbs) {
-        if (!mbar_wait(empty_bar(stage), phase ^ 1u, err)) break;
+        if (!mbar_wait(empty_bar(stage), phase ^ 1u, err)) {
+          drain_ring(full_bar(0), n_stages, kb / kbs, err);
+          break;
+        }
         const uint32_t a_dst = base + stage * stage_bytes, b_dst = a_dst + x_bytes;
         mbar_expect_tx(full_bar(stage), stage_bytes);
         tma_load_3d(a_dst, &xmap, full_bar(stage), 0, 0, kb, kEvictLast);

@@ -70,6 +70,13 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint32_
   }
 }
 
+// After an abort: waits, each time with the same limit, for the copies that a ring still has under way, so that none lands in
+// shared memory once the CTA has left. `issued` stages were filled, stage i in slot i % slots with its barrier at
+// full + 8 * slot.
+__device__ __forceinline__ void drain_ring(uint32_t full, int slots, int issued, uint32_t* err) {
+  for (int i = max(0, issued - slots); i < issued; ++i) mbar_wait(full + 8u * (uint32_t)(i % slots), (uint32_t)(i / slots) & 1u, err);
+}
+
 // ---- TMA -----------------------------------------------------------------------
 
 constexpr uint64_t kEvictNormal = 0x1000000000000000ull;

@@ -93,11 +93,6 @@ __global__ void __launch_bounds__(kThreads, 1)
     mbar_expect_tx(full_w(slot), w_bytes);
     tma_load_3d(base + (uint32_t)slot * slot_bytes + x_bytes, &wmap, full_w(slot), 0, tile * a.tn, (st0 + i) * a.kbs, kEvictFirst);
   };
-  // after an abort: no copy may land in shared memory once the CTA has left
-  auto drain = [&](uint32_t first_bar, int issued) {
-    for (int i = max(0, issued - a.slots); i < issued; ++i)
-      mbar_wait(first_bar + 8u * (i % a.slots), (uint32_t)(i / a.slots) & 1u, a.err);
-  };
 
   if (threadIdx.x == 0) {
     prefetch_tensormap(&wmap);
@@ -122,7 +117,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       uint32_t phase = 0;
       for (int i = a.slots; i < n_st; ++i) {
         if (!mbar_wait(empty(slot), phase, a.err)) {
-          drain(full_w(0), i);
+          drain_ring(full_w(0), a.slots, i, a.err);
           break;
         }
         load_w(i, slot);
@@ -137,7 +132,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       uint32_t phase = 0;
       for (int i = 0; i < n_st; ++i) {
         if (i >= a.slots && !mbar_wait(empty(slot), phase ^ 1u, a.err)) {
-          drain(full_x(0), i);
+          drain_ring(full_x(0), a.slots, i, a.err);
           break;
         }
         mbar_expect_tx(full_x(slot), x_bytes);

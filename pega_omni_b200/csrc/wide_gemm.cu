@@ -44,6 +44,13 @@ __device__ __forceinline__ uint32_t map_shared(uint32_t addr, uint32_t rank) {
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
   return r;
 }
+__device__ __forceinline__ void store_remote(uint32_t cluster_addr, uint32_t v) {
+  asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(cluster_addr), "r"(v) : "memory");
+}
+// `bytes` that will not arrive count as arrived on a barrier of this CTA.
+__device__ __forceinline__ void forgo_tx(uint32_t bar, uint32_t bytes) {
+  asm volatile("mbarrier.complete_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
 __device__ __forceinline__ void arrive_remote(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
@@ -99,6 +106,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kWideThreads, 1)
   extern __shared__ unsigned char wide_smem_raw[];
   __shared__ __align__(8) uint64_t bars_s[2 * kWideMaxSlots + 4];
   __shared__ uint32_t tmem_slot_s;
+  __shared__ int gave_up_s, issued_s[2];  // a wait of the pair ran out; stages its producers had filled by then (-1: all; the leader's)
   const uint32_t base = (smem_addr(wide_smem_raw) + 1023u) & ~1023u, bars = smem_addr(bars_s);
   auto full = [&](int s) { return bars + 8u * s; };  // the leader's counts the bytes of both CTAs
   auto empty = [&](int s) { return bars + 8u * (kWideMaxSlots + s); };
@@ -113,7 +121,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kWideThreads, 1)
     const int band = tile / (kBand * a.n_tiles), in = tile % (kBand * a.n_tiles), height = min(kBand, a.m_tiles - band * kBand);
     m = band * kBand + in % height, n = in / height;
   };
+  auto give_up = [&]() {  // known to both CTAs
+    store_remote(map_shared(smem_addr(&gave_up_s), 0), 1u);
+    store_remote(map_shared(smem_addr(&gave_up_s), 1), 1u);
+  };
   if (threadIdx.x == 0) {
+    gave_up_s = 0, issued_s[0] = issued_s[1] = -1;
     prefetch_tensormap(&xmap);
     prefetch_tensormap(&wmap);
     for (int s = 0; s < a.slots; ++s) mbar_init(full(s), 1), mbar_init(empty(s), 1);
@@ -135,7 +148,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kWideThreads, 1)
   if (warp == 0) {
     if (lane == 0) {
       fence_async_global();  // rows written by ordinary stores, read by TMA
-      int slot = 0;
+      int slot = 0, done = 0;
       uint32_t phase = 1;
       bool alive = true;
       for (int tile = first; tile < tiles && alive; tile += stride) {
@@ -149,12 +162,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kWideThreads, 1)
           const uint32_t dst = base + (uint32_t)slot * slot_bytes, bar = map_shared(full(slot), 0);
           pair_load_3d(dst, &xmap, bar, 0, x_row, kb, kEvictNormal);
           pair_load_3d(dst + x_bytes, &wmap, bar, 0, w_row, kb, kEvictNormal);
+          ++done;
           if (++slot == a.slots) slot = 0, phase ^= 1u;
         }
       }
-      if (!alive) {  // copies under way count on the leader's barriers, which the peer cannot wait on: give them time to land
-        const uint64_t start = global_timer_ns();
-        while (global_timer_ns() - start < 2000000ull) {}
+      if (!alive) {
+        store_remote(map_shared(smem_addr(&issued_s[rank]), 0), (uint32_t)done);
+        give_up();
       }
     }
   } else if (warp == 1) {
@@ -193,6 +207,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kWideThreads, 1)
         __syncwarp();
         if (++acc == 2) acc = 0, acc_phase ^= 1u;
       }
+      if (!alive && lane == 0) give_up();
     }
   } else {
     const int quad = warp & 3;
@@ -264,6 +279,19 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kWideThreads, 1)
   tc_fence_before_sync();
   __syncthreads();
   cluster_sync();  // no CTA leaves while the other may still arrive on its barriers or read its operands
+  if (*reinterpret_cast<volatile int*>(&gave_up_s)) {
+    // ... nor while copies are under way, which count on the leader's barriers: a stage that only one CTA filled is
+    // completed from here for the other, so that its barrier, too, tells when the copy is there
+    if (rank == 0 && threadIdx.x == 0) {
+      const int per = (a.nkb + kPer - 1) / kPer, all = (tiles - first + stride - 1) / stride * per;
+      const int mine = issued_s[0] < 0 ? all : issued_s[0], peer = issued_s[1] < 0 ? all : issued_s[1];
+      for (int i = peer; i < mine; ++i) forgo_tx(full(i % a.slots), slot_bytes);
+      for (int i = mine; i < peer; ++i) mbar_expect_tx(full(i % a.slots), slot_bytes);
+      drain_ring(full(0), a.slots, max(mine, peer), a.err);
+    }
+    __syncthreads();
+    cluster_sync();
+  }
   if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * kAccCols) : "memory");
 }
 
