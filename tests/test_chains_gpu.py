@@ -395,3 +395,24 @@ def test_norms_of_rows_that_end_inside_a_warp(ops, dim):
         ops.sync()
         close(out, norm(x.float()), steps=1.0)
         close(out2, norm((x.float() + y.float()).bfloat16().float()), steps=1.0)
+
+
+@pytest.mark.parametrize("vocab", [2047, 2048, 2049, 32768, 40001])
+@pytest.mark.parametrize("top_k", [1, 5, 250])
+def test_duplex_sampler_keeps_the_top_k(ops, vocab, top_k):
+    """Nearly flat logits, where the noise decides: every draw is one of the top k (ties with the k-th included) and the one
+    the host's restatement of the hash and the score takes (`__logf` against `logf` may move a near-tie)."""
+    from oracle import duplex as O
+    rows, col = 64, 2
+    logits = (torch.rand((rows, vocab), generator=torch.Generator().manual_seed(vocab + top_k)) * 0.5 - 0.25).to(torch.bfloat16).cuda()
+    force = torch.full((rows, 9), -1, dtype=torch.int32, device="cuda")
+    drawn = torch.full((rows, 9), -7, dtype=torch.int32, device="cuda")
+    seeds = [[r * 7919 + 1, r % 3] for r in range(rows)]
+    torch.cuda.synchronize()
+    ops.lm_sample(logits, 0.8, top_k, force, i32(seeds), col, drawn)
+    ops.sync()
+    got, host = drawn[:, col].cpu().numpy(), logits.float().cpu().numpy()
+    kth = np.sort(host, axis=1)[:, -top_k]
+    assert (host[np.arange(rows), got] >= kth).all()
+    want = np.array([O.sample(host[r], 0.8, top_k, seeds[r][0], seeds[r][1], col) for r in range(rows)])
+    assert (got == want).sum() >= rows - 1, (got, want)
