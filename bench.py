@@ -843,7 +843,8 @@ def main():
                 # grows with the KV length as they do
                 "traffic": int(tick_bytes * 6230.8 / 6129.2) if launches_per_tick <= 2 else None,
                 "traffic_note": "ncu dram__bytes_read+write of one captured tick (6.231 GB for 6.129 GB algorithmic), "
-                                "scaled by this run's algorithmic bytes"}
+                                "scaled by this run's algorithmic bytes" if launches_per_tick <= 2 else
+                                "not captured: the tick is a graph of several hundred kernels"}
         line = {
             "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": K, "warmup": W,
             "ms_per_step": 1e3 * elapsed_max / K, "higher_is_better": True, "scaling": "weak", "vs_baseline": None,

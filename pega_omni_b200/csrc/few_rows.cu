@@ -9,9 +9,10 @@
 // rows' arrival and the shared memory they take from the rings: at 16 rows a talker step took 3,526 us against 3,361 with the
 // tcgen05 kernel, a Higgs step 2,375 against 2,326, a duplex tick 4,604 against 4,548.
 // The add + norm before a projection is made by every CTA from the summands (L2 broadcast reads, 16 KB to 100 KB) while
-// one or two pieces a lane suffice (few_norm_fits); a kernel of its own takes 2.7 us and beyond that is faster. Measured as nodes of a chain
-// at one row: 1,024 x 3,072 2.5 us, 6,144 x 1,024 with norm and SwiGLU 4.7 us, 4,096 x 1,024 with norm 4.3 us (4.5 to
-// 5.3 us and 2.7 us for the norm with the tcgen05 kernel of stream_gemm.cu).
+// one or two pieces a lane suffice (few_norm_fits); a kernel of its own takes 2.7 us and beyond that is faster. Measured as nodes of a
+// traced chain (omni_talker_trace, whose stamp adds half a microsecond) at one row: 1,024 x 3,072 2.8 us, 6,144 x 1,024 with
+// norm and SwiGLU 4.1 us, 4,096 x 1,024 with norm 3.6 us (4.5 to 5.3 us and 2.7 us for the norm with the tcgen05 kernel of
+// stream_gemm.cu).
 #include "few_rows.h"
 
 #include <algorithm>

@@ -7,10 +7,11 @@
 // as the sum of three bf16, which is all of it, and sums are kept out of long chains of matrix instructions (decode_attend.cuh):
 // 0.01 to 0.02 % of the outputs of prompts of 77 to 512 rows are not the bf16 nearest to float64's (scalar kernel 0.01 to
 // 0.02 %, two bf16 a probability 0.17 to 0.22 %).
-// Measured at 8,700 rows of 28 ragged prompts, D = 128, G = 2: 146 us a layer, before page numbers were read a tile ahead
-// (scalar multiply-adds, each row reading its keys for itself: 1,184 us). Three CTAs an SM with fewer registers are no
-// faster. Bound by shared-memory reads (each warp reads the 16 KB of a stage for its sixteen rows: 512 cycles per 64 x 32
-// tile at G = 2 against 400 of the MMAs).
+// Measured alone with cold caches at 7,604 rows of 28 ragged prompts, D = 128, G = 2: 144 us a layer (109 us with two bf16 a
+// probability; scalar multiply-adds, each row reading its keys for itself: 1,184 us at 8,700 rows). Three CTAs an SM with
+// fewer registers are no faster. Bound by the matrix instructions' issue and shared-memory reads alike: 128 instructions a
+// warp and 64 x 32 tile at G = 2, and every warp reads the 16 KB of a stage for its sixteen rows (about 512 cycles each).
+// -Xptxas -v: 48 bytes of spill stores at <128, 2>, 12 at <128, 5>, 172 at <128, 8>.
 #pragma once
 #include "attend.cuh"
 #include "pdl.cuh"

@@ -139,8 +139,10 @@ struct Team {
   }
 
   // The same for keys of sixteen bits (rows of bf16 logits that no penalty has touched): the upper byte is found by counting
-  // four candidates a round from the largest key's byte down - the bytes of logits a few units wide are two or three - and
-  // the lower byte by one pass over counters, zeroed by the caller before its last barrier.
+  // four candidates a round from the largest key's byte down, and the lower byte by one pass over counters, zeroed by the
+  // caller before its last barrier. Where the k-th logit has the sign of the largest, their upper bytes are two or three apart
+  // and one round finds it; where fewer than k logits are positive the walk passes zero and takes up to 33 rounds of one
+  // barrier.
   static __device__ uint32_t kth_largest_key16(const uint32_t* key, uint32_t valid, uint32_t k, uint32_t top, int tid, Shared& sh) {
     const int lane = tid & 31;
     uint32_t left = k, digit = top >> 8;
@@ -179,7 +181,7 @@ struct Team {
   // The k-th largest key of the row (ties share it), most significant digit first, eight bits at a time. Logits are
   // a few units wide, so the keys' leading digits take a handful of values: counted one atomic per key, that pass would
   // serialise thousands of additions on two or three shared-memory words, so the first digit is found by counting
-  // (below). The other passes count through shared-memory atomics; every pass has its own 256 counters (zeroed once,
+  // (below; about 131 rounds where the walk passes zero). The other passes count through shared-memory atomics; every pass has its own 256 counters (zeroed once,
   // up front), and after the pass's one team barrier EVERY warp picks the digit by itself from the counters (lane l
   // sums counters 8l .. 8l + 7, a shuffle scan gives the keys above each lane's range).
   static __device__ uint32_t kth_largest_key(const uint32_t* key, int vocab, uint32_t k, uint32_t top_digit, int tid,

@@ -4,7 +4,7 @@
 // rows to shared memory by TMA, the MMAs' issue, commit, TMEM to registers, stores. Hence the rows on M (64 or 128 TMEM
 // lanes, a tile of weights as narrow as fills the chip once on N), weights asked for before the rows exist, four issuing
 // threads and split K without a reduction of its own. Measured as nodes of a chain at 64 rows: 12,288 x 2,048 with SwiGLU
-// 13.6 us (its weights alone take 7.7 us from DRAM), 12,288 x 4,096 23.8 us (15.4), 22,528 x 4,096 with SwiGLU 39.9 us
+// 13.3 us (its weights alone take 7.7 us from DRAM), 12,288 x 4,096 23.8 us (15.4), 22,528 x 4,096 with SwiGLU 39.9 us
 // (28.3), 4,096 x 1,024 4.7 us; a phase of the persistent tick kernel took 7 us at least.
 #include "stream_gemm.h"
 

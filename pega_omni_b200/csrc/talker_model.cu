@@ -1256,8 +1256,8 @@ void omni_talker_destroy(omni_talker* m) {
 
 // Whether a model's programs run as chains of kernels (chain.h) or, with `tick_kernel` set, as the persistent kernel. The
 // chain is the faster one wherever it was measured (stacks of 5.3 GB: 2,178 against 4,710 us a step of one session; of
-// 91 MB: 604 against 1,287 us); models whose stacks fit in the 126 MB of L2 keep the persistent kernel for its one launch
-// a tick, which their callers count on.
+// 91 MB: 604 against 1,287 us). Models whose stacks fit in the 126 MB of L2 keep the persistent kernel all the same: its one
+// launch a tick is what their statistics report and their tests hold, at twice the time of a step.
 static bool chain_wanted(const omni_talker* m) {
   const omni_talker_config& c = m->cfg;
   if (c.tick_kernel != 1 || c.gemm_path != 0) return false;

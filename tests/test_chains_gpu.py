@@ -39,7 +39,7 @@ def i32(v):
     return torch.tensor(v, dtype=torch.int32, device="cuda")
 
 
-# rows: one and two 8-row tiles of the warp-level kernel, then tcgen05 with M = 64, 128, two row tiles, SM pairs
+# rows: the warp-level kernel up to eight, then tcgen05 with M = 64, 128, two row tiles, SM pairs
 @pytest.mark.parametrize("rows", [1, 7, 8, 9, 16, 17, 64, 65, 128, 129, 256, 257, 300])
 @pytest.mark.parametrize("n,k,epilogue", [(200, 128, 0), (1000, 1088, 1), (4096, 64, 2), (24, 6144, 0)])
 def test_chain_gemm(ops, rows, n, k, epilogue):
