@@ -42,6 +42,24 @@ static cudaError_t order(cudaStream_t s) {
   return cudaGetLastError();
 }
 
+// go(qkv, out) on 16-byte aligned rows, which the attention kernels' vector accesses need: the caller's own where they are,
+// otherwise copies (out is written back; so are the rows of qkv, which may be rotated in place).
+template <typename Go>
+static cudaError_t on_aligned_rows(void* qkv, size_t qkv_bytes, void* out, size_t out_bytes, cudaStream_t s, Go&& go) {
+  if (((reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(out)) & 15) == 0) return go(qkv, out);
+  const size_t at = (qkv_bytes + 255) & ~(size_t)255;
+  char* tmp = nullptr;
+  cudaError_t e = cudaMalloc((void**)&tmp, at + out_bytes);
+  if (e != cudaSuccess) return e;
+  e = cudaMemcpyAsync(tmp, qkv, qkv_bytes, cudaMemcpyDeviceToDevice, s);
+  if (e == cudaSuccess) e = go(tmp, tmp + at);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(qkv, tmp, qkv_bytes, cudaMemcpyDeviceToDevice, s);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(out, tmp + at, out_bytes, cudaMemcpyDeviceToDevice, s);
+  const cudaError_t done = cudaStreamSynchronize(s);
+  cudaFree(tmp);
+  return e != cudaSuccess ? e : done;
+}
+
 #define OPS_CUDA(ctx, expr)                                                                       \
   do {                                                                                            \
     cudaError_t e_ = (expr);                                                                      \
@@ -178,9 +196,12 @@ int32_t omni_op_rope_attend(omni_ops* c, void* qkv, const void* q_norm, const vo
   map.indptr = indptr;
   map.pages = pages;
   const AttnShape a{q_heads, kv_heads, head_dim, eps, theta};
-  OPS_CUDA(c, launch_rope_kv((bf16*)qkv, (const bf16*)q_norm, (const bf16*)k_norm, (bf16*)kv, map, rows, a, kv_pages,
-                             c->err, c->stream));
-  OPS_CUDA(c, launch_attend((const bf16*)qkv, (const bf16*)kv, (bf16*)out, map, rows, a, c->err, c->stream));
+  const size_t head = (size_t)rows * head_dim * sizeof(bf16);
+  OPS_CUDA(c, on_aligned_rows(qkv, head * (q_heads + 2 * kv_heads), out, head * q_heads, c->stream, [&](void* x, void* y) {
+    const cudaError_t e = launch_rope_kv((bf16*)x, (const bf16*)q_norm, (const bf16*)k_norm, (bf16*)kv, map, rows, a, kv_pages,
+                                         c->err, c->stream);
+    return e != cudaSuccess ? e : launch_attend((const bf16*)x, (const bf16*)kv, (bf16*)y, map, rows, a, c->err, c->stream);
+  }));
   return OMNI_OK;
 }
 
@@ -193,8 +214,11 @@ int32_t omni_op_decode_attend(omni_ops* c, const void* qkv, const void* q_norm, 
   map.pos = pos, map.slot = slot, map.indptr = indptr, map.pages = pages;
   const AttnShape a{q_heads, kv_heads, head_dim, eps, theta};
   OPS_CUDA(c, order(c->stream));
-  OPS_CUDA(c, launch_rope_attend((const bf16*)qkv, {}, (const bf16*)q_norm, (const bf16*)k_norm, (bf16*)kv, (bf16*)out, map, rows,
-                                 a, kv_pages, c->sm_count, c->err, c->stream));
+  const size_t head = (size_t)rows * head_dim * sizeof(bf16);
+  OPS_CUDA(c, on_aligned_rows(const_cast<void*>(qkv), head * (q_heads + 2 * kv_heads), out, head * q_heads, c->stream, [&](void* x, void* y) {
+    return launch_rope_attend((const bf16*)x, {}, (const bf16*)q_norm, (const bf16*)k_norm, (bf16*)kv, (bf16*)y, map, rows, a,
+                              kv_pages, c->sm_count, c->err, c->stream);
+  }));
   return OMNI_OK;
 }
 

@@ -196,7 +196,7 @@ __global__ void __launch_bounds__(THREADS)
   const float uniform = uniforms[s * kGroups + prm.group];
   grid_wait();
   float mine[Team::PER];
-  if (prm.vocab % Team::PER == 0) {
+  if (prm.vocab % Team::PER == 0 && (reinterpret_cast<uintptr_t>(logits) & 7) == 0) {
     if (tid * Team::PER < prm.vocab) {
 #pragma unroll
       for (int j = 0; j < Team::PER; j += 4) {

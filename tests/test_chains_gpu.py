@@ -416,3 +416,57 @@ def test_duplex_sampler_keeps_the_top_k(ops, vocab, top_k):
     assert (host[np.arange(rows), got] >= kth).all()
     want = np.array([O.sample(host[r], 0.8, top_k, seeds[r][0], seeds[r][1], col) for r in range(rows)])
     assert (got == want).sum() >= rows - 1, (got, want)
+
+
+@pytest.mark.parametrize("vocab", [16, 1000, 2048, 3072, 4093])
+@pytest.mark.parametrize("top_k,top_p", [(50, 1.0), (0, 1.0), (40, 0.8), (1, 1.0)])
+def test_rows_without_a_penalty_draw_what_the_general_path_draws(ops, vocab, top_k, top_p):
+    """Unpenalised rows take sixteen-bit keys; a penalty of 1 over an empty bitmap takes the general path on the same logits,
+    infinities, NaN, ties and one-signed rows among them. Also from an address that vector loads cannot take."""
+    if top_p < 1 and top_k <= 0:
+        pytest.skip("refused")
+    rows, group = 64, 3
+    x = rand((rows, vocab), vocab + top_k, 2.0)
+    x[1], x[2], x[3] = -x[1].abs() - 1, 0.0, -float("inf")
+    x[4, 3], x[5, 3], x[6, 3] = float("nan"), float("inf"), -float("inf")
+    x[7] = torch.where(torch.arange(vocab, device="cuda") % 2 == 0, x[7].abs(), -x[7].abs())
+    x[8], x[9, :] = (x[8] * 4).round() / 4, torch.tensor(-0.0, device="cuda")
+    x[10, ::5], x[11, : vocab // 2] = float("nan"), -float("inf")
+    x[12] = x[12] * 1e30
+    x[13] = -x[13].abs() - 1
+    x[13, :3] = x[13, :3].abs()
+    odd = torch.empty(rows * vocab + 1, dtype=torch.bfloat16, device="cuda")[1:].view(rows, vocab).copy_(x)
+    stride = 4 * (16 + (vocab + 31) // 32 + 1) + 8
+    stride = (stride + 255) // 256 * 256
+    frames, uniforms = i32([2] * rows), torch.rand((rows, 16), generator=torch.Generator().manual_seed(vocab)).cuda()
+    force, lines = torch.full((rows, 16), -1, dtype=torch.int32, device="cuda"), i32(list(range(rows)))
+    got = []
+    for logits, penalize in ((x, 1), (x, 0), (odd, 0)):
+        state = torch.zeros((rows, stride // 4), dtype=torch.int32, device="cuda")
+        codes = torch.full((rows, 16), -9, dtype=torch.int32, device="cuda")
+        torch.cuda.synchronize()
+        ops.sample(logits, 0.9, top_k, top_p, 1.0, 0, 0, -1, 0, frames, uniforms, force, state, lines, stride, penalize, 0, codes, group)
+        ops.sync()
+        got.append(codes[:, group].tolist())
+    assert got[0] == got[1] == got[2]
+
+
+@pytest.mark.parametrize("prompt", [False, True])
+def test_attention_from_addresses_that_vector_loads_cannot_take(ops, prompt):
+    hq, hk, d, n = 4, 2, 128, 20
+    pos, slot = i32(list(range(n))), i32(list(range(n)))
+    seq, indptr, pages = (i32([0] * n), i32([0, 2]), i32([0, 1])) if prompt else (None, i32([2 * s for s in range(n + 1)]), i32([0, 1] * n))
+    x, qn, kn = rand((n, (hq + 2 * hk) * d), 91), rand((d,), 92, 0.2) + 1, rand((d,), 93, 0.2) + 1
+
+    def at(offset, like):
+        return torch.empty(like.numel() + 8, dtype=torch.bfloat16, device="cuda")[offset:offset + like.numel()].view(like.shape).copy_(like)
+    got = []
+    for offset in (0, 1):
+        qkv, out = at(offset, x), at(offset, torch.zeros((n, hq * d), dtype=torch.bfloat16, device="cuda"))
+        kv = torch.zeros((2, hk, 2, 16, d), dtype=torch.bfloat16, device="cuda")
+        torch.cuda.synchronize()
+        ops.rope_attend(qkv, qn, kn, kv, 2, pos, slot, seq, indptr, pages, hq, hk, d, 1e-6, 1e6, out)
+        ops.sync()
+        got.append((qkv, out, kv))
+    for a, b in zip(*got):
+        assert torch.equal(a, b)
