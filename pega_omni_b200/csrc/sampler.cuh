@@ -254,19 +254,7 @@ struct Team {
       if ((tid & 31) == 0) sh.warp_max[tid >> 5] = top;
       Sync::sync();
       top = __reduce_max_sync(0xffffffffu, (tid & 31) < THREADS / 32 ? sh.warp_max[tid & 31] : 0u);
-      uint32_t largest = top;
-      if (top > 0xff80u) {  // a NaN is the largest key but, as to fmaxf, not the maximum
-        largest = 0;
-#pragma unroll
-        for (int j = 0; j < PER; ++j)
-          if ((valid >> j & 1u) && key[j] <= 0xff80u) largest = max(largest, key[j]);
-        largest = __reduce_max_sync(0xffffffffu, largest);
-        Sync::sync();
-        if ((tid & 31) == 0) sh.warp_max[tid >> 5] = largest;
-        Sync::sync();
-        largest = __reduce_max_sync(0xffffffffu, (tid & 31) < THREADS / 32 ? sh.warp_max[tid & 31] : 0u);
-      }
-      const float m = __uint_as_float((largest & 0x8000u ? largest & 0x7fffu : ~largest & 0xffffu) << 16) / temperature;
+      const float m = __uint_as_float((top & 0x8000u ? top & 0x7fffu : ~top & 0xffffu) << 16) / temperature;
       const uint32_t threshold = keep < vocab ? kth_largest_key16(key, valid, (uint32_t)keep, top, tid, sh) : 0u;
 #pragma unroll
       for (int j = 0; j < PER; ++j) {

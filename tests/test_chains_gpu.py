@@ -435,6 +435,8 @@ def test_rows_without_a_penalty_draw_what_the_general_path_draws(ops, vocab, top
     x[12] = x[12] * 1e30
     x[13] = -x[13].abs() - 1
     x[13, :3] = x[13, :3].abs()
+    bits = x.view(torch.int16)
+    bits[14, 3], bits[15, 3], bits[16, ::5] = 0x7fc0, 0x7fc0 - 0x8000, 0x7fff  # NaN of either sign
     odd = torch.empty(rows * vocab + 1, dtype=torch.bfloat16, device="cuda")[1:].view(rows, vocab).copy_(x)
     stride = 4 * (16 + (vocab + 31) // 32 + 1) + 8
     stride = (stride + 255) // 256 * 256
