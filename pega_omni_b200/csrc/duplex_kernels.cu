@@ -814,6 +814,11 @@ __global__ void lm_copy_kv_kernel(void* kv, const int32_t* __restrict__ src_slot
         reinterpret_cast<const float*>(from + 2 * 16 * kHeliumHeadDim + 64 * lane)[st];
 }
 
+// Rows are read eight bytes at a time, pages by bulk copies.
+bool ring_aligned(const void* qkv, const void* kv) {
+  return (reinterpret_cast<uintptr_t>(qkv) & 7) == 0 && (reinterpret_cast<uintptr_t>(kv) & 15) == 0;
+}
+
 bool row_dim_ok(int dim) { return dim % 8 == 0 && dim / 8 <= 1024 && dim / 8 >= 32; }
 
 }  // namespace
@@ -859,6 +864,7 @@ cudaError_t launch_lm_tp_add_norm(const bf16* mine, const bf16* peer, bf16* x, c
 
 cudaError_t launch_lm_rope_kv(bf16* qkv, const int32_t* pos, const int32_t* slots, void* kv, int rows, int heads,
                               float coef, int kv_pages, uint32_t* err, cudaStream_t s) {
+  if (!ring_aligned(qkv, kv)) return cudaErrorInvalidValue;
   return launch_pdl(lm_rope_kv_kernel, dim3(rows, kRopeParts), dim3(kRopeWarps * 32), 0, s, qkv, pos, slots, kv, heads, coef, kv_pages, err);
 }
 
@@ -899,6 +905,7 @@ static cudaError_t launch_lm_rope_attend_w(const bf16* qkv, void* kv, const int3
 cudaError_t launch_lm_rope_attend(const bf16* qkv, void* kv, const int32_t* pos, const int32_t* slots,
                                   const int32_t* indptr, const int32_t* pages, bf16* out, int rows, int heads, float coef,
                                   float scale, int context, int kv_pages, int sm_count, uint32_t* err, cudaStream_t s) {
+  if (!ring_aligned(qkv, kv)) return cudaErrorInvalidValue;
   if (rows * heads <= sm_count)  // one CTA per SM at most: more warps of it
     return launch_lm_rope_attend_w<16>(qkv, kv, pos, slots, indptr, pages, out, rows, heads, coef, scale, context, kv_pages, err, s);
   return launch_lm_rope_attend_w<4>(qkv, kv, pos, slots, indptr, pages, out, rows, heads, coef, scale, context, kv_pages, err, s);

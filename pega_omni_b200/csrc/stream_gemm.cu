@@ -266,6 +266,7 @@ int stream_plan(StreamGemmPlan* plan, const bf16* w, int N, int K, const bf16* x
   if (out == kStreamPartials && N % 8) return -2;
   if (out == kStreamSwiglu && (N % (2 * kGateGroup) || ldy % 8)) return -2;
   if ((reinterpret_cast<uintptr_t>(w) & 15) || (reinterpret_cast<uintptr_t>(x) & 15)) return -3;
+  if (out == kStreamSwiglu && (reinterpret_cast<uintptr_t>(y) & 15)) return -3;
   StreamGemmPlan& p = *plan;
   p.N = N, p.K = K, p.rows = rows, p.out = out, p.y = y, p.ldy = ldy, p.part = part, p.epi = epi;
   p.M = rows <= 64 ? 64 : 128;

@@ -316,6 +316,7 @@ int wide_plan(WidePlan* plan, const bf16* w, int N, int K, const bf16* x, int ro
               int sm_count, int granule) {
   if (rows < 1 || N < 1 || K < kWideKb || K % kWideKb || out == kStreamPartials) return -2;
   if ((reinterpret_cast<uintptr_t>(w) & 15) || (reinterpret_cast<uintptr_t>(x) & 15)) return -3;
+  if (out == kStreamSwiglu && (reinterpret_cast<uintptr_t>(y) & 15)) return -3;
   WidePlan& p = *plan;
   p.N = N, p.K = K, p.rows = rows, p.out = out, p.y = y, p.ldy = ldy, p.epi = epi, p.granule = granule;
   const int pairs = std::max(1, sm_count / 2), m_tiles = (rows + kWideRows - 1) / kWideRows;

@@ -472,3 +472,19 @@ def test_attention_from_addresses_that_vector_loads_cannot_take(ops, prompt):
         got.append((qkv, out, kv))
     for a, b in zip(*got):
         assert torch.equal(a, b)
+
+
+def test_operands_that_vector_accesses_cannot_take_are_refused(ops):
+    from pega_omni_b200.ops import OpsError
+    w, x = rand((128, 64), 1), rand((300, 64), 2)
+    y = torch.zeros(300 * 64 + 1, dtype=torch.bfloat16, device="cuda")[1:].view(300, 64)
+    for rows in (40, 300):
+        with pytest.raises(OpsError):
+            ops.chain_gemm(w, x[:rows], y[:rows], swiglu=True)
+    qkv = torch.zeros(3 * 2 * 128 + 1, dtype=torch.bfloat16, device="cuda")[1:].view(1, -1)
+    kv = torch.zeros(1, 2, 2 * 16 * 128 + 2 * 16 * 4, dtype=torch.uint8, device="cuda")
+    out = torch.zeros((1, 256), dtype=torch.bfloat16, device="cuda")
+    for call in (ops.lm_decode_attend, lambda q, k, n, p, s, *rest: ops.lm_rope_attend(q, k, n, p, s, None, *rest)):
+        with pytest.raises(OpsError):
+            call(qkv, kv, 1, i32([0]), i32([0]), i32([0, 1]), i32([0]), 2, -0.14, 0.1, 16, out)
+    ops.sync()
