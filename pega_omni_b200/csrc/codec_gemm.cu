@@ -50,14 +50,6 @@ struct ConvArgs {
   uint32_t acc_cols, tmem_cols;  // TMEM columns per accumulator (a power of two >= tn) and in all
 };
 
-__device__ __forceinline__ bool elect_one() {
-  uint32_t p;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}\n"
-      : "=r"(p));
-  return p != 0;
-}
-
 // The walk over a launch's tiles without a division per tile: tile = n + n_tiles * (t + t_tiles * s).
 struct TileWalk {
   int n, t, s, dn, dt, ds;

@@ -12,17 +12,11 @@
 // The K dimension of an MMA may be permuted as long as both operands agree: a lane takes 16 consecutive bytes of a key
 // (or query) row, which serve as its share of two consecutive steps, so every load is one 16-byte access.
 #pragma once
+#include "sm100.cuh"
 #include "util.cuh"
 
 namespace omni {
 namespace dattn {
-
-__device__ __forceinline__ void mma16816(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
-                                         uint32_t b1) {
-  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
 
 __device__ __forceinline__ uint32_t word(const uint4& u, int i) { return i == 0 ? u.x : i == 1 ? u.y : i == 2 ? u.z : u.w; }
 
@@ -87,8 +81,8 @@ struct State {
     float s[4] = {0.f, 0.f, 0.f, 0.f}, s2[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
     for (int j = 0; j < D / 32; ++j) {
-      mma16816(s, pg.k[0][j].x, pg.k[1][j].x, pg.k[0][j].y, pg.k[1][j].y, q[j].x, q[j].y);
-      mma16816(s2, pg.k[0][j].z, pg.k[1][j].z, pg.k[0][j].w, pg.k[1][j].w, q[j].z, q[j].w);
+      sm100::mma_16816(s, pg.k[0][j].x, pg.k[1][j].x, pg.k[0][j].y, pg.k[1][j].y, q[j].x, q[j].y);
+      sm100::mma_16816(s2, pg.k[0][j].z, pg.k[1][j].z, pg.k[0][j].w, pg.k[1][j].w, q[j].z, q[j].w);
     }
     if (next) pg.load_k(next, lane);
 #pragma unroll
@@ -137,7 +131,7 @@ struct State {
         const uint32_t a2 = __byte_perm(v2, v3, 0x5410), a3 = __byte_perm(v2, v3, 0x7632);
         float sum[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-        for (int x = 2; x >= 0; --x) mma16816(sum, a0, a1, a2, a3, b0[x], b1[x]);
+        for (int x = 2; x >= 0; --x) sm100::mma_16816(sum, a0, a1, a2, a3, b0[x], b1[x]);
 #pragma unroll
         for (int k = 0; k < 4; ++k) acc[4 * i + e][k] = fmaf(acc[4 * i + e][k], corr[k & 1], sum[k]);
       }

@@ -15,6 +15,7 @@
 #pragma once
 #include "attend.cuh"
 #include "pdl.cuh"
+#include "sm100.cuh"
 
 namespace omni {
 namespace pattn {
@@ -30,24 +31,6 @@ __device__ __forceinline__ void cp16(uint32_t dst, const void* src, bool fetch) 
 __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-
-__device__ __forceinline__ void ldsm4(uint32_t addr, uint32_t (&r)[4]) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-               : "r"(addr)
-               : "memory");
-}
-__device__ __forceinline__ void ldsm4t(uint32_t addr, uint32_t (&r)[4]) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-               : "r"(addr)
-               : "memory");
-}
-__device__ __forceinline__ void mma(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
 
 template <int D, int G>
 __global__ void __launch_bounds__(kRows * G * 2, G >= 4 ? 1 : 2)
@@ -145,9 +128,9 @@ __global__ void __launch_bounds__(kRows * G * 2, G >= 4 ? 1 : 2)
         for (int jj = 0; jj < 2; ++jj) {  // 16 keys: matrices (keys 0-7, k 0-7), (keys 0-7, k 8-15), (keys 8-15, ...)
           const int tok = jj * 16 + (lane & 7) + ((lane >> 4) << 3);
           uint32_t b[4];
-          ldsm4(kb + (uint32_t)(tok * C + ((k * 2 + ((lane >> 3) & 1)) ^ (tok & 7))) * 16u, b);
-          mma(k & 1 ? s2[jj * 2] : s[jj * 2], q[k], b[0], b[1]);
-          mma(k & 1 ? s2[jj * 2 + 1] : s[jj * 2 + 1], q[k], b[2], b[3]);
+          sm100::ldsm4(kb + (uint32_t)(tok * C + ((k * 2 + ((lane >> 3) & 1)) ^ (tok & 7))) * 16u, b);
+          sm100::mma_16816(k & 1 ? s2[jj * 2] : s[jj * 2], q[k], b[0], b[1]);
+          sm100::mma_16816(k & 1 ? s2[jj * 2 + 1] : s[jj * 2 + 1], q[k], b[2], b[3]);
         }
       }
 #pragma unroll
@@ -206,11 +189,11 @@ __global__ void __launch_bounds__(kRows * G * 2, G >= 4 ? 1 : 2)
         for (int kk = 0; kk < 2; ++kk) {
           const int tok = kk * 16 + (lane & 15);
           uint32_t b[4];
-          ldsm4t(vb + (uint32_t)(tok * C + ((i * 2 + (lane >> 4)) ^ (tok & 7))) * 16u, b);
+          sm100::ldsm4t(vb + (uint32_t)(tok * C + ((i * 2 + (lane >> 4)) ^ (tok & 7))) * 16u, b);
 #pragma unroll
           for (int x = 2; x >= 0; --x) {
-            mma(o[0], p[kk][x], b[0], b[1]);
-            mma(o[1], p[kk][x], b[2], b[3]);
+            sm100::mma_16816(o[0], p[kk][x], b[0], b[1]);
+            sm100::mma_16816(o[1], p[kk][x], b[2], b[3]);
           }
         }
 #pragma unroll

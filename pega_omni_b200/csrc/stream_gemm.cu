@@ -31,39 +31,17 @@ struct StreamArgs {
   uint32_t acc_cols, tmem_cols;
 };
 
-__device__ __forceinline__ bool elect_one() {
-  uint32_t p;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}\n"
-      : "=r"(p));
-  return p != 0;
-}
-
-__device__ __forceinline__ void tmem_ld8_issue(uint32_t taddr, uint32_t (&r)[8]) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-               : "r"(taddr)
-               : "memory");
-}
-template <int NR>
-__device__ __forceinline__ void tmem_ld8_fence(uint32_t (&r)[NR][8]) {
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-  for (int i = 0; i < NR; ++i)
-    asm volatile("" : "+r"(r[i][0]), "+r"(r[i][1]), "+r"(r[i][2]), "+r"(r[i][3]), "+r"(r[i][4]), "+r"(r[i][5]), "+r"(r[i][6]), "+r"(r[i][7])::"memory");
-}
-
 // Eight columns of the accumulators, summed in issuer order.
 __device__ __forceinline__ void acc_cols8(uint32_t lane_addr, int col, const StreamArgs& a, float (&v)[8]) {
   uint32_t r[kIssuers][8];
 #pragma unroll
   for (int i = 0; i < kIssuers; ++i)
-    if (i < a.issuers) tmem_ld8_issue(lane_addr + (uint32_t)i * a.acc_cols + col, r[i]);
+    if (i < a.issuers) sm100::tmem_ld8_issue(lane_addr + (uint32_t)i * a.acc_cols + col, r[i]);
     else {
 #pragma unroll
       for (int j = 0; j < 8; ++j) r[i][j] = 0u;
     }
-  tmem_ld8_fence<kIssuers>(r);
+  sm100::tmem_ld8_fence<kIssuers>(r);
 #pragma unroll
   for (int j = 0; j < 8; ++j) v[j] = (__uint_as_float(r[0][j]) + __uint_as_float(r[1][j])) + (__uint_as_float(r[2][j]) + __uint_as_float(r[3][j]));
 }

@@ -62,13 +62,6 @@ __device__ __forceinline__ void pair_load_3d(uint32_t dst, const CUtensorMap* ma
       ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(x), "r"(y), "r"(z), "l"(hint)
       : "memory");
 }
-__device__ __forceinline__ bool elect_one() {
-  uint32_t p;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}\n"
-      : "=r"(p));
-  return p != 0;
-}
 __device__ __forceinline__ void pair_mma(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
       "{\n\t"
@@ -85,20 +78,6 @@ __device__ __forceinline__ void pair_commit(uint32_t bar) {
                "h"((uint16_t)3)
                : "memory");
 }
-__device__ __forceinline__ void ld8_issue(uint32_t taddr, uint32_t (&r)[8]) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-               : "r"(taddr)
-               : "memory");
-}
-template <int NR>
-__device__ __forceinline__ void ld8_fence(uint32_t (&r)[NR][8]) {
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-  for (int i = 0; i < NR; ++i)
-    asm volatile("" : "+r"(r[i][0]), "+r"(r[i][1]), "+r"(r[i][2]), "+r"(r[i][3]), "+r"(r[i][4]), "+r"(r[i][5]), "+r"(r[i][6]), "+r"(r[i][7])::"memory");
-}
-
 template <int OUT>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kWideThreads, 1)
     wide_gemm_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap wmap, const WideArgs a) {
@@ -229,9 +208,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kWideThreads, 1)
             const int ch0 = (n * groups + gr) * a.granule, half = min(a.granule, inter - ch0), at = gr * 2 * a.granule;
             for (int c = 0; c < half; c += 8) {
               uint32_t r[2][8];
-              ld8_issue(lane_addr + at + c, r[0]);
-              ld8_issue(lane_addr + at + half + c, r[1]);
-              ld8_fence<2>(r);
+              tmem_ld8_issue(lane_addr + at + c, r[0]);
+              tmem_ld8_issue(lane_addr + at + half + c, r[1]);
+              tmem_ld8_fence<2>(r);
               float o[8];
 #pragma unroll
               for (int j = 0; j < 8; ++j) {
@@ -245,8 +224,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kWideThreads, 1)
           for (int c = 0; c < cols; c += 32) {  // tn is a multiple of 32
             uint32_t r[4][8];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) ld8_issue(lane_addr + c + i * 8, r[i]);
-            ld8_fence<4>(r);
+            for (int i = 0; i < 4; ++i) tmem_ld8_issue(lane_addr + c + i * 8, r[i]);
+            tmem_ld8_fence<4>(r);
             if (!live) continue;
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
