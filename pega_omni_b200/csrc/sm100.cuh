@@ -284,5 +284,21 @@ __device__ __forceinline__ void tmem_ld8_fence(uint32_t (&r)[NR][8]) {
     asm volatile("" : "+r"(r[i][0]), "+r"(r[i][1]), "+r"(r[i][2]), "+r"(r[i][3]), "+r"(r[i][4]), "+r"(r[i][5]), "+r"(r[i][6]), "+r"(r[i][7])::"memory");
 }
 
+// Sixteen lanes of TMEM (the address' own, the first or the second half of the warp's quadrant) and eight f32 columns,
+// laid out as an m16n8 fragment: r[0], r[1] are columns 2 (lane % 4) and the next of TMEM lane lane / 4, r[2], r[3] those of
+// lane / 4 + 8. And the wait for any number of such loads.
+__device__ __forceinline__ void tmem_ld_16x8_issue(uint32_t taddr, uint32_t (&r)[4]) {
+  asm volatile("tcgen05.ld.sync.aligned.16x256b.x1.b32 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(taddr)
+               : "memory");
+}
+template <int NR>
+__device__ __forceinline__ void tmem_ld_16x8_fence(uint32_t (&r)[NR][4]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+  for (int i = 0; i < NR; ++i) asm volatile("" : "+r"(r[i][0]), "+r"(r[i][1]), "+r"(r[i][2]), "+r"(r[i][3])::"memory");
+}
+
 }  // namespace sm100
 }  // namespace omni

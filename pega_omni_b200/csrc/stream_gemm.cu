@@ -3,9 +3,9 @@
 // Bound by its weights' bytes where they are many, by the path from the rows' arrival to the stores where they are few:
 // rows to shared memory by TMA, the MMAs' issue, commit, TMEM to registers, stores. Hence the rows on M (64 or 128 TMEM
 // lanes, a tile of weights as narrow as fills the chip once on N), weights asked for before the rows exist, four issuing
-// threads and split K without a reduction of its own. Measured as nodes of a chain at 64 rows: 12,288 x 2,048 with SwiGLU
-// 13.3 us (its weights alone take 7.7 us from DRAM), 12,288 x 4,096 23.8 us (15.4), 22,528 x 4,096 with SwiGLU 39.9 us
-// (28.3), 4,096 x 1,024 4.7 us; a phase of the persistent tick kernel took 7 us at least.
+// threads and split K without a reduction of its own. Measured as nodes of a chain at 64 rows, from the rows' being there to the
+// CTAs' end: 12,288 x 2,048 with SwiGLU 9.9 us (its weights alone take 7.7 us from DRAM), 12,288 x 4,096 18.1 us (15.4),
+// 22,528 x 4,096 with SwiGLU 33.5 us (28.3), 4,096 x 1,024 3.0 us; a phase of the persistent tick kernel took 7 us at least.
 #include "stream_gemm.h"
 
 #include <algorithm>
@@ -20,7 +20,7 @@ namespace {
 
 constexpr int kKb = 64;  // K elements per k-block: one 128-byte swizzle row
 constexpr int kMaxSlots = 8, kIssuers = 4;
-constexpr int kThreads = 32 * (2 + kIssuers);  // W producer, X producer, four MMA issuers that are also the epilogue
+constexpr int kThreads = 256;  // W producer, X producer, four MMA issuers, two more: all eight are the epilogue
 
 struct StreamArgs {
   bf16* y;
@@ -31,19 +31,26 @@ struct StreamArgs {
   uint32_t acc_cols, tmem_cols;
 };
 
-// Eight columns of the accumulators, summed in issuer order.
-__device__ __forceinline__ void acc_cols8(uint32_t lane_addr, int col, const StreamArgs& a, float (&v)[8]) {
-  uint32_t r[kIssuers][8];
+// P pieces of eight columns of 16 accumulator rows, `step` columns apart, the accumulators summed in issuer order: rows
+// lane / 4 (v[p][0], v[p][1]) and lane / 4 + 8, columns 2 (lane % 4) and the next. Every load is under way before the wait.
+template <int P>
+__device__ __forceinline__ void acc_pieces(uint32_t addr, int step, int pieces, const StreamArgs& a, float (&v)[P][4]) {
+  uint32_t r[kIssuers * P][4];
 #pragma unroll
   for (int i = 0; i < kIssuers; ++i)
-    if (i < a.issuers) sm100::tmem_ld8_issue(lane_addr + (uint32_t)i * a.acc_cols + col, r[i]);
-    else {
 #pragma unroll
-      for (int j = 0; j < 8; ++j) r[i][j] = 0u;
+    for (int p = 0; p < P; ++p) {
+      if (i < a.issuers && p < pieces) sm100::tmem_ld_16x8_issue(addr + (uint32_t)i * a.acc_cols + (uint32_t)(p * step), r[i * P + p]);
+      else r[i * P + p][0] = r[i * P + p][1] = r[i * P + p][2] = r[i * P + p][3] = 0u;
     }
-  sm100::tmem_ld8_fence<kIssuers>(r);
+  sm100::tmem_ld_16x8_fence<kIssuers * P>(r);
 #pragma unroll
-  for (int j = 0; j < 8; ++j) v[j] = (__uint_as_float(r[0][j]) + __uint_as_float(r[1][j])) + (__uint_as_float(r[2][j]) + __uint_as_float(r[3][j]));
+  for (int p = 0; p < P; ++p)
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      auto f = [&](int i) { return __uint_as_float(r[i * P + p][k]); };
+      v[p][k] = (f(0) + f(1)) + (f(2) + f(3));
+    }
 }
 
 template <int OUT>
@@ -54,6 +61,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   extern __shared__ unsigned char stream_smem_raw[];
   __shared__ __align__(8) uint64_t bars_s[3 * kMaxSlots + 1];
   __shared__ uint32_t tmem_slot_s;
+  __shared__ float bias_s[OUT == kStreamBf16 ? 256 : 1];
   const uint32_t base = (smem_addr(stream_smem_raw) + 1023u) & ~1023u;
   const uint32_t bars = smem_addr(bars_s);
   auto full_w = [&](int s) { return bars + 8u * s; };
@@ -81,6 +89,9 @@ __global__ void __launch_bounds__(kThreads, 1)
     prefetch_tensormap(&xmap);
   }
   if (warp == 2) tmem_alloc(smem_addr(&tmem_slot_s), a.tmem_cols);
+  if constexpr (OUT == kStreamBf16) {
+    if (a.kind != kEpiNone && (int)threadIdx.x < min(a.tn, a.N - tile * a.tn)) bias_s[threadIdx.x] = __bfloat162float(a.bias[tile * a.tn + threadIdx.x]);
+  }
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
@@ -118,11 +129,10 @@ __global__ void __launch_bounds__(kThreads, 1)
         if (++slot == a.slots) slot = 0, phase ^= 1u;
       }
     }
-  } else {
+  } else if (warp < 2 + kIssuers) {
     // issuer `me` takes stages me, me + issuers, ... into its own accumulator: one thread issues an MMA only every
     // 80 cycles or so, half of what the tensor pipe takes at these shapes
     const int me = warp - 2;
-    grid_wait();
     if (me < a.issuers) {
       const uint32_t idesc = idesc_bf16_f32(a.M, a.tn), acc = tmem + (uint32_t)me * a.acc_cols;
       bool alive = true;
@@ -150,54 +160,78 @@ __global__ void __launch_bounds__(kThreads, 1)
       if (alive && elect_one()) mma_commit(acc_bar);
       __syncwarp();
     }
-    const bool ok = mbar_wait(acc_bar, 0, a.err);
-    tc_fence_after_sync();
-    const int quad = warp & 3;
-    const uint32_t lane_addr = tmem + ((uint32_t)(quad * 32) << 16);
-    // M = 128: row = TMEM lane; M = 64: rows 16 q .. 16 q + 15 sit in the first sixteen lanes of quadrant q
-    const int r = a.M == 128 ? quad * 32 + lane : quad * 16 + lane;
-    const int m = m0 + r;
-    const bool row_live = m < a.rows && (a.M == 128 || lane < 16);
-    const bool warp_live = m0 + (a.M == 128 ? quad * 32 : quad * 16) < a.rows;
-    if (ok && warp_live) {
-      if constexpr (OUT == kStreamSwiglu) {
-        // the tile's rows are groups of gates and their ups
-        const int ch0 = tile * (a.tn >> 1), half = min(a.tn >> 1, (a.N >> 1) - ch0);
-        for (int c = 0; c < half; c += kGateGroup) {
-          float g[8], u[8];
-          acc_cols8(lane_addr, 2 * c, a, g);
-          acc_cols8(lane_addr, 2 * c + kGateGroup, a, u);
-          if (!row_live) continue;
-          float o[8];
+  }
+  __syncwarp();
+
+  // ---- epilogue: two warps a TMEM quadrant, sixteen rows at a time as m16n8 fragments, so that every lane has work where
+  // M = 64 leaves half of a quadrant's lanes empty. M = 64: the quadrant's rows are 16 q .. 16 q + 15, and its warps share
+  // the columns; M = 128: 32 q .. 32 q + 31, sixteen a warp. From the last product to the CTA's end at 64 rows, before
+  // (four warps, a row a lane, eight columns at a time) and now: 48 columns with SwiGLU 1.9 and 1.0 us, 176 columns 4.9 and
+  // 2.6, 96 columns of bf16 4.5 and 1.9, 32 columns 2.0 and 1.1, 64 columns of partial sums 1.4 and 0.9.
+  const int quad = warp & 3, half = warp >> 2, g = lane >> 2, t2 = (lane & 3) * 2;
+  const int r0 = a.M == 128 ? quad * 32 + half * 16 : quad * 16;
+  const uint32_t lane_addr = tmem + ((uint32_t)(quad * 32 + (a.M == 128 ? half * 16 : 0)) << 16);
+  const int m_lo = m0 + r0 + g, m_hi = m_lo + 8;
+  const bool lo = m_lo < a.rows, hi = m_hi < a.rows;
+  // units of this warp: groups of gates and their ups, or pieces of eight columns
+  const int n0 = tile * a.tn, width = min(a.tn, a.N - n0), unit = OUT == kStreamSwiglu ? 2 * kGateGroup : 8;
+  const int units = (width + unit - 1) / unit, share = a.M == 128 ? units : (units + 1) >> 1;
+  const int u0 = a.M == 128 ? 0 : half * share, u1 = min(units, u0 + share);
+  grid_wait();
+  const bool ok = mbar_wait(acc_bar, 0, a.err);
+  tc_fence_after_sync();
+  if (ok && m0 + r0 < a.rows) {
+    if constexpr (OUT == kStreamSwiglu) {
+      constexpr int P = 2;
+      bf16* const y = a.y + (size_t)m_lo * a.ldy + (n0 >> 1) + t2;
+      for (int u = u0; u < u1; u += P) {
+        float v[2 * P][4];
+        acc_pieces<2 * P>(lane_addr + (uint32_t)(u * 16), 8, 2 * (u1 - u), a, v);
 #pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            o[j] = silu_bf16(bf16_round(g[j])) * bf16_round(u[j]);
+        for (int p = 0; p < P; ++p) {
+          float o[4];
+#pragma unroll
+          for (int k = 0; k < 4; ++k) o[k] = silu_bf16(bf16_round(v[2 * p][k])) * bf16_round(v[2 * p + 1][k]);
+          if (u + p < u1) {
+            if (lo) *reinterpret_cast<__nv_bfloat162*>(y + (u + p) * kGateGroup) = __floats2bfloat162_rn(o[0], o[1]);
+            if (hi) *reinterpret_cast<__nv_bfloat162*>(y + (size_t)8 * a.ldy + (u + p) * kGateGroup) = __floats2bfloat162_rn(o[2], o[3]);
           }
-          st8(a.y + (size_t)m * a.ldy + ch0 + c, o);
         }
-      } else {
-        const int n0 = tile * a.tn;
-        for (int c = 0; c < a.tn; c += 8) {
-          float v[8];
-          acc_cols8(lane_addr, c, a, v);
-          if (!row_live || n0 + c >= a.N) continue;
-          if constexpr (OUT == kStreamPartials) {
-            float* dst = a.part + ((size_t)split * a.rows + m) * a.N + n0 + c;
-            *reinterpret_cast<float4*>(dst) = make_float4(v[0], v[1], v[2], v[3]);
-            *reinterpret_cast<float4*>(dst + 4) = make_float4(v[4], v[5], v[6], v[7]);
-          } else {
-            bf16* dst = a.y + (size_t)m * a.ldy + n0 + c;
+      }
+    } else {
+      constexpr int P = 4;
+      for (int u = u0; u < u1; u += P) {
+        float v[P][4];
+        acc_pieces<P>(lane_addr + (uint32_t)(u * 8), 8, u1 - u, a, v);
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-              v[j] = bf16_round(v[j]);
-              if (a.kind != kEpiNone && n0 + c + j < a.N) {
-                v[j] = bf16_round(v[j] + __bfloat162float(a.bias[n0 + c + j]));
-                if (a.kind == kEpiBiasSilu) v[j] = v[j] / (1.f + __expf(-v[j]));
+        for (int p = 0; p < P; ++p) {
+          if (u + p >= u1) break;
+          const int c = (u + p) * 8 + t2, n = n0 + c;
+          if constexpr (OUT == kStreamPartials) {
+            float* dst = a.part + ((size_t)split * a.rows + m_lo) * a.N + n;
+            if (lo) *reinterpret_cast<float2*>(dst) = make_float2(v[p][0], v[p][1]);
+            if (hi) *reinterpret_cast<float2*>(dst + (size_t)8 * a.N) = make_float2(v[p][2], v[p][3]);
+          } else {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+              v[p][k] = bf16_round(v[p][k]);
+              if (a.kind != kEpiNone) {  // (past the row's end: a sum that is not stored)
+                v[p][k] = bf16_round(v[p][k] + bias_s[c + (k & 1)]);
+                if (a.kind == kEpiBiasSilu) v[p][k] = v[p][k] / (1.f + __expf(-v[p][k]));
               }
             }
-            if (a.vec) st8(dst, v);
-            else
-              for (int j = 0; j < 8 && n0 + c + j < a.N; ++j) dst[j] = __float2bfloat16(v[j]);
+            bf16* dst = a.y + (size_t)m_lo * a.ldy + n;
+            bf16* dst8 = dst + (size_t)8 * a.ldy;
+            if (a.vec) {
+              if (lo) *reinterpret_cast<__nv_bfloat162*>(dst) = __floats2bfloat162_rn(v[p][0], v[p][1]);
+              if (hi) *reinterpret_cast<__nv_bfloat162*>(dst8) = __floats2bfloat162_rn(v[p][2], v[p][3]);
+            } else {
+#pragma unroll
+              for (int k = 0; k < 2; ++k) {
+                if (lo && n + k < a.N) dst[k] = __float2bfloat16(v[p][k]);
+                if (hi && n + k < a.N) dst8[k] = __float2bfloat16(v[p][2 + k]);
+              }
+            }
           }
         }
       }

@@ -57,6 +57,19 @@ def test_chain_gemm(ops, rows, n, k, epilogue):
     assert (y[rows] == 7.0).all()  # nothing past the last row
 
 
+# the tcgen05 epilogue's fragments: rows that end inside one, columns that leave a warp of a pair without any, one to four sums
+@pytest.mark.parametrize("rows", [10, 24, 25, 57, 73, 121])
+@pytest.mark.parametrize("n,k", [(199, 64), (176, 192), (40, 320), (8, 1024)])
+def test_chain_gemm_fragments(ops, rows, n, k):
+    w, x = rand((n, k), 41, k ** -0.5), rand((rows, k), 42)
+    y = torch.full((rows + 1, n), 7.0, dtype=torch.bfloat16, device="cuda")
+    torch.cuda.synchronize()
+    ops.chain_gemm(w, x, y[:rows])
+    ops.sync()
+    close(y[:rows], product(x, w))
+    assert (y[rows] == 7.0).all()
+
+
 @pytest.mark.parametrize("rows", [1, 9, 17, 128, 129, 257])
 @pytest.mark.parametrize("inter,k", [(256, 64), (3072, 1024), (4096, 576)])
 def test_chain_swiglu(ops, rows, inter, k):
