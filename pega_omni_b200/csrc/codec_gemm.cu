@@ -89,7 +89,7 @@ __global__ void __launch_bounds__(kConvThreads, 1)
   auto empty_bar = [&](int s) { return bars + 8u * (kConvMaxStages + s); };
   auto acc_full = [&](int b) { return bars + 8u * (2 * kConvMaxStages + b); };
   auto acc_empty = [&](int b) { return bars + 8u * (2 * kConvMaxStages + 2 + b); };
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const int steps = a.taps * a.cpb / a.kbs;
   // weights first in a stage, then the activation box (whose MMA reads may run past the stage)
   auto load_w = [&](int n0, int tap, int cb, int stage) {

@@ -135,7 +135,7 @@ __global__ void __launch_bounds__(kWarps * 32, 2) few_rows_kernel(const __grid_c
   extern __shared__ unsigned char few_smem_raw[];
   __shared__ __align__(8) uint64_t bars_s[kWarps * kFewSlots];
   __shared__ __align__(16) float ss_s[8][kWarps];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const int tile = blockIdx.x, split = blockIdx.y;
   // k-blocks: `span` per split, `per` per warp, the last of each fewer
   const int kb0 = few_first(warp, split, a.span, a.per), nk = few_count(warp, split, a.span, a.per, a.nkb);

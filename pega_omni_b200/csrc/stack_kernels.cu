@@ -384,7 +384,7 @@ __global__ void __launch_bounds__(W * TEAMS * 32, W == 8 ? 1 : 3)
   grid_trigger();
   __shared__ RopeShared<D, G> shared[TEAMS];
   __shared__ MergeShared<D, G, W> merge;
-  const int lane = threadIdx.x & 31, warp = (threadIdx.x >> 5) % W, team = (threadIdx.x >> 5) / W;
+  const int lane = threadIdx.x & 31, warp = warp_index() % W, team = warp_index() / W;
   const int item = blockIdx.x * TEAMS + team, seq = item / hk, kh = item % hk;
   const bool live = item < items;
   RopeShared<D, G>& sh = shared[team];

@@ -68,7 +68,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   auto full_x = [&](int s) { return bars + 8u * (kMaxSlots + s); };
   auto empty = [&](int s) { return bars + 8u * (2 * kMaxSlots + s); };
   const uint32_t acc_bar = bars + 8u * (3 * kMaxSlots);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const int tile = blockIdx.x, split = blockIdx.y, m0 = blockIdx.z * 128;
   const int st0 = (int)((int64_t)a.stages * split / a.splits), st1 = (int)((int64_t)a.stages * (split + 1) / a.splits);
   const int n_st = st1 - st0;
