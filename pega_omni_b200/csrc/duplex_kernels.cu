@@ -113,27 +113,27 @@ __global__ void lm_add_norm_kernel(const bf16* y, bf16* x, const bf16* __restric
   if (out) norm_row(v, alpha, out + (int64_t)blockIdx.x * dim, dim, eps, scratch);
 }
 
-// The same over a GEMM's summands: every load of a thread's eight columns is under way at once.
-template <int S>
+// The same over a GEMM's summands: every load of a thread's E columns is under way at once.
+template <int S, int E>
 __global__ void lm_add_norm_sum_kernel(const Summands y, bf16* __restrict__ x, const bf16* __restrict__ alpha,
                                        bf16* __restrict__ out, int dim, float eps) {
   grid_trigger();
   __shared__ float scratch[32];
-  const int c = threadIdx.x * 8, lane = threadIdx.x & 31;
+  const int c = threadIdx.x * E, lane = threadIdx.x & 31;
   const int64_t at = (int64_t)blockIdx.x * dim + c;
   const bool on = c < dim;  // the block is a whole number of warps
-  float v[8], u[8], a[8], ss = 0.f;
-  if (out && on) ld8(alpha + c, a);
+  float v[E], u[E], a[E], ss = 0.f;
+  if (out && on) Run<E>::ld(alpha + c, a);
   grid_wait();
   if (on) {
-    ld8cg(x + at, v);
-    load_sum8<S>(y, blockIdx.x, c, u);
+    Run<E>::ldcg(x + at, v);
+    load_sum<S, E>(y, blockIdx.x, c, u);
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
+    for (int k = 0; k < E; ++k) {
       v[k] = bf16_round(v[k] + u[k]);
       ss += v[k] * v[k];
     }
-    st8(x + at, v);
+    Run<E>::st(x + at, v);
   }
   if (!out) return;
   ss = warp_add(ss);
@@ -142,8 +142,8 @@ __global__ void lm_add_norm_sum_kernel(const Summands y, bf16* __restrict__ x, c
   const float r = rsqrtf(warp_add(lane < (int)blockDim.x >> 5 ? scratch[lane] : 0.f) / dim + eps);
   if (!on) return;
 #pragma unroll
-  for (int k = 0; k < 8; ++k) v[k] = v[k] * (a[k] * r);
-  st8(out + at, v);
+  for (int k = 0; k < E; ++k) v[k] = v[k] * (a[k] * r);
+  Run<E>::st(out + at, v);
 }
 
 // ---- tensor-parallel pair: all-reduce of a projection's partial rows, fused with the add + norm that follows -----
@@ -850,7 +850,10 @@ cudaError_t launch_lm_add_norm_sum(const Summands& y, bf16* x, const bf16* alpha
                                    cudaStream_t s) {
   if (!row_dim_ok(dim)) return cudaErrorInvalidValue;
   return with_summands(y.splits, [&](auto sums) {
-    return launch_pdl(lm_add_norm_sum_kernel<decltype(sums)::value>, dim3(rows), dim3(row_threads(dim)), 0, s, y, x, alpha, out, dim, eps);
+    return with_columns(dim, rows, [&](auto columns) {
+      constexpr int E = decltype(columns)::value;
+      return launch_pdl(lm_add_norm_sum_kernel<decltype(sums)::value, E>, dim3(rows), dim3((dim + E * 32 - 1) / (E * 32) * 32), 0, s, y, x, alpha, out, dim, eps);
+    });
   });
 }
 

@@ -89,28 +89,28 @@ __global__ void silu_mul_kernel(const bf16* gate_up, bf16* __restrict__ act, int
   st8(act + (int64_t)i * 8, g);
 }
 
-// add_norm over a GEMM's S summands: a thread owns eight columns, and all its loads - the partial sums, the residual, the
+// add_norm over a GEMM's S summands: a thread owns E columns, and all its loads - the partial sums, the residual, the
 // gain - are under way together, so the kernel is one L2 round trip and one block reduction long. What is left is the
-// number of instructions, executed once: the count of summands is a template argument.
-template <int S>
+// number of instructions, executed once: the counts of summands and columns are template arguments.
+template <int S, int E>
 __global__ void add_norm_sum_kernel(const Summands x, bf16* __restrict__ res, const bf16* __restrict__ w,
                                     bf16* __restrict__ out, int dim, float eps, int every, int which) {
   grid_trigger();
   __shared__ float scratch[32];
-  const int n = blockIdx.x, c = threadIdx.x * 8, lane = threadIdx.x & 31;
+  const int n = blockIdx.x, c = threadIdx.x * E, lane = threadIdx.x & 31;
   const bool on = c < dim;  // the block is a whole number of warps
-  float g[8], v[8], rv[8], ss = 0.f;
-  if (on) ld8(w + c, g);
+  float g[E], v[E], rv[E], ss = 0.f;
+  if (on) Run<E>::ld(w + c, g);
   grid_wait();
   if (on) {
-    ld8cg(res + (int64_t)n * dim + c, rv);
-    load_sum8<S>(x, n, c, v);
+    Run<E>::ldcg(res + (int64_t)n * dim + c, rv);
+    load_sum<S, E>(x, n, c, v);
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
+    for (int k = 0; k < E; ++k) {
       v[k] += rv[k];
       ss += v[k] * v[k];
     }
-    st8(res + (int64_t)n * dim + c, v);
+    Run<E>::st(res + (int64_t)n * dim + c, v);
   }
   ss = warp_add(ss);
   if (lane == 0) scratch[threadIdx.x >> 5] = ss;
@@ -119,15 +119,19 @@ __global__ void add_norm_sum_kernel(const Summands x, bf16* __restrict__ res, co
   const float r = rsqrtf(warp_add(lane < (int)blockDim.x >> 5 ? scratch[lane] : 0.f) / dim + eps);
   if (!on) return;
 #pragma unroll
-  for (int k = 0; k < 8; ++k) v[k] = v[k] * r * g[k];
-  st8(out + (int64_t)(n / every) * dim + c, v);
+  for (int k = 0; k < E; ++k) v[k] = v[k] * r * g[k];
+  Run<E>::st(out + (int64_t)(n / every) * dim + c, v);
 }
 
 cudaError_t launch_add_norm_sum(const Summands& x, bf16* res, const bf16* w, bf16* out, int rows, int dim, float eps,
                                 int every, int which, cudaStream_t s) {
   if (dim % 8 || dim / 8 > 1024) return cudaErrorInvalidValue;
   return with_summands(x.splits, [&](auto sums) {
-    return launch_pdl(add_norm_sum_kernel<decltype(sums)::value>, dim3(rows), dim3(row_threads(dim)), 0, s, x, res, w, out, dim, eps, every, which);
+    return with_columns(dim, rows, [&](auto columns) {
+      constexpr int E = decltype(columns)::value;
+      return launch_pdl(add_norm_sum_kernel<decltype(sums)::value, E>, dim3(rows), dim3((dim + E * 32 - 1) / (E * 32) * 32), 0, s, x, res, w, out, dim, eps,
+                        every, which);
+    });
   });
 }
 

@@ -22,25 +22,27 @@ struct Summands {
   int ld = 0;                // elements per row
 };
 
-// Eight columns of row n from column c on, of S summands (0: bf16 rows): the bf16 values, widened.
-template <int S>
-__device__ __forceinline__ void load_sum8(const Summands& x, int n, int c, float (&v)[8]) {
+// E columns (2, 4 or 8) of row n from column c on, of S summands (0: bf16 rows): the bf16 values, widened.
+template <int S, int E>
+__device__ __forceinline__ void load_sum(const Summands& x, int n, int c, float (&v)[E]) {
   if constexpr (S == 0) {
-    unpack8v(__ldcg(reinterpret_cast<const uint4*>(x.done + (int64_t)n * x.ld + c)), v);
+    Run<E>::ldcg(x.done + (int64_t)n * x.ld + c, v);
   } else {
+    using Word = std::conditional_t<E == 2, float2, float4>;
+    constexpr int H = E == 8 ? 2 : 1;
     const float* p = x.part + (int64_t)n * x.ld + c;
-    float4 f[S][2];
+    Word f[S][H];
 #pragma unroll
     for (int s = 0; s < S; ++s)
 #pragma unroll
-      for (int h = 0; h < 2; ++h) f[s][h] = __ldcg(reinterpret_cast<const float4*>(p + s * x.split_stride) + h);
+      for (int h = 0; h < H; ++h) f[s][h] = __ldcg(reinterpret_cast<const Word*>(p + s * x.split_stride) + h);
 #pragma unroll
-    for (int s = 1; s < S; ++s) {
-      f[0][0].x += f[s][0].x, f[0][0].y += f[s][0].y, f[0][0].z += f[s][0].z, f[0][0].w += f[s][0].w;
-      f[0][1].x += f[s][1].x, f[0][1].y += f[s][1].y, f[0][1].z += f[s][1].z, f[0][1].w += f[s][1].w;
+    for (int k = 0; k < E; ++k) {
+      float sum = reinterpret_cast<const float*>(f[0])[k];
+#pragma unroll
+      for (int s = 1; s < S; ++s) sum += reinterpret_cast<const float*>(f[s])[k];
+      v[k] = bf16_round(sum);
     }
-    v[0] = bf16_round(f[0][0].x), v[1] = bf16_round(f[0][0].y), v[2] = bf16_round(f[0][0].z), v[3] = bf16_round(f[0][0].w);
-    v[4] = bf16_round(f[0][1].x), v[5] = bf16_round(f[0][1].y), v[6] = bf16_round(f[0][1].z), v[7] = bf16_round(f[0][1].w);
   }
 }
 
@@ -55,6 +57,17 @@ cudaError_t with_summands(int splits, F&& go) {
     case 8: return go(std::integral_constant<int, 8>());
     default: return cudaErrorInvalidValue;
   }
+}
+
+// go(std::integral_constant<int, E>): columns a thread of the add + norm of `rows` rows of `dim` elements. What is behind its
+// wait runs once, so few columns a thread and up to 1,024 threads. Eight columns and this, one pass, us: a talker step of 8
+// sessions (1,024 and 2,048 wide) 2,653 and 2,586, of 64 3,714 and 3,613, of 128 5,004 and 4,910, a duplex tick of 64 (4,096)
+// 5,713 and 5,652, a Higgs step of 32 (2,560) 3,010 and 2,980. Prompts are many rows whose bytes count.
+template <typename F>
+cudaError_t with_columns(int dim, int rows, F&& go) {
+  if (rows <= 256 && dim <= 2048) return go(std::integral_constant<int, 2>());
+  if (rows <= 256 && dim <= 4096) return go(std::integral_constant<int, 4>());
+  return go(std::integral_constant<int, 8>());
 }
 
 enum StreamOut : int { kStreamBf16 = 0, kStreamPartials = 1, kStreamSwiglu = 2 };

@@ -5,6 +5,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <type_traits>
+
 namespace omni {
 
 // threadIdx.x / 32 as a value that is the same in every lane, which the compiler cannot see by itself: what follows from it -
@@ -94,6 +96,28 @@ __device__ __forceinline__ void st8(bf16* dst, const float* v) { st8v(dst, v); }
 
 // The same past L1, for rows that another SM wrote while this kernel had already started.
 __device__ __forceinline__ void ld8cg(const bf16* src, float* v) { unpack8v(__ldcg(reinterpret_cast<const uint4*>(src)), v); }
+
+// E = 2, 4 or 8 bf16 as one access, widened to f32.
+template <int E>
+struct Run {
+  using Word = std::conditional_t<E == 8, uint4, std::conditional_t<E == 4, uint2, uint32_t>>;
+  static __device__ __forceinline__ void widen(const Word& u, float* v) {
+    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&u);
+#pragma unroll
+    for (int i = 0; i < E / 2; ++i) {
+      const float2 f = __bfloat1622float2(h[i]);
+      v[2 * i] = f.x, v[2 * i + 1] = f.y;
+    }
+  }
+  static __device__ __forceinline__ void ld(const bf16* src, float* v) { widen(__ldg(reinterpret_cast<const Word*>(src)), v); }
+  static __device__ __forceinline__ void ldcg(const bf16* src, float* v) { widen(__ldcg(reinterpret_cast<const Word*>(src)), v); }
+  static __device__ __forceinline__ void st(bf16* dst, const float* v) {
+    Word u;
+#pragma unroll
+    for (int i = 0; i < E / 2; ++i) reinterpret_cast<__nv_bfloat162*>(&u)[i] = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
+    *reinterpret_cast<Word*>(dst) = u;
+  }
+};
 
 // Two f32 values as the sum of three bf16 each (value, rest of it, rest of that), packed: 24 bits of a value, its whole
 // mantissa. A matrix instruction on bf16 then multiplies it as f32 would.

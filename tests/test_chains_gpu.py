@@ -132,6 +132,13 @@ def test_decode_attention_in_one_kernel(ops, hq, hk, d, sessions):
     close(a, b, steps=1.5, floor=0.25)
 
 
+# two, four and eight columns a thread, rows that end inside a warp of each
+@pytest.mark.parametrize("rows", [9, 250])
+@pytest.mark.parametrize("d", [1984, 2048, 2112, 4096, 4160])
+def test_chain_norm_columns(ops, rows, d):
+    test_chain_norm_gemm(ops, rows, d, 64, 64)
+
+
 @pytest.mark.parametrize("heads,sessions", [(4, 1), (4, 37), (32, 5), (16, 16)])
 def test_fp8_ring_attention_in_one_kernel(ops, heads, sessions):
     """Positions before, at and past the end of a ring of 40 tokens."""
