@@ -356,48 +356,50 @@ cudaError_t launch_attend(const bf16* qkv, const bf16* kv, bf16* out, const RowM
 }
 
 // ---- decode: q/k norm + RoPE + KV write + attention in one kernel ------------------------------------------------
-// A team of W warps per (sequence, kv head). The G query heads, the key and the value of a row are dealt to the team's
-// warps; q, k and v go to shared memory (k and v also to the row's slot), and the team attends to them with the page step
+// A CTA of W warps per (sequence, kv head) of paged rows. The G query heads, the key and the value of a row are dealt to the
+// warps; q, k and v go to shared memory (k and v also to the row's slot), and the CTA attends to them with the page step
 // of decode_attend.cuh, each warp on its own pages. A page is 16 loads of 16 bytes a lane, straight into registers.
-// Paged rows: a warp's first page is asked for before grid_wait() - what earlier calls wrote does not depend on the
+// A warp's first page is asked for before grid_wait() - what earlier calls wrote does not depend on the
 // projection this kernel waits for - and the row's own token is patched in from shared memory.
-// Dense frames (the predictor): one page per sequence, W = 1, four sequences' heads per CTA; the page is asked for
-// together with the row, and the tokens this kernel itself writes are patched in.
 
-template <int D, int G>
+template <int D>
 struct RopeShared {
   alignas(16) bf16 q[8][D];
-  alignas(16) bf16 k[2][D];
-  alignas(16) bf16 v[2][D];
+  alignas(16) bf16 k[D];
+  alignas(16) bf16 v[D];
 };
 template <int D, int G, int W>
 struct MergeShared {
   float m[W][8], l[W][8];
   float o[W][G][D];
 };
-template <int D, int G>
-struct MergeShared<D, G, 1> {};
 
-template <int D, int G, int W, int TEAMS>
-__global__ void __launch_bounds__(W * TEAMS * 32, W == 8 ? 1 : 3)
-    rope_attend_kernel(const bf16* qkv, const QkvTable lookup, const bf16* __restrict__ q_norm,
-                       const bf16* __restrict__ k_norm, bf16* kv, bf16* __restrict__ out, RowMap map, int items, int hq,
-                       int hk, float eps, float theta, float scale, int kv_pages, uint32_t* err) {
-  static_assert(W == 1 || TEAMS == 1, "a team of several warps is a CTA");
+// Resident CTAs an SM: registers for one page in a lane's hands and the next on its way.
+constexpr int rope_attend_ctas(int W) { return W == 8 ? 1 : 12 / W; }
+
+// A lane's elements of both halves of a head, as they lie in memory.
+template <int D>
+__device__ __forceinline__ void ld_halves(const bf16* src, int lane, uint32_t (&raw)[2]) {
+  using Half = std::conditional_t<D == 128, uint32_t, uint16_t>;
+  raw[0] = __ldcg(reinterpret_cast<const Half*>(src) + lane), raw[1] = __ldcg(reinterpret_cast<const Half*>(src + D / 2) + lane);
+}
+template <int D>
+__device__ __forceinline__ void widen_halves(const uint32_t (&raw)[2], float (&lo)[D / 64], float (&hi)[D / 64]) {
+  lo[0] = __uint_as_float(raw[0] << 16), hi[0] = __uint_as_float(raw[1] << 16);
+  if constexpr (D == 128) lo[1] = __uint_as_float(raw[0] & 0xffff0000u), hi[1] = __uint_as_float(raw[1] & 0xffff0000u);
+}
+
+template <int D, int G, int W>
+__global__ void __launch_bounds__(W * 32, rope_attend_ctas(W))
+    rope_attend_kernel(const bf16* qkv, const bf16* __restrict__ q_norm, const bf16* __restrict__ k_norm, bf16* kv,
+                       bf16* __restrict__ out, RowMap map, int hq, int hk, float eps, float theta, float scale, int kv_pages,
+                       uint32_t* err) {
   constexpr int E = D / 64;
   grid_trigger();
-  __shared__ RopeShared<D, G> shared[TEAMS];
+  __shared__ RopeShared<D> sh;
   __shared__ MergeShared<D, G, W> merge;
-  const int lane = threadIdx.x & 31, warp = warp_index() % W, team = warp_index() / W;
-  const int item = blockIdx.x * TEAMS + team, seq = item / hk, kh = item % hk;
-  const bool live = item < items;
-  RopeShared<D, G>& sh = shared[team];
-  auto team_sync = [&]() {
-    if constexpr (W == 1) __syncwarp();
-    else __syncthreads();
-  };
-  const bool paged = map.pages != nullptr;
-  const int per = paged ? 1 : map.per;
+  const int lane = threadIdx.x & 31, warp = warp_index();
+  const int n = blockIdx.x / hk, kh = blockIdx.x % hk;
   float qwl[E], qwh[E], kwl[E], kwh[E];
 #pragma unroll
   for (int e = 0; e < E; ++e) {
@@ -406,124 +408,203 @@ __global__ void __launch_bounds__(W * TEAMS * 32, W == 8 ? 1 : 3)
   }
   for (int i = warp * 32 + lane; i < (8 - G) * D / 8; i += W * 32)  // heads past G: zero rows
     *reinterpret_cast<uint4*>(&sh.q[G][0] + i * 8) = make_uint4(0u, 0u, 0u, 0u);
-  const int32_t* pages = paged && live ? map.pages + map.indptr[seq] : nullptr;
+  const int32_t* pages = map.pages + map.indptr[n];
   dattn::Page<D> pg;
   dattn::State<D> st;
-  for (int r = 0; r < per; ++r) {
-    const int n = live ? seq * per + r : 0;
-    const int pos = paged ? map.pos[n] : map.base + r;
-    const int npages = paged ? (pos + 16) >> 4 : 1, last = npages - 1;
-    float cs[E], sn[E];
-    rope_angles<D>(lane, pos, theta, cs, sn);
-    const int64_t slot = paged ? map.slot[n] : (int64_t)seq * 16 + pos;
-    int64_t own = slot >> 4;
-    const int tok = (int)(slot & 15);
-    const bool owned = own >= 0 && own < kv_pages;  // otherwise the row stores nothing: page 0 is somebody's
-    if (!owned) {
-      if (live && warp == 0 && lane == 0) raise(err, kErrBadIndex);
-      own = 0;
+  const int pos = map.pos[n], npages = (pos + 16) >> 4, last = npages - 1;
+  float cs[E], sn[E];
+  rope_angles<D>(lane, pos, theta, cs, sn);
+  const int64_t slot = map.slot[n];
+  int64_t own = slot >> 4;
+  const int tok = (int)(slot & 15);
+  const bool owned = own >= 0 && own < kv_pages;  // otherwise the row stores nothing: page 0 is somebody's
+  if (!owned) {
+    if (warp == 0 && lane == 0) raise(err, kErrBadIndex);
+    own = 0;
+  }
+  auto block = [&](int pi) {
+    int64_t page = pi == last ? own : pages[pi];
+    if (page < 0 || page >= kv_pages) {
+      if (lane == 0) raise(err, kErrBadIndex);
+      page = 0;
     }
-    auto block = [&](int pi) {
-      int64_t page = pi == last ? own : pages[pi];
-      if (page < 0 || page >= kv_pages) {
-        if (lane == 0) raise(err, kErrBadIndex);
-        page = 0;
-      }
-      return kv + kv_offset<D>(page, hk, kh, 0, 0);
-    };
-    if (paged && live && warp < npages) pg.load(block(warp), lane);
-    if (r == 0) grid_wait();
-    if (W == 1 && !live) return;  // (a dead team of several warps does not exist: TEAMS is 1 there)
-    if (!paged) pg.load(block(0), lane);
-    const bf16* row = lookup.table ? lookup.table + (int64_t)__ldcg(lookup.codes + n * 16 + lookup.group) * ((hq + 2 * hk) * D)
-                                   : qkv + (int64_t)n * ((hq + 2 * hk) * D);
-    constexpr int JOBS = (G + 2 + W - 1) / W;
-    uint32_t raw[JOBS][2];
+    return kv + kv_offset<D>(page, hk, kh, 0, 0);
+  };
+  if (warp < npages) pg.load(block(warp), lane);
+  grid_wait();
+  const bf16* row = qkv + (int64_t)n * ((hq + 2 * hk) * D);
+  constexpr int JOBS = (G + 2 + W - 1) / W;
+  uint32_t raw[JOBS][2];
 #pragma unroll
-    for (int jj = 0; jj < JOBS; ++jj) {  // every head of this warp's share is asked for before the first is used
-      const int job = warp + jj * W;
-      const bf16* src = row + (job < G ? kh * G + job : job == G ? hq + kh : hq + hk + kh) * D;
-      if (job < G + 2) {
-        if constexpr (E == 2) {
-          raw[jj][0] = __ldcg(reinterpret_cast<const uint32_t*>(src) + lane), raw[jj][1] = __ldcg(reinterpret_cast<const uint32_t*>(src + D / 2) + lane);
-        } else {
-          raw[jj][0] = __ldcg(reinterpret_cast<const uint16_t*>(src) + lane), raw[jj][1] = __ldcg(reinterpret_cast<const uint16_t*>(src + D / 2) + lane);
-        }
+  for (int jj = 0; jj < JOBS; ++jj) {  // every head of this warp's share is asked for before the first is used
+    const int job = warp + jj * W;
+    if (job < G + 2) ld_halves<D>(row + (job < G ? kh * G + job : job == G ? hq + kh : hq + hk + kh) * D, lane, raw[jj]);
+  }
+#pragma unroll
+  for (int jj = 0; jj < JOBS; ++jj) {
+    const int job = warp + jj * W;
+    if (job >= G + 2) continue;
+    float lo[E], hi[E];
+    widen_halves<D>(raw[jj], lo, hi);
+    if (job < G) rope_head<D>(lo, hi, qwl, qwh, cs, sn, eps);
+    else if (job == G) rope_head<D>(lo, hi, kwl, kwh, cs, sn, eps);
+    st_half<D>(job < G ? sh.q[job] : job == G ? sh.k : sh.v, lane, lo, hi);
+    if (job >= G && owned) st_half<D>(kv + kv_offset<D>(own, hk, kh, job - G, tok), lane, lo, hi);
+  }
+  __syncthreads();
+  uint4 q[D / 32];
+#pragma unroll
+  for (int j = 0; j < D / 32; ++j) q[j] = *reinterpret_cast<const uint4*>(sh.q[lane >> 2] + 8 * (lane & 3) + 32 * j);
+  st.reset();
+  for (int pi = warp; pi < npages; pi += W) {
+    if (pi == last) pg.patch(tok, sh.k, sh.v, lane);
+    st.step(pg, q, min(16, pos + 1 - pi * 16), scale, lane, pi + W < npages ? block(pi + W) : nullptr);
+  }
+  st.finish();
+  const int g = lane >> 2, t = lane & 3;
+#pragma unroll
+  for (int h = 0; h < 2; ++h)
+    if (2 * t + h < G) {
+      if (g == 0) merge.m[warp][2 * t + h] = st.m[h], merge.l[warp][2 * t + h] = st.l[h];
+#pragma unroll
+      for (int i = 0; i < D / 64; ++i) {
+        float v[8];
+        st.dims8(i, h, v);
+        float4* dst = reinterpret_cast<float4*>(&merge.o[warp][2 * t + h][64 * i + 8 * g]);
+        dst[0] = make_float4(v[0], v[1], v[2], v[3]), dst[1] = make_float4(v[4], v[5], v[6], v[7]);
       }
     }
+  __syncthreads();
+  // a warp per head and 64 dims at a time; lane w has the weight of warp w's state (0 where it held no page)
+  for (int i = warp; i < G * (D / 64); i += W) {
+    const int h = i / (D / 64), d = i % (D / 64) * 64 + 2 * lane;
+    const float mw = lane < W ? merge.m[lane][h] : -INFINITY;
+    const float e = __expf(mw - warp_fmax(mw));
+    const float den = warp_add(lane < W ? e * merge.l[lane][h] : 0.f);
+    float o0 = 0.f, o1 = 0.f;
 #pragma unroll
-    for (int jj = 0; jj < JOBS; ++jj) {
-      const int job = warp + jj * W;
-      if (job >= G + 2) continue;
-      float lo[E], hi[E];
-      lo[0] = __uint_as_float(raw[jj][0] << 16), hi[0] = __uint_as_float(raw[jj][1] << 16);
-      if constexpr (E == 2) lo[1] = __uint_as_float(raw[jj][0] & 0xffff0000u), hi[1] = __uint_as_float(raw[jj][1] & 0xffff0000u);
-      if (job < G) rope_head<D>(lo, hi, qwl, qwh, cs, sn, eps);
-      else if (job == G) rope_head<D>(lo, hi, kwl, kwh, cs, sn, eps);
-      bf16* dst = job < G ? sh.q[job] : job == G ? sh.k[r & 1] : sh.v[r & 1];
-      bf16* page = job < G || !owned ? nullptr : kv + kv_offset<D>(own, hk, kh, job - G, tok);
-      st_half<D>(dst, lane, lo, hi);
-      if (page) st_half<D>(page, lane, lo, hi);
+    for (int w = 0; w < W; ++w) {
+      const float ew = __shfl_sync(0xffffffffu, e, w);
+      const float2 o = *reinterpret_cast<const float2*>(&merge.o[w][h][d]);
+      o0 += ew * o.x, o1 += ew * o.y;
     }
-    team_sync();
-    uint4 q[D / 32];
+    const float inv = 1.f / den;
+    *reinterpret_cast<__nv_bfloat162*>(out + ((int64_t)n * hq + kh * G + h) * D + d) = __floats2bfloat162_rn(o0 * inv, o1 * inv);
+  }
+}
+
+// The same for dense frames (the predictor: one page a sequence, one row or the first two of it at once). What is behind the
+// wait runs once, at five to six cycles an instruction, so four warps share a (row, kv head): each makes some of the q, k and v
+// heads and brings a quarter of the page, all weigh the keys, each sums a quarter of the values' dims. The queries are the M of
+// m16n8k16 (rows past G are zero), keys and then dims the N: a lane has one head's scores, and its probabilities are
+// the next product's operand as they are. Shared-memory rows are 16 bytes apart modulo 128, so no ldmatrix has a bank conflict.
+template <int D, int G>
+__global__ void __launch_bounds__(128)
+    frame_attend_kernel(const bf16* qkv, const QkvTable lookup, const bf16* __restrict__ q_norm, const bf16* __restrict__ k_norm,
+                        bf16* kv, bf16* __restrict__ out, int base, int hq, int hk, float eps, float theta, float scale,
+                        int kv_pages, uint32_t* err) {
+  constexpr int E = D / 64, W = 4, P = D + 8;
+  grid_trigger();
+  extern __shared__ __align__(16) bf16 frame_rows[];  // rows of P: zeros, the G queries, the keys 0..pos, their values
+  static_assert(P * 2 % 16 == 0);
+  const int lane = threadIdx.x & 31, warp = warp_index();
+  const int seq = blockIdx.x / hk, kh = blockIdx.x % hk, r = blockIdx.y, per = gridDim.y;
+  const int n = seq * per + r, pos = base + r;
+  bf16* const qs = frame_rows + P;
+  bf16* const kvs[2] = {qs + G * P, qs + (G + 1 + pos) * P};
+  float cs[E], sn[E], cs0[E], sn0[E], qwl[E], qwh[E], kwl[E], kwh[E];
+  rope_angles<D>(lane, pos, theta, cs, sn);
+  if (r > 0) rope_angles<D>(lane, pos - 1, theta, cs0, sn0);  // the row before is this CTA's key, too
 #pragma unroll
-    for (int j = 0; j < D / 32; ++j) q[j] = *reinterpret_cast<const uint4*>(sh.q[lane >> 2] + 8 * (lane & 3) + 32 * j);
-    st.reset();
-    for (int pi = warp; pi < npages; pi += W) {
-      if (pi == last) {
-        if (!paged && r > 0) pg.patch(tok - 1, sh.k[(r - 1) & 1], sh.v[(r - 1) & 1], lane);  // (per <= 2)
-        pg.patch(tok, sh.k[r & 1], sh.v[r & 1], lane);
-      }
-      st.step(pg, q, min(16, pos + 1 - pi * 16), scale, lane, pi + W < npages ? block(pi + W) : nullptr);
+  for (int e = 0; e < E; ++e) {
+    qwl[e] = __bfloat162float(q_norm[lane * E + e]), qwh[e] = __bfloat162float(q_norm[D / 2 + lane * E + e]);
+    kwl[e] = __bfloat162float(k_norm[lane * E + e]), kwh[e] = __bfloat162float(k_norm[D / 2 + lane * E + e]);
+  }
+  if (threadIdx.x < P / 8) *reinterpret_cast<uint4*>(frame_rows + threadIdx.x * 8) = make_uint4(0u, 0u, 0u, 0u);
+  const bool owned = seq < kv_pages;  // otherwise the row stores nothing: page 0 is somebody's
+  if (!owned && threadIdx.x == 0) raise(err, kErrBadIndex);
+  bf16* const page = kv + kv_offset<D>(owned ? seq : 0, hk, kh, 0, 0);
+  grid_wait();
+
+  constexpr int JOBS = (G + 4 + W - 1) / W;
+  const int jobs = G + 2 + 2 * r, width = (hq + 2 * hk) * D;
+  uint32_t raw[JOBS][2];
+#pragma unroll
+  for (int jj = 0; jj < JOBS; ++jj) {
+    const int job = warp + jj * W, m = job < G + 2 ? n : n - 1, part = job < G + 2 ? job : job - 2;
+    if (job >= jobs) continue;
+    const bf16* row = lookup.table ? lookup.table + (int64_t)__ldcg(lookup.codes + m * 16 + lookup.group) * width : qkv + (int64_t)m * width;
+    ld_halves<D>(row + (part < G ? kh * G + part : part == G ? hq + kh : hq + hk + kh) * D, lane, raw[jj]);
+  }
+  // the tokens that earlier passes wrote
+  for (int i = threadIdx.x; i < 2 * base * (D / 8); i += W * 32) {
+    const int half = i >= base * (D / 8), at = i - half * base * (D / 8), tok = at / (D / 8), c = at % (D / 8) * 8;
+    pattn::cp16(sm100::smem_addr(kvs[half] + tok * P + c), page + (half * 16 + tok) * D + c, true);
+  }
+#pragma unroll
+  for (int jj = 0; jj < JOBS; ++jj) {
+    const int job = warp + jj * W;
+    if (job >= jobs) continue;
+    const bool before = job >= G + 2;
+    const int part = before ? job - 2 : job, tok = before ? pos - 1 : pos;
+    float lo[E], hi[E];
+    widen_halves<D>(raw[jj], lo, hi);
+    if (part < G) rope_head<D>(lo, hi, qwl, qwh, cs, sn, eps);
+    else if (part == G && !before) rope_head<D>(lo, hi, kwl, kwh, cs, sn, eps);
+    else if (part == G) rope_head<D>(lo, hi, kwl, kwh, cs0, sn0, eps);
+    st_half<D>(part < G ? qs + part * P : kvs[part - G] + tok * P, lane, lo, hi);
+    if (part >= G && !before && owned) st_half<D>(page + ((part - G) * 16 + tok) * D, lane, lo, hi);
+  }
+  pattn::cp_commit(), pattn::cp_wait<0>();
+  __syncthreads();
+
+  // S[heads, keys] = q . K^T: two accumulators for each eight keys
+  const int g = lane >> 2, t = lane & 3;
+  // ldmatrix rows of this lane: heads past G and tokens to come are the row of zeros (no value may meet a zero weight as Inf)
+  const int head = lane & 7, k_tok = (lane & 7) + (lane >> 4) * 8, v_tok = lane & 15;
+  const uint32_t q_at = sm100::smem_addr((head < G ? qs + head * P : frame_rows) + (lane >> 3) * 8);
+  const uint32_t k_at = sm100::smem_addr((k_tok <= pos ? kvs[0] + k_tok * P : frame_rows) + ((lane >> 3) & 1) * 8);
+  float s[2][2][4] = {};
+#pragma unroll
+  for (int j = 0; j < D / 32; ++j) {
+    uint32_t a[4];
+    sm100::ldsm4(q_at + j * 64, a);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      uint32_t b[4];
+      sm100::ldsm4(k_at + j * 64 + h * 32, b);
+      sm100::mma_16816(s[0][h], a[2 * h], 0u, a[2 * h + 1], 0u, b[0], b[1]);
+      sm100::mma_16816(s[1][h], a[2 * h], 0u, a[2 * h + 1], 0u, b[2], b[3]);
     }
-    st.finish();
-    const int g = lane >> 2, t = lane & 3;
-    if constexpr (W == 1) {
+  }
+  float p[4], mx = -INFINITY, l = 0.f;  // head g, keys 2 t, 2 t + 1, 2 t + 8, 2 t + 9
 #pragma unroll
-      for (int h = 0; h < 2; ++h)
-        if (2 * t + h < G) {
-          const float inv = 1.f / st.l[h];
+  for (int k = 0; k < 4; ++k) {
+    const int key = 2 * t + (k & 1) + 8 * (k >> 1);
+    p[k] = key <= pos ? (s[k >> 1][0][k & 1] + s[k >> 1][1][k & 1]) * scale : -INFINITY;
+    mx = fmaxf(mx, p[k]);
+  }
+  mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1)), mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
 #pragma unroll
-          for (int i = 0; i < D / 64; ++i) {
-            float v[8];
-            st.dims8(i, h, v);
+  for (int k = 0; k < 4; ++k) p[k] = __expf(p[k] - mx), l += p[k];
+  l += __shfl_xor_sync(0xffffffffu, l, 1), l += __shfl_xor_sync(0xffffffffu, l, 2);
+  uint32_t a0[3], a2[3];
+  split3(p[0], p[1], a0), split3(p[2], p[3], a2);
+  const float inv = 1.f / l;
+
+  // O[heads, dims] = P . V, this warp's quarter of the dims
+  const uint32_t v_at = sm100::smem_addr((v_tok <= pos ? kvs[1] + v_tok * P : frame_rows) + warp * (D / 4) + (lane >> 4) * 8);
+  bf16* const dst = out + ((int64_t)n * hq + kh * G + g) * D + warp * (D / 4) + 2 * t;
 #pragma unroll
-            for (int e = 0; e < 8; ++e) v[e] *= inv;
-            st8(out + ((int64_t)n * hq + kh * G + 2 * t + h) * D + 64 * i + 8 * g, v);
-          }
-        }
-      __syncwarp();  // q is free for the next row
-    } else {
+  for (int i = 0; i < D / 64; ++i) {
+    uint32_t b[4];
+    sm100::ldsm4t(v_at + i * 32, b);
 #pragma unroll
-      for (int h = 0; h < 2; ++h)
-        if (2 * t + h < G) {
-          if (g == 0) merge.m[warp][2 * t + h] = st.m[h], merge.l[warp][2 * t + h] = st.l[h];
+    for (int h = 0; h < 2; ++h) {
+      float o[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-          for (int i = 0; i < D / 64; ++i) {
-            float v[8];
-            st.dims8(i, h, v);
-            float4* dst = reinterpret_cast<float4*>(&merge.o[warp][2 * t + h][64 * i + 8 * g]);
-            dst[0] = make_float4(v[0], v[1], v[2], v[3]), dst[1] = make_float4(v[4], v[5], v[6], v[7]);
-          }
-        }
-      __syncthreads();
-      // a warp per head and 64 dims at a time; lane w has the weight of warp w's state (0 where it held no page)
-      for (int i = warp; i < G * (D / 64); i += W) {
-        const int h = i / (D / 64), d = i % (D / 64) * 64 + 2 * lane;
-        const float mw = lane < W ? merge.m[lane][h] : -INFINITY;
-        const float e = __expf(mw - warp_fmax(mw));
-        const float den = warp_add(lane < W ? e * merge.l[lane][h] : 0.f);
-        float o0 = 0.f, o1 = 0.f;
-#pragma unroll
-        for (int w = 0; w < W; ++w) {
-          const float ew = __shfl_sync(0xffffffffu, e, w);
-          const float2 o = *reinterpret_cast<const float2*>(&merge.o[w][h][d]);
-          o0 += ew * o.x, o1 += ew * o.y;
-        }
-        const float inv = 1.f / den;
-        *reinterpret_cast<__nv_bfloat162*>(out + ((int64_t)n * hq + kh * G + h) * D + d) = __floats2bfloat162_rn(o0 * inv, o1 * inv);
-      }
+      for (int x = 2; x >= 0; --x) sm100::mma_16816(o, a0[x], 0u, a2[x], 0u, b[2 * h], b[2 * h + 1]);
+      if (g < G) *reinterpret_cast<__nv_bfloat162*>(dst + i * 16 + h * 8) = __floats2bfloat162_rn(o[0] * inv, o[1] * inv);
     }
   }
 }
@@ -532,22 +613,24 @@ template <int D, int G>
 static cudaError_t launch_rope_attend_dg(const bf16* qkv, const QkvTable& lookup, const bf16* q_norm, const bf16* k_norm,
                                          bf16* kv, bf16* out, const RowMap& map, int rows, const AttnShape& a,
                                          int kv_pages, int sm_count, uint32_t* err, cudaStream_t s) {
-  const int items = (map.pages ? rows : rows / map.per) * a.kv_heads;
   const float scale = 1.f / sqrtf((float)D);
   if (!map.pages) {
-    if (map.per > 2) return cudaErrorInvalidValue;
-    return launch_pdl(rope_attend_kernel<D, G, 1, 4>, dim3((items + 3) / 4), dim3(128), 0, s, qkv, lookup, q_norm, k_norm, kv, out,
-                      map, items, a.q_heads, a.kv_heads, a.rms_eps, a.rope_theta, scale, kv_pages, err);
+    if (map.per < 1 || map.per > 2 || map.base < 0 || map.base + map.per > 16) return cudaErrorInvalidValue;
+    return launch_pdl(frame_attend_kernel<D, G>, dim3(rows / map.per * a.kv_heads, map.per), dim3(128),
+                      (size_t)(1 + G + 2 * (map.base + map.per)) * (D + 8) * sizeof(bf16), s, qkv, lookup, q_norm, k_norm, kv, out, map.base, a.q_heads, a.kv_heads, a.rms_eps, a.rope_theta, scale, kv_pages, err);
   }
-  if (map.seq) return cudaErrorInvalidValue;  // one row per sequence
+  if (map.seq || lookup.table) return cudaErrorInvalidValue;  // one row per sequence
+  const int items = rows * a.kv_heads;
   auto go = [&](auto kernel, int warps) {
-    return launch_pdl(kernel, dim3(items), dim3(warps * 32), 0, s, qkv, lookup, q_norm, k_norm, kv, out, map, items, a.q_heads,
+    return launch_pdl(kernel, dim3(items), dim3(warps * 32), 0, s, qkv, q_norm, k_norm, kv, out, map, a.q_heads,
                       a.kv_heads, a.rms_eps, a.rope_theta, scale, kv_pages, err);
   };
   // items that leave SMs idle: eight warps each, so that 128 keys are one round (sixteen would have to spill: 2,282 against
-  // 2,242 us a step of one session, 2,133 against 2,042 us for Higgs at three); more items: four warps, three CTAs an SM
-  // (two warps with more CTAs: 4,485 against 4,024 us at 64 sessions, four CTAs an SM with spills 5,655 against 5,228 at 128)
-  return items <= sm_count ? go(rope_attend_kernel<D, G, 8, 1>, 8) : go(rope_attend_kernel<D, G, 4, 1>, 4);
+  // 2,242 us a step of one session, 2,133 against 2,042 us for Higgs at three); more items: four warps, three CTAs an SM, or
+  // three, four CTAs an SM, where that saves a second wave (64 sessions, 512 items: 3,654 against 3,789 us a step; 1,024
+  // items, three waves and two: 5,070 against 5,022)
+  if (items <= sm_count) return go(rope_attend_kernel<D, G, 8>, 8);
+  return items > 3 * sm_count && items <= 4 * sm_count ? go(rope_attend_kernel<D, G, 3>, 3) : go(rope_attend_kernel<D, G, 4>, 4);
 }
 
 template <int D>

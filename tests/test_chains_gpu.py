@@ -132,6 +132,13 @@ def test_decode_attention_in_one_kernel(ops, hq, hk, d, sessions):
     close(a, b, steps=1.5, floor=0.25)
 
 
+# around the counts at which the warps of a team change: 148, 444 and 592 items on 148 SMs
+@pytest.mark.parametrize("items", [147, 149, 443, 445, 500, 591, 593])
+@pytest.mark.parametrize("hq,hk,d", [(2, 1, 128), (4, 1, 64), (5, 1, 128)])
+def test_decode_attention_teams(ops, hq, hk, d, items):
+    test_decode_attention_in_one_kernel(ops, hq, hk, d, items)
+
+
 # two, four and eight columns a thread, rows that end inside a warp of each
 @pytest.mark.parametrize("rows", [9, 250])
 @pytest.mark.parametrize("d", [1984, 2048, 2112, 4096, 4160])
@@ -210,7 +217,7 @@ def test_codec_conv(ops, n, T, C, N, taps, dil, kind):
 
 
 @pytest.mark.parametrize("sessions", [1, 5, 20])
-def test_talker_as_a_chain_agrees_with_per_op_kernels(built_lib, sessions):
+def test_talker_as_a_chain_agrees_with_per_op_kernels(built_lib, sessions, predictor={}):
     """Stacks too large for the L2 run as chains: forced frames give the logits of the per-op kernels."""
     from pega_omni_b200.config import presets
     from pega_omni_b200.model import Draw, Limits, Model, Prompt
@@ -218,7 +225,8 @@ def test_talker_as_a_chain_agrees_with_per_op_kernels(built_lib, sessions):
     base = presets["mid"]()
     cfg = dataclasses.replace(base, talker=dataclasses.replace(base.talker, hidden_size=1024, intermediate_size=3072,
                                                                num_hidden_layers=6, num_attention_heads=16,
-                                                               num_key_value_heads=8, head_dim=128))
+                                                               num_key_value_heads=8, head_dim=128),
+                              predictor=dataclasses.replace(base.predictor, **predictor))
     ck = random_checkpoint(cfg, seed=3, device="cuda")
     rng = np.random.default_rng(sessions)
     lens = [9 + (31 * s) % 90 for s in range(sessions)]
@@ -241,6 +249,12 @@ def test_talker_as_a_chain_agrees_with_per_op_kernels(built_lib, sessions):
     a, b = got
     step = np.exp2(np.floor(np.log2(np.maximum(np.abs(b), 2.0))) - 7)
     assert float((np.abs(a - b) / step).max()) <= 2.0
+
+
+# a frame's attention: head widths and query heads a kv head, one row a sequence and the first two
+@pytest.mark.parametrize("hq,hk,d", [(4, 4, 64), (8, 4, 64), (8, 2, 128), (5, 1, 128), (16, 2, 64)])
+def test_frame_attention_agrees_with_per_op_kernels(built_lib, hq, hk, d):
+    test_talker_as_a_chain_agrees_with_per_op_kernels(built_lib, 19, dict(num_attention_heads=hq, num_key_value_heads=hk, head_dim=d))
 
 
 @pytest.mark.parametrize("bad", [-9, (1 << 20) + 9])  # tokens 7 and 9, which no other row writes
