@@ -51,6 +51,11 @@ struct Chain {
   int* launches = nullptr;
   ChainPlans* plans = nullptr;
   const ChainTrace* trace = nullptr;
+  // The pass's attention keeps its rows in shared memory (frame_attend_kernel): beside a tcgen05 GEMM under the default carve-out
+  // its CTAs find no room before the GEMM ends. One pass, default and whole, us: a talker step of 64 sessions 3,605 and 3,453,
+  // of 128 4,906 and 4,836. The talker's own passes want the L1 that this takes away: their attention holds its pages under
+  // way in registers, 4,836 and 5,170.
+  bool whole_smem = false;
 
   // Behind every launch: counted, and stamped where the program is traced.
   cudaError_t done(cudaError_t launched, const char* what, int N, int K, int rows) const {
@@ -102,7 +107,7 @@ struct Chain {
     const int out = p.few ? p.f.out : p.s.out;
     const char* what = norm.kind ? (out == kStreamSwiglu ? "norm_gemm_swiglu" : "norm_gemm") : out == kStreamSwiglu ? "gemm_swiglu" : "gemm";
     return p.few ? done(few_launch(p.f, norm, err, stream), what, p.f.N, p.f.K, p.f.rows)
-                 : done(stream_launch(p.s, err, stream), what, p.s.N, p.s.K, p.s.rows);
+                 : done(stream_launch(p.s, err, stream, whole_smem), what, p.s.N, p.s.K, p.s.rows);
   }
 };
 
@@ -124,10 +129,11 @@ inline bool chain_supports(int hidden, int inter, int q_width, int head_dim) {
 
 // gate_up(l) and down(l) pick a layer's MLP; `inter` is its width, its gate|up rows lie in groups of kGateGroup.
 template <typename Layer, typename GateUp, typename Down>
-cudaError_t chain_pass(const Chain& c, const std::vector<Layer>& layers, const GateUp& gate_up, const Down& down, int hidden,
+cudaError_t chain_pass(Chain c, const std::vector<Layer>& layers, const GateUp& gate_up, const Down& down, int hidden,
                        int inter, const AttnShape& a, ChainBuffers b, int rows, const RowMap& map,
                        const std::vector<bf16*>& kv, int kv_pages, const bf16* final_gain, bf16* keep_out, int every,
                        int which, const QkvTable& lookup = {}, bool prompt = false) {
+  c.whole_smem = !map.pages;
   const int qd = a.q_heads * a.head_dim, qw = (a.q_heads + 2 * a.kv_heads) * a.head_dim;
   Summands sum;
   FewNorm norm;

@@ -319,7 +319,7 @@ int stream_plan(StreamGemmPlan* plan, const bf16* w, int N, int K, const bf16* x
   return 0;
 }
 
-cudaError_t stream_launch(const StreamGemmPlan& p, uint32_t* err, cudaStream_t stream) {
+cudaError_t stream_launch(const StreamGemmPlan& p, uint32_t* err, cudaStream_t stream, bool whole_smem) {
   StreamArgs a;
   a.y = p.y, a.part = p.part, a.bias = p.epi.bias, a.err = err, a.kind = p.epi.kind;
   a.N = p.N, a.rows = p.rows, a.M = p.M, a.bn = p.bn, a.tn = p.tn, a.splits = p.splits, a.kbs = p.kbs;
@@ -331,9 +331,9 @@ cudaError_t stream_launch(const StreamGemmPlan& p, uint32_t* err, cudaStream_t s
   const size_t smem = std::max<size_t>(kMinSmem, 1024 + (size_t)p.slots * p.kbs * (p.bn + p.tn) * 128 + (size_t)(p.M - p.bn) * 128);
   const dim3 grid((p.N + p.tn - 1) / p.tn, p.splits, (p.rows + 127) / 128);
   switch (p.out) {
-    case kStreamBf16: return launch_pdl(stream_gemm_kernel<0>, grid, dim3(kThreads), smem, stream, p.wmap, p.xmap, a);
-    case kStreamPartials: return launch_pdl(stream_gemm_kernel<1>, grid, dim3(kThreads), smem, stream, p.wmap, p.xmap, a);
-    default: return launch_pdl(stream_gemm_kernel<2>, grid, dim3(kThreads), smem, stream, p.wmap, p.xmap, a);
+    case kStreamBf16: return launch_pdl_smem(whole_smem, stream_gemm_kernel<0>, grid, dim3(kThreads), smem, stream, p.wmap, p.xmap, a);
+    case kStreamPartials: return launch_pdl_smem(whole_smem, stream_gemm_kernel<1>, grid, dim3(kThreads), smem, stream, p.wmap, p.xmap, a);
+    default: return launch_pdl_smem(whole_smem, stream_gemm_kernel<2>, grid, dim3(kThreads), smem, stream, p.wmap, p.xmap, a);
   }
 }
 
