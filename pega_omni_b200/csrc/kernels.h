@@ -26,6 +26,8 @@ struct RowMap {
   const int32_t* seq = nullptr;
   const int32_t* indptr = nullptr;
   const int32_t* pages = nullptr;
+  // one row per sequence: the rows as their attention is to start, the longest first (nullptr: as they are)
+  const int32_t* order = nullptr;
   // dense (pages == nullptr): `per` consecutive rows per sequence at positions
   // base, base+1, ...; sequence s uses page s.
   int per = 1, base = 0;

@@ -401,7 +401,7 @@ __global__ void __launch_bounds__(W * 32, rope_attend_ctas(W))
   __shared__ RopeShared<D> sh;
   __shared__ MergeShared<D, G, W> merge;
   const int lane = threadIdx.x & 31, warp = warp_index();
-  const int n = blockIdx.x / hk, kh = blockIdx.x % hk;
+  const int at = blockIdx.x / hk, n = map.order ? map.order[at] : at, kh = blockIdx.x % hk;
   float qwl[E], qwh[E], kwl[E], kwh[E];
 #pragma unroll
   for (int e = 0; e < E; ++e) {
@@ -618,13 +618,14 @@ __global__ void __launch_bounds__(128)
 
 template <int D, int G>
 static cudaError_t launch_rope_attend_dg(const bf16* qkv, const QkvTable& lookup, const bf16* q_norm, const bf16* k_norm,
-                                         bf16* kv, bf16* out, const RowMap& map, int rows, const AttnShape& a,
+                                         bf16* kv, bf16* out, RowMap map, int rows, const AttnShape& a,
                                          int kv_pages, int sm_count, uint32_t* err, cudaStream_t s) {
   const float scale = 1.f / sqrtf((float)D);
   if (!map.pages) {
     if (map.per < 1 || map.per > 2 || map.base < 0 || map.base + map.per > 16) return cudaErrorInvalidValue;
     return launch_pdl(frame_attend_kernel<D, G>, dim3(rows / map.per * a.kv_heads, map.per), dim3(128),
-                      (size_t)(1 + G + 2 * (map.base + map.per)) * (D + 8) * sizeof(bf16), s, qkv, lookup, q_norm, k_norm, kv, out, map.base, a.q_heads, a.kv_heads, a.rms_eps, a.rope_theta, scale, kv_pages, err);
+                      (size_t)(1 + G + 2 * (map.base + map.per)) * (D + 8) * sizeof(bf16), s, qkv, lookup, q_norm, k_norm, kv, out, map.base,
+                      a.q_heads, a.kv_heads, a.rms_eps, a.rope_theta, scale, kv_pages, err);
   }
   if (map.seq || lookup.table) return cudaErrorInvalidValue;  // one row per sequence
   const int items = rows * a.kv_heads;
@@ -633,11 +634,13 @@ static cudaError_t launch_rope_attend_dg(const bf16* qkv, const QkvTable& lookup
                       a.kv_heads, a.rms_eps, a.rope_theta, scale, kv_pages, err);
   };
   // items that leave SMs idle: eight warps each, so that 128 keys are one round (sixteen would have to spill: 2,282 against
-  // 2,242 us a step of one session, 2,133 against 2,042 us for Higgs at three); more items: four warps, three CTAs an SM, or
-  // three, four CTAs an SM, where that saves a second wave (64 sessions, 512 items: 3,654 against 3,789 us a step; 1,024
-  // items, three waves and two: 5,070 against 5,022)
-  if (items <= sm_count) return go(rope_attend_kernel<D, G, 8>, 8);
-  return items > 3 * sm_count && items <= 4 * sm_count ? go(rope_attend_kernel<D, G, 3>, 3) : go(rope_attend_kernel<D, G, 4>, 4);
+  // 2,242 us a step of one session, 2,133 against 2,042 us for Higgs at three); up to three CTAs an SM, four warps; beyond, three
+  // warps and four CTAs an SM, one wave of 512 items instead of two (64 sessions: 3,416 against 3,513 us a step), and the longest
+  // rows first where there is more than a wave. Prompts of 32 to 512 tokens, four warps as the rows come and this: 80 sessions
+  // 4,418 and 4,256 us, 128 4,747 and 4,697 (four warps in order 4,757, two 4,707).
+  if (items > 3 * sm_count) return go(rope_attend_kernel<D, G, 3>, 3);
+  map.order = nullptr;
+  return items <= sm_count ? go(rope_attend_kernel<D, G, 8>, 8) : go(rope_attend_kernel<D, G, 4>, 4);
 }
 
 template <int D>

@@ -151,7 +151,7 @@ struct omni_talker {
 
   // staged inputs: one host (pinned) block mirrored on the device
   struct Inputs {
-    size_t lines, pos, force, uniforms, indptr, d_pos, d_slot, pages;  // front block: every graph call
+    size_t lines, pos, force, uniforms, indptr, d_pos, d_slot, order, pages;  // front block: every graph call
     size_t t_ids, t_codec, t_pos, t_slot, t_seq, last_row;             // prefill only
     size_t front_fixed_bytes, total_bytes;
   } in;
@@ -484,6 +484,7 @@ int enqueue_advance(omni_talker* m, int b) {
     rows.slot = m->din<int32_t>(m->in.d_slot);
     rows.indptr = m->din<int32_t>(m->in.indptr);
     rows.pages = m->din<int32_t>(m->in.pages);
+    rows.order = m->din<int32_t>(m->in.order);
     return chain_layers(m, m->talker, m->T, b, rows, m->kv, m->pages_total, m->hidden, 1, 0, {}, false);
   }
   LAUNCH(m, launch_frame_embed(slots(m), m->pad_embed, m->codec_emb, c.talker.vocab, m->p_emb, c.predictor.vocab,
@@ -1051,6 +1052,7 @@ void layout_inputs(omni_talker* m) {
   in.indptr = take((B + 1) * 4);
   in.d_pos = take(B * 4);
   in.d_slot = take(B * 4);
+  in.order = take(B * 4);
   in.front_fixed_bytes = at;
   in.pages = take((size_t)m->page_table * 4);
   in.t_ids = take(T * 4);
@@ -1083,6 +1085,7 @@ size_t stage_graph_inputs(omni_talker* m, char* host, const std::vector<FrameRow
   int32_t* indptr = reinterpret_cast<int32_t*>(host + in.indptr);
   int32_t* d_pos = reinterpret_cast<int32_t*>(host + in.d_pos);
   int32_t* d_slot = reinterpret_cast<int32_t*>(host + in.d_slot);
+  int32_t* order = reinterpret_cast<int32_t*>(host + in.order);
   int32_t* pages = reinterpret_cast<int32_t*>(host + in.pages);
   int np = 0;
   indptr[0] = 0;
@@ -1105,6 +1108,8 @@ size_t stage_graph_inputs(omni_talker* m, char* host, const std::vector<FrameRow
     }
     indptr[s + 1] = np;
   }
+  for (int s = 0; s < b; ++s) order[s] = s;
+  std::stable_sort(order, order + b, [&](int x, int y) { return d_pos[x] / OMNI_PAGE > d_pos[y] / OMNI_PAGE; });
   return in.pages + (size_t)np * 4;
 }
 
