@@ -429,120 +429,276 @@ __global__ void __launch_bounds__(kAttendWarps * 32)
   }
 }
 
-// Decode: rotary embedding, FP8 KV write and ring attention of one row per session in one kernel, a CTA of W warps per
-// (session, head). Warps 0, 1 and 2 take the head's query, key and value; meanwhile every warp already has two pages of
-// the ring on their way - the pages earlier ticks filled do not depend on the projection this kernel waits for. The page
-// the row is written to comes last: its writers' stores are fenced for the bulk copy that reads them back.
+// Decode: rotary embedding, FP8 KV write and ring attention of one row per session in one kernel, W warps per (session, head),
+// each on its own pages, which come straight into registers: a page's keys while the values before them are summed, the page
+// behind on its way to L2. FP8 is exact in f16, so a page's products run on m16n8k16:
+//   S[16 keys] = K[16, 128] . q      A = K (one conversion for two values), B = q. Step c of eight has its share of q in column c
+//                                    and zeros elsewhere, so no sum runs through two instructions; the columns are added in f32.
+//   O[dims] += V^T[dims, 16] . p     A = pairs of value rows, B = p in columns 0, 1, 2: three f16 whose sum is all of an f32,
+//                                    scaled by powers of two that keep them clear of f16's range.
+// q is bf16 already; scaled by a power of two so that its largest element is near the top of f16, what it loses is below
+// 2^-38 of that. The lane 4 g + t that a q element belongs to as an operand also rotates it. Every page's products start from
+// zero; maxima, sums and the running output are f32, as in the reference.
+// Two conversions of a word are one asm block: the header's intrinsic gives two 16-bit halves, whose packing cost 110 instructions
+// a page (41.0 us). Calls one behind the other, 64 rows of 32 heads, f32 arithmetic on staged pages and this: 252 keys
+// 43.1 and 30.8 us, 500 keys 74.1 and 51.8, that is 21 us for each further 138 MB (6.6 TB/s); 16 rows of 252 16.5 and 16.2.
+struct RingPage {
+  uint4 k[2][2], v[4];  // keys g, g + 8: 16 values from 64 j + 16 t on; values of keys 2 t, 2 t + 1, 2 t + 8, 2 t + 9 from 16 g on
+  float ks[2], vs[2];   // scales of keys g and g + 8
+  __device__ __forceinline__ void load_k(const uint8_t* blk, int g, int t) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+#pragma unroll
+      for (int j = 0; j < 2; ++j) k[h][j] = __ldcg(reinterpret_cast<const uint4*>(blk + (g + 8 * h) * kHeliumHeadDim + 64 * j + 16 * t));
+      ks[h] = __ldcg(reinterpret_cast<const float*>(blk + 2 * 16 * kHeliumHeadDim) + g + 8 * h);
+    }
+  }
+  __device__ __forceinline__ void load_v(const uint8_t* blk, int g, int t) {
+#pragma unroll
+    for (int r = 0; r < 4; ++r) v[r] = __ldcg(reinterpret_cast<const uint4*>(blk + (16 + 2 * t + (r & 1) + 8 * (r >> 1)) * kHeliumHeadDim + 16 * g));
+#pragma unroll
+    for (int h = 0; h < 2; ++h) vs[h] = __ldcg(reinterpret_cast<const float*>(blk + 2 * 16 * kHeliumHeadDim + 64) + g + 8 * h);
+  }
+};
+
+__device__ __forceinline__ uint32_t ring_word(const uint4& u, int i) { return i == 0 ? u.x : i == 1 ? u.y : i == 2 ? u.z : u.w; }
+// Four e4m3 (a word) as f16: bytes 0, 1 in lo, bytes 2, 3 in hi.
+__device__ __forceinline__ void e4m3_to_f16(uint32_t four, uint32_t& lo, uint32_t& hi) {
+  asm("{\n.reg .b16 l, h;\nmov.b32 {l, h}, %2;\ncvt.rn.f16x2.e4m3x2 %0, l;\ncvt.rn.f16x2.e4m3x2 %1, h;\n}" : "=r"(lo), "=r"(hi) : "r"(four));
+}
+__device__ __forceinline__ uint32_t half_pair(float lo, float hi) {
+  const __half2 h = __floats2half2_rn(lo, hi);
+  return *reinterpret_cast<const uint32_t*>(&h);
+}
+
 template <int W>
-__global__ void __launch_bounds__(W * 32)
+__global__ void __launch_bounds__(W < 4 ? 128 : W * 32, W < 4 ? 4 : 16 / W)
     lm_rope_attend_kernel(const bf16* qkv, void* kv, const int32_t* __restrict__ pos,
                           const int32_t* __restrict__ slots, const int32_t* __restrict__ indptr,
-                          const int32_t* __restrict__ pages, bf16* __restrict__ out, int heads, float coef, float scale,
+                          const int32_t* __restrict__ pages, bf16* __restrict__ out, int items, int heads, float coef, float scale,
                           int context, int kv_pages, uint32_t* err) {
+  constexpr int TEAMS = W < 4 ? 4 / W : 1, WARPS = TEAMS * W, D = kHeliumHeadDim;
   grid_trigger();
-  extern __shared__ __align__(128) unsigned char lra_slots[];
-  __shared__ float q[kHeliumHeadDim], ms[W], ls[W], os[W][kHeliumHeadDim];
-  __shared__ __align__(8) uint64_t bars[W][2];
-  const int n = blockIdx.x, h = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int at = pos[n], len = min(at + 1, context), npages = (len + 15) >> 4, own = (at % context) >> 4;
+  __shared__ alignas(16) uint8_t own_s[TEAMS][2][D];  // the row's own key and value
+  __shared__ float own_scale_s[TEAMS][2];
+  __shared__ float ms[WARPS], ls[WARPS];
+  __shared__ alignas(16) float os[W == 1 ? 1 : WARPS][D];
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3, warp = warp_index() % W, team = warp_index() / W;
+  const int item = blockIdx.x * TEAMS + team;
+  const bool live = item < items;
+  const int n = live ? item / heads : 0, h = live ? item % heads : 0;
+  const int at = pos[n], len = min(at + 1, context), npages = live ? (len + 15) >> 4 : 0, own = (at % context) >> 4;
   const int32_t* my_pages = pages + indptr[n];
   int64_t slot_id = slots[n];
   const bool owned = slot_id >= 0 && (slot_id >> 4) < kv_pages;  // otherwise the row stores nothing: page 0 is some session's
   if (!owned) {
-    if (threadIdx.x == 0) raise(err, kErrBadIndex);
+    if (live && warp == 0 && lane == 0) raise(err, kErrBadIndex);
     slot_id = 0;
   }
-  if (lane == 0) {
-    sm100::mbar_init(sm100::smem_addr(&bars[warp][0]), 1);
-    sm100::mbar_init(sm100::smem_addr(&bars[warp][1]), 1);
-    sm100::mbar_init_fence();
-  }
-  __syncwarp();
-  unsigned char* mine = lra_slots + (size_t)warp * 2 * kAttendSlotBytes;
-  auto page_of = [&](int v) { return v == npages - 1 ? own : v < own ? v : v + 1; };  // the row's own page last
-  auto fetch = [&](int v, int slot) {  // lane 0: one bulk copy of the v-th page's block for this head
-    int64_t page = v == npages - 1 ? slot_id >> 4 : my_pages[page_of(v)];
+  auto block = [&](int pi) -> const uint8_t* {
+    int64_t page = pi == own ? slot_id >> 4 : my_pages[pi];
     if (page < 0 || page >= kv_pages) {
-      raise(err, kErrBadIndex);
+      if (lane == 0) raise(err, kErrBadIndex);
       page = 0;
     }
-    const uint32_t bar = sm100::smem_addr(&bars[warp][slot]);
-    sm100::mbar_expect_tx(bar, kDuplexPageHeadBytes);
-    sm100::bulk_load(sm100::smem_addr(mine + (size_t)slot * kAttendSlotBytes), page_head(kv, page, heads, h), kDuplexPageHeadBytes, bar);
+    return page_head(kv, page, heads, h);
   };
-  if (lane == 0) {
-    if (warp < npages - 1) fetch(warp, 0);
-    if (warp + W < npages - 1) fetch(warp + W, 1);
+  auto ask = [&](int pi) {
+    if (lane == 0 && pi < npages) sm100::prefetch_l2(block(pi), kDuplexPageHeadBytes);
+  };
+  RingPage pg;
+  if (warp < npages) {
+    const uint8_t* first = block(warp);
+    pg.load_k(first, g, t), pg.load_v(first, g, t);
   }
+  ask(warp + W);
+  const int d0 = 64 * (g >> 2) + 16 * t + 4 * (g & 3);  // the four elements of a row this lane takes: step g's
   float cs[2], sn[2];
 #pragma unroll
-  for (int k = 0; k < 2; ++k) sincosf(expf((float)(2 * lane + k) * coef) * (float)at, &sn[k], &cs[k]);
+  for (int k = 0; k < 2; ++k) sincosf(expf((float)(d0 / 2 + k) * coef) * (float)at, &sn[k], &cs[k]);
   grid_wait();
-  if (warp < 3) {
-    const uint2 raw = __ldcg(reinterpret_cast<const uint2*>(qkv + ((int64_t)n * 3 * heads + warp * heads + h) * kHeliumHeadDim) + lane);
+
+  const bool mine = live && own % W == warp;  // the own page is this warp's: so are the row's key and value
+  auto row4 = [&](int part) { return __ldcg(reinterpret_cast<const uint2*>(qkv + ((int64_t)n * 3 * heads + part * heads + h) * D + d0)); };
+  auto widen = [](const uint2& raw, float (&v)[4]) {
     const float2 p0 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.x));
     const float2 p1 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.y));
-    float v[4] = {p0.x, p0.y, p1.x, p1.y};
-    if (warp < 2) {  // pairs (2i, 2i + 1) rotated by angle i
+    v[0] = p0.x, v[1] = p0.y, v[2] = p1.x, v[3] = p1.y;
+  };
+  auto rotate = [&](float (&v)[4]) {  // pairs (2i, 2i + 1) by angle i
 #pragma unroll
-      for (int k = 0; k < 2; ++k) {
-        const float r = v[2 * k], im = v[2 * k + 1];
-        v[2 * k] = r * cs[k] - im * sn[k];
-        v[2 * k + 1] = r * sn[k] + im * cs[k];
-      }
+    for (int k = 0; k < 2; ++k) {
+      const float r = v[2 * k], im = v[2 * k + 1];
+      v[2 * k] = r * cs[k] - im * sn[k];
+      v[2 * k + 1] = r * sn[k] + im * cs[k];
     }
-    if (warp == 0) {
+  };
+  const uint2 raw_q = row4(0);
+  if (mine) {
+    uint2 raw[2] = {row4(1), row4(2)};
 #pragma unroll
-      for (int k = 0; k < 4; ++k) q[lane * 4 + k] = bf16_round(v[k]);
-    } else if (owned) {
+    for (int is_v = 0; is_v < 2; ++is_v) {
+      float v[4];
+      widen(raw[is_v], v);
+      if (!is_v) rotate(v);
       const float amax = warp_fmax(fmaxf(fmaxf(fabsf(v[0]), fabsf(v[1])), fmaxf(fabsf(v[2]), fabsf(v[3]))));
       const float sc = e4m3_scale(amax), inv = 1.f / sc;
-      uint8_t* block = page_head(kv, slot_id >> 4, heads, h);
-      const int tok = (int)(slot_id & 15), is_v = warp - 1;
       const uint32_t lo = __nv_cvt_float2_to_fp8x2(make_float2(v[0] * inv, v[1] * inv), __NV_SATFINITE, __NV_E4M3);
       const uint32_t hi = __nv_cvt_float2_to_fp8x2(make_float2(v[2] * inv, v[3] * inv), __NV_SATFINITE, __NV_E4M3);
-      *reinterpret_cast<uint32_t*>(block + (is_v * 16 + tok) * kHeliumHeadDim + lane * 4) = lo | hi << 16;
-      if (lane == 0) reinterpret_cast<float*>(block + 2 * 16 * kHeliumHeadDim + is_v * 64)[tok] = sc;
-      sm100::fence_async_global();
+      const uint32_t four = lo | hi << 16;
+      *reinterpret_cast<uint32_t*>(&own_s[team][is_v][d0]) = four;
+      if (lane == 0) own_scale_s[team][is_v] = sc;
+      if (owned) {
+        uint8_t* blk = page_head(kv, slot_id >> 4, heads, h);
+        const int tok = (int)(slot_id & 15);
+        *reinterpret_cast<uint32_t*>(blk + (is_v * 16 + tok) * D + d0) = four;
+        if (lane == 0) reinterpret_cast<float*>(blk + 2 * 16 * D + is_v * 64)[tok] = sc;
+      }
     }
+    __syncwarp();
   }
-  __syncthreads();
-  if (lane == 0) {  // the own page, where it is one of the warp's first two
-    if (warp == npages - 1) fetch(warp, 0);
-    else if (warp + W == npages - 1) fetch(warp + W, 1);
+  // the query as the B operand: this lane's four elements are column g of step g
+  uint32_t q0, q1;
+  float q_scale = scale;
+  {
+    float v[4];
+    widen(raw_q, v);
+    rotate(v);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) v[k] = bf16_round(v[k]);
+    const float top = sm100::redux_max(fmaxf(fmaxf(fabsf(v[0]), fabsf(v[1])), fmaxf(fabsf(v[2]), fabsf(v[3]))));
+    // 2^(14 - its exponent), within what f32 can hold; a row of zeros, infinities or NaN as it is
+    const uint32_t e = __float_as_uint(top) >> 23;
+    const bool plain = e < 16 || e > 240;
+    const float up = plain ? 1.f : __uint_as_float((268u - e) << 23);
+    q_scale *= plain ? 1.f : __uint_as_float((e - 14u) << 23);
+    q0 = half_pair(v[0] * up, v[1] * up), q1 = half_pair(v[2] * up, v[3] * up);
   }
-  float m = -INFINITY, l = 0.f, acc[4] = {0.f, 0.f, 0.f, 0.f};
-  const int tok = lane & 15, half = lane >> 4;
-  uint32_t parity[2] = {0, 0};
-  int slot = 0;
-  for (int vi = warp; vi < npages; vi += W, slot ^= 1) {
-    if (!sm100::mbar_wait(sm100::smem_addr(&bars[warp][slot]), parity[slot], err)) {
-      if (vi + W < npages) sm100::mbar_wait(sm100::smem_addr(&bars[warp][slot ^ 1]), parity[slot ^ 1], err);  // nothing may land later
-      break;
+
+  const float w0 = t == 0 ? 1.f : t == 1 ? 0x1p-22f : 0.f, w1 = t == 0 ? 0x1p-11f : 0.f;  // of columns 2 t and 2 t + 1
+  float m = -INFINITY, l = 0.f, acc[16];
+#pragma unroll
+  for (int i = 0; i < 16; ++i) acc[i] = 0.f;
+  for (int pi = warp; pi < npages; pi += W) {
+    ask(pi + 2 * W);
+    const int ntok = min(16, len - pi * 16);
+    if (pi == own) {
+      const int tok = (int)(slot_id & 15);
+#pragma unroll
+      for (int x = 0; x < 2; ++x)
+        if (g + 8 * x == tok) {
+          pg.k[x][0] = *reinterpret_cast<const uint4*>(&own_s[team][0][16 * t]), pg.k[x][1] = *reinterpret_cast<const uint4*>(&own_s[team][0][64 + 16 * t]);
+          pg.ks[x] = own_scale_s[team][0], pg.vs[x] = own_scale_s[team][1];
+        }
+#pragma unroll
+      for (int r = 0; r < 4; ++r)
+        if (2 * t + (r & 1) + 8 * (r >> 1) == tok) pg.v[r] = *reinterpret_cast<const uint4*>(&own_s[team][1][16 * g]);
     }
-    parity[slot] ^= 1u;
-    const unsigned char* blk = mine + (size_t)slot * kAttendSlotBytes;
-    const int ntok = min(16, len - page_of(vi) * 16);
-    page_step(blk, q, ntok, scale, tok, half, lane, m, l, acc);
-    __syncwarp();  // every lane is done with this slot
-    if (lane == 0 && vi + 2 * W < npages) fetch(vi + 2 * W, slot);
-  }
-  if (lane == 0) ms[warp] = m, ls[warp] = l;
+    if (ntok < 16) {  // tokens past the end: whatever lies there must not meet a zero weight as NaN
 #pragma unroll
-  for (int d = 0; d < 4; ++d) os[warp][lane * 4 + d] = acc[d];
-  __syncthreads();
-  for (int d = threadIdx.x; d < kHeliumHeadDim; d += W * 32) {
-    float top = -INFINITY;
+      for (int r = 0; r < 4; ++r)
+        if (2 * t + (r & 1) + 8 * (r >> 1) >= ntok) pg.v[r] = make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll
-    for (int w = 0; w < W; ++w) top = fmaxf(top, ms[w]);
-    float num = 0.f, den = 0.f;
-#pragma unroll
-    for (int w = 0; w < W; ++w) {
-      const float e = ms[w] == -INFINITY ? 0.f : __expf(ms[w] - top);
-      num += os[w][d] * e;
-      den += ls[w] * e;
+      for (int x = 0; x < 2; ++x)
+        if (g + 8 * x >= ntok) pg.vs[x] = 0.f;
     }
-    out[((int64_t)n * heads + h) * kHeliumHeadDim + d] = __float2bfloat16(num / den);
+    float s[2][4] = {};
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+      uint32_t a0, a1, a2, a3;
+      e4m3_to_f16(ring_word(pg.k[0][c >> 2], c & 3), a0, a2), e4m3_to_f16(ring_word(pg.k[1][c >> 2], c & 3), a1, a3);
+      sm100::mma_16816_f16(s[c & 1], a0, a1, a2, a3, g == c ? q0 : 0u, g == c ? q1 : 0u);
+    }
+    float sv[2], p[2];
+#pragma unroll
+    for (int x = 0; x < 2; ++x) {  // key g + 8 x
+      float dot = (s[0][2 * x] + s[0][2 * x + 1]) + (s[1][2 * x] + s[1][2 * x + 1]);
+      dot += __shfl_xor_sync(0xffffffffu, dot, 1);
+      dot += __shfl_xor_sync(0xffffffffu, dot, 2);
+      sv[x] = g + 8 * x < ntok ? dot * (pg.ks[x] * q_scale) : -INFINITY;
+    }
+    const bool more = pi + W < npages;
+    const uint8_t* next = more ? block(pi + W) : nullptr;
+    if (more) pg.load_k(next, g, t);
+    const float m2 = fmaxf(m, sm100::redux_max(fmaxf(sv[0], sv[1]))), corr = __expf(m - m2);
+    p[0] = __expf(sv[0] - m2), p[1] = __expf(sv[1] - m2);
+    l = l * corr + (p[0] + p[1]);
+    m = m2;
+    // weights p * v_scale, times 2^(14 - the largest scale's exponent)
+    const uint32_t ve = max(15u, min(254u, __float_as_uint(sm100::redux_max(fmaxf(pg.vs[0], pg.vs[1]))) >> 23));
+    const float up = __uint_as_float((268u - ve) << 23), down = __uint_as_float((ve - 14u) << 23);
+    const float pv[2] = {p[0] * pg.vs[0] * up, p[1] * pg.vs[1] * up};
+    float x[4];  // of keys 2 t, 2 t + 1, 2 t + 8, 2 t + 9
+#pragma unroll
+    for (int r = 0; r < 4; ++r) x[r] = __shfl_sync(0xffffffffu, pv[r >> 1], 4 * (2 * t + (r & 1)));
+    uint32_t b[2];
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      float y0 = x[2 * half], y1 = x[2 * half + 1];
+      uint32_t piece = 0u;
+#pragma unroll
+      for (int i = 0; i < 3; ++i) {
+        const uint32_t two = half_pair(y0, y1);
+        if (g == i) piece = two;
+        const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&two));
+        y0 = (y0 - f.x) * 2048.f, y1 = (y1 - f.y) * 2048.f;
+      }
+      b[half] = piece;
+    }
+    const float f0 = w0 * down, f1 = w1 * down;
+#pragma unroll
+    for (int w = 0; w < 4; ++w) {
+      const uint32_t u0 = ring_word(pg.v[0], w), u1 = ring_word(pg.v[1], w), u2 = ring_word(pg.v[2], w), u3 = ring_word(pg.v[3], w);
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {  // dims 4 w + 2 half and the next are rows g and g + 8
+        uint32_t a0, a1, a2, a3;
+        e4m3_to_f16(__byte_perm(u0, u1, half ? 0x7362 : 0x5140), a0, a1), e4m3_to_f16(__byte_perm(u2, u3, half ? 0x7362 : 0x5140), a2, a3);
+        float sum[4] = {0.f, 0.f, 0.f, 0.f};
+        sm100::mma_16816_f16(sum, a0, a1, a2, a3, b[0], b[1]);
+#pragma unroll
+        for (int d = 0; d < 2; ++d)
+          acc[4 * w + 2 * half + d] = fmaf(acc[4 * w + 2 * half + d], corr, fmaf(sum[2 * d + 1], f1, sum[2 * d] * f0));
+      }
+    }
+    if (more) pg.load_v(next, g, t);
+  }
+  // the three columns are lanes t = 0 and 1: each adds the other's and takes eight of the sixteen dims
+#pragma unroll
+  for (int o = 4; o < 32; o <<= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
+  float o[8];
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    const float theirs = __shfl_xor_sync(0xffffffffu, t & 1 ? acc[k] : acc[8 + k], 1);
+    o[k] = (t & 1 ? acc[8 + k] : acc[k]) + theirs;
+  }
+  bf16* const dst = out + ((int64_t)n * heads + h) * D;
+  if constexpr (W == 1) {
+    if (!live || t > 1) return;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) o[k] /= l;
+    st8(dst + 16 * g + 8 * t, o);
+  } else {
+    const int w = team * W + warp;
+    if (t < 2) {
+      float4* to = reinterpret_cast<float4*>(&os[w][16 * g + 8 * t]);
+      to[0] = make_float4(o[0], o[1], o[2], o[3]), to[1] = make_float4(o[4], o[5], o[6], o[7]);
+    }
+    if (lane == 0) ms[w] = m, ls[w] = l;
+    __syncthreads();
+    if (!live) return;
+    for (int d = warp * 32 + lane; d < D; d += W * 32) {
+      float top = -INFINITY;
+#pragma unroll
+      for (int x = 0; x < W; ++x) top = fmaxf(top, ms[team * W + x]);
+      float num = 0.f, den = 0.f;
+#pragma unroll
+      for (int x = 0; x < W; ++x) {
+        const float e = ms[team * W + x] == -INFINITY ? 0.f : __expf(ms[team * W + x] - top);
+        num += os[team * W + x][d] * e;
+        den += ls[team * W + x] * e;
+      }
+      dst[d] = __float2bfloat16(num / den);
+    }
   }
 }
 
@@ -886,32 +1042,23 @@ cudaError_t launch_lm_attend(const bf16* qkv, const void* kv, const int32_t* pos
   return launch_pdl(lm_attend_kernel, dim3(rows, heads), dim3(kAttendWarps * 32), smem, s, qkv, kv, pos, seq, indptr, pages, out, heads, scale, context, kv_pages, err);
 }
 
-template <int W>
-static cudaError_t launch_lm_rope_attend_w(const bf16* qkv, void* kv, const int32_t* pos, const int32_t* slots,
-                                           const int32_t* indptr, const int32_t* pages, bf16* out, int rows, int heads,
-                                           float coef, float scale, int context, int kv_pages, uint32_t* err, cudaStream_t s) {
-  constexpr size_t smem = (size_t)W * 2 * kAttendSlotBytes;
-  if (smem > 40 * 1024) {
-    static bool raised[64] = {};  // per device: above the default limit of dynamic shared memory
-    int device = 0;
-    if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= 64) return cudaErrorInvalidDevice;
-    if (!raised[device]) {
-      const cudaError_t e = cudaFuncSetAttribute(lm_rope_attend_kernel<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      if (e != cudaSuccess) return e;
-      raised[device] = true;
-    }
-  }
-  return launch_pdl(lm_rope_attend_kernel<W>, dim3(rows, heads), dim3(W * 32), smem, s, qkv, kv, pos, slots, indptr, pages, out,
-                    heads, coef, scale, context, kv_pages, err);
-}
-
 cudaError_t launch_lm_rope_attend(const bf16* qkv, void* kv, const int32_t* pos, const int32_t* slots,
                                   const int32_t* indptr, const int32_t* pages, bf16* out, int rows, int heads, float coef,
                                   float scale, int context, int kv_pages, int sm_count, uint32_t* err, cudaStream_t s) {
   if (!ring_aligned(qkv, kv)) return cudaErrorInvalidValue;
-  if (rows * heads <= sm_count)  // one CTA per SM at most: more warps of it
-    return launch_lm_rope_attend_w<16>(qkv, kv, pos, slots, indptr, pages, out, rows, heads, coef, scale, context, kv_pages, err, s);
-  return launch_lm_rope_attend_w<4>(qkv, kv, pos, slots, indptr, pages, out, rows, heads, coef, scale, context, kv_pages, err, s);
+  const int items = rows * heads;
+  auto go = [&](auto kernel, int warps) {
+    const int teams = warps < 4 ? 4 / warps : 1;
+    return launch_pdl(kernel, dim3((items + teams - 1) / teams), dim3(teams * warps * 32), 0, s, qkv, kv, pos, slots, indptr, pages, out,
+                      items, heads, coef, scale, context, kv_pages, err);
+  };
+  // As many warps an item as run at once, sixteen an SM: 64 rows of 252 keys 30.8 us with one warp an item, 34.6 with two, 36.9
+  // with four (a merge through shared memory and fewer pages a warp).
+  const int64_t room = (int64_t)16 * sm_count;
+  if (items * 16 <= room) return go(lm_rope_attend_kernel<16>, 16);
+  if (items * 8 <= room) return go(lm_rope_attend_kernel<8>, 8);
+  if (items * 4 <= room) return go(lm_rope_attend_kernel<4>, 4);
+  return items * 2 <= room ? go(lm_rope_attend_kernel<2>, 2) : go(lm_rope_attend_kernel<1>, 1);
 }
 
 cudaError_t launch_lm_dep_embed_norm(const bf16* projected, int k, const bf16* table, int table_rows,

@@ -176,6 +176,12 @@ def test_fp8_ring_attention_in_one_kernel(ops, heads, sessions):
     close(a, b, steps=1.5, floor=0.25)
 
 
+# one, two, four, eight and sixteen warps an item, and a last CTA that is not full
+@pytest.mark.parametrize("heads,sessions", [(4, 296), (1, 1187), (3, 231), (32, 19), (4, 73), (1, 147)])
+def test_fp8_ring_attention_teams(ops, heads, sessions):
+    test_fp8_ring_attention_in_one_kernel(ops, heads, sessions)
+
+
 @pytest.mark.parametrize("vocab", [1, 2047, 2048, 2049, 32768, 40001])
 def test_duplex_sampler_takes_the_largest(ops, vocab):
     """top_k = 1 leaves the largest logit whatever the noise, at both ends of each register budget."""
