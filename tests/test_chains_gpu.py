@@ -57,6 +57,13 @@ def test_chain_gemm(ops, rows, n, k, epilogue):
     assert (y[rows] == 7.0).all()  # nothing past the last row
 
 
+# few rows whose share of a CTA's shared memory, or whose weights, the tcgen05 kernel takes: both sides of either line
+@pytest.mark.parametrize("rows,n,k", [(5, 48, 4288), (5, 48, 4352), (8, 48, 2560), (8, 48, 2752), (8, 48, 11264), (2, 8208, 8192), (3, 8208, 8192),
+                                      (3, 8176, 8192)])
+def test_chain_gemm_of_few_long_rows(ops, rows, n, k):
+    test_chain_gemm(ops, rows, n, k, 0)
+
+
 # the tcgen05 epilogue's fragments: rows that end inside one, columns that leave a warp of a pair without any, one to four sums
 @pytest.mark.parametrize("rows", [10, 24, 25, 57, 73, 121])
 @pytest.mark.parametrize("n,k", [(199, 64), (176, 192), (40, 320), (8, 1024)])
