@@ -4,6 +4,7 @@
 // rows the add + norm is part of the GEMM behind it: five kernels.
 // Op order and rounding points of `Stack::forward` (crates/omni-qwen3/src/stack.rs:152-203).
 #pragma once
+#include <algorithm>
 #include <map>
 #include <tuple>
 #include <vector>
@@ -40,6 +41,7 @@ struct ChainTrace {
   }
 };
 
+constexpr size_t kAheadBytes = 8 << 20;
 constexpr int kChainRows = 256;  // beyond this the GEMMs are contractions, not streams of weights: wide_gemm.h
 
 struct Chain {
@@ -56,6 +58,18 @@ struct Chain {
   // of 128 4,906 and 4,836. The talker's own passes want the L1 that this takes away: their attention holds its pages under
   // way in registers, 4,836 and 5,170.
   bool whole_smem = false;
+
+  // What the next GEMM asks into L2 on its way: the first of the weights that the GEMM behind it reads, whose own requests start
+  // one kernel before they are needed. For passes that leave DRAM idle. One pass without and with 8 MB, us: a talker step of 1
+  // session 1,875 and 1,831, of 8 2,548 and 2,514, of 64 3,456 and 3,394, a start of one prompt 2,697 and 2,650, a duplex tick of
+  // 64 with the depformer's 5,174 and 5,129 (32 MB: 1,865, 2,560, 3,449, 2,662, 5,279). A Higgs step of 3, at half the copy rate,
+  // 1,913 and 1,938, a duplex tick of 1 3,174 and 3,198: none there.
+  size_t ahead_cap = 0;
+  sm100::Ahead ahead;
+  void next(const bf16* w, int N, int K) {
+    ahead.at = reinterpret_cast<const char*>(w);
+    ahead.bytes = w ? (uint32_t)std::min((size_t)N * K * sizeof(bf16), ahead_cap) : 0u;
+  }
 
   // Behind every launch: counted, and stamped where the program is traced.
   cudaError_t done(cudaError_t launched, const char* what, int N, int K, int rows) const {
@@ -106,8 +120,8 @@ struct Chain {
     if (sum) *sum = p.few ? p.f.summands() : p.s.summands();
     const int out = p.few ? p.f.out : p.s.out;
     const char* what = norm.kind ? (out == kStreamSwiglu ? "norm_gemm_swiglu" : "norm_gemm") : out == kStreamSwiglu ? "gemm_swiglu" : "gemm";
-    return p.few ? done(few_launch(p.f, norm, err, stream), what, p.f.N, p.f.K, p.f.rows)
-                 : done(stream_launch(p.s, err, stream, whole_smem), what, p.s.N, p.s.K, p.s.rows);
+    return p.few ? done(few_launch(p.f, norm, err, stream, ahead), what, p.f.N, p.f.K, p.f.rows)
+                 : done(stream_launch(p.s, err, stream, whole_smem, ahead), what, p.s.N, p.s.K, p.s.rows);
   }
 };
 
@@ -150,6 +164,7 @@ cudaError_t chain_pass(Chain c, const std::vector<Layer>& layers, const GateUp& 
   for (size_t i = 0; i < layers.size(); ++i) {
     const Layer& L = layers[i];
     const QkvTable& from = i == 0 ? lookup : QkvTable{};
+    c.next(gate_up(L), 2 * inter, hidden);
     if (i > 0) OMNI_CHAIN(norm_gemm(L.ln1, L.qkv, qw, kStreamBf16, b.qkv, qw));
     else if (!from.table) OMNI_CHAIN(c.gemm(L.qkv, qw, hidden, b.x, rows, kStreamBf16, b.qkv, qw));
     if (prompt) {  // rows of one sequence attend to one another: every key is written before the first is read
@@ -160,8 +175,11 @@ cudaError_t chain_pass(Chain c, const std::vector<Layer>& layers, const GateUp& 
                                        c.stream),
                         "rope_attend", 0, 0, rows));
     }
+    c.next(down(L), inter, hidden);
     OMNI_CHAIN(c.gemm(L.o, hidden, qd, b.attn, rows, kStreamPartials, nullptr, hidden, &sum));
+    c.next(i + 1 < layers.size() ? layers[i + 1].qkv : nullptr, qw, hidden);
     OMNI_CHAIN(norm_gemm(L.ln2, gate_up(L), 2 * inter, kStreamSwiglu, b.act, inter));
+    c.next(i + 1 < layers.size() ? layers[i + 1].o : nullptr, qd, hidden);
     OMNI_CHAIN(c.gemm(down(L), hidden, inter, b.act, rows, kStreamPartials, nullptr, hidden, &sum));
   }
   return c.done(launch_add_norm_sum(sum, b.res, final_gain, keep_out, rows, hidden, a.rms_eps, every, which, c.stream), "add_norm",

@@ -318,7 +318,8 @@ int depformer_step(omni_duplex* m, int n, const int32_t* force, const int32_t* s
   const omni_duplex_config& c = m->cfg;
   const int D = c.dep_dim, H = c.dep_hidden, S = c.max_sessions;
   const float scale = 1.f / std::sqrt((float)kDepHeadDim);
-  const Chain chain = m->chain();
+  Chain chain = m->chain();
+  if (n > kFewRows) chain.ahead_cap = kAheadBytes;
   // the out projections' rows, which the add + norm behind them takes: partial sums up to kChainRows sessions, finished
   // rows beyond (the GEMM of that size makes no partial sums)
   Summands y;
@@ -345,13 +346,21 @@ int depformer_step(omni_duplex* m, int n, const int32_t* force, const int32_t* s
     for (int i = 0; i < c.dep_layers; ++i) {
       const DepLayer& L = m->d[i];
       const bf16* qkv = L.qkv + (size_t)k * 3 * D * D;
+      const bool last = i + 1 == c.dep_layers;  // the next pass has its own weights
+      const DepLayer* Ln = !last ? &m->d[i + 1] : k + 1 < kDepSteps ? &m->d[0] : nullptr;
+      const size_t kn = last ? k + 1 : k;
+      chain.next(L.gate_in + (size_t)k * 2 * H * D, 2 * H, D);
       if (i > 0) DTRY(behind_norm(kNormLm, L.norm1, qkv, 3 * D, kStreamBf16, m->dqkv));
       else DTRY(gemm(m, qkv, 3 * D, D, m->dxn, n, m->dqkv, 3 * D));
       DLAUNCH(m, launch_lm_dep_kv_attend(m->dqkv, m->dkv[i], k, m->dattn, n, c.dep_heads, scale, m->stream));
+      chain.next(L.gate_out + (size_t)k * D * H, D, H);
       DTRY(projected(L.out + (size_t)k * D * D, D, m->dattn));
+      chain.next(Ln ? Ln->qkv + kn * 3 * D * D : nullptr, 3 * D, D);
       DTRY(behind_norm(kNormLm, L.norm2, L.gate_in + (size_t)k * 2 * H * D, 2 * H, kStreamSwiglu, m->dact));
+      chain.next(Ln ? Ln->out + kn * D * D : nullptr, D, D);
       DTRY(projected(L.gate_out + (size_t)k * D * H, H, m->dact));
     }
+    chain.next(nullptr, 0, 0);
     bf16* logits = m->audio_logits + (size_t)k * S * c.card;
     DTRY(behind_norm(kAddLm, nullptr, m->d_heads + (size_t)k * c.card * D, c.card, kStreamBf16, logits));
     DLAUNCH(m, launch_lm_sample(logits, c.card, c.card, c.audio_temperature, c.audio_top_k, force, seeds, 1 + k,

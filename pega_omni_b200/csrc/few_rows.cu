@@ -36,6 +36,7 @@ struct FewArgs {
   const bf16* bias;
   uint32_t* err;
   FewNorm norm;
+  sm100::Ahead ahead;
   float inv_k;
   int N, K, rows, R, slots, ldy, kind, nkb, span, per, xk, lanes_log2, rounds;
 };
@@ -157,6 +158,7 @@ __global__ void __launch_bounds__(kWarps * 32, 2) few_rows_kernel(const __grid_c
     for (int i = 0; i < ahead; ++i) load_w(i, i);
   }
   grid_trigger();
+  if (warp == kWarps - 1 && lane == 0) ask_ahead(a.ahead, blockIdx.y * gridDim.x + blockIdx.x, gridDim.x * gridDim.y);
   __syncwarp();
 
   // ---- everything that does not depend on the rows comes before grid_wait(), the first weights' arrival included ----
@@ -392,12 +394,12 @@ int few_plan(FewPlan* plan, const bf16* w, int N, int K, const bf16* x, int rows
   return tc_encode_bf16(&p.wmap, w, 3, wd, ws, wb) == 0 ? 0 : -4;
 }
 
-cudaError_t few_launch(const FewPlan& p, const FewNorm& norm, uint32_t* err, cudaStream_t stream) {
+cudaError_t few_launch(const FewPlan& p, const FewNorm& norm, uint32_t* err, cudaStream_t stream, const sm100::Ahead& ahead) {
   const int sums = norm.sum.splits;
   if (norm.kind && sums != 1 && sums != 2 && sums != 4) return cudaErrorInvalidValue;
   FewArgs a;
   a.x = p.x, a.y = p.y, a.part = p.part, a.bias = p.epi.bias, a.err = err, a.norm = norm, a.kind = p.epi.kind;
-  a.inv_k = 1.f / (float)p.K;
+  a.inv_k = 1.f / (float)p.K, a.ahead = ahead;
   a.N = p.N, a.K = p.K, a.rows = p.rows, a.R = p.R, a.slots = p.slots, a.ldy = p.ldy;
   a.nkb = p.K / kKb, a.span = few_span(a.nkb, p.splits), a.per = few_per(a.nkb, p.splits), a.xk = p.xk;
   a.lanes_log2 = few_lanes_log2(p.rows), a.rounds = few_rounds(a.nkb, p.splits, p.rows);

@@ -47,6 +47,6 @@ bool few_norm_fits(int K, int rows);
 // Nonzero where the shape is not one of this kernel's. x == nullptr: the rows come from a FewNorm.
 int few_plan(FewPlan* plan, const bf16* w, int N, int K, const bf16* x, int rows, int out, bf16* y, int ldy, float* part,
              Epilogue epi, int sm_count);
-cudaError_t few_launch(const FewPlan& plan, const FewNorm& norm, uint32_t* err, cudaStream_t stream);
+cudaError_t few_launch(const FewPlan& plan, const FewNorm& norm, uint32_t* err, cudaStream_t stream, const sm100::Ahead& ahead = {});
 
 }  // namespace omni

@@ -129,6 +129,16 @@ __device__ __forceinline__ void prefetch_l2(const void* p, uint32_t bytes) {
   asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
 }
 
+// Weights of a later kernel, which a GEMM asks into L2 on its way: CTA `cta` of `ctas` asks for its share.
+struct Ahead {
+  const char* at = nullptr;
+  uint32_t bytes = 0;
+};
+__device__ __forceinline__ void ask_ahead(const Ahead& a, uint32_t cta, uint32_t ctas) {
+  constexpr uint32_t kPiece = 8192;
+  for (uint32_t o = cta * kPiece; o < a.bytes; o += ctas * kPiece) prefetch_l2(a.at + o, min(kPiece, a.bytes - o));
+}
+
 // Between ordinary stores to global memory (another kernel's, ordered before this thread) and the copies above that read
 // them, issued by this thread: the copies are accesses of another proxy. The boundary between two kernels covers them;
 // griddepcontrol.wait is not said to.

@@ -27,6 +27,7 @@ struct StreamArgs {
   float* part;
   const bf16* bias;
   uint32_t* err;
+  sm100::Ahead ahead;
   int N, rows, M, bn, tn, splits, kbs, stages, slots, issuers, ldy, kind, vec;
   uint32_t acc_cols, tmem_cols;
 };
@@ -161,6 +162,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       __syncwarp();
     }
   }
+  else if (warp == 7 && elect_one()) ask_ahead(a.ahead, (blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x, gridDim.x * gridDim.y * gridDim.z);
   __syncwarp();
 
   // ---- epilogue: two warps a TMEM quadrant, sixteen rows at a time as m16n8 fragments, so that every lane has work where
@@ -319,8 +321,9 @@ int stream_plan(StreamGemmPlan* plan, const bf16* w, int N, int K, const bf16* x
   return 0;
 }
 
-cudaError_t stream_launch(const StreamGemmPlan& p, uint32_t* err, cudaStream_t stream, bool whole_smem) {
+cudaError_t stream_launch(const StreamGemmPlan& p, uint32_t* err, cudaStream_t stream, bool whole_smem, const sm100::Ahead& ahead) {
   StreamArgs a;
+  a.ahead = ahead;
   a.y = p.y, a.part = p.part, a.bias = p.epi.bias, a.err = err, a.kind = p.epi.kind;
   a.N = p.N, a.rows = p.rows, a.M = p.M, a.bn = p.bn, a.tn = p.tn, a.splits = p.splits, a.kbs = p.kbs;
   a.stages = p.stages, a.slots = p.slots, a.issuers = p.issuers, a.ldy = p.ldy;

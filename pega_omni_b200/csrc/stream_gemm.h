@@ -8,6 +8,7 @@
 #include <type_traits>
 
 #include "gemm.h"
+#include "sm100.cuh"
 #include "util.cuh"
 
 namespace omni {
@@ -98,6 +99,6 @@ bool stream_supports(int N, int K, int rows);
 constexpr int kGateGroup = 8;
 int stream_plan(StreamGemmPlan* plan, const bf16* w, int N, int K, const bf16* x, int rows, int out, bf16* y, int ldy,
                 float* part, Epilogue epi, int sm_count, int force_splits = 0);
-cudaError_t stream_launch(const StreamGemmPlan& plan, uint32_t* err, cudaStream_t stream, bool whole_smem = false);
+cudaError_t stream_launch(const StreamGemmPlan& plan, uint32_t* err, cudaStream_t stream, bool whole_smem = false, const sm100::Ahead& ahead = {});
 
 }  // namespace omni

@@ -175,8 +175,10 @@ struct omni_talker {
   std::map<std::tuple<const void*, const void*, const void*, int, int>, TcGemmPlan> plans;
   ChainPlans stream_plans;
   Chain chain() {
-    return Chain{stream, err, sm_count, gemm_scratch.partials, gemm_scratch.partial_floats, &launches, &stream_plans,
-                 chain_trace.lines ? &chain_trace : nullptr};
+    Chain c{stream, err, sm_count, gemm_scratch.partials, gemm_scratch.partial_floats, &launches, &stream_plans,
+            chain_trace.lines ? &chain_trace : nullptr};
+    c.ahead_cap = kAheadBytes;
+    return c;
   }
   bool use_chain = false;  // programs run as chains of kernels (chain.h) rather than as the persistent kernel
   std::map<std::pair<int, int>, cudaGraphExec_t> graphs;  // (program, bucket)
