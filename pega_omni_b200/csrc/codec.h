@@ -61,7 +61,6 @@ cudaError_t launch_codec_add_norm(const bf16* add, int64_t add_stride, bf16* res
                                   int dim, float eps, cudaStream_t stream);
 cudaError_t launch_codec_window_attend(const bf16* qkv, CodecStateRef st, int64_t ring_offset, bf16* out, int n, int heads,
                                        float theta, cudaStream_t stream);
-cudaError_t launch_codec_silu_mul(const bf16* gate_up, bf16* out, int rows, int inter, cudaStream_t stream);
 cudaError_t launch_codec_bias_gelu(bf16* x, const bf16* bias, int64_t rows, int cols, cudaStream_t stream);
 cudaError_t launch_codec_bias_snake(const bf16* x, const bf16* bias, const float* alpha, const float* inv_b, bf16* out,
                                     int64_t rows, int cols, cudaStream_t stream);

@@ -171,21 +171,6 @@ __global__ void __launch_bounds__(kWindowWarps * 32)
   }
 }
 
-__global__ void codec_silu_mul_kernel(const bf16* gate_up, bf16* __restrict__ out, int inter, int64_t total) {
-  grid_trigger();
-  grid_wait();
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= total) return;
-  const int per = inter / 8;
-  const int64_t r = i / per, c = i % per * 8;
-  float g[8], u[8];
-  ld8cg(gate_up + r * 2 * inter + c, g);
-  ld8cg(gate_up + r * 2 * inter + inter + c, u);
-#pragma unroll
-  for (int k = 0; k < 8; ++k) g[k] = bf16_round(g[k] / (1.f + __expf(-g[k]))) * u[k];
-  st8v(out + i * 8, g);
-}
-
 __global__ void codec_bias_gelu_kernel(bf16* x, const bf16* __restrict__ bias, int cols, int64_t total) {
   grid_trigger();
   grid_wait();
@@ -454,11 +439,6 @@ cudaError_t launch_codec_add_norm(const bf16* add, int64_t add_stride, bf16* res
 cudaError_t launch_codec_window_attend(const bf16* qkv, CodecStateRef st, int64_t ring_offset, bf16* out, int n, int heads,
                                        float theta, cudaStream_t stream) {
   return launch_pdl(codec_window_attend_kernel, dim3(n, heads), dim3(kWindowWarps * 32), 0, stream, qkv, st, ring_offset, out, heads, theta);
-}
-
-cudaError_t launch_codec_silu_mul(const bf16* gate_up, bf16* out, int rows, int inter, cudaStream_t stream) {
-  const int64_t total = (int64_t)rows * inter / 8;
-  return launch_pdl(codec_silu_mul_kernel, dim3(blocks_for(total, 256)), dim3(256), 0, stream, gate_up, out, inter, total);
 }
 
 cudaError_t launch_codec_bias_gelu(bf16* x, const bf16* bias, int64_t rows, int cols, cudaStream_t stream) {

@@ -324,8 +324,12 @@ int load_weights(omni_codec* m, const Index& idx) {
     CTRY(put(m, ln2, &L.ln2));
     CTRY(fetch(m, idx, q + "mlp.gate_proj.weight", {inter, h}, &gate));
     CTRY(fetch(m, idx, q + "mlp.up_proj.weight", {inter, h}, &up));
-    gate.insert(gate.end(), up.begin(), up.end());
-    CTRY(put(m, gate, &L.gate_up));
+    Vec grouped;  // as the SwiGLU epilogue wants them: eight gate rows, their eight up rows, the next eight
+    for (size_t at = 0, run = (size_t)kGateGroup * h; at < gate.size(); at += run) {
+      grouped.insert(grouped.end(), gate.begin() + at, gate.begin() + at + run);
+      grouped.insert(grouped.end(), up.begin() + at, up.begin() + at + run);
+    }
+    CTRY(put(m, grouped, &L.gate_up));
     CTRY(fetch(m, idx, q + "mlp.down_proj.weight", {h, inter}, &down));
     CTRY(fetch(m, idx, q + "mlp_layer_scale.scale", {h}, &sm));
     CTRY(put(m, scale_rows(down, sm), &L.down));
@@ -489,17 +493,52 @@ int enqueue_frame(omni_codec* m, int n) {
   CTRY(dense(m, m->pre_w, lat, 3 * dim, COL, n, B));
   CTRY(dense(m, m->in_w, h, lat, B, n, RES));
   CLAUNCH(m, launch_codec_add_norm(m->in_b, 0, RES, m->ln1_0, X, n, h, c.rms_norm_eps, s));
-  for (const TLayer& L : m->layers) {
-    CTRY(dense(m, L.qkv, 3 * qd, h, X, n, COL));
+  // A layer is a chain's: the out projections leave partial sums (finished rows beyond kChainRows streams) for the add + norm
+  // behind them, which for a few streams is part of the next GEMM, as SwiGLU is of its own. A frame with a kernel for each op
+  // and this, us: 1 stream 475 and 429, 8 590 and 531, 16 708 and 656, 64 1,146 and 1,129.
+  Chain chain = m->chain();
+  chain.ahead_cap = kAheadBytes;
+  Summands y;
+  bf16 *res = RES, *spare = PAD;
+  FewNorm norm;
+  norm.kind = kNormStack, norm.eps = c.rms_norm_eps;
+  auto projected = [&](const bf16* w, int K, const bf16* x) -> int {
+    if (n <= kChainRows) {
+      CCUDA(m, chain.gemm(w, h, K, x, n, kStreamPartials, nullptr, h, &y));
+    } else {
+      CCUDA(m, chain.gemm(w, h, K, x, n, kStreamBf16, X, h));
+      y.done = X, y.splits = 0, y.ld = h;
+    }
+    return OMNI_OK;
+  };
+  auto behind_norm = [&](const bf16* gain, const bf16* w, int N, int out, bf16* to) -> int {
+    norm.sum = y, norm.gain = gain;
+    CCUDA(m, chain.norm_gemm(norm, &res, &spare,
+                             [&](const Summands& from, bf16* rows) { return launch_add_norm_sum(from, rows, gain, X, n, h, c.rms_norm_eps, 1, 0, s); },
+                             w, N, h, X, n, out, to, out == kStreamSwiglu ? N / 2 : N));
+    return OMNI_OK;
+  };
+  for (size_t i = 0; i < m->layers.size(); ++i) {
+    const TLayer& L = m->layers[i];
+    const TLayer* Ln = i + 1 < m->layers.size() ? &L + 1 : nullptr;
+    chain.next(L.gate_up, 2 * inter, h);
+    if (i > 0) CTRY(behind_norm((&L - 1)->next, L.qkv, 3 * qd, kStreamBf16, COL));
+    else CTRY(dense(m, L.qkv, 3 * qd, h, X, n, COL));
     CLAUNCH(m, launch_codec_window_attend(COL, st, L.ring, A, n, c.num_attention_heads, c.rope_theta, s));
-    CTRY(dense(m, L.o, h, qd, A, n, X));
-    CLAUNCH(m, launch_codec_add_norm(X, h, RES, L.ln2, X, n, h, c.rms_norm_eps, s));
-    CTRY(dense(m, L.gate_up, 2 * inter, h, X, n, COL));
-    CLAUNCH(m, launch_codec_silu_mul(COL, A, n, inter, s));
-    CTRY(dense(m, L.down, h, inter, A, n, X));
-    CLAUNCH(m, launch_codec_add_norm(X, h, RES, L.next, X, n, h, c.rms_norm_eps, s));
+    chain.next(L.down, h, inter);
+    CTRY(projected(L.o, qd, A));
+    chain.next(Ln ? Ln->qkv : m->out_w, Ln ? 3 * qd : lat, h);
+    if (n <= kFewRows) {
+      CTRY(behind_norm(L.ln2, L.gate_up, 2 * inter, kStreamSwiglu, A));
+    } else {  // (a frame of many streams is 134 kernels, which its statistics report and tests hold)
+      CTRY(behind_norm(L.ln2, L.gate_up, 2 * inter, kStreamBf16, COL));
+      CLAUNCH(m, launch_silu_mul(COL, A, n, inter, kGateGroup, s));
+    }
+    chain.next(Ln ? Ln->o : nullptr, h, qd);
+    CTRY(projected(L.down, inter, A));
   }
-  CTRY(dense(m, m->out_w, lat, h, X, n, A));
+  chain.next(nullptr, 0, 0);
+  CTRY(behind_norm(m->layers.back().next, m->out_w, lat, kStreamBf16, A));
   bf16 *cur = A, *tmp = B;
   int t = 1;
   for (int i = 0; i < c.n_upsampling_ratios; ++i) {
