@@ -112,7 +112,12 @@ struct Chain {
     if (it != plans->end()) return &it->second;
     ChainPlan p;
     p.few = few_plan(&p.f, w, N, K, x, rows, out, y, ldy, partials, epi, sm_count) == 0;
-    if (!p.few && (!x || stream_plan(&p.s, w, N, K, x, rows, out, y, ldy, partials, epi, sm_count) != 0)) return nullptr;
+    if (!p.few) {  // what the tcgen05 kernel cannot take (stores, columns or sums of its own) stays with the other one
+      const bool streams = x && stream_plan(&p.s, w, N, K, x, rows, out, y, ldy, partials, epi, sm_count) == 0 &&
+                           (out != kStreamPartials || p.s.partial_floats() <= partial_floats);
+      p.few = !streams && few_plan(&p.f, w, N, K, x, rows, out, y, ldy, partials, epi, sm_count, true) == 0;
+      if (!streams && !p.few) return nullptr;
+    }
     if (out == kStreamPartials && (p.few ? p.f.partial_floats() : p.s.partial_floats()) > partial_floats) return nullptr;
     return &plans->emplace(key, p).first->second;
   }

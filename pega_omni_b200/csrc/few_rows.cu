@@ -358,7 +358,7 @@ static FewShape few_shape(int N, int K, int rows, int R, int splits, int sm_coun
 }
 
 int few_plan(FewPlan* plan, const bf16* w, int N, int K, const bf16* x, int rows, int out, bf16* y, int ldy, float* part,
-             Epilogue epi, int sm_count) {
+             Epilogue epi, int sm_count, bool any_shape) {
   if (rows < 1 || rows > kFewRows || K % kKb || N < 1) return -2;
   if (!x && !few_norm_fits(K, rows)) return -2;
   if (out == kStreamSwiglu && N % (2 * kGateGroup)) return -2;
@@ -385,7 +385,7 @@ int few_plan(FewPlan* plan, const bf16* w, int N, int K, const bf16* x, int rows
   // one: 8 rows of 12,288 x 4,096 (32 layers) -103, 22,528 x 4,096 -314, 4,096 x 11,264 -109, but 2,560 x 9,728 (36) +129,
   // 19,456 x 2,560 -6; 4 rows of 22,528 x 4,096 -108, but 12,288 x 4,096 +111; 1 row of 22,528 x 4,096 +97.
   const size_t x_share = (size_t)few_per(K / kKb, best.splits) * kKb * kWarps * rows * 2;
-  if (x && (x_share > 42 * 1024 || (rows > 2 && (int64_t)N * K > 64 << 20))) return -2;
+  if (x && !any_shape && (x_share > 42 * 1024 || (rows > 2 && (int64_t)N * K > 64 << 20))) return -2;
   p.R = best.R, p.splits = best.splits, p.slots = best.slots, p.smem = best.smem;
   p.xk = few_per(K / kKb, p.splits) * kKb + 8;
   const int nkb = K / kKb;

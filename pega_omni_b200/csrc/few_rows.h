@@ -44,9 +44,10 @@ constexpr int kFewRows = 8;  // one tile of m16n8k16; beyond, the tcgen05 kernel
 void few_configure();
 // Whether the norm of `rows` rows of K elements can be made by every CTA of the projection.
 bool few_norm_fits(int K, int rows);
-// Nonzero where the shape is not one of this kernel's. x == nullptr: the rows come from a FewNorm.
+// Nonzero where the shape is not one of this kernel's, or (any_shape: taken all the same) is left to stream_gemm.h. x == nullptr:
+// the rows come from a FewNorm.
 int few_plan(FewPlan* plan, const bf16* w, int N, int K, const bf16* x, int rows, int out, bf16* y, int ldy, float* part,
-             Epilogue epi, int sm_count);
+             Epilogue epi, int sm_count, bool any_shape = false);
 cudaError_t few_launch(const FewPlan& plan, const FewNorm& norm, uint32_t* err, cudaStream_t stream, const sm100::Ahead& ahead = {});
 
 }  // namespace omni

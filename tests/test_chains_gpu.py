@@ -64,6 +64,18 @@ def test_chain_gemm_of_few_long_rows(ops, rows, n, k):
     test_chain_gemm(ops, rows, n, k, 0)
 
 
+@pytest.mark.parametrize("k", [64, 4096])
+def test_swiglu_of_few_long_rows_at_any_address(ops, k):
+    """The tcgen05 kernel refuses an activation row that vector stores cannot take: few rows stay with the other one."""
+    w, x = rand((64, k), 51, k ** -0.5), rand((8, k), 52)
+    y = torch.zeros(8 * 32 + 1, dtype=torch.bfloat16, device="cuda")[1:].view(8, 32)
+    torch.cuda.synchronize()
+    ops.chain_gemm(w, x, y, swiglu=True)
+    ops.sync()
+    gate, up = product(x, w[:32]).bfloat16().float(), product(x, w[32:]).bfloat16().float()
+    close(y, torch.nn.functional.silu(gate).bfloat16().float() * up, steps=3.0)
+
+
 # the tcgen05 epilogue's fragments: rows that end inside one, columns that leave a warp of a pair without any, one to four sums
 @pytest.mark.parametrize("rows", [10, 24, 25, 57, 73, 121])
 @pytest.mark.parametrize("n,k", [(199, 64), (176, 192), (40, 320), (8, 1024)])
