@@ -567,11 +567,11 @@ __global__ void __launch_bounds__(W < 4 ? 128 : W * 32, W < 4 ? 4 : 16 / W)
 #pragma unroll
     for (int k = 0; k < 4; ++k) v[k] = bf16_round(v[k]);
     const float top = sm100::redux_max(fmaxf(fmaxf(fabsf(v[0]), fabsf(v[1])), fmaxf(fabsf(v[2]), fabsf(v[3]))));
-    // 2^(14 - its exponent), within what f32 can hold; a row of zeros, infinities or NaN as it is
-    const uint32_t e = __float_as_uint(top) >> 23;
-    const bool plain = e < 16 || e > 240;
-    const float up = plain ? 1.f : __uint_as_float((268u - e) << 23);
-    q_scale *= plain ? 1.f : __uint_as_float((e - 14u) << 23);
+    // times 2^(14 - the largest element's exponent); below 2^-112 the factor stays 2^126, where f16 holds every bf16, and
+    // infinities and NaN stay what they are
+    const uint32_t e = max(15u, min(254u, __float_as_uint(top) >> 23));
+    const float up = __uint_as_float((268u - e) << 23);
+    q_scale *= __uint_as_float((e - 14u) << 23);
     q0 = half_pair(v[0] * up, v[1] * up), q1 = half_pair(v[2] * up, v[3] * up);
   }
 

@@ -201,6 +201,31 @@ def test_fp8_ring_attention_teams(ops, heads, sessions):
     test_fp8_ring_attention_in_one_kernel(ops, heads, sessions)
 
 
+@pytest.mark.parametrize("top", [2.0 ** -130, 2.0 ** -113, 2.0 ** -112, 1.5 * 2.0 ** 113, 2.0 ** 114, 2.0 ** 115])
+def test_fp8_ring_attention_of_a_query_of_any_size(ops, top):
+    """Queries whose largest element is near either end of f32: the sums of the scalar kernel are finite, and so are these."""
+    heads, sessions, per, context = 4, 3, 2, 32
+    at, table, indptr = i32([7, 31, 50]), i32([4, 1, 0, 2, 5, 3]), i32([0, 2, 4, 6])
+    slot = i32([4 * 16 + 7, 2 * 16 + 15, 3 * 16 + 2])
+    kv = torch.zeros(sessions * per, heads, 2 * 16 * 128 + 2 * 16 * 4, dtype=torch.uint8, device="cuda")
+    kv[:, :, :4096] = (rand((sessions * per, heads, 4096), 131).float() * 0.5).to(torch.float8_e4m3fn).view(torch.uint8)
+    kv[:, :, 4096:] = torch.full((sessions * per, heads, 32), 0.01, device="cuda").view(torch.uint8)
+    x = torch.randn((sessions, 3 * heads * 128), generator=torch.Generator().manual_seed(7)).clamp(-2, 2)
+    q = x[:, :heads * 128].view(sessions, heads, 64, 2)
+    q[:, :, 5] = torch.tensor([4.0, 0.0])
+    q *= top / 4.0  # rotation keeps a pair's length: 2^0 to 2^-0.5 of it is in its larger element
+    qkv = x.to(torch.bfloat16).cuda()
+    qkv_b, kv_b = qkv.clone(), kv.clone()
+    a, b = (torch.zeros((sessions, heads * 128), dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    torch.cuda.synchronize()
+    coef = float(np.float32(-np.log(10000.0) * 2.0 / 128))
+    ops.lm_decode_attend(qkv, kv, sessions * per, at, slot, indptr, table, heads, coef, 128 ** -0.5, context, a)
+    ops.lm_rope_attend(qkv_b, kv_b, sessions * per, at, slot, None, indptr, table, heads, coef, 128 ** -0.5, context, b)
+    ops.sync()
+    assert torch.equal(kv, kv_b) and torch.isfinite(b.float()).all()
+    close(a, b, steps=1.5, floor=1e-3)
+
+
 @pytest.mark.parametrize("vocab", [1, 2047, 2048, 2049, 32768, 40001])
 def test_duplex_sampler_takes_the_largest(ops, vocab):
     """top_k = 1 leaves the largest logit whatever the noise, at both ends of each register budget."""
