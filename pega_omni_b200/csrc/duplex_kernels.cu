@@ -1053,12 +1053,13 @@ cudaError_t launch_lm_rope_attend(const bf16* qkv, void* kv, const int32_t* pos,
                       items, heads, coef, scale, context, kv_pages, err);
   };
   // As many warps an item as run at once, sixteen an SM: 64 rows of 252 keys 30.8 us with one warp an item, 34.6 with two, 36.9
-  // with four (a merge through shared memory and fewer pages a warp).
+  // with four (a merge through shared memory and fewer pages a warp). One warp stores 16 bytes a lane, so rows at addresses that
+  // do not take them have two.
   const int64_t room = (int64_t)16 * sm_count;
   if (items * 16 <= room) return go(lm_rope_attend_kernel<16>, 16);
   if (items * 8 <= room) return go(lm_rope_attend_kernel<8>, 8);
   if (items * 4 <= room) return go(lm_rope_attend_kernel<4>, 4);
-  return items * 2 <= room ? go(lm_rope_attend_kernel<2>, 2) : go(lm_rope_attend_kernel<1>, 1);
+  return items * 2 <= room || (reinterpret_cast<uintptr_t>(out) & 15) ? go(lm_rope_attend_kernel<2>, 2) : go(lm_rope_attend_kernel<1>, 1);
 }
 
 cudaError_t launch_lm_dep_embed_norm(const bf16* projected, int k, const bf16* table, int table_rows,

@@ -201,6 +201,24 @@ def test_fp8_ring_attention_teams(ops, heads, sessions):
     test_fp8_ring_attention_in_one_kernel(ops, heads, sessions)
 
 
+# sixteen, eight, four, two warps an item and one, which stores whole rows as vectors where it may
+@pytest.mark.parametrize("per_sm", [1, 2, 4, 8, 9])
+def test_fp8_ring_attention_into_rows_at_any_address(ops, per_sm):
+    sessions, context = per_sm * torch.cuda.get_device_properties(0).multi_processor_count, 16
+    kv = torch.zeros(sessions, 1, 2 * 16 * 128 + 2 * 16 * 4, dtype=torch.uint8, device="cuda")
+    qkv, table = rand((sessions, 3 * 128), 141), i32(list(range(sessions)))
+    at, slot, indptr = i32([3] * sessions), i32([16 * s + 3 for s in range(sessions)]), i32(list(range(sessions + 1)))
+    outs = []
+    for offset in (0, 1):
+        out = torch.zeros(sessions * 128 + 1, dtype=torch.bfloat16, device="cuda")[offset:offset + sessions * 128].view(sessions, 128)
+        torch.cuda.synchronize()
+        ops.lm_decode_attend(qkv, kv, sessions, at, slot, indptr, table, 1, -0.14, 0.1, context, out)
+        ops.sync()
+        outs.append(out)
+    close(outs[1], outs[0], steps=1.0, floor=1e-3)  # (one warp's sums merged by two)
+    assert outs[0].any()
+
+
 @pytest.mark.parametrize("top", [2.0 ** -130, 2.0 ** -113, 2.0 ** -112, 1.5 * 2.0 ** 113, 2.0 ** 114, 2.0 ** 115])
 def test_fp8_ring_attention_of_a_query_of_any_size(ops, top):
     """Queries whose largest element is near either end of f32: the sums of the scalar kernel are finite, and so are these."""
