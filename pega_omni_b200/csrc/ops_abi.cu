@@ -34,8 +34,8 @@ struct omni_ops {
 };
 
 // Nothing of the next launch starts before everything in front of it in the stream has ended. Attention kernels ask for their
-// pages, GEMMs for their weights before they wait for the kernel in front of them, because no other kernel of a model's call
-// writes those; calls made one by one here may.
+// pages, GEMMs for their weights and biases before they wait for the kernel in front of them, because no other kernel of a
+// model's call writes those; calls made one by one here may.
 __global__ void order_kernel() {}
 static cudaError_t order(cudaStream_t s) {
   order_kernel<<<1, 1, 0, s>>>();
@@ -232,6 +232,7 @@ int32_t omni_op_chain_gemm(omni_ops* c, const void* w, int32_t N, int32_t K, con
   if (!swiglu) {
     Epilogue epi;
     epi.bias = static_cast<const bf16*>(bias), epi.kind = epilogue;
+    OPS_CUDA(c, order(c->stream));
     OPS_CUDA(c, chain.gemm((const bf16*)w, N, K, (const bf16*)x, rows, kStreamBf16, (bf16*)y, ldy, nullptr, 0, epi));
     return OMNI_OK;
   }
@@ -255,6 +256,7 @@ int32_t omni_op_chain_norm_gemm(omni_ops* c, const void* w1, int32_t D, int32_t 
   int launches = 0;
   ChainPlans plans;
   const Chain chain{c->stream, c->err, c->sm_count, c->scratch.partials, c->scratch.partial_floats, &launches, &plans};
+  OPS_CUDA(c, order(c->stream));
   bf16* tmp = nullptr;  // the rows of a norm of its own, the other residual of a folded one
   const size_t row_bytes = (size_t)rows * D * sizeof(bf16);
   OPS_CUDA(c, cudaMalloc((void**)&tmp, 2 * row_bytes));
@@ -499,6 +501,7 @@ int32_t omni_op_codec_conv(omni_ops* c, const void* w, int32_t N, int32_t C, int
   const int rc = conv_plan(&plan, (const bf16*)w, N, C, taps, dil, (const bf16*)padded, T, n_streams, (bf16*)y, epilogue,
                            (const bf16*)bias, alpha, inv_b, c->sm_count);
   if (rc != 0) return c->fail(OMNI_ERR_UNSUPPORTED, "conv plan refused (%d): N=%d C=%d taps=%d T=%d", rc, N, C, taps, T);
+  OPS_CUDA(c, order(c->stream));
   OPS_CUDA(c, conv_launch(plan, c->err, c->stream));
   return OMNI_OK;
 }

@@ -57,6 +57,23 @@ def test_chain_gemm(ops, rows, n, k, epilogue):
     assert (y[rows] == 7.0).all()  # nothing past the last row
 
 
+def test_a_gemm_waits_for_the_call_that_makes_its_bias(ops):
+    """The second call's bias is the first one's output, which takes a few CTAs some time; nobody waits in between."""
+    w1, x1, w2, x2 = rand((64, 32768), 151, 32768 ** -0.5), rand((16, 32768), 152), rand((64, 64), 153, 0.125), rand((16, 64), 154)
+    outs = []
+    for wait in (True, False):
+        made = torch.zeros((16, 64), dtype=torch.bfloat16, device="cuda")
+        y = torch.zeros((16, 64), dtype=torch.bfloat16, device="cuda")
+        torch.cuda.synchronize()
+        ops.chain_gemm(w1, x1, made)
+        if wait:
+            ops.sync()
+        ops.chain_gemm(w2, x2, y, bias=made[15], epilogue=1)
+        ops.sync()
+        outs.append(y)
+    assert torch.equal(outs[0], outs[1])
+
+
 # few rows whose share of a CTA's shared memory, or whose weights, the tcgen05 kernel takes: both sides of either line
 @pytest.mark.parametrize("rows,n,k", [(5, 48, 4288), (5, 48, 4352), (8, 48, 2560), (8, 48, 2752), (8, 48, 11264), (2, 8208, 8192), (3, 8208, 8192),
                                       (3, 8176, 8192)])
