@@ -212,7 +212,7 @@ def test_fp8_ring_attention_in_one_kernel(ops, heads, sessions):
     close(a, b, steps=1.5, floor=0.25)
 
 
-# one, two, four, eight and sixteen warps an item, and a last CTA that is not full
+# one, two, eight and sixteen warps an item, and a last CTA that is not full (four, and more than one page a warp: further down)
 @pytest.mark.parametrize("heads,sessions", [(4, 296), (1, 1187), (3, 231), (32, 19), (4, 73), (1, 147)])
 def test_fp8_ring_attention_teams(ops, heads, sessions):
     test_fp8_ring_attention_in_one_kernel(ops, heads, sessions)
@@ -464,6 +464,68 @@ def test_swiglu_of_every_gate(ops, rows):
     assert int((y[0] != want.to(torch.bfloat16)).sum()) <= 1
     # half a bf16 step of the value and 2^-22 of it for the f32 arithmetic; below the smallest normal f32 a step is fixed
     assert ((y[0].double() - want).abs() <= want.abs() * (2.0 ** -8 + 2.0 ** -22) + 2.0 ** -134).all()
+
+
+def ring64(q, kv, pages, length, heads, scale):
+    """One row of the FP8 ring in float64, from the bf16 query and the bytes and scales the kernels read."""
+    block = kv[pages.long()].view(-1, heads, 2 * 16 * 128 + 2 * 16 * 4)
+    byte = block[:, :, :4096].reshape(-1, heads, 2, 16, 128).view(torch.float8_e4m3fn).double()
+    scales = block[:, :, 4096:].contiguous().view(torch.float32).view(-1, heads, 2, 16).double()
+    k, v = ((byte[:, :, i] * scales[:, :, i, :, None]).permute(1, 0, 2, 3).reshape(heads, -1, 128)[:, :length] for i in range(2))
+    p = torch.softmax(torch.einsum("hd,hld->hl", q.double().reshape(heads, 128), k) * scale, -1)
+    return torch.einsum("hl,hld->hd", p, v).reshape(heads * 128)
+
+
+# Both sides of the item counts at which the warps an item change (16, 8, 4, 2 and 1 of them, from few items to many), a last CTA
+# that is not full among them. Full rings are 63 pages, so that every warp of sixteen takes three at least; the row's own page is
+# the first, one in the middle and the last, of rings that are not full, full and wrapped. Token scales differ by 2^9 (keys, which
+# keeps the scores below ten, as f32 sums need) and 2^16 (values); what lies behind a row's end is NaN; some queries are zero.
+@pytest.mark.parametrize("heads", [1, 4])
+@pytest.mark.parametrize("per_sm,more", [(1, 0), (1, 1), (2, 0), (2, 1), (4, 0), (4, 1), (8, 0), (8, 1)])
+def test_fp8_ring_attention_keeps_f32_weights(ops, per_sm, more, heads):
+    context, per = 1000, 63
+    sessions = per_sm * torch.cuda.get_device_properties(0).multi_processor_count // heads + more
+    rng = np.random.default_rng(sessions)
+    table = rng.permutation(sessions * per).reshape(sessions, per)
+    at = [[0, 5, 15, 16, 40, 255, 256, 500, 991, 992, 999, 1000, 1007, 1008, 1500, 1991, 1999, 2000, 2640][s % 19] for s in range(sessions)]
+    slot = [int(table[s, p % context // 16]) * 16 + p % context % 16 for s, p in enumerate(at)]
+    pages, indptr = torch.tensor(table, device="cuda"), i32([s * per for s in range(sessions + 1)])
+    g = torch.Generator(device="cuda").manual_seed(sessions)
+    kv = torch.empty((sessions * per, heads, 2 * 16 * 128 + 2 * 16 * 4), dtype=torch.uint8, device="cuda")
+    for i in range(0, sessions * per, 4096):
+        part = kv[i:i + 4096]
+        part[:, :, :4096] = (torch.randn((len(part), heads, 4096), generator=g, device="cuda") * 40).to(torch.float8_e4m3fn).view(torch.uint8)
+        e = torch.rand((len(part), heads, 32), generator=g, device="cuda")
+        e[:, :, :16] = e[:, :, :16] * 9 - 14.5
+        e[:, :, 16:] = e[:, :, 16:] * 16 - 14
+        part[:, :, 4096:] = torch.exp2(e).view(torch.uint8)
+    ends = torch.tensor([min(p + 1, context) for p in at], device="cuda")
+    behind = torch.arange(per * 16, device="cuda").view(1, per, 16) >= ends.view(-1, 1, 1)  # [session, page, token]
+    s_at, p_at, t_at = behind.nonzero(as_tuple=True)
+
+    def plant(pool):
+        lost = pages[s_at, p_at]
+        for i in range(2):
+            pool[:, :, :4096].view(-1, heads, 2, 16, 128)[lost, :, i, t_at] = 0x7f
+            pool[:, :, 4096 + 64 * i:4160 + 64 * i].view(torch.int32)[lost, :, t_at] = 0x7fc00000
+    qkv = rand((sessions, 3 * heads * 128), 161)
+    qkv[7::19, :heads * 128] = 0
+    qkv_b, kv_b = qkv.clone(), kv.clone()
+    a, b = (torch.zeros((sessions, heads * 128), dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    plant(kv)  # (the scalar kernel wants numbers there)
+    torch.cuda.synchronize()
+    coef, scale, lists = float(np.float32(-np.log(10000.0) * 2.0 / 128)), 128 ** -0.5, i32(table.ravel().tolist())
+    ops.lm_decode_attend(qkv, kv, sessions * per, i32(at), i32(slot), indptr, lists, heads, coef, scale, context, a)
+    ops.lm_rope_attend(qkv_b, kv_b, sessions * per, i32(at), i32(slot), None, indptr, lists, heads, coef, scale, context, b)
+    ops.sync()
+    rows = rng.permutation(sessions)[:160]
+    want = torch.stack([ring64(qkv_b[s, :heads * 128], kv_b, pages[s], min(at[s] + 1, context), heads, scale) for s in rows])
+    close(a, b, steps=1.5, floor=0.25)
+    plant(kv_b)
+    assert torch.equal(kv, kv_b)
+    # as NOT_NEAREST, for scores up to ten instead of two or three: twice the error, two to four times the rounding boundaries crossed
+    for got in (a, b):
+        assert float((got[torch.tensor(rows, device="cuda")] != want.to(torch.bfloat16)).double().mean()) <= 2 * NOT_NEAREST
 
 
 @pytest.mark.parametrize("lens,broken", [([10, 9], 0), ([10, 9], 1), ([33, 5, 40], 1), ([3, 3, 3, 3], 2)])
