@@ -150,7 +150,7 @@ def paged(lens, seed, spare=3):
     return i32(pos), i32(slot), i32(indptr), i32(pages), count
 
 
-# up to 148 (sequence, kv head) items a team has eight warps, beyond that four
+# up to 148 (sequence, kv head) items a team has eight warps, up to 444 four, beyond that three
 @pytest.mark.parametrize("hq,hk,d", [(16, 8, 128), (4, 4, 64), (5, 1, 128), (8, 2, 64), (8, 1, 128)])
 @pytest.mark.parametrize("sessions", [1, 40, 160])
 def test_decode_attention_in_one_kernel(ops, hq, hk, d, sessions):
@@ -302,7 +302,7 @@ def test_codec_conv(ops, n, T, C, N, taps, dil, kind):
 
 
 @pytest.mark.parametrize("sessions", [1, 5, 20])
-def test_talker_as_a_chain_agrees_with_per_op_kernels(built_lib, sessions, predictor={}):
+def test_talker_as_a_chain_agrees_with_per_op_kernels(built_lib, sessions, predictor={}, ticks=4, max_tokens=2048):
     """Stacks too large for the L2 run as chains: forced frames give the logits of the per-op kernels."""
     from pega_omni_b200.config import presets
     from pega_omni_b200.model import Draw, Limits, Model, Prompt
@@ -317,13 +317,13 @@ def test_talker_as_a_chain_agrees_with_per_op_kernels(built_lib, sessions, predi
     lens = [9 + (31 * s) % 90 for s in range(sessions)]
     prompts = [Prompt(list(rng.integers(0, cfg.text_vocab_size, n)), [-1] * n) for n in lens]
     hi = min(cfg.talker.vocab_size - cfg.control_tokens, cfg.predictor.vocab_size)
-    forced = rng.integers(0, hi, (4, sessions, 16)).astype(np.int32)
+    forced = rng.integers(0, hi, (ticks, sessions, 16)).astype(np.int32)
     forced[:, :, cfg.num_code_groups:] = 0
     got = []
     for tick_kernel in (True, False):
-        m = Model.load(0, ck, cfg, Limits(max_batch=max(sessions, 8), max_tokens=2048, kv_gib=0.5), tick_kernel=tick_kernel)
+        m = Model.load(0, ck, cfg, Limits(max_batch=max(sessions, 8), max_tokens=max_tokens, kv_gib=0.5), tick_kernel=tick_kernel)
         seqs, rows = [m.open(n, 8) for n in lens], []
-        for t in range(4):
+        for t in range(ticks):
             draws = [Draw([0.5] * 16, list(forced[t, s])) for s in range(sessions)]
             out = m.start(list(zip(seqs, prompts, draws))) if t == 0 else m.step(list(zip(seqs, draws)))
             assert (out.codes == forced[t]).all()
@@ -334,6 +334,16 @@ def test_talker_as_a_chain_agrees_with_per_op_kernels(built_lib, sessions, predi
     a, b = got
     step = np.exp2(np.floor(np.log2(np.maximum(np.abs(b), 2.0))) - 7)
     assert float((np.abs(a - b) / step).max()) <= 2.0
+
+
+# More than 444 rows and kv heads: the longest rows' attention starts first. Buckets of 64 (one wave of three-warp CTAs) and 128
+# rows, with padding; prompts of one to seven pages in no order of length, which changes between the ticks of the replayed graph.
+@pytest.mark.parametrize("sessions", [60, 70])
+def test_talker_rows_started_by_length_agree_with_per_op_kernels(built_lib, sessions):
+    pages = [[(9 + (31 * s) % 90 + t) // 16 for s in range(sessions)] for t in range(5)]
+    orders = [sorted(range(sessions), key=lambda s: -p[s]) for p in pages]  # as the staged inputs have it, ties as they come
+    assert all(o != list(range(sessions)) for o in orders) and orders[2] != orders[3] != orders[4]
+    test_talker_as_a_chain_agrees_with_per_op_kernels(built_lib, sessions, ticks=6, max_tokens=8192)
 
 
 # a frame's attention: head widths and query heads a kv head, one row a sequence and the first two
