@@ -83,6 +83,11 @@ int32_t omni_op_chain_gemm(omni_ops* ctx, const void* w, int32_t N, int32_t K, c
 int32_t omni_op_chain_norm_gemm(omni_ops* ctx, const void* w1, int32_t D, int32_t K, const void* x, int32_t rows,
                                 void* res, const void* gain, float eps, const void* w2, int32_t N, void* y);
 
+/* The add + norm of the chains by itself: v = res + bf16(sum over `splits` (1, 2, 4 or 8) of part[split][rows][dim], in their
+ * order), where `lm` is set rounded to bf16; res = bf16(v); out = norm(v) * gain. All of it at 16-byte addresses. */
+int32_t omni_op_add_norm_sum(omni_ops* ctx, const float* part, int32_t splits, void* res, const void* gain, void* out,
+                             int32_t rows, int32_t dim, float eps, int32_t lm);
+
 /* `talker_sample` (crates/omni-qwen3-tts/kernels/talker.cu:259-293). state:
  * per-sequence slots of `stride` bytes, each i32 last_frame[16], u32
  * seen[ceil(vocab/32)], then (8-byte aligned) the u64 Philox seed. */

@@ -279,6 +279,20 @@ int32_t omni_op_chain_norm_gemm(omni_ops* c, const void* w1, int32_t D, int32_t 
   return OMNI_OK;
 }
 
+int32_t omni_op_add_norm_sum(omni_ops* c, const float* part, int32_t splits, void* res, const void* gain, void* out,
+                             int32_t rows, int32_t dim, float eps, int32_t lm) {
+  if (!c || !part || !res || !gain || !out || splits < 1 || rows < 1 || dim < 1) return OMNI_ERR_INVALID;
+  const uintptr_t at = reinterpret_cast<uintptr_t>(part) | reinterpret_cast<uintptr_t>(res) | reinterpret_cast<uintptr_t>(gain) |
+                       reinterpret_cast<uintptr_t>(out);
+  if (at & 15) return c->fail(OMNI_ERR_INVALID, "rows that are not at 16-byte addresses");
+  Summands sum;
+  sum.part = part, sum.splits = splits, sum.split_stride = (int64_t)rows * dim, sum.ld = dim;
+  OPS_CUDA(c, order(c->stream));  // the gain is read early
+  if (lm) OPS_CUDA(c, launch_lm_add_norm_sum(sum, (bf16*)res, (const bf16*)gain, (bf16*)out, rows, dim, eps, c->stream));
+  else OPS_CUDA(c, launch_add_norm_sum(sum, (bf16*)res, (const bf16*)gain, (bf16*)out, rows, dim, eps, 1, 0, c->stream));
+  return OMNI_OK;
+}
+
 int32_t omni_op_sample(omni_ops* c, const void* logits, int32_t vocab, float temperature, int32_t top_k, float top_p,
                        float penalty, int32_t suppress_lo, int32_t suppress_hi, int32_t exempt, int32_t min_frames,
                        const int32_t* frames, const float* uniforms, const int32_t* force, void* state,

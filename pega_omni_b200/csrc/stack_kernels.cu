@@ -89,9 +89,10 @@ __global__ void silu_mul_kernel(const bf16* gate_up, bf16* __restrict__ act, int
   st8(act + (int64_t)i * 8, g);
 }
 
-// add_norm over a GEMM's S summands: a thread owns E columns, and all its loads - the partial sums, the residual, the
-// gain - are under way together, so the kernel is one L2 round trip and one block reduction long. What is left is the
-// number of instructions, executed once: the counts of summands and columns are template arguments.
+// add_norm over a GEMM's S summands: a thread owns E columns, and its loads - the partial sums, the residual, the
+// gain - are under way together, so the kernel is one L2 round trip and one block reduction long (eight sums of four or eight
+// columns are more than the 32 and 46 registers that the compiler gives them: it loads those in batches, a round trip each).
+// What is left is the number of instructions, executed once: the counts of summands and columns are template arguments.
 template <int S, int E>
 __global__ void add_norm_sum_kernel(const Summands x, bf16* __restrict__ res, const bf16* __restrict__ w,
                                     bf16* __restrict__ out, int dim, float eps, int every, int which) {

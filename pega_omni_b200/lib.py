@@ -127,6 +127,7 @@ SYMBOLS = {
     "omni_op_decode_attend": (I32, [VP, VP, VP, VP, VP, I32, VP, VP, VP, VP, I32, I32, I32, I32, C.c_float, C.c_float, VP]),
     "omni_op_chain_gemm": (I32, [VP, VP, I32, I32, VP, I32, VP, I32, VP, I32, I32]),
     "omni_op_chain_norm_gemm": (I32, [VP, VP, I32, I32, VP, I32, VP, VP, C.c_float, VP, I32, VP]),
+    "omni_op_add_norm_sum": (I32, [VP, VP, I32, VP, VP, VP, I32, I32, C.c_float, I32]),
     "omni_op_sample": (I32, [VP, VP, I32, C.c_float, I32, C.c_float, C.c_float, I32, I32, I32, I32, VP, VP, VP, VP,
                              VP, C.c_int64, I32, I32, VP, I32, I32]),
     "omni_op_gemm_noalloc": (I32, [VP, I32, I32, VP, I32, VP, I32, I32, VP, I32, VP, C.c_char_p, C.c_size_t]),

@@ -88,6 +88,11 @@ class Ops:
         self._check(self._lib.omni_op_chain_norm_gemm(self._h, _p(w1), w1.shape[0], w1.shape[1], _p(x), x.shape[0],
                                                       _p(res), _p(gain), eps, _p(w2), w2.shape[0], _p(y)))
 
+    def add_norm_sum(self, part, res, gain, out, eps, lm=False):
+        splits, rows, dim = part.shape
+        self._check(self._lib.omni_op_add_norm_sum(self._h, _p(part), splits, _p(res), _p(gain), _p(out), rows, dim, eps,
+                                                   int(lm)))
+
     def sample(self, logits, temperature, top_k, top_p, penalty, suppress_lo, suppress_hi, exempt, min_frames, frames,
                uniforms, force, state, lines, stride, penalize, philox, codes, group):
         rows, vocab = logits.shape

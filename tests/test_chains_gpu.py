@@ -175,11 +175,33 @@ def test_decode_attention_teams(ops, hq, hk, d, items):
     test_decode_attention_in_one_kernel(ops, hq, hk, d, items)
 
 
-# two, four and eight columns a thread, rows that end inside a warp of each
+# two, four and eight columns a thread, rows that end inside a warp of each; one sum, of products that are one k-block long
 @pytest.mark.parametrize("rows", [9, 250])
 @pytest.mark.parametrize("d", [1984, 2048, 2112, 4096, 4160])
 def test_chain_norm_columns(ops, rows, d):
     test_chain_norm_gemm(ops, rows, d, 64, 64)
+
+
+# every count of sums by every count of columns a thread (the last by the rows, too)
+@pytest.mark.parametrize("lm", [False, True])
+@pytest.mark.parametrize("splits", [1, 2, 4, 8])
+@pytest.mark.parametrize("rows,d", [(9, 1984), (250, 2048), (9, 2112), (256, 4096), (9, 4160), (5, 8192), (257, 1024)])
+def test_add_norm_of_split_sums(ops, rows, d, splits, lm):
+    g = torch.Generator(device="cuda").manual_seed(d + splits)
+    part = torch.randn((splits, rows, d), generator=g, device="cuda")
+    res, gain = rand((rows, d), 171), rand((d,), 172, 0.2) + 1
+    total = part[0].clone()
+    for p in part[1:]:
+        total += p
+    v = res.float() + total.bfloat16().float()
+    if lm:
+        v = v.bfloat16().float()
+    out = torch.zeros((rows, d), dtype=torch.bfloat16, device="cuda")
+    torch.cuda.synchronize()
+    ops.add_norm_sum(part, res, gain, out, 1e-6, lm=lm)
+    ops.sync()
+    assert torch.equal(res, v.bfloat16())
+    close(out, v * torch.rsqrt((v * v).mean(1, keepdim=True) + 1e-6) * gain.float(), steps=1.0)
 
 
 @pytest.mark.parametrize("heads,sessions", [(4, 1), (4, 37), (32, 5), (16, 16)])
