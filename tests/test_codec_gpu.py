@@ -184,3 +184,39 @@ def test_full_size_decoder_at_64_streams_matches_the_oracle(built_lib):
     ms, launches = m.stats()
     assert launches == 134
     m.close()
+
+
+# up to eight streams the transformer's norms and SwiGLU are inside its GEMMs; beyond, and in the frame of the test above, apart
+@pytest.mark.parametrize("n", [1, 3, 8, 9])
+def test_full_size_decoder_of_few_streams_matches_the_oracle(built_lib, n):
+    c = CODEC_PRESETS["qwen3-tts-12hz"]
+    ck = codec_random_checkpoint(c, 0)
+    W, frames = oc.fold(ck, c), 4
+    codes = np.random.default_rng(n).integers(0, c.codebook_size, size=(frames, n, 16)).astype(np.int32)
+    m = Codec(c, ck, max_batch=n)
+    m.warmup()
+    streams = [m.open() for _ in range(n)]
+    got = np.stack([m.decode(streams, codes[f]) for f in range(frames)])
+    launches = m.stats()[1]
+    m.close()
+    assert np.isfinite(got).all() and np.abs(got).max() <= 1.0 and launches <= 134
+    for s in {0, n - 1}:  # the bounds of the test above
+        so = oc.StreamOracle(c, W)
+        want = np.stack([so.step(codes[f, s]) for f in range(frames)])
+        truth = oc.whole_utterance(ck, c, codes[:, s]).reshape(frames, -1)
+        assert oc.snr_db(got[:, s], truth) > oc.snr_db(want, truth) - 1.0, s
+        assert oc.snr_db(got[:, s], want) > 21.0, s
+        assert oc.snr_db(got[0, s], want[0]) > 25.0, s
+
+
+def test_more_streams_than_the_weight_streaming_gemms_take(built_lib):
+    """Beyond 256 streams the out projections leave finished rows: the first and the last stream of 300 against the oracle."""
+    c, ck, codes, want = _setup("codec-tiny", 4)
+    m = Codec(c, ck, max_batch=300)
+    streams = [m.open() for _ in range(300)]
+    rows = np.random.default_rng(2).integers(0, c.codebook_size, (4, 300, 16)).astype(np.int32)
+    rows[:, 0] = rows[:, 299] = codes
+    got = np.stack([m.decode(streams, r) for r in rows])
+    m.close()
+    assert np.array_equal(got[:, 0], got[:, 299])
+    assert oc.snr_db(got[:, 0], want) > 25.0 and oc.snr_db(got[0, 0], want[0]) > 33.0
