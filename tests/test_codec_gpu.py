@@ -182,7 +182,7 @@ def test_full_size_decoder_at_64_streams_matches_the_oracle(built_lib):
         assert oc.snr_db(got[:, s], want) > 21.0, s
         assert oc.snr_db(got[0, s], want[0]) > 25.0, s
     ms, launches = m.stats()
-    assert launches == 134
+    assert launches <= 134
     m.close()
 
 
