@@ -27,7 +27,7 @@ def rand(shape, seed, scale=1.0):
 def close(got, want, steps=2.0, floor=0.05):
     """Within `steps` bf16 steps of the fp32 value; `floor`: the size of what was rounded on the way, where sums cancel."""
     g, w = got.float(), want.float()
-    bad = (g - w).abs() > steps * 2.0 ** -7 * w.abs().clamp_min(floor)
+    bad = ~((g - w).abs() <= steps * 2.0 ** -7 * w.abs().clamp_min(floor))  # NaN is a difference
     assert not bad.any(), (int(bad.sum()), float((g - w).abs().max()))
 
 
