@@ -59,11 +59,13 @@ struct Chain {
   // way in registers, 4,836 and 5,170.
   bool whole_smem = false;
 
-  // What the next GEMM asks into L2 on its way: the first of the weights that the GEMM behind it reads, whose own requests start
-  // one kernel before they are needed. For passes that leave DRAM idle. One pass without and with 8 MB, us: a talker step of 1
-  // session 1,875 and 1,831, of 8 2,548 and 2,514, of 64 3,456 and 3,394, a start of one prompt 2,697 and 2,650, a duplex tick of
-  // 64 with the depformer's 5,174 and 5,129 (32 MB: 1,865, 2,560, 3,449, 2,662, 5,279). A Higgs step of 3, at half the copy rate,
-  // 1,913 and 1,938, a duplex tick of 1 3,174 and 3,198: none there.
+  // What the next GEMM asks into L2 on its way: the first of the weights of the GEMM after it, whose own requests start one
+  // kernel before they are needed. For passes that leave DRAM idle, as measured; in brackets the share of the copy rate that the
+  // call moves without it. One pass without and with 8 MB, us: a talker step of 1 session (0.25) 1,875 and 1,831, of 8 (0.2) 2,548
+  // and 2,514, of 64 (0.2) 3,456 and 3,394, a start of one prompt (0.2) 2,697 and 2,650, a duplex tick of 64 with the depformer's
+  // (its passes below 0.2) 5,174 and 5,129 (32 MB: 1,865, 2,560, 3,449, 2,662, 5,279). Where a call moves more, the requests
+  // compete with the GEMMs' own: a Higgs step of 3 (0.5) 1,913 and 1,938, a duplex tick of 1 (0.7) 3,174 and 3,198: none there.
+  // A pass's last GEMM asks for nothing.
   size_t ahead_cap = 0;
   sm100::Ahead ahead;
   void next(const bf16* w, int N, int K) {
@@ -169,7 +171,7 @@ cudaError_t chain_pass(Chain c, const std::vector<Layer>& layers, const GateUp& 
   for (size_t i = 0; i < layers.size(); ++i) {
     const Layer& L = layers[i];
     const QkvTable& from = i == 0 ? lookup : QkvTable{};
-    c.next(gate_up(L), 2 * inter, hidden);
+    if (!from.table) c.next(gate_up(L), 2 * inter, hidden);
     if (i > 0) OMNI_CHAIN(norm_gemm(L.ln1, L.qkv, qw, kStreamBf16, b.qkv, qw));
     else if (!from.table) OMNI_CHAIN(c.gemm(L.qkv, qw, hidden, b.x, rows, kStreamBf16, b.qkv, qw));
     if (prompt) {  // rows of one sequence attend to one another: every key is written before the first is read

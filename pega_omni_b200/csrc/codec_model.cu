@@ -521,9 +521,12 @@ int enqueue_frame(omni_codec* m, int n) {
   for (size_t i = 0; i < m->layers.size(); ++i) {
     const TLayer& L = m->layers[i];
     const TLayer* Ln = i + 1 < m->layers.size() ? &L + 1 : nullptr;
-    chain.next(L.gate_up, 2 * inter, h);
-    if (i > 0) CTRY(behind_norm((&L - 1)->next, L.qkv, 3 * qd, kStreamBf16, COL));
-    else CTRY(dense(m, L.qkv, 3 * qd, h, X, n, COL));
+    if (i > 0) {
+      chain.next(L.gate_up, 2 * inter, h);
+      CTRY(behind_norm((&L - 1)->next, L.qkv, 3 * qd, kStreamBf16, COL));
+    } else {
+      CTRY(dense(m, L.qkv, 3 * qd, h, X, n, COL));
+    }
     CLAUNCH(m, launch_codec_window_attend(COL, st, L.ring, A, n, c.num_attention_heads, c.rope_theta, s));
     chain.next(L.down, h, inter);
     CTRY(projected(L.o, qd, A));

@@ -349,9 +349,12 @@ int depformer_step(omni_duplex* m, int n, const int32_t* force, const int32_t* s
       const bool last = i + 1 == c.dep_layers;  // the next pass has its own weights
       const DepLayer* Ln = !last ? &m->d[i + 1] : k + 1 < kDepSteps ? &m->d[0] : nullptr;
       const size_t kn = last ? k + 1 : k;
-      chain.next(L.gate_in + (size_t)k * 2 * H * D, 2 * H, D);
-      if (i > 0) DTRY(behind_norm(kNormLm, L.norm1, qkv, 3 * D, kStreamBf16, m->dqkv));
-      else DTRY(gemm(m, qkv, 3 * D, D, m->dxn, n, m->dqkv, 3 * D));
+      if (i > 0) {
+        chain.next(L.gate_in + (size_t)k * 2 * H * D, 2 * H, D);
+        DTRY(behind_norm(kNormLm, L.norm1, qkv, 3 * D, kStreamBf16, m->dqkv));
+      } else {
+        DTRY(gemm(m, qkv, 3 * D, D, m->dxn, n, m->dqkv, 3 * D));
+      }
       DLAUNCH(m, launch_lm_dep_kv_attend(m->dqkv, m->dkv[i], k, m->dattn, n, c.dep_heads, scale, m->stream));
       chain.next(L.gate_out + (size_t)k * D * H, D, H);
       DTRY(projected(L.out + (size_t)k * D * D, D, m->dattn));
