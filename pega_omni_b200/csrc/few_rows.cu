@@ -380,10 +380,12 @@ int few_plan(FewPlan* plan, const bf16* w, int N, int K, const bf16* x, int rows
     }
   if (even.early) best = even;
   if (best.cost > 1e29) return -2;
-  // Left to the tcgen05 kernel: rows that take so much of an SM's shared memory that the rings hold too little of the weights, and
-  // from three rows on weights that no ring holds much of. As nodes of a tick or step, us for all of them, this kernel and that
-  // one: 8 rows of 12,288 x 4,096 (32 layers) -103, 22,528 x 4,096 -314, 4,096 x 11,264 -109, but 2,560 x 9,728 (36) +129,
-  // 19,456 x 2,560 -6; 4 rows of 22,528 x 4,096 -108, but 12,288 x 4,096 +111; 1 row of 22,528 x 4,096 +97.
+  // Left to the tcgen05 kernel: rows that take so much of an SM's shared memory that the rings hold too little of the weights
+  // (the line lies between the 40 and 48 KB of the nearest measured shapes), and from three rows on weights beyond the 126 MB of
+  // L2, which no ring holds much of. As nodes of a tick or step, us for all of them, this kernel and that one, the rows' share in
+  // brackets: 8 rows of 12,288 x 4,096 (32 layers, 64 KB) -103, 22,528 x 4,096 (64) -314, 4,096 x 11,264 (48) -109, but
+  // 2,560 x 9,728 (36 layers, 40) +129, 19,456 x 2,560 (40) -6; 4 rows (32 KB) of 22,528 x 4,096, 185 MB, -108, but 12,288 x 4,096,
+  // 101 MB, +111; 1 row of 22,528 x 4,096 +97.
   const size_t x_share = (size_t)few_per(K / kKb, best.splits) * kKb * kWarps * rows * 2;
   if (x && !any_shape && (x_share > 42 * 1024 || (rows > 2 && (int64_t)N * K > 64 << 20))) return -2;
   p.R = best.R, p.splits = best.splits, p.slots = best.slots, p.smem = best.smem;

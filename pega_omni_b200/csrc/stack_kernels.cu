@@ -636,9 +636,9 @@ static cudaError_t launch_rope_attend_dg(const bf16* qkv, const QkvTable& lookup
   };
   // items that leave SMs idle: eight warps each, so that 128 keys are one round (sixteen would have to spill: 2,282 against
   // 2,242 us a step of one session, 2,133 against 2,042 us for Higgs at three); up to three CTAs an SM, four warps; beyond, three
-  // warps and four CTAs an SM, one wave of 512 items instead of two (64 sessions: 3,416 against 3,513 us a step), and the longest
-  // rows first where there is more than a wave. Prompts of 32 to 512 tokens, four warps as the rows come and this: 80 sessions
-  // 4,418 and 4,256 us, 128 4,747 and 4,697 (four warps in order 4,757, two 4,707).
+  // warps and four CTAs an SM, one wave of 512 items instead of two (64 sessions: 3,416 against 3,513 us a step), and there the
+  // longest rows first, which counts from the second wave (592 items) on. Prompts of 32 to 512 tokens, four warps as the rows come
+  // and this: 80 sessions 4,418 and 4,256 us, 128 4,747 and 4,697 (four warps in order 4,757, two 4,707).
   if (items > 3 * sm_count) return go(rope_attend_kernel<D, G, 3>, 3);
   map.order = nullptr;
   return items <= sm_count ? go(rope_attend_kernel<D, G, 8>, 8) : go(rope_attend_kernel<D, G, 4>, 4);

@@ -261,9 +261,9 @@ void stream_configure() {
 bool stream_supports(int N, int K, int rows) { return K % kKb == 0 && K >= kKb && N >= 1 && rows >= 1; }
 
 // Weight rows per tile (tn) and K splits: the shape with the shortest estimated time after the inputs are there. A CTA
-// pulls its tile's rows at about 120 GB/s whatever the number of CTAs (they all read the same rows; with 170, as its weights, a talker
-// step of 64 sessions took 3,375 us instead of 3,351, of 128 4,629 and 4,596; with 90 3,335, 4,596, but a duplex tick of 64 5,175
-// instead of 5,135), the tensor pipe
+// pulls its tile's rows at about 120 GB/s whatever the number of CTAs (they all read the same rows, while the weights of later
+// GEMMs are on their way). That is a fit: with 170, as its weights, a talker step of 64 sessions took 3,375 us instead of 3,351,
+// of 128 4,629 and 4,596; with 90 3,335, 4,596, but a duplex tick of 64 5,175 instead of 5,135. The tensor pipe
 // takes (M + tn) / 4 cycles per 16 elements of K, stores leave an SM at 57 GB/s, and weights only count where a shape
 // loads some SMs more than others, since they were asked for before the inputs were there.
 static double stream_cost(int N, int K, int rows, int M, int bn, int tn, int S, int out, int sms, int row_tiles) {
