@@ -495,7 +495,8 @@ int enqueue_frame(omni_codec* m, int n) {
   CLAUNCH(m, launch_codec_add_norm(m->in_b, 0, RES, m->ln1_0, X, n, h, c.rms_norm_eps, s));
   // A layer is a chain's: the out projections leave partial sums (finished rows beyond kChainRows streams) for the add + norm
   // behind them, which for a few streams is part of the next GEMM, as SwiGLU is of its own. A frame with a kernel for each op
-  // and this, us: 1 stream 475 and 429, 8 590 and 531, 16 708 and 656, 64 1,146 and 1,129.
+  // and this, us: 1 stream 475 and 429, 8 590 and 531, 16 708 and 656, 64 1,146 and 1,129. Relative distance from float64 over 60
+  // frames of three utterances (1 to 64 streams): 0.0148 to 0.0152 for both.
   Chain chain = m->chain();
   chain.ahead_cap = kAheadBytes;
   Summands y;
@@ -533,7 +534,7 @@ int enqueue_frame(omni_codec* m, int n) {
     chain.next(Ln ? Ln->qkv : m->out_w, Ln ? 3 * qd : lat, h);
     if (n <= kFewRows) {
       CTRY(behind_norm(L.ln2, L.gate_up, 2 * inter, kStreamSwiglu, A));
-    } else {  // (a frame of many streams is 134 kernels, which its statistics report and tests hold)
+    } else {  // still a kernel of its own: inside the GEMM a frame takes 598 us instead of 608 at 12 streams, 1,041 and 1,052 at 64
       CTRY(behind_norm(L.ln2, L.gate_up, 2 * inter, kStreamBf16, COL));
       CLAUNCH(m, launch_silu_mul(COL, A, n, inter, kGateGroup, s));
     }
